@@ -348,6 +348,14 @@ struct BuiltHT {
     bool unit_mult = false;
 };
 
+// A scan that tests a filter runs in the direct form below this many key
+// pages. Device time of the scan of N rows against tables of 400 to 8,000
+// kept keys, 2% of them (staged filter against direct, one B200): 0.1M rows
+// 13.4 / 12.4 us, 1M 13.6 / 12.5, 3M 13.6 / 20.7, 24M 38 / 155. Without a
+// filter the direct form is never slower: 100K keys of which 35% are kept,
+// all matching: 1M rows 36 / 18 us.
+constexpr uint32_t kDirectFilterPages = 512;
+
 // Streamed scans (Executor::streamed_scan): windows of 16 MiB, three in flight.
 constexpr uint32_t kWindowPages = 2048;
 constexpr uint32_t kWindowRing = 3;
@@ -581,8 +589,8 @@ class Executor {
     }
 
     // A fused chain of the unique-key stages s, s + 1, ... (up to kMaxChain)
-    // over `in`: the stages, the outputs (room for in.count items) and the
-    // items it leaves, whose count is on the device.
+    // over `in` (unit: every multiplicity is 1): the stages, the outputs (room
+    // for in.count items) and the items it leaves, whose count is on the device.
     struct ChainRun {
         ProbeChain ch{};
         ItemsOut out{};
@@ -593,9 +601,8 @@ class Executor {
     };
     ChainRun plan_chain(const PipelinePlan& pp, const std::vector<uint32_t>& order,
                         const std::vector<HTView>& by_stage, const std::vector<double>& rate, size_t s,
-                        const Items& in) {
+                        const Items& in, bool unit) {
         ChainRun r;
-        bool unit = in.mult == nullptr;
         size_t s2 = s;
         while (s2 < order.size() && r.ch.n < kMaxChain && hts_[pp.probes[order[s2]].child].unique) {
             const uint32_t k2 = order[s2];
@@ -690,6 +697,52 @@ class Executor {
                 launched(probe_chain_unique(scanned, chain->ch, chain->out, chain->cursor, chain->cap, ctx_->d_err,
                                             ctx_->num_sms, st_, marks + i, marks + i + 1));
         }
+    }
+
+    // The scan stage as scan_probe_direct (k_direct.cu) with the unique-key
+    // stages after it, when that form takes it: updates s and items. Not
+    // taken: repeated build keys, pages in host memory (their loads are sized
+    // for the link), shapes tuned to the split form, and long scans of a
+    // selective probe, which the staged filter serves better.
+    bool direct_scan(const PipelinePlan& pp, const std::vector<uint32_t>& order, const std::vector<HTView>& by_stage,
+                     const std::vector<double>& rate, size_t& s, Items& items) {
+        if (items.rows != nullptr || s != 0) return false;
+        const uint32_t k = order[s];
+        const PipelinePlan::Probe& pr = pp.probes[k];
+        const BuiltHT& bh = hts_[pr.child];
+        const DevColumn& key = col(pr.probe_attr);
+        const HTView& ht = by_stage[s];
+        if (!bh.unique || (key.flags & kColHostPages) || (ctx_->scan_split && ctx_->tune.scan_split)) return false;
+        const bool bloom = ht.bloom && rate[k] < 0.5;
+        if (bloom && key.npages > kDirectFilterPages) return false;
+        Items next{};
+        next.count = key.nrows;
+        next.nprobes = 1;
+        ItemsOut out{};
+        uint32_t* cursor = nullptr;
+        ChainRun chain;
+        const bool fuse = s + 1 < order.size() && hts_[pp.probes[order[s + 1]].child].unique;
+        if (fuse) {
+            chain = plan_chain(pp, order, by_stage, rate, s + 1, next, bh.unit_mult);
+            out = chain.out;
+            cursor = chain.cursor;
+            next = chain.result;
+        } else {
+            next.rows = out.rows = alloc<uint32_t>(key.nrows);
+            next.ents[0] = out.ents[0] = alloc<uint32_t>(key.nrows);
+            next.mult = out.mult = bh.unit_mult ? nullptr : alloc<uint64_t>(key.nrows);
+            cursor = alloc<uint32_t>(1);
+            next.dcount = cursor;
+            BJ_CK(cudaMemsetAsync(cursor, 0, sizeof(uint32_t), st_));
+        }
+        if (ctx_->profile) begin_timed();
+        launched(scan_probe_direct(key, ht, bloom, fuse ? &chain.ch : nullptr, out, cursor, key.nrows, ctx_->d_err,
+                                   ctx_->num_sms, st_));
+        if (ctx_->profile) end_timed(uint64_t(key.npages) * kPageSize);
+        trace("direct scan enqueued");
+        items = next;
+        if (fuse) s = chain.s2 - 1;
+        return true;
     }
 
     // Exclusive scan of tile counts; returns the total (synchronises).
@@ -825,6 +878,7 @@ class Executor {
         for (size_t s = 0; s < np; s++) {
             uint32_t k = order[s];
             const HTView& ht = by_stage[s];
+            if (direct_scan(pp, order, by_stage, rate, s, items)) continue;
             if (items.rows == nullptr && col(pp.probes[k].probe_attr).type == kInt32) {
                 // Scan stage: stream the key pages of the scanned table. (An
                 // INT64 key column takes the item stages below, over the
@@ -859,7 +913,7 @@ class Executor {
                         // the next windows' copies.
                         const bool fuse = s + 1 < np && hts_[pp.probes[order[s + 1]].child].unique;
                         ChainRun chain;
-                        if (fuse) chain = plan_chain(pp, order, by_stage, rate, s + 1, next);
+                        if (fuse) chain = plan_chain(pp, order, by_stage, rate, s + 1, next, bh.unit_mult);
                         streamed_scan(key, ht, bloom, cursor, out, cap, fuse ? &chain : nullptr, next);
                         if (timed) end_timed(page_bytes);
                         trace("streamed scan enqueued");
@@ -929,7 +983,7 @@ class Executor {
             if (bh.unique) {
                 // This stage and the unique-key stages right after it run as
                 // one fused chain.
-                ChainRun chain = plan_chain(pp, order, by_stage, rate, s, items);
+                ChainRun chain = plan_chain(pp, order, by_stage, rate, s, items, items.mult == nullptr);
                 launched(probe_chain_unique(items, chain.ch, chain.out, chain.cursor, chain.cap, ctx_->d_err,
                                             ctx_->num_sms, st_));
                 trace("probe chain enqueued");

@@ -260,6 +260,15 @@ int scan_probe_split(const DevColumn& key, const HTView& ht, uint32_t* cursor, u
                      uint32_t* cand_count, uint32_t cand_cap, uint32_t* err, int num_sms, cudaStream_t st,
                      uint32_t row_base = 0);
 
+// The stage against a table with unique keys without staging a filter, a CTA
+// a page (k_direct.cu), INT32 or INT64 keys; pages in device memory. `chain`
+// (optional): the unique-key stages right after the scan, run in the same
+// launch (their payload sources may be the scan's own match, stage 0); the
+// items then carry one entry per stage. Appends at *cursor (zero before).
+int scan_probe_direct(const DevColumn& key, const HTView& ht, bool use_bloom, const ProbeChain* chain,
+                      const ItemsOut& out, uint32_t* cursor, uint32_t capacity, uint32_t* err, int num_sms,
+                      cudaStream_t st);
+
 // ---- hash table build (k_build.cu) ----
 // Tuples of a build pipeline, one per item: key from `key` (NULL key ->
 // mult 0), payload from `src`, mult from the item.

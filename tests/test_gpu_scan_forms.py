@@ -1,0 +1,90 @@
+"""The scan-side probe in its forms, against the oracle, at the sizes where
+they can go wrong: part groups of 32 rows, part pages, pages with NULLs (their
+rows taken by the null bitmap), unit boundaries, tables probed with and
+without a filter, the fused unique-key stages, INT32 and INT64 keys."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle_lib
+
+pytestmark = pytest.mark.gpu
+
+
+def column(pkg, dtype, values, valid=None):
+    values = np.ascontiguousarray(values)
+    h = ctypes.c_void_p()
+    st = pkg.wlib().bjw_encode_column(dtype, len(values), values.ctypes.data,
+                                      None if valid is None else valid.ctypes.data, None, None, ctypes.byref(h))
+    assert st == 0
+    n, ptrs = pkg.wlib().bjw_pages_count(h), pkg.wlib().bjw_pages_ptrs(h)
+    data = b"".join(ctypes.string_at(ptrs[i], 8192) for i in range(n))
+    pkg.wlib().bjw_pages_free(h)
+    return pkg.Column(dtype, data)
+
+
+def star(pkg, seed, fact, dims, keep, nulls, wide, copies=1):
+    """fact(id, k0, ...) joined with dims[j] keys of which a share `keep` is present, each `copies` times."""
+    rng = np.random.default_rng(seed)
+    kt, kn = (pkg.INT64, np.int64) if wide else (pkg.INT32, np.int32)
+    spread = (lambda k: k.astype(np.int64) | ((k.astype(np.int64) % 8 - 4) << 32)) if wide else \
+             (lambda k: (k.astype(np.int64) - 7).astype(np.int32))  # INT32 keys around zero
+    p = pkg.Plan()
+    cols = [column(pkg, pkg.INT32, np.arange(fact, dtype=np.int32))]
+    for d in dims:
+        valid = None if not nulls else (rng.random(fact) >= nulls).astype(np.uint8)
+        cols.append(column(pkg, kt, spread(rng.integers(0, d, fact)).astype(kn), valid))
+    p.new_input(pkg.ColumnarTable(fact, cols))
+    left = p.new_scan_node(0, [(0, pkg.INT32)] + [(1 + j, kt) for j in range(len(dims))])
+    width = 1 + len(dims)
+    for j, d in enumerate(dims):
+        own = np.repeat(rng.permutation(d)[:max(1, int(d * keep))], copies)
+        t = p.new_input(pkg.ColumnarTable(len(own), [
+            column(pkg, kt, spread(own).astype(kn)),
+            column(pkg, pkg.INT32, rng.integers(0, 1 << 30, len(own), dtype=np.int32))]))
+        right = p.new_scan_node(t, [(0, kt), (1, pkg.INT32)])
+        attrs = [(i, pkg.INT32 if i == 0 else kt) for i in range(1 + len(dims))]
+        attrs += [(i, pkg.INT32) for i in range(1 + len(dims), width)] + [(width + 1, pkg.INT32)]
+        left = p.new_join_node(False, left, right, 1 + j, 0, attrs)
+        width += 1
+    p.root = left
+    return pkg.CPlan(p)
+
+
+def check(pkg, ctx, oracle, cp, label):
+    want = oracle.execute(cp.ref())
+    with ctx.execute_raw(cp) as r:
+        got, keep = r.table_struct()
+        oracle_lib.assert_same_rows(oracle, ctypes.byref(got), want.view(), label + " host")
+    plan = cp.struct
+    res = [ctx.upload(plan.inputs[i]) for i in range(plan.num_inputs)]
+    try:
+        for run in range(3):  # recorded, captured, replayed
+            with ctx.execute_resident(cp, res) as r:
+                got, keep = r.table_struct()
+                oracle_lib.assert_same_rows(oracle, ctypes.byref(got), want.view(), f"{label} resident {run}")
+    finally:
+        for x in res:
+            x.free()
+
+
+# Rows: a lone row, group and batch edges, page edges (1,984 INT32 rows, 1,007 INT64 rows), several pages.
+@pytest.mark.parametrize("fact", [1, 31, 33, 127, 128, 129, 1023, 1025, 1007, 1008, 1984, 1985, 4001, 40_003])
+@pytest.mark.parametrize("nulls", [0.0, 0.1, 0.9])
+@pytest.mark.parametrize("wide", [False, True])
+def test_direct_scan(pkg, ctx, oracle, fact, nulls, wide):
+    check(pkg, ctx, oracle, star(pkg, fact, fact, [300], 0.5, nulls, wide), f"fact {fact} nulls {nulls} wide {wide}")
+
+
+@pytest.mark.parametrize("dims", [[500, 200], [4000, 900, 60], [70_000, 5, 300, 20]])
+@pytest.mark.parametrize("keep", [0.05, 0.6, 1.0])
+@pytest.mark.parametrize("wide", [False, True])
+def test_fused_stages(pkg, ctx, oracle, dims, keep, wide):
+    check(pkg, ctx, oracle, star(pkg, len(dims), 30_011, dims, keep, 0.05, wide), f"dims {dims} keep {keep}")
+
+
+# Either side of the line where a filtered scan takes the staged form (512 pages).
+@pytest.mark.parametrize("fact", [512 * 1984, 512 * 1984 + 1])
+def test_filter_form_line(pkg, ctx, oracle, fact):
+    check(pkg, ctx, oracle, star(pkg, 5, fact, [3000, 700], 0.1, 0.0, False), f"fact {fact}")
