@@ -228,43 +228,60 @@ __device__ __forceinline__ uint32_t bloom_bits_fast(uint32_t hh, uint32_t hh5) {
 inline uint32_t key_hash_hi(uint32_t key) { return uint32_t(key_hash(key) >> 32); }
 #endif
 
-// A built hash table: entries grouped by bucket (CSR), keys 32-bit, a
-// multiplicity per entry (eager aggregation folds identical tuples into one
-// entry, engine/op/Hashtable.cpp:236-248), `width` 64-bit payload slots per
-// entry with a NULL mask.
+// A built hash table. A bucket is 16 bytes, read by one load: the position and
+// number of its entries and the (low halves of the) keys of its first two, so
+// a probe of a bucket with at most two entries (93% of them at the sizing
+// rule's fullest, one key per bucket) touches nothing else. Measured against
+// 8-byte buckets with one key, whose length took the next bucket's start, on
+// a B200: 8M probes of 1M keys, all matching: 89 -> 67 us.
+// An entry is one run of words: its key slot, then `width` payload slots.
+// Entries of a bucket lie side by side; buckets lie in no particular order.
 struct HTView {
-    // nbuckets + 1: x = position of the bucket's first entry (the last x is
-    // the entry count), y = that entry's key when the bucket is not empty,
-    // so one 8-byte load answers a probe of a bucket with a single key.
-    const uint2* buckets;
-    const uint32_t* keys;        // nentries
-    const uint64_t* mult;        // nentries
-    const uint64_t* pay;         // nentries * width
-    const uint32_t* pnull;       // nentries (bit j: slot j is NULL)
-    const uint32_t* bloom;       // 1 << bloom_log2 words, or null (always null for INT64 keys)
-    const uint32_t* keys_hi;     // INT64 keys: high halves (keys holds the low ones); null for INT32
-    uint32_t shift;              // bucket = key_hash >> shift
+    const uint4* buckets;   // per bucket: first entry, entries, first key, second key
+    const uint64_t* ent;    // nentries * (1 + width)
+    const uint64_t* mult;   // nentries multiplicities (eager aggregation folds identical tuples
+                            // into one entry, engine/op/Hashtable.cpp:236-248); null: all 1
+    const uint32_t* pnull;  // nentries NULL masks (bit j: slot j is NULL); null: no slot is NULL
+    const uint32_t* bloom;  // 1 << bloom_log2 words, or null (always null for INT64 keys)
+    uint32_t shift;         // bucket = key_hash >> shift (33..63)
     uint32_t bloom_log2;
     uint32_t nentries;
     uint32_t width;
+    uint32_t wide;          // INT64 keys
 };
 
-// Bucket of key slot k in a table keyed on 64-bit (wide) or 32-bit keys.
-BJ_HD uint32_t bucket_of(uint64_t k, bool wide, uint32_t shift) {
-    return uint32_t((wide ? key_hash_any(k, kInt64) : key_hash(uint32_t(k))) >> shift);
-}
-
 #if defined(__CUDACC__)
-__device__ __forceinline__ uint32_t ht_bucket(const HTView& ht, uint64_t k) {
-    return bucket_of(k, ht.keys_hi != nullptr, ht.shift);
-}
-// Entry e's key equals key slot k.
-__device__ __forceinline__ bool ht_key_eq(const HTView& ht, uint32_t e, uint64_t k) {
-    return ht.keys[e] == uint32_t(k) && (!ht.keys_hi || ht.keys_hi[e] == uint32_t(k >> 32));
+// Bucket of key slot k in a table keyed on 64-bit (wide) or 32-bit keys.
+__device__ __forceinline__ uint32_t bucket_of(uint64_t k, bool wide, uint32_t shift) {
+    return wide ? uint32_t(key_hash_any(k, kInt64) >> shift) : key_hash_hi(uint32_t(k)) >> (shift - 32);
 }
 // Entry e's key as a value slot.
 __device__ __forceinline__ uint64_t ht_key(const HTView& ht, uint32_t e) {
-    return uint64_t(ht.keys[e]) | (ht.keys_hi ? uint64_t(ht.keys_hi[e]) << 32 : 0ull);
+    return ht.ent[size_t(e) * (1 + ht.width)];
+}
+__device__ __forceinline__ uint64_t ht_slot(const HTView& ht, uint32_t e, uint32_t slot) {
+    return ht.ent[size_t(e) * (1 + ht.width) + 1 + slot];
+}
+__device__ __forceinline__ bool ht_slot_null(const HTView& ht, uint32_t e, uint32_t slot) {
+    return ht.pnull && ((ht.pnull[e] >> slot) & 1);
+}
+__device__ __forceinline__ uint64_t ht_mult(const HTView& ht, uint32_t e) { return ht.mult ? ht.mult[e] : 1ull; }
+
+// Calls fn(entry) for the entries of bucket b with key slot `key`, until fn
+// returns false. The bucket's own keys decide without a look at the entries,
+// except where only their low halves are known (INT64).
+template <typename Fn>
+__device__ __forceinline__ void bucket_matches(const HTView& ht, const uint4& b, uint64_t key, Fn&& fn) {
+    if (b.y >= 1 && b.z == uint32_t(key) && (!ht.wide || ht_key(ht, b.x) == key))
+        if (!fn(b.x)) return;
+    if (b.y >= 2 && b.w == uint32_t(key) && (!ht.wide || ht_key(ht, b.x + 1) == key))
+        if (!fn(b.x + 1)) return;
+    for (uint32_t j = 2; j < b.y; j++)
+        if (ht_key(ht, b.x + j) == key)
+            if (!fn(b.x + j)) return;
+}
+__device__ __forceinline__ uint4 ht_bucket(const HTView& ht, uint64_t key) {
+    return __ldg(ht.buckets + bucket_of(key, ht.wide != 0, ht.shift));
 }
 
 __device__ __forceinline__ bool bloom_may_contain(const uint32_t* bloom, uint32_t log2w, uint32_t key) {

@@ -1050,49 +1050,45 @@ class Executor {
     // A build's buffers and sizes; the buffers that must start at zero lie
     // in one region of zbytes bytes, placed by place_zero.
     struct PreparedBuild {
-        BuildArgs ba{};
+        DevColumn key{};
         HTView ht{};
-        uint2* buckets = nullptr;
         uint32_t nb = 0;
-        bool with_bloom = false;
-        uint32_t wlog2 = 0;
-        size_t zb_table = 0, zb_counts = 0, zb_cursor = 0, zb_bloom = 0, zb_flags = 256, zb_scan = 0;
+        uint32_t* rank1 = nullptr;
+        size_t zb_table = 0, zb_counts = 0, zb_bloom = 0, zb_flags = 256;
         size_t zbytes = 0;
-        uint32_t* cursor = nullptr;
+        uint32_t* table = nullptr;   // aggregation table (builds fed by probes)
+        uint32_t tlog2 = 0;
+        uint32_t* counts = nullptr;
         uint32_t* bloom = nullptr;
-        uint32_t* dflags = nullptr;
-        void* scan_status = nullptr;
+        uint32_t* dflags = nullptr;  // table flags, then the entries placed
+        bool with_bloom = false;
     };
     static size_t round256(size_t x) { return (x + 255) & ~size_t(255); }
 
-    PreparedBuild prepare_build(size_t pi, const Items& items, const SlotSources& src,
-                                const std::vector<HTView>& probes, int32_t key_stage = -1) {
-        const PipelinePlan& pp = ex_.pipelines[pi];
+    // Whether some slot of a build can be NULL: a column with NULLs, or a
+    // payload slot of a table that has NULL masks.
+    static bool nullable(const SlotSources& src, const std::vector<HTView>& probes) {
+        for (int j = 0; j < src.n; j++) {
+            const SlotSource& s = src.s[j];
+            if (s.kind == 0 ? (s.col.flags & kColNulls) != 0 : s.kind == 1 && probes[size_t(s.probe)].pnull) return true;
+        }
+        return false;
+    }
+
+    // aggregate: equal tuples are folded. A leaf (items are the input's rows
+    // 0..n-1, multiplicity 1) is built without eager aggregation: its tuples
+    // can only repeat where whole rows repeat (or, without payload, where keys
+    // repeat), and such copies may stay separate entries of multiplicity 1
+    // (the same result rows; the table's flags then report repeated keys and
+    // probes take the path for them). Folding pays off in builds fed by
+    // probes, where one row comes back once per match.
+    PreparedBuild prepare_build(size_t pi, uint32_t n, const SlotSources& src, const std::vector<HTView>& probes,
+                                bool aggregate) {
         PreparedBuild pb;
-        const uint32_t n = items.count;
         const uint32_t width = uint32_t(src.n);
-        BuildArgs& ba = pb.ba;
-        ba.in = items;
-        ba.key = col(uint32_t(pp.build_key));
-        // Keyed on an attribute of a probed input (key_stage >= 0: the stage
-        // of that probe in this pipeline), carried as its payload.
-        ba.key_stage = key_stage;
-        ba.key_slot = key_stage >= 0 ? pp.build_key_slot : 0;
-        ba.src = src;
-        ba.ps = make_probe_set(probes.data(), items.nprobes);
-        TupleBuf& tb = ba.tb;
-        // INT64 keys (no reference counterpart) keep their high halves beside
-        // the low ones and build no bloom filter.
-        const bool wide = ba.key.type == kInt64;
-        tb.keys = alloc<uint32_t>(n);
-        tb.keys_hi = wide ? alloc<uint32_t>(n) : nullptr;
-        tb.mult = alloc<uint64_t>(n);
-        tb.pay = alloc<uint64_t>(size_t(n) * std::max<uint32_t>(width, 1));
-        tb.pnull = alloc<uint32_t>(n);
-        tb.count = n;
-        tb.width = width;
-        ba.is_rep = alloc<uint32_t>(n);
-        ba.err = ctx_->d_err;
+        pb.key = col(uint32_t(ex_.pipelines[pi].build_key));
+        // INT64 keys (no reference counterpart) build no bloom filter.
+        const bool wide = pb.key.type == kInt64;
         // Sizes. Aggregation table: at least 2n slots. Buckets:
         // 2^max(bit_width(n), 4) (engine/op/Hashtable.cpp:94-104), sized by the
         // tuple count n, an upper bound of the distinct tuples, so the build
@@ -1100,66 +1096,45 @@ class Executor {
         // most 128 KiB (shared-memory staging); none when that leaves fewer
         // than 8 bits per key (over 131,072 tuples), where it would pass
         // most keys and its build would be contended atomics for nothing.
-        // A leaf (items are the input's rows 0..n-1, multiplicity 1) is built
-        // without eager aggregation: its tuples can only repeat where whole
-        // rows repeat (or, without payload, where keys repeat), and such
-        // copies may stay separate entries of multiplicity 1 (the same result
-        // rows; the table's flags then report repeated keys and probes take
-        // the path for them). Folding pays off in builds fed by probes, where
-        // one row comes back once per match.
-        ba.distinct = items.rows == nullptr && items.mult == nullptr && items.nprobes == 0 ? 1u : 0u;
-        ba.tlog2 = ba.distinct ? 1u : std::max<uint32_t>(1, bit_width(uint64_t(n) * 2));
-        const uint32_t nrep = n;
+        pb.tlog2 = aggregate ? std::max<uint32_t>(1, bit_width(uint64_t(n) * 2)) : 1u;
         // Autotuned: bucket count (fill factor) and bloom bits per key.
         const TuneConfig& tc = ctx_->tune;
-        const uint32_t blog2 = std::min<uint32_t>(31, std::max<uint32_t>(bit_width(nrep), 4) + tc.bucket_extra);
-        ba.shift = 64 - blog2;
+        const uint32_t blog2 = std::min<uint32_t>(31, std::max<uint32_t>(bit_width(n), 4) + tc.bucket_extra);
         pb.nb = uint32_t(1) << blog2;
-        pb.with_bloom = !wide && uint64_t(nrep) * 8 <= (uint64_t(32) << kBloomMaxLog2);
-        pb.wlog2 = pb.with_bloom ? std::min<uint32_t>(kBloomMaxLog2,
-                                                      std::max<uint32_t>(5, bit_width((uint64_t(nrep) * tc.bloom_bits + 31) / 32 - 1)))
-                                 : 0;
-        pb.zb_table = sizeof(uint32_t) << ba.tlog2;
-        pb.zb_counts = sizeof(uint32_t) * pb.nb;
-        pb.zb_cursor = sizeof(uint32_t) * pb.nb;
-        pb.zb_bloom = pb.with_bloom ? sizeof(uint32_t) << pb.wlog2 : 0;
-        pb.zb_scan = scan_status_bytes(pb.nb);
-        pb.zbytes = round256(pb.zb_table) + round256(pb.zb_counts) + round256(pb.zb_cursor) + round256(pb.zb_bloom) +
-                    pb.zb_flags + round256(pb.zb_scan);
-        // Bucket offsets go into the x words of the interleaved bucket array;
-        // the scatter fills each non-empty bucket's y (its first key).
-        pb.buckets = alloc<uint2>(size_t(pb.nb) + 1);
+        pb.with_bloom = !wide && uint64_t(n) * 8 <= (uint64_t(32) << kBloomMaxLog2);
         HTView& ht = pb.ht;
-        ht.buckets = pb.buckets;
-        ht.keys = alloc<uint32_t>(nrep);
-        ht.keys_hi = wide ? alloc<uint32_t>(nrep) : nullptr;
-        ht.mult = alloc<uint64_t>(nrep);
-        ht.pay = alloc<uint64_t>(size_t(nrep) * std::max<uint32_t>(width, 1));
-        ht.pnull = alloc<uint32_t>(nrep);
-        ht.shift = ba.shift;
-        ht.nentries = nrep;
+        ht.bloom_log2 = pb.with_bloom ? std::min<uint32_t>(kBloomMaxLog2,
+                                                           std::max<uint32_t>(5, bit_width((uint64_t(n) * tc.bloom_bits + 31) / 32 - 1)))
+                                      : 0;
+        pb.zb_table = aggregate ? sizeof(uint32_t) << pb.tlog2 : 0;
+        pb.zb_counts = sizeof(uint32_t) * pb.nb;
+        pb.zb_bloom = pb.with_bloom ? sizeof(uint32_t) << ht.bloom_log2 : 0;
+        pb.zbytes = round256(pb.zb_table) + round256(pb.zb_counts) + round256(pb.zb_bloom) + pb.zb_flags;
+        pb.rank1 = alloc<uint32_t>(n);
+        ht.buckets = alloc<uint4>(pb.nb);
+        ht.ent = alloc<uint64_t>(size_t(n) * (1 + width));
+        ht.mult = nullptr;
+        ht.pnull = nullable(src, probes) ? alloc<uint32_t>(n) : nullptr;
+        ht.shift = 64 - blog2;
+        ht.nentries = n;
         ht.width = width;
+        ht.wide = wide ? 1u : 0u;
         return pb;
     }
 
     // Points the build's zero-start buffers into z (zbytes, zeroed by the caller).
     static void place_zero(PreparedBuild& pb, uint8_t* z) {
-        pb.ba.table = reinterpret_cast<uint32_t*>(z);
+        pb.table = reinterpret_cast<uint32_t*>(z);
         z += round256(pb.zb_table);
-        pb.ba.counts = reinterpret_cast<uint32_t*>(z);
+        pb.counts = reinterpret_cast<uint32_t*>(z);
         z += round256(pb.zb_counts);
-        pb.cursor = reinterpret_cast<uint32_t*>(z);
-        z += round256(pb.zb_cursor);
-        pb.bloom = reinterpret_cast<uint32_t*>(z);
+        pb.bloom = pb.with_bloom ? reinterpret_cast<uint32_t*>(z) : nullptr;
         z += round256(pb.zb_bloom);
         pb.dflags = reinterpret_cast<uint32_t*>(z);
-        z += pb.zb_flags;
-        pb.scan_status = pb.zb_scan ? z : nullptr;
     }
 
     void publish(size_t pi, PreparedBuild& pb) {
-        pb.ht.bloom = pb.with_bloom ? pb.bloom : nullptr;
-        pb.ht.bloom_log2 = pb.wlog2;
+        pb.ht.bloom = pb.bloom;
         hts_[pi].view = pb.ht;
         hts_[pi].empty = false;
         hts_[pi].dflags = pb.dflags;
@@ -1167,24 +1142,48 @@ class Executor {
 
     bool build(size_t pi, const Items& items, const SlotSources& src, const std::vector<HTView>& probes,
                int32_t key_stage) {
-        PreparedBuild pb = prepare_build(pi, items, src, probes, key_stage);
+        const PipelinePlan& pp = ex_.pipelines[pi];
+        const bool leaf = items.rows == nullptr && items.mult == nullptr && items.nprobes == 0;
+        PreparedBuild pb = prepare_build(pi, items.count, src, probes, !leaf);
+        BuildArgs ba{};
+        ba.in = items;
+        ba.key = pb.key;
+        // Keyed on an attribute of a probed input (key_stage >= 0: the stage
+        // of that probe in this pipeline), carried as its payload.
+        ba.key_stage = key_stage;
+        ba.key_slot = key_stage >= 0 ? pp.build_key_slot : 0;
+        ba.src = src;
+        ba.ps = make_probe_set(probes.data(), items.nprobes);
+        TupleBuf& tb = ba.tb;
+        tb.count = items.count;
+        tb.width = uint32_t(src.n);
+        tb.keys = alloc<uint64_t>(tb.count);
+        tb.mult = alloc<uint64_t>(tb.count);
+        tb.pay = alloc<uint64_t>(size_t(tb.count) * std::max<uint32_t>(tb.width, 1));
+        tb.pnull = pb.ht.pnull ? alloc<uint32_t>(tb.count) : nullptr;
+        pb.ht.mult = alloc<uint64_t>(tb.count);
         // Sideways restriction by a batched leaf's filter (built on the main
         // stream before any pipeline that probes).
-        const int32_t r = ex_.pipelines[pi].restrict_by;
+        const int32_t r = pp.restrict_by;
         if (r >= 0 && ctx_->sideways && batched_[size_t(r)] && restricted_by_[size_t(r)] < 0 &&
-            hts_[size_t(r)].view.bloom && pb.ba.key.type == kInt32) {
-            pb.ba.rbloom = hts_[size_t(r)].view.bloom;
-            pb.ba.rlog2w = hts_[size_t(r)].view.bloom_log2;
+            hts_[size_t(r)].view.bloom && pb.key.type == kInt32) {
+            ba.rbloom = hts_[size_t(r)].view.bloom;
+            ba.rlog2w = hts_[size_t(r)].view.bloom_log2;
             restricted_by_[pi] = r;
         }
         uint8_t* z = alloc<uint8_t>(pb.zbytes);
         BJ_CK(cudaMemsetAsync(z, 0, pb.zbytes, st_));
         place_zero(pb, z);
-        launched(emit_aggregate(pb.ba, st_));
-        launched(scan_exclusive_u32_zeroed(pb.ba.counts, reinterpret_cast<uint32_t*>(pb.buckets), pb.nb,
-                                           pb.scan_status, ctx_->d_err, st_, 2));
-        launched(scatter_bloom(pb.ba.tb, pb.ba.is_rep, pb.ba.shift, pb.buckets, pb.cursor, pb.ht,
-                               pb.with_bloom ? pb.bloom : nullptr, pb.wlog2, ctx_->d_err, st_));
+        ba.table = pb.table;
+        ba.tlog2 = pb.tlog2;
+        ba.rank1 = pb.rank1;
+        ba.counts = pb.counts;
+        ba.ht = pb.ht;
+        ba.bloom = pb.bloom;
+        ba.err = ctx_->d_err;
+        ba.distinct = leaf ? 1u : 0u;
+        launched(emit_aggregate(ba, st_));
+        launched(place_tuples(tb, pb.rank1, pb.counts, pb.dflags + 2, pb.nb, pb.ht, ctx_->d_err, st_));
         publish(pi, pb);
         if (ctx_->tape_mode != 2) launched(ht_flags(hts_[pi].view, pb.nb, pb.dflags, ctx_->num_sms, st_));
         return true;
@@ -1193,55 +1192,51 @@ class Executor {
     static_assert(size_t(kMaxLeafSlots) == kLeafBatchMaxSlots, "the planner marks restrictions on batched leaves");
     // The builds of the pipelines in `leaves` (inputs that probe nothing),
     // kMaxLeafBuilds at a time, each pass one launch over all of them on the
-    // current stream, with one memset for all their zero-start buffers.
+    // current stream, with one memset for all their zero-start buffers (one
+    // launch and no memset when all of them are small).
     // by[p] >= 0: leaf p's rows are restricted by the bloom filter of the
     // table of pipeline by[p] (built earlier on this stream), when it has one.
     void build_leaf_batch(const std::vector<size_t>& leaves, const std::vector<int32_t>& by) {
         for (size_t i0 = 0; i0 < leaves.size(); i0 += kMaxLeafBuilds) {
             const size_t i1 = std::min(leaves.size(), i0 + kMaxLeafBuilds);
             std::vector<PreparedBuild> pbs;
+            std::vector<SlotSources> srcs;
             size_t zbytes = 0;
+            bool small = true;
             for (size_t i = i0; i < i1; i++) {
                 const size_t pi = leaves[i];
                 pipes_++;
                 const PipelinePlan& pp = ex_.pipelines[pi];
-                Items items{};
-                items.count = uint32_t(ex_.inputs[pp.input].rows);
                 SlotSources src{};
                 src.n = int(pp.slots.size());
                 for (size_t j = 0; j < pp.slots.size(); j++) {
                     src.s[j].kind = 0;  // a leaf's slots are its own columns
                     src.s[j].col = col(pp.slots[j].attr);
                 }
-                pbs.push_back(prepare_build(pi, items, src, {}));
+                const uint32_t rows = uint32_t(ex_.inputs[pp.input].rows);
+                pbs.push_back(prepare_build(pi, rows, src, {}, false));
+                srcs.push_back(src);
                 zbytes += pbs.back().zbytes;
+                small = small && rows <= kClusterLeafRows;
             }
             uint8_t* z = alloc<uint8_t>(zbytes);
-            BJ_CK(cudaMemsetAsync(z, 0, zbytes, st_));
+            if (!small) BJ_CK(cudaMemsetAsync(z, 0, zbytes, st_));
             LeafBatch batch{};
             batch.err = ctx_->d_err;
             batch.flags = ctx_->tape_mode != 2 ? 1 : 0;
-            size_t zoff = 0;
             for (size_t k = 0; k < pbs.size(); k++) {
                 PreparedBuild& pb = pbs[k];
-                place_zero(pb, z + zoff);
-                zoff += pb.zbytes;
+                place_zero(pb, z);
+                z += pb.zbytes;
                 LeafBuild& L = batch.l[batch.n];
-                L.key = pb.ba.key;
-                L.nslots = pb.ba.src.n;
-                for (int j = 0; j < pb.ba.src.n; j++) L.cols[j] = pb.ba.src.s[j].col;
-                L.tb = pb.ba.tb;
-                L.table = pb.ba.table;
-                L.tlog2 = pb.ba.tlog2;
-                L.is_rep = pb.ba.is_rep;
-                L.counts = pb.ba.counts;
-                L.shift = pb.ba.shift;
-                L.distinct = pb.ba.distinct;
-                L.buckets = pb.buckets;
+                L.key = pb.key;
+                L.nslots = srcs[k].n;
+                for (int j = 0; j < srcs[k].n; j++) L.cols[j] = srcs[k].s[j].col;
+                L.rows = pb.ht.nentries;
+                L.rank1 = pb.rank1;
+                L.counts = pb.counts;
                 L.nb = pb.nb;
-                L.cursor = pb.cursor;
-                L.bloom = pb.with_bloom ? pb.bloom : nullptr;
-                L.log2w = pb.wlog2;
+                L.bloom = pb.bloom;
                 L.dflags = pb.dflags;
                 L.ht = pb.ht;
                 const int32_t r = by[leaves[i0 + k]];
@@ -1250,14 +1245,11 @@ class Executor {
                     L.rlog2w = hts_[size_t(r)].view.bloom_log2;
                     restricted_by_[leaves[i0 + k]] = r;
                 }
-                batch.tuple_start[batch.n + 1] = batch.tuple_start[batch.n] + pb.ba.tb.count;
-                batch.block_start[batch.n + 1] = batch.block_start[batch.n] + (pb.ba.tb.count + 255) / 256;
-                batch.tile_start[batch.n + 1] =
-                    batch.tile_start[batch.n] + (pb.nb + kLeafTileBuckets - 1) / kLeafTileBuckets;
+                batch.block_start[batch.n + 1] = batch.block_start[batch.n] + (L.rows + 255) / 256;
+                batch.tile_start[batch.n + 1] = batch.tile_start[batch.n] + (L.nb + kBucketTile - 1) / kBucketTile;
                 batch.n++;
             }
-            batch.tile_sums = alloc<uint32_t>(batch.tile_start[batch.n]);
-            launched(build_leaves(batch, st_));
+            launched(small ? build_cluster_leaves(batch, st_) : build_leaves(batch, st_));
             for (size_t k = 0; k < pbs.size(); k++) publish(leaves[i0 + k], pbs[k]);
         }
     }

@@ -782,8 +782,8 @@ BJ_API int bj_plan_scratch_estimate(bj_context* ctx, const bj_plan* plan, bj_res
             total += 2.0 * n * (12.0 + 4.0 * double(pp.probes.size()));  // items in and out of the stages
             if (pp.build_key >= 0) {
                 // tuples and table entries (key, mult, payload, NULL mask,
-                // representative flag), buckets, aggregation slots
-                total += n * (2.0 * (20.0 + 8.0 * w) + 8.0) + 16.0 * std::exp2(double(bit_width(uint64_t(n) + 1)));
+                // rank), buckets and their counts, aggregation slots
+                total += n * (2.0 * (20.0 + 8.0 * w) + 8.0) + 20.0 * std::exp2(double(bit_width(uint64_t(n) + 1)));
             } else {
                 total += n * 17.0 * double(ex.out_slot.size());  // flat values + result pages
             }

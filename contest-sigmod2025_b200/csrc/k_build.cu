@@ -7,40 +7,50 @@
 // key and payload are equal (eager aggregation, engine/op/Hashtable.cpp:
 // 208-263). Sizing: 2^max(bit_width(n), 4) buckets (Hashtable.cpp:94-104).
 //
-// On the GPU the build is three passes:
-//  1. emit (each thread writes its tuple: key, NULL mask, payload,
-//     multiplicity), then eager aggregation and bucket counts (K6) in the next
-//     launch: each tuple's index goes into an open-addressing table keyed by
-//     the whole tuple. The first copy of each distinct tuple claims a slot
-//     with atomicCAS and becomes its representative (and counts itself into
-//     its bucket); every other copy adds its multiplicity to the
-//     representative with atomicAdd. Unlike the reference, which only merges
-//     with the current bucket head, this folds every duplicate. Builds whose
-//     tuples cannot repeat (BuildArgs::distinct) count in the emit and skip
-//     the aggregation launch.
-//  2. an exclusive scan of the bucket counts (CSR offsets), then a scatter of
-//     the representatives into their bucket's contiguous range that also sets
-//     their bits in a blocked bloom filter (K3/K4). The same bucket index as
-//     the reference: key_hash(key) >> shift. The filter is at most 128 KiB so
-//     scans can stage it in shared memory; probes consult it before touching
-//     the buckets.
-//  3. flags of the finished table (repeated keys, multiplicities above 1).
+// On the GPU the build is a counting sort by bucket. Counting a row into its
+// bucket also gives its rank there (the atomic's return value), so the pass
+// that places the rows needs no second atomic; a bucket's range may lie
+// anywhere, so a block takes the ranges of its 1024 buckets with one atomic
+// instead of a device-wide prefix sum. The same bucket index as the
+// reference: key_hash(key) >> shift. The blocked bloom filter (K3) is set in
+// the counting pass; it is at most 128 KiB so scans can stage it in shared
+// memory, and probes consult it before touching the buckets.
+//
+//  * A leaf (an input that probes nothing) places its rows straight from the
+//    column pages: nothing is written between the passes but the ranks. When
+//    all leaves of a query are small, one launch builds them, a cluster of
+//    CTAs each (k_leaf_cluster).
+//  * A build fed by probes writes its tuples first (key, NULL mask, payload,
+//    multiplicity), then folds equal ones (eager aggregation, K6) in the next
+//    launch: each tuple's index goes into an open-addressing table keyed by
+//    the whole tuple. The first copy of each distinct tuple claims a slot with
+//    atomicCAS, becomes its representative and counts itself into its bucket;
+//    every other copy adds its multiplicity to the representative. Unlike the
+//    reference, which only merges with the current bucket head, this folds
+//    every duplicate. Builds whose tuples cannot repeat (BuildArgs::distinct)
+//    count in the emit and skip the aggregation launch.
+//  * The flags of the finished table (repeated keys, multiplicities above 1)
+//    come from one pass over the buckets.
 // Every buffer that must start at zero is cleared by one memset per build.
+//
+// Bound: the random sectors of the counts, buckets and entries in L2. The leaf
+// of 1M rows with one INT64 payload column, count + ranges + place: 55 us,
+// where writing the tuples first, an ordered prefix sum and a scatter into
+// separate key, multiplicity, NULL mask and payload arrays took 81 us.
 #include "launch.h"
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
-#include <cstdlib>
 
 namespace bj {
 namespace {
 
-__device__ __forceinline__ uint64_t tuple_key(const TupleBuf& t, uint32_t i) {
-    return uint64_t(t.keys[i]) | (t.keys_hi ? uint64_t(t.keys_hi[i]) << 32 : 0ull);
-}
+namespace cg = cooperative_groups;
 
 __device__ __forceinline__ uint64_t tuple_hash(const TupleBuf& t, uint32_t i) {
-    uint64_t h = mix64(uint64_t(t.keys[i]) ^ (uint64_t(t.pnull[i]) << 32));
-    if (t.keys_hi) h = mix64(h ^ t.keys_hi[i]);
+    uint64_t h = mix64(t.keys[i]);
+    if (t.pnull) h = mix64(h ^ t.pnull[i]);
     const uint64_t* p = t.pay + size_t(i) * t.width;
     for (uint32_t j = 0; j < t.width; j++) h = mix64(h ^ (p[j] + 0x9E3779B97F4A7C15ull * (j + 1)));
     return h;
@@ -48,8 +58,8 @@ __device__ __forceinline__ uint64_t tuple_hash(const TupleBuf& t, uint32_t i) {
 
 // Tuple a (written by another thread, read through L2) equals tuple b.
 __device__ __forceinline__ bool tuple_equal_cg(const TupleBuf& t, uint32_t a, uint32_t b) {
-    if (__ldcg(t.keys + a) != t.keys[b] || __ldcg(t.pnull + a) != t.pnull[b]) return false;
-    if (t.keys_hi && __ldcg(t.keys_hi + a) != t.keys_hi[b]) return false;
+    if (__ldcg(t.keys + a) != t.keys[b]) return false;
+    if (t.pnull && __ldcg(t.pnull + a) != t.pnull[b]) return false;
     const uint64_t* pa = t.pay + size_t(a) * t.width;
     const uint64_t* pb = t.pay + size_t(b) * t.width;
     for (uint32_t j = 0; j < t.width; j++)
@@ -57,55 +67,36 @@ __device__ __forceinline__ bool tuple_equal_cg(const TupleBuf& t, uint32_t a, ui
     return true;
 }
 
-// Where a build's tuples go (the parts of BuildArgs the emit writes).
-struct EmitTarget {
-    TupleBuf tb;
-    uint32_t* table;
-    uint32_t tlog2;
-    uint32_t* is_rep;
-    uint32_t* counts;
-    uint32_t shift;
-    uint32_t distinct;
-    uint32_t* err;
-};
+// Counts key kv into its bucket and the filter; returns 1 + its rank there.
+__device__ __forceinline__ uint32_t count_key(uint32_t* counts, const HTView& ht, uint32_t* bloom, uint64_t kv) {
+    if (bloom) {  // INT32 keys only (INT64 tables are built without a filter)
+        const uint32_t hh = key_hash_hi(uint32_t(kv));
+        atomicOr(&bloom[bloom_word_hi(hh, ht.bloom_log2)], bloom_bits_fast(hh, hh >> 5));
+    }
+    return 1 + atomicAdd(&counts[bucket_of(kv, ht.wide != 0, ht.shift)], 1u);
+}
 
-// Writes tuple i of a build (key kv; multiplicity m, 0 for a NULL key; the
-// slot values from slot(j, v), false for NULL). A zero-multiplicity tuple
-// represents nothing; a tuple of a distinct build represents itself and is
-// counted into its bucket here. The others are folded by aggregate_tuple in
-// a later launch, which sees every tuple written (no fence needed here).
-template <typename Slot>
-__device__ __forceinline__ void emit_tuple_to(const EmitTarget& a, uint32_t i, uint64_t kv, uint64_t m, int nslots,
-                                              Slot&& slot) {
-    const TupleBuf& t = a.tb;
-    t.keys[i] = uint32_t(kv);
-    if (t.keys_hi) t.keys_hi[i] = uint32_t(kv >> 32);
-    t.mult[i] = m;
-    uint32_t nulls = 0;
-    for (int j = 0; j < nslots; j++) {
-        uint64_t v = 0;
-        if (!slot(j, v)) {
-            nulls |= 1u << j;
-            v = 0;
-        }
-        t.pay[size_t(i) * t.width + j] = v;
+// Where the entry of key kv with this rank goes in a table whose buckets have
+// their ranges; the bucket's first two keys are written into it. False, with
+// an error, past the table's end.
+__device__ __forceinline__ bool place_key(const HTView& ht, uint64_t kv, uint32_t rank, uint32_t* err, uint32_t& pos) {
+    uint4* b = const_cast<uint4*>(ht.buckets) + bucket_of(kv, ht.wide != 0, ht.shift);
+    pos = __ldcg(&b->x) + rank;  // (another SM may have written it in this launch)
+    if (pos >= ht.nentries) {
+        record_error(err, kErrCapacity);
+        return false;
     }
-    t.pnull[i] = nulls;
-    if (m == 0) {
-        a.is_rep[i] = 0;
-        return;
-    }
-    if (a.distinct) {
-        a.is_rep[i] = 1;
-        atomicAdd(&a.counts[bucket_of(kv, t.keys_hi != nullptr, a.shift)], 1u);
-    }
+    if (rank == 0) b->z = uint32_t(kv);
+    if (rank == 1) b->w = uint32_t(kv);
+    const_cast<uint64_t*>(ht.ent)[size_t(pos) * (1 + ht.width)] = kv;
+    return true;
 }
 
 // Eager aggregation of tuple i (every tuple written by an earlier launch):
 // the first copy of a distinct tuple to claim a slot of the open-addressing
 // table keyed by the whole tuple represents it and is counted into its
 // bucket; every other copy adds its multiplicity to the representative.
-__device__ __forceinline__ void aggregate_tuple(const EmitTarget& a, uint32_t i) {
+__device__ __forceinline__ void aggregate_tuple(const BuildArgs& a, uint32_t i) {
     const TupleBuf& t = a.tb;
     const uint64_t m = t.mult[i];  // only a representative's grows, after it claimed its slot
     if (m == 0) return;
@@ -114,26 +105,25 @@ __device__ __forceinline__ void aggregate_tuple(const EmitTarget& a, uint32_t i)
     for (uint32_t step = 0; step <= mask; step++) {
         const uint32_t cur = atomicCAS(&a.table[pos], 0u, i + 1);
         if (cur == 0) {
-            a.is_rep[i] = 1;
-            atomicAdd(&a.counts[bucket_of(tuple_key(t, i), t.keys_hi != nullptr, a.shift)], 1u);
+            a.rank1[i] = count_key(a.counts, a.ht, a.bloom, t.keys[i]);
             return;
         }
         if (tuple_equal_cg(t, cur - 1, i)) {
             atomicAdd(reinterpret_cast<unsigned long long*>(&t.mult[cur - 1]), (unsigned long long)m);
-            a.is_rep[i] = 0;
+            a.rank1[i] = 0;
             return;
         }
         pos = (pos + 1) & mask;
     }
-    a.is_rep[i] = 0;
+    a.rank1[i] = 0;
     record_error(a.err, kErrCapacity);
 }
 
-__device__ __forceinline__ EmitTarget emit_target(const BuildArgs& a) {
-    return EmitTarget{a.tb, a.table, a.tlog2, a.is_rep, a.counts, a.shift, a.distinct, a.err};
-}
-
-// Writes tuple i of a build.
+// Writes tuple i of a build (multiplicity 0 for a NULL key or one that a
+// sideways filter cannot hold: such a tuple represents nothing). A tuple of a
+// distinct build represents itself and is counted into its bucket here; the
+// others are folded by aggregate_tuple in a later launch, which sees every
+// tuple written (no fence needed here).
 __device__ __forceinline__ void emit_tuple(const BuildArgs& a, uint32_t i) {
     const uint32_t row = item_row(a.in, i);
     uint64_t kv = 0;
@@ -142,16 +132,31 @@ __device__ __forceinline__ void emit_tuple(const BuildArgs& a, uint32_t i) {
         // The key is an attribute of an input probed by this pipeline.
         const HTView& src = a.ps.ht[a.key_stage];
         const uint32_t e = a.in.ents[a.key_stage][i];
-        key_ok = !((src.pnull[e] >> a.key_slot) & 1);
-        if (key_ok) kv = src.pay[size_t(e) * src.width + a.key_slot];
+        key_ok = !ht_slot_null(src, e, a.key_slot);
+        if (key_ok) kv = ht_slot(src, e, a.key_slot);
     } else {
         key_ok = row < a.key.nrows && col_get(a.key, row, kv);
         if (row >= a.key.nrows) record_error(a.err, kErrRowRange);
     }
     if (key_ok && a.rbloom && !bloom_may_contain(a.rbloom, a.rlog2w, uint32_t(kv))) key_ok = false;
     const uint64_t m = key_ok ? item_mult(a.in, i) : 0ull;
-    emit_tuple_to(emit_target(a), i, kv, m, a.src.n,
-                  [&](int j, uint64_t& v) { return slot_value(a.src.s[j], a.in, i, row, a.ps, v); });
+    const TupleBuf& t = a.tb;
+    t.keys[i] = kv;
+    t.mult[i] = m;
+    uint32_t nulls = 0;
+    for (int j = 0; j < a.src.n; j++) {
+        uint64_t v = 0;
+        if (!slot_value(a.src.s[j], a.in, i, row, a.ps, v)) {
+            nulls |= 1u << j;
+            v = 0;
+        }
+        t.pay[size_t(i) * t.width + j] = v;
+    }
+    if (t.pnull) t.pnull[i] = nulls;
+    if (m == 0)
+        a.rank1[i] = 0;
+    else if (a.distinct)
+        a.rank1[i] = count_key(a.counts, a.ht, a.bloom, kv);
 }
 
 __global__ void __launch_bounds__(256) k_emit(BuildArgs a) {
@@ -161,80 +166,23 @@ __global__ void __launch_bounds__(256) k_emit(BuildArgs a) {
 
 __global__ void __launch_bounds__(256) k_aggregate(BuildArgs a) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < a.tb.count) aggregate_tuple(emit_target(a), i);
+    if (i < a.tb.count) aggregate_tuple(a, i);
 }
 
-// Places representative i in its bucket's range and sets its bloom bits.
-__device__ __forceinline__ void scatter_tuple(const TupleBuf& t, const uint32_t* __restrict__ is_rep, uint32_t shift,
-                                              uint2* __restrict__ buckets, uint32_t* __restrict__ cursor,
-                                              const HTView& ht, uint32_t* __restrict__ bloom, uint32_t log2w,
-                                              uint32_t* __restrict__ err, uint32_t i) {
-    if (!is_rep[i]) return;
-    const uint32_t key = t.keys[i];
-    const uint32_t b = bucket_of(tuple_key(t, i), t.keys_hi != nullptr, shift);
-    const uint32_t first = buckets[b].x;
-    const uint32_t pos = first + atomicAdd(&cursor[b], 1u);
-    if (bloom) {  // INT32 keys only (INT64 tables are built without a filter)
-        const uint32_t hh = key_hash_hi(key);
-        atomicOr(&bloom[bloom_word_hi(hh, log2w)], bloom_bits_fast(hh, hh >> 5));
-    }
-    if (pos >= buckets[b + 1].x || pos >= ht.nentries) {
-        record_error(err, kErrCapacity);
-        return;
-    }
-    if (pos == first) buckets[b].y = key;  // the bucket's first entry
-    const_cast<uint32_t*>(ht.keys)[pos] = key;
-    if (t.keys_hi) const_cast<uint32_t*>(ht.keys_hi)[pos] = t.keys_hi[i];
+// Places the representatives as entries of their buckets.
+__global__ void __launch_bounds__(256) k_place(TupleBuf t, const uint32_t* __restrict__ rank1, HTView ht,
+                                               uint32_t* __restrict__ err) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= t.count) return;
+    const uint32_t r1 = rank1[i];
+    uint32_t pos;
+    if (!r1 || !place_key(ht, t.keys[i], r1 - 1, err, pos)) return;
     const_cast<uint64_t*>(ht.mult)[pos] = t.mult[i];
-    const_cast<uint32_t*>(ht.pnull)[pos] = t.pnull[i];
-    uint64_t* dst = const_cast<uint64_t*>(ht.pay) + size_t(pos) * t.width;
+    if (ht.pnull) const_cast<uint32_t*>(ht.pnull)[pos] = t.pnull[i];
+    uint64_t* dst = const_cast<uint64_t*>(ht.ent) + size_t(pos) * (1 + ht.width) + 1;
     const uint64_t* src = t.pay + size_t(i) * t.width;
     for (uint32_t j = 0; j < t.width; j++) dst[j] = src[j];
 }
-
-__global__ void k_scatter_bloom(TupleBuf t, const uint32_t* __restrict__ is_rep, uint32_t shift,
-                                uint2* __restrict__ buckets, uint32_t* __restrict__ cursor, HTView ht,
-                                uint32_t* __restrict__ bloom, uint32_t log2w, uint32_t* __restrict__ err) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < t.count) scatter_tuple(t, is_rep, shift, buckets, cursor, ht, bloom, log2w, err, i);
-}
-
-// Flags of entry e of a built table (see ht_flags).
-__device__ __forceinline__ void flag_entry(const HTView& ht, uint32_t e, uint32_t* __restrict__ flags) {
-    if (ht.mult[e] > 1) flags[1] = 1;
-    const uint64_t key = ht_key(ht, e);
-    uint32_t b = ht_bucket(ht, key);
-    uint32_t s = ht.buckets[b].x;
-    if (e - s > 256) {
-        flags[0] = 1;  // long bucket: assume repeats (only steers capacity choices)
-        return;
-    }
-    for (uint32_t j = s; j < e; j++)
-        if (ht_key_eq(ht, j, key)) {
-            flags[0] = 1;
-            break;
-        }
-}
-
-__global__ void k_ht_flags(HTView ht, uint32_t nbuckets, uint32_t* __restrict__ flags) {
-    const uint32_t n = ht.buckets[nbuckets].x;  // entries actually stored
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
-        flag_entry(ht, e, flags);
-}
-
-// ---- leaf builds of a query, batched ----
-//
-// Builds whose input probes nothing (a query's leaves) run together: each of
-// the passes above is one launch over all builds' tuples or buckets at once
-// (blocks find their build from prefix sums of the builds' sizes), so the
-// leaves of a query cost four launches (five with the table flags) instead
-// of three or four per build, and the builds' small grids fill the GPU
-// together: 1. emit + aggregation + bucket counts; 2a. sums of bucket tiles
-// of 1024 counts; 2b. each tile's exclusive offsets (the sums of the earlier
-// tiles of its build plus a block scan) into the buckets' x words, and the
-// build's total into bucket nb; 3. scatter + bloom; 4. table flags.
-
-constexpr uint32_t kLeafTile = 1024;  // bucket counts per tile in pass 2
 
 __device__ __forceinline__ int leaf_of(const uint32_t* start, int n, uint32_t x) {
     int b = 0;
@@ -242,20 +190,8 @@ __device__ __forceinline__ int leaf_of(const uint32_t* start, int n, uint32_t x)
     return b;
 }
 
-__device__ __forceinline__ uint32_t block_sum_u32(uint32_t v) {
-    __shared__ uint32_t ws[8];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
-    __syncthreads();
-    uint32_t t = 0;
-    for (int w = 0; w < int(blockDim.x >> 5); w++) t += ws[w];
-    __syncthreads();
-    return t;
-}
-
 // Exclusive prefix of v over the block (256 threads), in thread order.
-__device__ __forceinline__ uint32_t block_excl_u32(uint32_t v) {
+__device__ __forceinline__ uint32_t block_excl_u32(uint32_t v, uint32_t& total) {
     __shared__ uint32_t ws[8];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t inc = v;
@@ -267,99 +203,174 @@ __device__ __forceinline__ uint32_t block_excl_u32(uint32_t v) {
     if (lane == 31) ws[warp] = inc;
     __syncthreads();
     uint32_t base = 0;
-    for (uint32_t w = 0; w < warp; w++) base += ws[w];
-    __syncthreads();
+    total = 0;
+    for (uint32_t w = 0; w < 8; w++) {
+        if (w < warp) base += ws[w];
+        total += ws[w];
+    }
     return base + inc - v;
 }
 
-// Blocks of 256 tuples, each within one build (block_start: prefix of the
+// Bucket ranges: a block takes a tile of 1024 buckets of one build, reserves
+// the entries it counts with one atomic and writes each bucket's first entry
+// and length (thread k: counts 4k .. 4k + 3; nb is a multiple of 16).
+__global__ void __launch_bounds__(256) k_bucket_ranges(BucketTiles t) {
+    const int b = leaf_of(t.tile_start, t.n, blockIdx.x);
+    const uint32_t i0 = (blockIdx.x - t.tile_start[b]) * kBucketTile + 4 * threadIdx.x;
+    const BucketTiles::Build& B = t.b[b];
+    uint4 c = make_uint4(0, 0, 0, 0);
+    if (i0 < B.nb) c = *reinterpret_cast<const uint4*>(B.counts + i0);
+    uint32_t total;
+    uint32_t run = block_excl_u32(c.x + c.y + c.z + c.w, total);
+    __shared__ uint32_t base;
+    if (threadIdx.x == 0) base = total ? atomicAdd(B.entries, total) : 0u;
+    __syncthreads();
+    if (i0 >= B.nb) return;
+    run += base;
+    uint4* out = B.buckets + i0;
+    out[0] = make_uint4(run, c.x, 0, 0);
+    out[1] = make_uint4(run + c.x, c.y, 0, 0);
+    out[2] = make_uint4(run + c.x + c.y, c.z, 0, 0);
+    out[3] = make_uint4(run + c.x + c.y + c.z, c.w, 0, 0);
+}
+
+// Flags of bucket b's entries (see ht_flags).
+__device__ __forceinline__ void flag_bucket(const HTView& ht, uint32_t b, uint32_t* __restrict__ flags) {
+    const uint4 k = __ldcg(ht.buckets + b);
+    if (ht.mult)
+        for (uint32_t j = 0; j < k.y; j++)
+            if (ht.mult[k.x + j] > 1) flags[1] = 1;
+    if (k.y < 2) return;
+    if (k.y > 256) {
+        flags[0] = 1;  // long bucket: assume repeats (only steers capacity choices)
+        return;
+    }
+    if (k.y == 2 && k.z != k.w) return;
+    for (uint32_t i = 1; i < k.y; i++) {
+        const uint64_t key = __ldcg(ht.ent + size_t(k.x + i) * (1 + ht.width));
+        for (uint32_t j = 0; j < i; j++)
+            if (__ldcg(ht.ent + size_t(k.x + j) * (1 + ht.width)) == key) {
+                flags[0] = 1;
+                return;
+            }
+    }
+}
+
+__global__ void __launch_bounds__(256) k_ht_flags(HTView ht, uint32_t nbuckets, uint32_t* __restrict__ flags) {
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nbuckets; b += gridDim.x * blockDim.x)
+        flag_bucket(ht, b, flags);
+}
+
+// ---- leaf builds of a query, batched ----
+//
+// The leaves of a query build together, each pass one launch over all of
+// them (blocks find their build from prefix sums of the builds' sizes).
+
+// Row i's key when the row takes part in the build: not NULL and, under a
+// sideways restriction, possibly in the restricting filter (a row whose key
+// it cannot hold joins nothing).
+__device__ __forceinline__ bool leaf_key(const LeafBuild& L, uint32_t i, uint64_t& kv) {
+    return col_get(L.key, i, kv) && (!L.rbloom || bloom_may_contain(L.rbloom, L.rlog2w, uint32_t(kv)));
+}
+
+// Row i's entry: its key and the values of its payload columns.
+__device__ __forceinline__ void leaf_place(const LeafBuild& L, uint32_t i, uint64_t kv, uint32_t rank, uint32_t* err) {
+    uint32_t pos;
+    if (!place_key(L.ht, kv, rank, err, pos)) return;
+    uint64_t* dst = const_cast<uint64_t*>(L.ht.ent) + size_t(pos) * (1 + L.ht.width) + 1;
+    uint32_t nulls = 0;
+    for (int j = 0; j < L.nslots; j++) {
+        uint64_t v = 0;
+        if (!column_value(L.cols[j], i, v)) {
+            nulls |= 1u << j;
+            v = 0;
+        }
+        dst[j] = v;
+    }
+    if (L.ht.pnull) const_cast<uint32_t*>(L.ht.pnull)[pos] = nulls;
+}
+
+// Blocks of 256 rows, each within one build (block_start: prefix of the
 // builds' block counts), so a block's build and its arguments are uniform.
-__device__ __forceinline__ bool leaf_tuple(const LeafBatch& B, int& b, uint32_t& i) {
+__device__ __forceinline__ bool leaf_row(const LeafBatch& B, int& b, uint32_t& i) {
     b = leaf_of(B.block_start, B.n, blockIdx.x);
     i = (blockIdx.x - B.block_start[b]) * blockDim.x + threadIdx.x;
-    return i < B.tuple_start[b + 1] - B.tuple_start[b];
+    return i < B.l[b].rows;
 }
 
-__device__ __forceinline__ EmitTarget leaf_target(const LeafBatch& B, const LeafBuild& L) {
-    return EmitTarget{L.tb, L.table, L.tlog2, L.is_rep, L.counts, L.shift, L.distinct, B.err};
-}
-
-__global__ void __launch_bounds__(256) k_leaf_emit(LeafBatch B) {
+__global__ void __launch_bounds__(256) k_leaf_count(LeafBatch B) {
     int b;
     uint32_t i;
-    if (!leaf_tuple(B, b, i)) return;
+    if (!leaf_row(B, b, i)) return;
     const LeafBuild& L = B.l[b];
-    // A leaf's item i is row i, multiplicity 1; its slots are its own columns.
-    // A row whose key the restricting filter cannot hold joins nothing: it
-    // is written with multiplicity 0, like a NULL key.
     uint64_t kv = 0;
-    const bool key_ok = col_get(L.key, i, kv) && (!L.rbloom || bloom_may_contain(L.rbloom, L.rlog2w, uint32_t(kv)));
-    emit_tuple_to(leaf_target(B, L), i, kv, key_ok ? 1ull : 0ull, L.nslots,
-                  [&](int j, uint64_t& v) { return column_value(L.cols[j], i, v); });
+    L.rank1[i] = leaf_key(L, i, kv) ? count_key(L.counts, L.ht, L.bloom, kv) : 0u;
 }
 
-// Aggregation pass of the leaves that are not distinct (launched only when
-// some leaf of the batch is not).
-__global__ void __launch_bounds__(256) k_leaf_aggregate(LeafBatch B) {
+__global__ void __launch_bounds__(256) k_leaf_place(LeafBatch B) {
     int b;
     uint32_t i;
-    if (!leaf_tuple(B, b, i)) return;
+    if (!leaf_row(B, b, i)) return;
     const LeafBuild& L = B.l[b];
-    if (!L.distinct) aggregate_tuple(leaf_target(B, L), i);
+    const uint32_t r1 = L.rank1[i];
+    uint64_t kv = 0;
+    if (r1 && col_get(L.key, i, kv)) leaf_place(L, i, kv, r1 - 1, B.err);
 }
 
-// One block per tile of 1024 bucket counts.
-__global__ void __launch_bounds__(256) k_leaf_tile_sums(LeafBatch B) {
-    const uint32_t tile = blockIdx.x;
-    const int b = leaf_of(B.tile_start, B.n, tile);
-    const LeafBuild& L = B.l[b];
-    const uint32_t i0 = (tile - B.tile_start[b]) * kLeafTile, i1 = min(i0 + kLeafTile, L.nb);
-    uint32_t v = 0;
-    for (uint32_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) v += L.counts[i];
-    v = block_sum_u32(v);
-    if (threadIdx.x == 0) B.tile_sums[tile] = v;
-}
-
-// One block per tile; thread k takes counts 4k..4k+3 of the tile.
-__global__ void __launch_bounds__(256) k_leaf_offsets(LeafBatch B) {
-    const uint32_t tile = blockIdx.x;
-    const int b = leaf_of(B.tile_start, B.n, tile);
-    const LeafBuild& L = B.l[b];
-    const uint32_t first = B.tile_start[b];
-    uint32_t before = 0;
-    for (uint32_t k = first + threadIdx.x; k < tile; k += blockDim.x) before += B.tile_sums[k];
-    before = block_sum_u32(before);
-    const uint32_t i0 = (tile - first) * kLeafTile + 4 * threadIdx.x;
-    uint32_t c[4], own = 0;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        c[j] = i0 + j < L.nb ? L.counts[i0 + j] : 0u;
-        own += c[j];
-    }
-    uint32_t run = before + block_excl_u32(own);
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        if (i0 + j < L.nb) L.buckets[i0 + j].x = run;
-        run += c[j];
-    }
-    if (i0 < L.nb && i0 + 4 >= L.nb) L.buckets[L.nb].x = run;  // the build's total
-}
-
-__global__ void __launch_bounds__(256) k_leaf_scatter(LeafBatch B) {
-    int b;
-    uint32_t i;
-    if (!leaf_tuple(B, b, i)) return;
-    const LeafBuild& L = B.l[b];
-    scatter_tuple(L.tb, L.is_rep, L.shift, L.buckets, L.cursor, L.ht, L.bloom, L.log2w, B.err, i);
-}
-
-// Entries are numbered like tuples (a build stores at most its tuple count).
 __global__ void __launch_bounds__(256) k_leaf_flags(LeafBatch B) {
-    int b;
-    uint32_t e;
-    if (!leaf_tuple(B, b, e)) return;
+    const int b = leaf_of(B.tile_start, B.n, blockIdx.x);
     const LeafBuild& L = B.l[b];
-    if (e < L.buckets[L.nb].x) flag_entry(L.ht, e, L.dflags);
+    const uint32_t i0 = (blockIdx.x - B.tile_start[b]) * kBucketTile;
+    for (uint32_t i = i0 + threadIdx.x; i < min(i0 + kBucketTile, L.nb); i += blockDim.x) flag_bucket(L.ht, i, L.dflags);
+}
+
+// Leaves of at most kClusterLeafRows rows: a cluster of eight CTAs builds one
+// table in one launch. The passes are the ones above, over buffers in L2, with
+// a cluster barrier (its CTAs are resident together) where they have a launch;
+// the zeroing is a pass too, so no memset goes before.
+constexpr int kClusterCtas = 8;
+constexpr int kClusterThreads = 512;
+
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads) k_leaf_cluster(LeafBatch B) {
+    const cg::cluster_group cluster = cg::this_cluster();
+    const LeafBuild& L = B.l[blockIdx.x / kClusterCtas];
+    const uint32_t all = kClusterCtas * kClusterThreads;
+    const uint32_t t = (blockIdx.x % kClusterCtas) * kClusterThreads + threadIdx.x;
+    uint4* counts4 = reinterpret_cast<uint4*>(L.counts);
+    for (uint32_t i = t; i < L.nb / 4; i += all) counts4[i] = make_uint4(0, 0, 0, 0);
+    if (L.bloom)
+        for (uint32_t i = t; i < 1u << L.ht.bloom_log2; i += all) L.bloom[i] = 0;
+    if (t < 3) L.dflags[t] = 0;
+    cluster.sync();
+    for (uint32_t i = t; i < L.rows; i += all) {
+        uint64_t kv = 0;
+        L.rank1[i] = leaf_key(L, i, kv) ? count_key(L.counts, L.ht, L.bloom, kv) : 0u;
+    }
+    cluster.sync();
+    uint4* buckets = const_cast<uint4*>(L.ht.buckets);
+    for (uint32_t w = t >> 5; w * 32 < L.nb; w += all / 32) {  // a warp a run of 32 buckets (or all 16)
+        const uint32_t b = w * 32 + (t & 31);
+        const uint32_t n = b < L.nb ? __ldcg(L.counts + b) : 0u;
+        uint32_t inc = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+            if ((t & 31) >= uint32_t(o)) inc += u;
+        }
+        uint32_t first = 0;
+        if ((t & 31) == 31 && inc) first = atomicAdd(L.dflags + 2, inc);
+        first = __shfl_sync(0xffffffffu, first, 31);
+        if (b < L.nb) buckets[b] = make_uint4(first + inc - n, n, 0, 0);
+    }
+    cluster.sync();
+    for (uint32_t i = t; i < L.rows; i += all) {
+        const uint32_t r1 = L.rank1[i];  // this thread's own
+        uint64_t kv = 0;
+        if (r1 && col_get(L.key, i, kv)) leaf_place(L, i, kv, r1 - 1, B.err);
+    }
+    if (!B.flags) return;
+    cluster.sync();
+    for (uint32_t b = t; b < L.nb; b += all) flag_bucket(L.ht, b, L.dflags);
 }
 
 // Hit counts of evenly spaced sample rows against every probe of a pipeline:
@@ -371,12 +382,10 @@ __global__ void k_sample_probes(SampleSet set, uint32_t nsample, uint32_t* hits)
     const uint32_t row = uint32_t((uint64_t(i) * sp.key.nrows) / nsample);
     uint64_t v;
     if (!col_get(sp.key, row, v)) return;
-    const uint32_t b = ht_bucket(sp.ht, v);
-    for (uint32_t j = sp.ht.buckets[b].x; j < sp.ht.buckets[b + 1].x; j++)
-        if (ht_key_eq(sp.ht, j, v)) {
-            atomicAdd(hits + blockIdx.y, 1u);
-            return;
-        }
+    bucket_matches(sp.ht, ht_bucket(sp.ht, v), v, [&](uint32_t) {
+        atomicAdd(hits + blockIdx.y, 1u);
+        return false;
+    });
 }
 
 } // namespace
@@ -390,37 +399,47 @@ int emit_aggregate(const BuildArgs& a, cudaStream_t st) {
     return 2;
 }
 
-int scatter_bloom(TupleBuf t, const uint32_t* is_rep, uint32_t shift, uint2* buckets, uint32_t* cursor,
-                  HTView ht_mut, uint32_t* bloom, uint32_t log2w, uint32_t* err, cudaStream_t st) {
+int place_tuples(const TupleBuf& t, const uint32_t* rank1, const uint32_t* counts, uint32_t* entries, uint32_t nb,
+                 const HTView& ht, uint32_t* err, cudaStream_t st) {
     if (!t.count) return 0;
-    k_scatter_bloom<<<(t.count + 255) / 256, 256, 0, st>>>(t, is_rep, shift, buckets, cursor, ht_mut, bloom, log2w,
-                                                           err);
-    return 1;
+    BucketTiles tiles{};
+    tiles.b[0] = {counts, const_cast<uint4*>(ht.buckets), entries, nb};
+    tiles.tile_start[1] = (nb + kBucketTile - 1) / kBucketTile;
+    tiles.n = 1;
+    k_bucket_ranges<<<tiles.tile_start[1], 256, 0, st>>>(tiles);
+    k_place<<<(t.count + 255) / 256, 256, 0, st>>>(t, rank1, ht, err);
+    return 2;
 }
 
 int ht_flags(HTView ht, uint32_t nbuckets, uint32_t* flags, int num_sms, cudaStream_t st) {
     if (!ht.nentries) return 0;
-    uint32_t blocks = (ht.nentries + 255) / 256;
-    if (blocks > uint32_t(num_sms) * 8) blocks = uint32_t(num_sms) * 8;
+    const uint32_t blocks = std::min<uint32_t>((nbuckets + 255) / 256, uint32_t(num_sms) * 8);
     k_ht_flags<<<blocks, 256, 0, st>>>(ht, nbuckets, flags);
     return 1;
 }
 
+int build_cluster_leaves(const LeafBatch& batch, cudaStream_t st) {
+    if (batch.n <= 0) return 0;
+    k_leaf_cluster<<<unsigned(batch.n * kClusterCtas), kClusterThreads, 0, st>>>(batch);
+    return 1;
+}
+
 int build_leaves(const LeafBatch& batch, cudaStream_t st) {
-    const uint32_t tuples = batch.tuple_start[batch.n], tiles = batch.tile_start[batch.n];
-    if (batch.n <= 0 || tuples == 0) return 0;
-    const uint32_t blocks = batch.block_start[batch.n];
-    bool all_distinct = true;
-    for (int b = 0; b < batch.n; b++) all_distinct = all_distinct && batch.l[b].distinct;
-    k_leaf_emit<<<blocks, 256, 0, st>>>(batch);
-    if (!all_distinct) k_leaf_aggregate<<<blocks, 256, 0, st>>>(batch);
-    k_leaf_tile_sums<<<tiles, 256, 0, st>>>(batch);
-    k_leaf_offsets<<<tiles, 256, 0, st>>>(batch);
-    k_leaf_scatter<<<blocks, 256, 0, st>>>(batch);
-    const int launches = all_distinct ? 4 : 5;
-    if (!batch.flags) return launches;
-    k_leaf_flags<<<blocks, 256, 0, st>>>(batch);
-    return launches + 1;
+    const uint32_t blocks = batch.block_start[batch.n], tiles = batch.tile_start[batch.n];
+    if (batch.n <= 0 || blocks == 0) return 0;
+    BucketTiles bt{};
+    bt.n = batch.n;
+    for (int b = 0; b < batch.n; b++) {
+        const LeafBuild& L = batch.l[b];
+        bt.b[b] = {L.counts, const_cast<uint4*>(L.ht.buckets), L.dflags + 2, L.nb};
+        bt.tile_start[b + 1] = batch.tile_start[b + 1];
+    }
+    k_leaf_count<<<blocks, 256, 0, st>>>(batch);
+    k_bucket_ranges<<<tiles, 256, 0, st>>>(bt);
+    k_leaf_place<<<blocks, 256, 0, st>>>(batch);
+    if (!batch.flags) return 3;
+    k_leaf_flags<<<tiles, 256, 0, st>>>(batch);
+    return 4;
 }
 
 int sample_probes(const SampleSet& set, uint32_t nsample, uint32_t* hits, cudaStream_t st) {

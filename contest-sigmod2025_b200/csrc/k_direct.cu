@@ -16,11 +16,11 @@
 // on the collected rows before they leave (JoinPipeline.hpp:111-131 fuses the
 // same stages), which saves their launch and the items between.
 //
-// Bound: the bucket lookups' L2 sectors (8M probes of a 1M-key table: 89 us),
+// Bound: the bucket lookups' L2 sectors (8M probes of a 1M-key table: 67 us),
 // below a few thousand pages the latency of one page. Measured on a B200
 // against the staged form, device time of the scan (with the stages after
-// it): 30K rows in 16 pages 30 -> 13 us; 1M rows, two tables 28 -> 18 us; 8M
-// rows with 10% NULLs 145 -> 112 us.
+// it): 30K rows in 16 pages 30 -> 10 us; 1M rows, two tables 28 -> 16 us; 8M
+// rows with 10% NULLs 145 -> 75 us.
 #include "launch.h"
 
 #include <algorithm>
@@ -72,41 +72,40 @@ __device__ __forceinline__ uint32_t probe_groups(const DirectArgs& a, const uint
         for (int k = 0; k < kGroups; k++)
             if (((valid >> k) & 1) && !bloom_may_contain(ht.bloom, ht.bloom_log2, uint32_t(key[k]))) valid &= ~(1u << k);
     }
-    uint2 b0[kGroups];
-    uint32_t hi[kGroups];
+    uint4 b[kGroups];
 #pragma unroll
     for (int k = 0; k < kGroups; k++) {
-        b0[k] = make_uint2(0, 0);
-        hi[k] = 0;
-        if ((valid >> k) & 1) {
-            const uint2* b = ht.buckets + bucket_of(key[k], kWide, ht.shift);
-            b0[k] = __ldg(b);
-            hi[k] = __ldg(&b[1].x);
+        b[k] = make_uint4(0, 0, 0, 0);
+        if ((valid >> k) & 1) b[k] = __ldg(ht.buckets + bucket_of(key[k], kWide, ht.shift));
+    }
+    uint32_t hit = 0;
+#pragma unroll
+    for (int k = 0; k < kGroups; k++) {
+        e[k] = 0;
+        if (!kWide) {
+            const uint32_t kk = uint32_t(key[k]);
+            const bool first = b[k].y >= 1 && b[k].z == kk, second = b[k].y >= 2 && b[k].w == kk;
+            e[k] = b[k].x + (second ? 1u : 0u);
+            if (first || second) hit |= 1u << k;
         }
     }
-    uint32_t hit = 0, more = 0;
 #pragma unroll
     for (int k = 0; k < kGroups; k++) {
-        e[k] = b0[k].x;
-        if (e[k] >= hi[k]) continue;
-        if (b0[k].y == uint32_t(key[k]) && (!kWide || __ldg(ht.keys_hi + e[k]) == uint32_t(key[k] >> 32)))
-            hit |= 1u << k;
-        else if (e[k] + 1 < hi[k])
-            more |= 1u << k;
-    }
-    // The rest of the buckets that hold several keys, the groups in step.
-    while (more) {
-#pragma unroll
-        for (int k = 0; k < kGroups; k++) {
-            if (!((more >> k) & 1)) continue;
-            e[k]++;
-            if (__ldg(ht.keys + e[k]) == uint32_t(key[k]) &&
-                (!kWide || __ldg(ht.keys_hi + e[k]) == uint32_t(key[k] >> 32))) {
+        if ((hit >> k) & 1) continue;
+        if (kWide) {
+            bucket_matches(ht, b[k], key[k], [&](uint32_t j) {
+                e[k] = j;
                 hit |= 1u << k;
-                more &= ~(1u << k);
-            } else if (e[k] + 1 >= hi[k]) {
-                more &= ~(1u << k);
-            }
+                return false;
+            });
+        } else {
+            // Buckets of three entries and more.
+            for (uint32_t j = 2; j < b[k].y; j++)
+                if (uint32_t(ht_key(ht, b[k].x + j)) == uint32_t(key[k])) {
+                    e[k] = b[k].x + j;
+                    hit |= 1u << k;
+                    break;
+                }
         }
     }
     return hit;
@@ -115,15 +114,13 @@ __device__ __forceinline__ uint32_t probe_groups(const DirectArgs& a, const uint
 // First entry of `ht` with this key (unique keys), or false.
 __device__ __forceinline__ bool find_entry(const HTView& ht, uint64_t key, bool use_bloom, uint32_t& e) {
     if (use_bloom && ht.bloom && !bloom_may_contain(ht.bloom, ht.bloom_log2, uint32_t(key))) return false;
-    const uint2* b = ht.buckets + ht_bucket(ht, key);
-    const uint2 b0 = *b;
-    const uint32_t hi = b[1].x;
-    e = b0.x;
-    if (e >= hi) return false;
-    if (b0.y == uint32_t(key) && (!ht.keys_hi || ht.keys_hi[e] == uint32_t(key >> 32))) return true;
-    for (e++; e < hi; e++)
-        if (ht_key_eq(ht, e, key)) return true;
-    return false;
+    bool found = false;
+    bucket_matches(ht, ht_bucket(ht, key), key, [&](uint32_t j) {
+        e = j;
+        found = true;
+        return false;
+    });
+    return found;
 }
 
 template <bool kWide, bool kChain>
@@ -202,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_scan_direct(DirectArgs a) {
                 const uint2 f = found[i];
                 a.out.rows[o] = f.x;
                 a.out.ents[0][o] = f.y;
-                if (a.out.mult) a.out.mult[o] = a.ht.mult[f.y];
+                if (a.out.mult) a.out.mult[o] = ht_mult(a.ht, f.y);
             }
             __syncthreads();  // `found` and `nfound` are reused
         } else {
@@ -220,8 +217,8 @@ __global__ void __launch_bounds__(kThreads, 6) k_scan_direct(DirectArgs a) {
                     const ChainStage& c = a.chain.st[t];
                     uint64_t v = 0;
                     if (c.src.stage >= 0) {  // the scan's own match (stage 0)
-                        hit = !((c.src.ht.pnull[f.y] >> c.src.slot) & 1);
-                        if (hit) v = c.src.ht.pay[size_t(f.y) * c.src.ht.width + c.src.slot];
+                        hit = !ht_slot_null(c.src.ht, f.y, c.src.slot);
+                        if (hit) v = ht_slot(c.src.ht, f.y, c.src.slot);
                     } else if (f.x >= c.key.nrows) {
                         record_error(a.err, kErrRowRange);
                         hit = false;
@@ -245,12 +242,12 @@ __global__ void __launch_bounds__(kThreads, 6) k_scan_direct(DirectArgs a) {
                 }
                 a.out.rows[o] = f.x;
                 a.out.ents[0][o] = f.y;
-                uint64_t mult = a.out.mult ? a.ht.mult[f.y] : 1ull;
+                uint64_t mult = ht_mult(a.ht, f.y);
 #pragma unroll
                 for (int t = 0; t < kMaxChain; t++) {
                     if (t >= a.chain.n) continue;
                     a.out.ents[1 + t][o] = e[t];
-                    if (a.out.mult) mult *= a.chain.st[t].ht.mult[e[t]];
+                    if (a.out.mult) mult *= ht_mult(a.chain.st[t].ht, e[t]);
                 }
                 if (a.out.mult) a.out.mult[o] = mult;
             }

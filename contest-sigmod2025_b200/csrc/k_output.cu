@@ -138,8 +138,8 @@ __device__ __forceinline__ uint32_t gather_direct(const OutColumns& cols, const 
     for (int k = 0; k < 8; k++) {
         if (!((live >> k) & 1)) continue;
         const uint32_t e = a8[k];
-        v8[k] = ht.pay[size_t(e) * ht.width + s.slot];
-        if (!((ht.pnull[e] >> s.slot) & 1)) bits |= 1u << k;
+        v8[k] = ht_slot(ht, e, s.slot);
+        if (!ht_slot_null(ht, e, s.slot)) bits |= 1u << k;
     }
     return bits;
 }

@@ -25,27 +25,13 @@ namespace bj {
 namespace {
 
 
-// Entries of `ht` whose key equals `key`: calls fn(entry) for each.
-// `key` is a value slot: an INT32 key zero-extended, or an INT64 key (the
-// table then carries keys_hi and no bloom filter).
+// Entries of `ht` whose key equals `key`: calls fn(entry) for each, until it
+// returns false. `key` is a value slot: an INT32 key zero-extended, or an
+// INT64 key (the table is then wide and carries no bloom filter).
 template <typename Fn>
-__device__ __forceinline__ uint32_t for_matches(const HTView& ht, uint64_t key, bool use_bloom, Fn&& fn) {
-    if (use_bloom && ht.bloom && !bloom_may_contain(ht.bloom, ht.bloom_log2, uint32_t(key))) return 0;
-    const uint32_t b = ht_bucket(ht, key);
-    const uint2 b0 = ht.buckets[b];
-    const uint32_t e = ht.buckets[b + 1].x;
-    uint32_t n = 0;
-    if (b0.x < e && b0.y == uint32_t(key) && (!ht.keys_hi || ht.keys_hi[b0.x] == uint32_t(key >> 32))) {
-        fn(b0.x);
-        n++;
-    }
-    for (uint32_t j = b0.x + 1; j < e; j++) {
-        if (ht_key_eq(ht, j, key)) {
-            fn(j);
-            n++;
-        }
-    }
-    return n;
+__device__ __forceinline__ void for_matches(const HTView& ht, uint64_t key, bool use_bloom, Fn&& fn) {
+    if (use_bloom && ht.bloom && !bloom_may_contain(ht.bloom, ht.bloom_log2, uint32_t(key))) return;
+    bucket_matches(ht, ht_bucket(ht, key), key, fn);
 }
 
 template <typename T>
@@ -101,7 +87,10 @@ __global__ void __launch_bounds__(256) k_probe_stage(Items in, DevColumn key, HT
         uint32_t row = item_row(in, i);
         uint64_t v;
         if (!stage_key(key, src, in, i, row, err, v)) continue;
-        mine += for_matches(ht, v, use_bloom != 0, [](uint32_t) {});
+        for_matches(ht, v, use_bloom != 0, [&](uint32_t) {
+            mine++;
+            return true;
+        });
     }
     __shared__ unsigned long long total;
     const unsigned long long base = block_exclusive_sum<unsigned long long>(mine, &total);
@@ -123,13 +112,14 @@ __global__ void __launch_bounds__(256) k_probe_stage(Items in, DevColumn key, HT
         for_matches(ht, v, use_bloom != 0, [&](uint32_t e) {
             if (o >= capacity) {
                 record_error(err, kErrCapacity);
-                return;
+                return false;
             }
             out.rows[o] = row;
             for (int p = 0; p < in.nprobes; p++) out.ents[p][o] = in.ents[p][i];
             out.ents[in.nprobes][o] = e;
-            out.mult[o] = m * ht.mult[e];
+            out.mult[o] = m * ht_mult(ht, e);
             o++;
+            return true;
         });
     }
 }
@@ -166,8 +156,9 @@ __global__ void __launch_bounds__(256) k_probe_chain(Items in, ProbeChain ch, It
             } else {
                 bool found = false;
                 for_matches(c.ht, v, c.use_bloom != 0, [&](uint32_t j) {
-                    if (!found) e[t] = j;
+                    e[t] = j;
                     found = true;
+                    return false;  // unique keys: no other match
                 });
                 hit = found;
             }
@@ -190,7 +181,7 @@ __global__ void __launch_bounds__(256) k_probe_chain(Items in, ProbeChain ch, It
         for (int t = 0; t < kMaxChain; t++) {
             if (t >= ch.n) continue;
             out.ents[in.nprobes + t][o] = e[t];
-            m *= ch.st[t].ht.mult[e[t]];
+            m *= ht_mult(ch.st[t].ht, e[t]);
         }
         if (out.mult) out.mult[o] = m;
     }

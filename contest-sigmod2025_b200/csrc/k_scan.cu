@@ -134,35 +134,25 @@ struct WarpState {
 __device__ __forceinline__ void probe_batch(const ScanArgs& a, WarpState& w, const uint32_t (&key)[kPerLane],
                                             const uint32_t (&row)[kPerLane], uint32_t has, uint32_t unit) {
     const uint32_t lane = lane_id();
-    // One load per candidate gives its bucket's range and first key; only
-    // buckets with more entries (few: about one key per bucket) loop.
-    uint32_t lo[kPerLane], hi[kPerLane], k0[kPerLane];
+    // One load per candidate gives its bucket's range and first two keys;
+    // only buckets with more entries (few: at most one key per bucket on
+    // average) are walked.
+    uint4 bk[kPerLane];
 #pragma unroll
     for (int i = 0; i < kPerLane; i++) {
-        lo[i] = hi[i] = 0;
-        k0[i] = ~key[i];
-        if ((has >> i) & 1) {
-            const uint32_t b = uint32_t(key_hash(key[i]) >> a.ht.shift);
-            const uint2 b0 = a.ht.buckets[b];
-            lo[i] = b0.x;
-            hi[i] = a.ht.buckets[b + 1].x;
-            k0[i] = b0.y;
-        }
+        bk[i] = make_uint4(0, 0, 0, 0);
+        if ((has >> i) & 1) bk[i] = __ldg(a.ht.buckets + (key_hash_hi(key[i]) >> (a.ht.shift - 32)));
     }
-#pragma unroll
-    for (int i = 0; i < kPerLane; i++)
-        if (lo[i] >= hi[i]) k0[i] = ~key[i];
     uint32_t cnt = 0;
-    uint32_t cj[kPerLane];
+    uint32_t cj[kPerLane], lo[kPerLane];  // matches, the first one
 #pragma unroll
     for (int i = 0; i < kPerLane; i++) {
-        uint32_t c = k0[i] == key[i] ? 1u : 0u, first = c ? lo[i] : hi[i];
-        // Mode 2 (unique build keys): nothing after the first match.
-        for (uint32_t e = lo[i] + 1; e < hi[i] && !(a.mode == 2 && c); e++)
-            if (a.ht.keys[e] == key[i]) {
-                first = c ? first : e;
-                c++;
-            }
+        uint32_t c = 0, first = 0;
+        bucket_matches(a.ht, bk[i], key[i], [&](uint32_t e) {
+            if (!c) first = e;
+            c++;
+            return a.mode != 2;  // mode 2 (unique build keys): nothing after the first match
+        });
         lo[i] = first;
         cj[i] = c;
         cnt += c;
@@ -183,7 +173,7 @@ __device__ __forceinline__ void probe_batch(const ScanArgs& a, WarpState& w, con
             if (o < a.capacity) {
                 a.out_rows[o] = r;
                 a.out_ents[o] = e;
-                if (a.out_mult) a.out_mult[o] = a.ht.mult[e];
+                if (a.out_mult) a.out_mult[o] = ht_mult(a.ht, e);
             } else {
                 record_error(a.err, kErrCapacity);
             }
@@ -195,7 +185,7 @@ __device__ __forceinline__ void probe_batch(const ScanArgs& a, WarpState& w, con
             emit(row[i], lo[i]);  // the first match, found above
             uint32_t left = cj[i] - 1;
             for (uint32_t e = lo[i] + 1; left; e++) {
-                if (a.ht.keys[e] != key[i]) continue;
+                if (uint32_t(ht_key(a.ht, e)) != key[i]) continue;
                 left--;
                 emit(row[i], e);
             }

@@ -6,8 +6,7 @@
 // inclusive prefixes 32 at a time until it meets an inclusive one, and
 // publishes its own inclusive prefix. One launch (plus one memset of the
 // tile status words) for any n. Used for page row offsets, tile offsets of
-// the pipeline stages, bucket offsets of the hash build and output row
-// offsets.
+// the pipeline stages and output row offsets.
 #include "launch.h"
 
 #include <algorithm>
@@ -63,8 +62,7 @@ __device__ __forceinline__ unsigned long long ld_status(const unsigned long long
 // One tile of a single-pass scan (the calling CTA takes its tile by ticket).
 template <typename T>
 __device__ __forceinline__ void scan_tile_lookback(const T* __restrict__ in, T* __restrict__ out, size_t n,
-                                                   unsigned long long* status, uint32_t* ticket, uint32_t* err,
-                                                   uint32_t ostride = 1) {
+                                                   unsigned long long* status, uint32_t* ticket, uint32_t* err) {
     __shared__ uint32_t s_tile;
     __shared__ T s_prefix;
     if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
@@ -128,9 +126,9 @@ __device__ __forceinline__ void scan_tile_lookback(const T* __restrict__ in, T* 
 #pragma unroll
     for (int k = 0; k < kScanPer; k++) {
         if (base + k < n) {
-            out[(base + k) * ostride] = run;
+            out[base + k] = run;
             run += v[k];
-            if (base + k == n - 1) out[n * ostride] = run;
+            if (base + k == n - 1) out[n] = run;
         }
     }
 }
@@ -138,8 +136,8 @@ __device__ __forceinline__ void scan_tile_lookback(const T* __restrict__ in, T* 
 template <typename T>
 __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(const T* __restrict__ in, T* __restrict__ out,
                                                                 size_t n, unsigned long long* status,
-                                                                uint32_t* ticket, uint32_t* err, uint32_t ostride) {
-    scan_tile_lookback<T>(in, out, n, status, ticket, err, ostride);
+                                                                uint32_t* ticket, uint32_t* err) {
+    scan_tile_lookback<T>(in, out, n, status, ticket, err);
 }
 
 // Independent scans of several u32 arrays (blockIdx.y = array); array k's
@@ -158,10 +156,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_segs(ScanSegs segs, unsig
                                  err);
 }
 
-// Output i goes to out[i * ostride].
 template <typename T>
-__global__ void k_tile_scan(const T* __restrict__ in, T* __restrict__ out, size_t n, const T* __restrict__ base_ex,
-                            uint32_t ostride = 1) {
+__global__ void k_tile_scan(const T* __restrict__ in, T* __restrict__ out, size_t n, const T* __restrict__ base_ex) {
     size_t base = size_t(blockIdx.x) * kScanTile + size_t(threadIdx.x) * kScanPer;
     T v[kScanPer];
     T local = 0;
@@ -175,9 +171,9 @@ __global__ void k_tile_scan(const T* __restrict__ in, T* __restrict__ out, size_
 #pragma unroll
     for (int k = 0; k < kScanPer; k++) {
         if (base + k < n) {
-            out[(base + k) * ostride] = run;
+            out[base + k] = run;
             run += v[k];
-            if (base + k == n - 1) out[n * ostride] = run;
+            if (base + k == n - 1) out[n] = run;
         }
     }
 }
@@ -217,21 +213,20 @@ size_t status_bytes(size_t n) {
 }
 
 // status: status_bytes(n) zero bytes (null when that is 0).
-// Output i goes to out[i * ostride].
 template <typename T>
-int scan_launch(const T* in, T* out, size_t n, void* status, uint32_t* err, cudaStream_t st, uint32_t ostride = 1) {
+int scan_launch(const T* in, T* out, size_t n, void* status, uint32_t* err, cudaStream_t st) {
     if (n == 0) {
         k_zero_one<T><<<1, 1, 0, st>>>(out);
         return 1;
     }
     const size_t nt = (n + kScanTile - 1) / kScanTile;
     if (nt == 1) {
-        k_tile_scan<T><<<1, kScanThreads, 0, st>>>(in, out, n, nullptr, ostride);
+        k_tile_scan<T><<<1, kScanThreads, 0, st>>>(in, out, n, nullptr);
         return 1;
     }
     auto* words = static_cast<unsigned long long*>(status);
     k_scan_lookback<T><<<unsigned(nt), kScanThreads, 0, st>>>(in, out, n, words, reinterpret_cast<uint32_t*>(words + nt),
-                                                              err, ostride);
+                                                              err);
     return 1;
 }
 
@@ -297,8 +292,6 @@ int scan_exclusive_u64_batch(const ScanBatch64& b, size_t n, Scratch& s, cudaStr
     return 1;
 }
 
-size_t scan_status_bytes(size_t n) { return status_bytes(n); }
-
 int scan_exclusive_u32_segs(ScanSegs segs, Scratch& s, cudaStream_t st) {
     if (segs.n <= 0) return 0;
     size_t words = 0, max_nt = 1;
@@ -320,10 +313,6 @@ int gather_values(const GatherList& g, uint64_t* dst, cudaStream_t st) {
     if (g.n <= 0) return 0;
     k_gather_values<<<1, kMaxGather, 0, st>>>(g, dst);
     return 1;
-}
-int scan_exclusive_u32_zeroed(const uint32_t* in, uint32_t* out, size_t n, void* status, uint32_t* err,
-                              cudaStream_t st, uint32_t out_stride) {
-    return scan_launch<uint32_t>(in, out, n, status, err, st, out_stride);
 }
 int fill_u32(uint32_t* p, uint32_t v, size_t n, cudaStream_t st) {
     if (!n) return 0;

@@ -24,12 +24,6 @@ struct Scratch {
 // Exclusive scan of n values into out[0..n]; out[n] receives the total.
 int scan_exclusive_u32(const uint32_t* in, uint32_t* out, size_t n, Scratch& s, cudaStream_t st);
 int scan_exclusive_u64(const uint64_t* in, uint64_t* out, size_t n, Scratch& s, cudaStream_t st);
-// The same scan with its tile status words supplied: scan_status_bytes(n)
-// bytes (possibly 0) that the caller has zeroed, so no memset is issued.
-// Output i goes to out[i * out_stride].
-size_t scan_status_bytes(size_t n);
-int scan_exclusive_u32_zeroed(const uint32_t* in, uint32_t* out, size_t n, void* status, uint32_t* err,
-                              cudaStream_t st, uint32_t out_stride = 1);
 // Independent exclusive scans of up to kMaxScanSegs u32 arrays of any
 // lengths, in one launch (status_off is filled in by the wrapper).
 constexpr int kMaxScanSegs = 64;
@@ -187,8 +181,8 @@ inline ProbeSet make_probe_set(const HTView* probes, int n) {
 __device__ __forceinline__ bool payload_key(const KeySource& src, const uint32_t* const* ents, uint32_t i,
                                             uint64_t& v) {
     const uint32_t e = ents[src.stage][i];
-    if ((src.ht.pnull[e] >> src.slot) & 1) return false;
-    v = src.ht.pay[size_t(e) * src.ht.width + src.slot];
+    if (ht_slot_null(src.ht, e, src.slot)) return false;
+    v = ht_slot(src.ht, e, src.slot);
     return true;
 }
 __device__ __forceinline__ uint32_t item_row(const Items& in, uint32_t i) { return in.rows ? in.rows[i] : i; }
@@ -215,8 +209,8 @@ __device__ __forceinline__ bool slot_value(const SlotSource& s, const Items& in,
         return true;
     }
     const HTView& ht = ps.ht[s.probe];
-    if ((ht.pnull[e] >> s.slot) & 1) return false;
-    v = ht.pay[size_t(e) * ht.width + s.slot];
+    if (ht_slot_null(ht, e, s.slot)) return false;
+    v = ht_slot(ht, e, s.slot);
     return true;
 }
 #endif
@@ -270,20 +264,19 @@ int scan_probe_direct(const DevColumn& key, const HTView& ht, bool use_bloom, co
                       cudaStream_t st);
 
 // ---- hash table build (k_build.cu) ----
-// Tuples of a build pipeline, one per item: key from `key` (NULL key ->
-// mult 0), payload from `src`, mult from the item.
+// Tuples of a build fed by probes, one per item: key slot from `key` (NULL key
+// -> mult 0), payload from `src`, mult from the item.
 struct TupleBuf {
-    uint32_t* keys;
-    uint32_t* keys_hi; // INT64 build keys: high halves; null for INT32
+    uint64_t* keys;
     uint64_t* mult;
     uint64_t* pay;     // count * width
-    uint32_t* pnull;
+    uint32_t* pnull;   // null when no slot can be NULL
     uint32_t count;
     uint32_t width;
 };
-// Emit, eager aggregation and bucket counts of a hash build (emit_aggregate:
-// two launches, one when the build is distinct). table (1 << tlog2 words)
-// and counts (one per bucket) must be zero.
+// Emit, eager aggregation, bucket counts and filter of a hash build
+// (emit_aggregate: two launches, one when the build is distinct). table
+// (1 << tlog2 words), counts (one per bucket) and the filter must be zero.
 struct BuildArgs {
     Items in;
     DevColumn key;       // key column of the scanned input, or (key_stage >= 0) only its type
@@ -294,9 +287,10 @@ struct BuildArgs {
     TupleBuf tb;
     uint32_t* table;   // slot: index + 1 of the tuple representing it, 0 = empty
     uint32_t tlog2;
-    uint32_t* is_rep;  // per tuple: 1 if it represents its distinct tuple
+    uint32_t* rank1;   // per tuple: 1 + its rank in its bucket, 0 if it represents no distinct tuple
     uint32_t* counts;  // per bucket: representatives
-    uint32_t shift;    // bucket = key_hash >> shift
+    HTView ht;         // the table to build (its sizes and key width)
+    uint32_t* bloom;   // its filter (null: none)
     uint32_t* err;
     uint32_t distinct; // 1: no two tuples can be equal (each is its own representative; no table)
     // Sideways restriction (INT32 keys): the bloom filter (1 << rlog2w words)
@@ -306,34 +300,25 @@ struct BuildArgs {
     uint32_t rlog2w;
 };
 int emit_aggregate(const BuildArgs& a, cudaStream_t st);
-// Scatters the representatives into their buckets' ranges (cursor: one zero
-// word per bucket) and sets their bloom bits (bloom: zero, 1 << log2w words;
-// null: no filter).
-int scatter_bloom(TupleBuf t, const uint32_t* is_rep, uint32_t shift, uint2* buckets, uint32_t* cursor,
-                  HTView ht_mut, uint32_t* bloom, uint32_t log2w, uint32_t* err, cudaStream_t st);
+// Gives the buckets their ranges (entries: one zero word) and places the
+// representatives as entries.
+int place_tuples(const TupleBuf& t, const uint32_t* rank1, const uint32_t* counts, uint32_t* entries, uint32_t nb,
+                 const HTView& ht, uint32_t* err, cudaStream_t st);
 // The builds of inputs that probe nothing, up to kMaxLeafBuilds at a time,
 // each pass one launch over all of them (k_build.cu). Each build's zero
-// region (table, counts, cursor, bloom, flags) must be zero before;
-// tile_sums holds tile_start[n] words.
+// region (counts, bloom, flags) must be zero before.
 constexpr int kMaxLeafBuilds = 6;
 constexpr int kMaxLeafSlots = 4;  // leaves with more payload columns build one by one
 struct LeafBuild {
     DevColumn key;                  // build key column
     DevColumn cols[kMaxLeafSlots];  // payload columns (slot j)
     int nslots;
-    TupleBuf tb;
-    uint32_t* table;    // aggregation table, 1 << tlog2 zero words (unused when distinct)
-    uint32_t tlog2;
-    uint32_t* is_rep;
+    uint32_t rows;
+    uint32_t* rank1;    // per row: 1 + its rank in its bucket, 0 if it is not inserted
     uint32_t* counts;   // nb zero words
-    uint32_t shift;
-    uint32_t distinct;  // see BuildArgs::distinct
-    uint2* buckets;     // nb + 1: offsets written into x, first keys into y
     uint32_t nb;
-    uint32_t* cursor;   // nb zero words
-    uint32_t* bloom;    // zero, 1 << log2w words; null: no filter
-    uint32_t log2w;
-    uint32_t* dflags;   // two zero words: table flags (pass 4)
+    uint32_t* bloom;    // zero, 1 << ht.bloom_log2 words; null: no filter
+    uint32_t* dflags;   // three zero words: table flags (last pass), entries placed
     HTView ht;          // the table's arrays to fill
     // Sideways restriction: the bloom filter (1 << rlog2w words) of another
     // table built on the same key class; a row whose key it cannot hold is
@@ -344,21 +329,34 @@ struct LeafBuild {
 struct LeafBatch {
     LeafBuild l[kMaxLeafBuilds];
     int n;
-    uint32_t tuple_start[kMaxLeafBuilds + 1];  // prefix of the builds' tuple counts
-    uint32_t block_start[kMaxLeafBuilds + 1];  // prefix of their blocks of 256 tuples
-    uint32_t tile_start[kMaxLeafBuilds + 1];   // prefix of their bucket tiles (1024 buckets each)
-    uint32_t* tile_sums;
+    uint32_t block_start[kMaxLeafBuilds + 1];  // prefix of the builds' blocks of 256 rows
+    uint32_t tile_start[kMaxLeafBuilds + 1];   // prefix of their bucket tiles
     uint32_t* err;
     int flags;          // 1: compute the table flags
 };
 static_assert(sizeof(LeafBatch) <= 4096, "a LeafBatch is one kernel parameter block; kept within 4 KiB");
 // Returns the launches made.
 int build_leaves(const LeafBatch& batch, cudaStream_t st);
-constexpr uint32_t kLeafTileBuckets = 1024;
+constexpr uint32_t kBucketTile = 1024;
+struct BucketTiles {
+    struct Build {
+        const uint32_t* counts;
+        uint4* buckets;
+        uint32_t* entries;  // entries reserved so far (zero before)
+        uint32_t nb;
+    } b[kMaxLeafBuilds];
+    uint32_t tile_start[kMaxLeafBuilds + 1];
+    int n;
+};
+// The same when every leaf has at most kClusterLeafRows rows (a row a thread):
+// one launch, and nothing needs to be zero before. Build phase in a replayed
+// graph on a B200, one or three leaves: 1,000 rows 11.5 us against 13.8 for
+// the separate passes, 8,000 rows 15.7 against 13.6.
+constexpr uint32_t kClusterLeafRows = 4096;
+int build_cluster_leaves(const LeafBatch& batch, cudaStream_t st);
 
 // Flags of a built table: [0] = 1 if some key repeats, [1] = 1 if some mult > 1
-// (both words must be zero before). The entry count is read on the device
-// from buckets[nbuckets].x.
+// (both words must be zero before).
 int ht_flags(HTView ht, uint32_t nbuckets, uint32_t* flags, int num_sms, cudaStream_t st);
 // Counts, for nsample evenly spaced rows of each probe's key column, how many
 // hit its table: hits[p] for probe p, all probes in one launch (the role of

@@ -88,3 +88,29 @@ def test_fused_stages(pkg, ctx, oracle, dims, keep, wide):
 @pytest.mark.parametrize("fact", [512 * 1984, 512 * 1984 + 1])
 def test_filter_form_line(pkg, ctx, oracle, fact):
     check(pkg, ctx, oracle, star(pkg, 5, fact, [3000, 700], 0.1, 0.0, False), f"fact {fact}")
+
+
+# Build sizes: bucket counts' edges, the cluster build's last size, the filter's last size, a large build; each key
+# once, twice (both keys in the bucket) and seven times (buckets walked); NULL keys and NULL payloads.
+@pytest.mark.parametrize("rows", [1, 15, 16, 1025, 4096, 4097, 131_072, 131_073])
+@pytest.mark.parametrize("copies", [1, 2, 7])
+@pytest.mark.parametrize("wide", [False, True])
+def test_builds(pkg, ctx, oracle, rows, copies, wide):
+    rng = np.random.default_rng(rows * 10 + copies)
+    kt = pkg.INT64 if wide else pkg.INT32
+    spread = (lambda k: k.astype(np.int64) | ((k.astype(np.int64) % 8 - 4) << 32)) if wide else \
+             (lambda k: (k.astype(np.int64) - 7).astype(np.int32))
+    own = rng.permutation(np.repeat(np.arange(-(-rows // copies)), copies)[:rows])
+    fact = 150_000 if rows > 5000 else 9_001
+    fk = rng.integers(0, 2 * len(own) // copies + 2, fact)
+    some = lambda n, p: (rng.random(n) >= p).astype(np.uint8)  # noqa: E731
+    p = pkg.Plan()
+    p.new_input(pkg.ColumnarTable(fact, [column(pkg, kt, spread(fk)), column(pkg, pkg.INT32, np.arange(fact, dtype=np.int32))]))
+    p.new_input(pkg.ColumnarTable(rows, [
+        column(pkg, kt, spread(own), some(rows, 0.1)),
+        column(pkg, pkg.INT64, rng.integers(0, 1 << 50, rows), some(rows, 0.3)),
+        column(pkg, pkg.FP64, rng.random(rows))]))
+    a = p.new_scan_node(0, [(0, kt), (1, pkg.INT32)])
+    b = p.new_scan_node(1, [(0, kt), (1, pkg.INT64), (2, pkg.FP64)])
+    p.root = p.new_join_node(False, a, b, 0, 0, [(0, kt), (1, pkg.INT32), (3, pkg.INT64), (4, pkg.FP64)])
+    check(pkg, ctx, oracle, pkg.CPlan(p), f"rows {rows} copies {copies} wide {wide}")
