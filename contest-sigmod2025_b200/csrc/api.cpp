@@ -127,6 +127,7 @@ BJ_API int bj_context_create(int device, bj_context** out) {
     if (cudaMalloc(&ctx->d_err, 256) != cudaSuccess) return BJ_ERR_OOM;
     ctx->arena.err = ctx->d_err;
     if (cudaMalloc(&ctx->d_small, sizeof(uint64_t) * 64) != cudaSuccess) return BJ_ERR_OOM;
+    if (cudaMalloc(&ctx->d_result, 256) != cudaSuccess) return BJ_ERR_OOM;
     if (cudaHostAlloc(reinterpret_cast<void**>(&ctx->h_small), sizeof(uint64_t) * 64, cudaHostAllocDefault) != cudaSuccess)
         return BJ_ERR_OOM;
     cudaMemset(ctx->d_err, 0, 256);
@@ -172,6 +173,7 @@ BJ_API void bj_context_destroy(bj_context* ctx) {
     if (ctx->stage.p) cudaFreeHost(ctx->stage.p);
     if (ctx->h_small) cudaFreeHost(ctx->h_small);
     if (ctx->d_small) cudaFree(ctx->d_small);
+    if (ctx->d_result) cudaFree(ctx->d_result);
     if (ctx->d_err) cudaFree(ctx->d_err);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);

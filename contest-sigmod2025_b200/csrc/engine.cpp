@@ -1003,7 +1003,7 @@ class Executor {
             ItemsOut out{};
             out.rows = alloc<uint32_t>(total);
             for (size_t j = 0; j <= s; j++) out.ents[j] = alloc<uint32_t>(total);
-            out.mult = alloc<uint64_t>(total);
+            out.mult = !items.mult && bh.unit_mult ? nullptr : alloc<uint64_t>(total);
             launched(probe_stage(items, key, ht, 1, nullptr, toff, out, bloom, ctx_->d_err, st_, total, ksrc));
             Items next{};
             next.rows = out.rows;
@@ -1385,7 +1385,10 @@ class Executor {
         }
         res.total_pages = total;
         uint8_t* dst = nullptr;
-        if (ctx_->graph_output) {
+        uint8_t* const* dst_at = nullptr;
+        if (ctx_->graph_output && (flags & BJ_RESULT_DEVICE)) {
+            dst_at = ctx_->d_result;  // each replay writes its own result's memory
+        } else if (ctx_->graph_output) {
             dst = alloc<uint8_t>(total * kPageSize);
             res.arena_pages = dst;
         } else if (flags & BJ_RESULT_DEVICE) {
@@ -1445,7 +1448,8 @@ class Executor {
                 }
             }
             const uint64_t pages = res.page_base[c1 - 1] + res.npages[c1 - 1] - res.page_base[c0];
-            launched(write_pages(oc, uint32_t(pages), dst + res.page_base[c0] * kPageSize, ctx_->d_err, st_));
+            oc.out_offset = res.page_base[c0] * kPageSize;
+            launched(write_pages(oc, uint32_t(pages), dst_at ? nullptr : dst + oc.out_offset, dst_at, ctx_->d_err, st_));
         }
         if (!ctx_->graph_output && !(flags & BJ_RESULT_DEVICE) && total) {
             res.host = ctx_->take_pinned(total * kPageSize);

@@ -331,6 +331,7 @@ struct bj_context {
     std::unique_ptr<bj::ThreadPool> pool;
     std::string last_error;
     uint32_t* d_err = nullptr;         // device error word
+    uint8_t** d_result = nullptr;      // device word: where a replayed graph writes its result pages
     uint64_t* h_small = nullptr;       // pinned readback slots
     uint64_t* d_small = nullptr;       // device readback slots
     bj::GatherList gather{};               // values queued for the next read-back

@@ -151,17 +151,21 @@ int replay_graph(bj_context* ctx, GraphEntry& g, const std::vector<int32_t>& typ
     try {
         res->types = types;
         ctx->h_small[63] = 0;  // the graph's last node writes the low half
-        BJ_CK(cudaEventRecord(ctx->ev0, ctx->stream));
-        BJ_CK(cudaGraphLaunch(g.exec, ctx->stream));
         res->rows = g.rows;
         res->npages = g.npages;
         res->page_base = g.page_base;
         res->total_pages = g.total_pages;
-        size_t bytes = g.total_pages * kPageSize;
+        const size_t bytes = g.total_pages * kPageSize;
+        BJ_CK(cudaEventRecord(ctx->ev0, ctx->stream));
         if (bytes && (flags & BJ_RESULT_DEVICE)) {
+            // The graph writes the pages where this word says, in stream
+            // order (8 pageable bytes: staged by the call, so replays in
+            // flight keep theirs).
             BJ_CK(cudaMallocAsync(reinterpret_cast<void**>(&res->dev), bytes, ctx->stream));
-            BJ_CK(cudaMemcpyAsync(res->dev, g.pages, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-        } else if (bytes) {
+            BJ_CK(cudaMemcpyAsync(ctx->d_result, &res->dev, sizeof(res->dev), cudaMemcpyHostToDevice, ctx->stream));
+        }
+        BJ_CK(cudaGraphLaunch(g.exec, ctx->stream));
+        if (bytes && !(flags & BJ_RESULT_DEVICE)) {
             res->host = ctx->take_pinned(bytes);
             BJ_CK(cudaMemcpyAsync(res->host.p, g.pages, bytes, cudaMemcpyDeviceToHost, ctx->stream));
             res->stats.d2h_bytes = bytes;

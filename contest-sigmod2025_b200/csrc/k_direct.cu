@@ -11,16 +11,18 @@
 // Here a CTA of 256 threads takes a page. Lane l of a warp has row l of a
 // group of 32 rows, so keys, items and the null bitmap are read and written
 // coalesced, and four groups at a time are probed with their bucket loads in
-// flight together. Matches collect in shared memory and leave in one append
-// (one global atomic a page). The unique-key stages that follow the scan run
-// on the collected rows before they leave (JoinPipeline.hpp:111-131 fuses the
-// same stages), which saves their launch and the items between.
+// flight together. Matches leave in one append (one global atomic a page),
+// from the registers that found them, or, when unique-key stages follow the
+// scan, from shared memory after those stages ran on them (JoinPipeline.hpp:
+// 111-131 fuses the same stages), which saves their launch and the items
+// between.
 //
-// Bound: the bucket lookups' L2 sectors (8M probes of a 1M-key table: 67 us),
-// below a few thousand pages the latency of one page. Measured on a B200
-// against the staged form, device time of the scan (with the stages after
-// it): 30K rows in 16 pages 30 -> 10 us; 1M rows, two tables 28 -> 16 us; 8M
-// rows with 10% NULLs 145 -> 75 us.
+// Bound: the bucket lookups' L2 sectors (8M probes of a 1M-key table: 58 us,
+// 140 G sectors/s), below a few thousand pages the latency of one page.
+// Measured on a B200 against the staged form, device time of the scan (with
+// the stages after it): 30K rows in 16 pages 30 -> 10 us; 1M rows, two tables
+// 28 -> 16 us; 8M rows with 10% NULLs 145 -> 63 us (75 us with the matches
+// staged in shared memory and 1,184 CTAs looping over the pages).
 #include "launch.h"
 
 #include <algorithm>
@@ -123,136 +125,209 @@ __device__ __forceinline__ bool find_entry(const HTView& ht, uint64_t key, bool 
     return found;
 }
 
-template <bool kWide, bool kChain>
-__global__ void __launch_bounds__(kThreads, 6) k_scan_direct(DirectArgs a) {
+// A page's shape: rows, whether some are NULL, its first row and chunk.
+struct PageShape {
+    uint32_t n, row0, chunk0;
+    bool nulls;
+};
+__device__ __forceinline__ PageShape page_shape(const DevColumn& c, uint32_t p) {
+    const uint32_t hdr = __ldg(reinterpret_cast<const uint32_t*>(c.pages + size_t(p) * kPageSize));
+    PageShape s;
+    s.n = hdr & 0xffff;
+    s.nulls = (hdr >> 16) != s.n;
+    s.row0 = c.rpp ? p * c.rpp : __ldg(c.row_start + p);
+    s.chunk0 = s.nulls ? __ldg(c.chunk_base + p) : 0u;
+    return s;
+}
+
+// The keys of kGroups groups of 32 rows of a page from row r0 (a multiple of
+// 64, below `end`), a row a lane, none at or beyond row `end`; the result
+// flags the lanes' rows that have one.
+template <bool kWide>
+__device__ __forceinline__ uint32_t load_groups(const DirectArgs& a, const uint8_t* pg, const PageShape& s, uint32_t r0,
+                                                uint32_t end, uint64_t (&key)[kGroups]) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t valid = 0;
+    if (!s.nulls) {
+#pragma unroll
+        for (int k = 0; k < kGroups; k++) {
+            const uint32_t r = r0 + 32 * k + lane;
+            key[k] = 0;
+            if (r < end) {
+                key[k] = load_value<kWide>(pg, r);
+                valid |= 1u << k;
+            }
+        }
+        return valid;
+    }
+    // The value index of a row comes from the page index and the bitmap.
+    uint32_t word = 0;
+    if (lane < kGroups && r0 + 32 * lane < end) {
+        word = bitmap_word(pg, (s.n + 7) >> 3, r0 / 32 + lane);
+        const uint32_t left = end - (r0 + 32 * lane);
+        if (left < 32) word &= (1u << left) - 1;
+    }
+    uint32_t dense = __ldg(a.key.dense_base + s.chunk0 + (r0 >> 6));
+#pragma unroll
+    for (int k = 0; k < kGroups; k++) {
+        const uint32_t w = __shfl_sync(0xffffffffu, word, k);
+        const uint32_t d = dense + __popc(w & ((1u << lane) - 1));
+        dense += __popc(w);
+        key[k] = 0;
+        if (((w >> lane) & 1) && d < kPageValues) {
+            key[k] = load_value<kWide>(pg, d);
+            valid |= 1u << k;
+        }
+    }
+    return valid;
+}
+
+// The scan alone: a warp keeps its rows' matches in registers until the block
+// has reserved the page's items, and writes them in place.
+template <bool kWide>
+__global__ void __launch_bounds__(kThreads, 5) k_scan_direct(DirectArgs a) {
+    constexpr int kRounds = 3;  // rounds of kGroups groups a warp holds
+    __shared__ uint32_t count[kWarps], base;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t below = (1u << lane) - 1;
+    const uint32_t p = blockIdx.x;
+    const uint8_t* pg = a.key.pages + size_t(p) * kPageSize;
+    const PageShape s = page_shape(a.key, p);
+    // Rows a warp, in chunks of 64: 256 on a full page without NULLs, more on
+    // one with; a page of more than 3,072 rows takes several turns.
+    const uint32_t share = min((s.n + 64 * kWarps - 1) / (64 * kWarps) * 64, uint32_t(kRounds * kGroups * 32));
+    for (uint32_t span = 0; span < s.n; span += share * kWarps) {
+        const uint32_t first = span + warp * share, end = min(first + share, s.n);
+        uint32_t e[kRounds][kGroups], hit[kRounds], total = 0;
+#pragma unroll
+        for (int h = 0; h < kRounds; h++) {
+            const uint32_t r0 = first + h * (kGroups * 32);
+            hit[h] = 0;
+            if (r0 >= end) continue;
+            uint64_t key[kGroups];
+            const uint32_t valid = load_groups<kWide>(a, pg, s, r0, end, key);
+            hit[h] = probe_groups<kWide>(a, key, valid, e[h]);
+        }
+#pragma unroll
+        for (int h = 0; h < kRounds; h++) total += __popc(hit[h]);
+        for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+        if (lane == 0) count[warp] = total;
+        __syncthreads();
+        uint32_t o = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) {
+            if (w == int(warp)) o = all;
+            all += count[w];
+        }
+        if (threadIdx.x == 0 && all) base = atomicAdd(a.cursor, all);
+        __syncthreads();
+        o += base;
+        if (base + all > a.capacity || base + all < all) {
+            if (threadIdx.x == 0 && all) record_error(a.err, kErrCapacity);
+            return;
+        }
+#pragma unroll
+        for (int h = 0; h < kRounds; h++) {
+            if (first + h * (kGroups * 32) >= end) continue;
+#pragma unroll
+            for (int k = 0; k < kGroups; k++) {
+                const bool mine = (hit[h] >> k) & 1;
+                const uint32_t m = __ballot_sync(0xffffffffu, mine);
+                if (mine) {
+                    const uint32_t at = o + __popc(m & below);
+                    a.out.rows[at] = s.row0 + first + (h * kGroups + k) * 32 + lane;
+                    a.out.ents[0][at] = e[h][k];
+                    if (a.out.mult) a.out.mult[at] = ht_mult(a.ht, e[h][k]);
+                }
+                o += __popc(m);
+            }
+        }
+    }
+}
+
+// The scan with the stages after it: a page's matches collect in shared
+// memory, then each takes its further probes.
+template <bool kWide>
+__global__ void __launch_bounds__(kThreads, 6) k_scan_chain(DirectArgs a) {
     __shared__ uint2 found[kPageValues];  // (row, entry) of the page's matches
     __shared__ uint32_t nfound, base, nkept[2];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t below = (1u << lane) - 1;
-    for (uint32_t p = blockIdx.x; p < a.key.npages; p += gridDim.x) {
-        if (threadIdx.x == 0) nfound = 0;
-        __syncthreads();
-        const uint8_t* pg = a.key.pages + size_t(p) * kPageSize;
-        const uint32_t hdr = __ldg(reinterpret_cast<const uint32_t*>(pg));
-        const uint32_t n = hdr & 0xffff, nn = hdr >> 16;
-        const uint32_t row0 = a.key.rpp ? p * a.key.rpp : __ldg(a.key.row_start + p);
-        const uint32_t nbytes = (n + 7) >> 3;
-        const uint32_t cb = nn != n ? __ldg(a.key.chunk_base + p) : 0u;
-        for (uint32_t r0 = warp * (32 * kGroups); r0 < n; r0 += kWarps * 32 * kGroups) {
-            uint64_t key[kGroups];
-            uint32_t e[kGroups], valid = 0;
-            uint32_t word = 0, dense = r0;
-            if (nn != n) {
-                // Rows with NULLs before them: the value index comes from the
-                // page index (r0 is a multiple of 64) and the bitmap.
-                if (lane < kGroups) word = bitmap_word(pg, nbytes, r0 / 32 + lane);
-                dense = __ldg(a.key.dense_base + cb + (r0 >> 6));
-            }
+    const uint32_t p = blockIdx.x;
+    if (threadIdx.x == 0) nfound = 0;
+    __syncthreads();
+    const uint8_t* pg = a.key.pages + size_t(p) * kPageSize;
+    const PageShape s = page_shape(a.key, p);
+    for (uint32_t r0 = warp * (32 * kGroups); r0 < s.n; r0 += kWarps * 32 * kGroups) {
+        uint64_t key[kGroups];
+        uint32_t e[kGroups];
+        const uint32_t valid = load_groups<kWide>(a, pg, s, r0, s.n, key);
+        const uint32_t hit = probe_groups<kWide>(a, key, valid, e);
+        uint32_t m[kGroups], total = 0;
 #pragma unroll
-            for (int k = 0; k < kGroups; k++) {
-                key[k] = 0;
-                uint32_t d = dense + lane;
-                bool ok = r0 + 32 * k + lane < n;
-                if (nn != n) {
-                    uint32_t w = __shfl_sync(0xffffffffu, word, k);
-                    const uint32_t left = n - min(n, r0 + 32 * k);
-                    if (left < 32) w &= (1u << left) - 1;
-                    ok = (w >> lane) & 1;
-                    d = dense + __popc(w & below);
-                    dense += __popc(w);
-                } else {
-                    dense += 32;
-                }
-                if (ok && d < kPageValues - 1) {
-                    key[k] = load_value<kWide>(pg, d);
-                    valid |= 1u << k;
-                }
-            }
-            const uint32_t hit = probe_groups<kWide>(a, key, valid, e);
-            uint32_t m[kGroups], total = 0;
-#pragma unroll
-            for (int k = 0; k < kGroups; k++) {
-                m[k] = __ballot_sync(0xffffffffu, (hit >> k) & 1);
-                total += __popc(m[k]);
-            }
-            if (!total) continue;
-            uint32_t o = 0;
-            if (lane == 0) o = atomicAdd(&nfound, total);
-            o = __shfl_sync(0xffffffffu, o, 0);
-#pragma unroll
-            for (int k = 0; k < kGroups; k++) {
-                if ((hit >> k) & 1) found[o + __popc(m[k] & below)] = make_uint2(row0 + r0 + 32 * k + lane, e[k]);
-                o += __popc(m[k]);
-            }
+        for (int k = 0; k < kGroups; k++) {
+            m[k] = __ballot_sync(0xffffffffu, (hit >> k) & 1);
+            total += __popc(m[k]);
         }
-        __syncthreads();
-        const uint32_t cnt = nfound;
-        if (!kChain) {
-            if (threadIdx.x == 0 && cnt) base = atomicAdd(a.cursor, cnt);
-            __syncthreads();
-            for (uint32_t i = threadIdx.x; i < cnt; i += kThreads) {
-                const uint32_t o = base + i;
-                if (o >= a.capacity) {
-                    record_error(a.err, kErrCapacity);
-                    break;
-                }
-                const uint2 f = found[i];
-                a.out.rows[o] = f.x;
-                a.out.ents[0][o] = f.y;
-                if (a.out.mult) a.out.mult[o] = ht_mult(a.ht, f.y);
-            }
-            __syncthreads();  // `found` and `nfound` are reused
-        } else {
-            for (uint32_t i0 = 0, turn = 0; i0 < cnt; i0 += kThreads, turn ^= 1) {
-                if (threadIdx.x == 0) nkept[turn] = 0;
-                __syncthreads();
-                const uint32_t i = i0 + threadIdx.x;
-                bool hit = i < cnt;
-                const uint2 f = hit ? found[i] : make_uint2(0, 0);
-                uint32_t e[kMaxChain];
+        if (!total) continue;
+        uint32_t o = 0;
+        if (lane == 0) o = atomicAdd(&nfound, total);
+        o = __shfl_sync(0xffffffffu, o, 0);
 #pragma unroll
-                for (int t = 0; t < kMaxChain; t++) {
-                    e[t] = 0;
-                    if (t >= a.chain.n || !hit) continue;
-                    const ChainStage& c = a.chain.st[t];
-                    uint64_t v = 0;
-                    if (c.src.stage >= 0) {  // the scan's own match (stage 0)
-                        hit = !ht_slot_null(c.src.ht, f.y, c.src.slot);
-                        if (hit) v = ht_slot(c.src.ht, f.y, c.src.slot);
-                    } else if (f.x >= c.key.nrows) {
-                        record_error(a.err, kErrRowRange);
-                        hit = false;
-                    } else {
-                        hit = col_get(c.key, f.x, v);
-                    }
-                    hit = hit && find_entry(c.ht, v, c.use_bloom != 0, e[t]);
-                }
-                const uint32_t m = __ballot_sync(0xffffffffu, hit);
-                uint32_t o = 0;
-                if (lane == 0 && m) o = atomicAdd(&nkept[turn], __popc(m));
-                o = __shfl_sync(0xffffffffu, o, 0) + __popc(m & below);
-                __syncthreads();
-                if (threadIdx.x == 0 && nkept[turn]) base = atomicAdd(a.cursor, nkept[turn]);
-                __syncthreads();
-                if (!hit) continue;
-                o += base;
-                if (o >= a.capacity) {
-                    record_error(a.err, kErrCapacity);
-                    continue;
-                }
-                a.out.rows[o] = f.x;
-                a.out.ents[0][o] = f.y;
-                uint64_t mult = ht_mult(a.ht, f.y);
-#pragma unroll
-                for (int t = 0; t < kMaxChain; t++) {
-                    if (t >= a.chain.n) continue;
-                    a.out.ents[1 + t][o] = e[t];
-                    if (a.out.mult) mult *= ht_mult(a.chain.st[t].ht, e[t]);
-                }
-                if (a.out.mult) a.out.mult[o] = mult;
-            }
-            __syncthreads();
+        for (int k = 0; k < kGroups; k++) {
+            if ((hit >> k) & 1) found[o + __popc(m[k] & below)] = make_uint2(s.row0 + r0 + 32 * k + lane, e[k]);
+            o += __popc(m[k]);
         }
+    }
+    __syncthreads();
+    const uint32_t cnt = nfound;
+    for (uint32_t i0 = 0, turn = 0; i0 < cnt; i0 += kThreads, turn ^= 1) {
+        if (threadIdx.x == 0) nkept[turn] = 0;
+        __syncthreads();
+        const uint32_t i = i0 + threadIdx.x;
+        bool hit = i < cnt;
+        const uint2 f = hit ? found[i] : make_uint2(0, 0);
+        uint32_t e[kMaxChain];
+#pragma unroll
+        for (int t = 0; t < kMaxChain; t++) {
+            e[t] = 0;
+            if (t >= a.chain.n || !hit) continue;
+            const ChainStage& c = a.chain.st[t];
+            uint64_t v = 0;
+            if (c.src.stage >= 0) {  // the scan's own match (stage 0)
+                hit = !ht_slot_null(c.src.ht, f.y, c.src.slot);
+                if (hit) v = ht_slot(c.src.ht, f.y, c.src.slot);
+            } else if (f.x >= c.key.nrows) {
+                record_error(a.err, kErrRowRange);
+                hit = false;
+            } else {
+                hit = col_get(c.key, f.x, v);
+            }
+            hit = hit && find_entry(c.ht, v, c.use_bloom != 0, e[t]);
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, hit);
+        uint32_t o = 0;
+        if (lane == 0 && m) o = atomicAdd(&nkept[turn], __popc(m));
+        o = __shfl_sync(0xffffffffu, o, 0) + __popc(m & below);
+        __syncthreads();
+        if (threadIdx.x == 0 && nkept[turn]) base = atomicAdd(a.cursor, nkept[turn]);
+        __syncthreads();
+        if (!hit) continue;
+        o += base;
+        if (o >= a.capacity) {
+            record_error(a.err, kErrCapacity);
+            continue;
+        }
+        a.out.rows[o] = f.x;
+        a.out.ents[0][o] = f.y;
+        uint64_t mult = ht_mult(a.ht, f.y);
+#pragma unroll
+        for (int t = 0; t < kMaxChain; t++) {
+            if (t >= a.chain.n) continue;
+            a.out.ents[1 + t][o] = e[t];
+            if (a.out.mult) mult *= ht_mult(a.chain.st[t].ht, e[t]);
+        }
+        if (a.out.mult) a.out.mult[o] = mult;
     }
 }
 
@@ -271,14 +346,12 @@ int scan_probe_direct(const DevColumn& key, const HTView& ht, bool use_bloom, co
     a.capacity = capacity;
     a.err = err;
     if (chain) a.chain = *chain;
-    const uint32_t blocks = std::min<uint32_t>(key.npages, uint32_t(num_sms) * 8);
-    const bool wide = key.type == kInt64, fused = chain && chain->n > 0;
-    if (wide)
-        fused ? k_scan_direct<true, true><<<blocks, kThreads, 0, st>>>(a)
-              : k_scan_direct<true, false><<<blocks, kThreads, 0, st>>>(a);
+    const uint32_t blocks = key.npages;
+    const bool wide = key.type == kInt64;
+    if (chain && chain->n > 0)
+        wide ? k_scan_chain<true><<<blocks, kThreads, 0, st>>>(a) : k_scan_chain<false><<<blocks, kThreads, 0, st>>>(a);
     else
-        fused ? k_scan_direct<false, true><<<blocks, kThreads, 0, st>>>(a)
-              : k_scan_direct<false, false><<<blocks, kThreads, 0, st>>>(a);
+        wide ? k_scan_direct<true><<<blocks, kThreads, 0, st>>>(a) : k_scan_direct<false><<<blocks, kThreads, 0, st>>>(a);
     return 1;
 }
 

@@ -3,11 +3,16 @@
 // Replaces the reference's output writers (impl::WriterT, engine/op/
 // TableTarget.cpp:111-391, and the long-string page copy :243-250). The
 // reference fills pages greedily per worker thread; here every page is built
-// by one CTA in shared memory and stored with 16-byte writes:
+// by one CTA:
 //  * fixed width: a page holds a fixed number of rows (the most that fit when
 //    none is NULL: 1984 for INT32, 1007 for INT64/FP64), so page p covers
-//    rows [p*R, p*R+R) and all pages are independent. A block scan of the
-//    validity flags places the non-null values densely, as the format wants.
+//    rows [p*R, p*R+R) and all pages are independent. Where a value can be
+//    NULL, a block scan of the validity flags places the non-null values
+//    densely in shared memory, as the format wants, and the page is stored
+//    with 16-byte writes; where none can, it is written in place
+//    (write_dense_column). Bound there: the gathers' L2 sectors. 7.2M rows of
+//    an INT32 column and an INT64 payload on a B200: 126 us staged, 64 us
+//    (78 us while sharing the other forms' registers: 5 CTAs an SM, not 8).
 //  * VARCHAR: per-row lengths first; then a greedy packer walks blocks of 4096
 //    rows (one thread per block, same fill rule as the contest's converter,
 //    src/build_table.cpp:640-660) and emits page descriptors; a string longer
@@ -142,6 +147,67 @@ __device__ __forceinline__ uint32_t gather_direct(const OutColumns& cols, const 
         if (!ht_slot_null(ht, e, s.slot)) bits |= 1u << k;
     }
     return bits;
+}
+
+// Page pidx of a direct fixed-width column that cannot be NULL: row i's value
+// is word i after the header, so the page goes straight to global memory,
+// thread t taking rows t, t + 256, ...: items, values and stores coalesced,
+// the kPer gathers of a thread in flight together, no staging and no prefix
+// sums. value(a) is the value of item row (or matched entry) a.
+template <typename T, int kPer, typename Value>
+__device__ __forceinline__ void write_dense_page(const uint32_t* __restrict__ from, uint64_t nrows, uint32_t rpp,
+                                                 uint32_t pidx, uint8_t* __restrict__ dst, Value&& value) {
+    const uint64_t r0 = uint64_t(pidx) * rpp;
+    const uint32_t nr = uint32_t(nrows - r0 < rpp ? nrows - r0 : rpp);
+    const uint32_t t = threadIdx.x;
+    uint32_t a[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        const uint32_t i = t + 256 * k;
+        a[k] = 0;
+        if (i < nr) a[k] = from ? __ldg(from + r0 + i) : uint32_t(r0 + i);  // null: the item's own number
+    }
+    T v[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; k++)
+        if (t + 256 * k < nr) v[k] = value(a[k]);
+    T* data = reinterpret_cast<T*>(dst) + 1;  // values start at byte 4 (INT32) or 8
+#pragma unroll
+    for (int k = 0; k < kPer; k++)
+        if (t + 256 * k < nr) data[t + 256 * k] = v[k];
+    // Header, zeros up to the bitmap, the bitmap (bits beyond the rows zero).
+    if (t == 0) *reinterpret_cast<uint32_t*>(dst) = nr | (nr << 16);
+    if (sizeof(T) == 8 && t == 32) *reinterpret_cast<uint32_t*>(dst + 4) = 0;
+    const uint32_t bm = kPageSize - (nr + 7) / 8;
+    for (uint32_t b = sizeof(T) * (nr + 1) + t; b < kPageSize; b += 256) {
+        const uint32_t left = b >= bm ? nr - 8 * (b - bm) : 0u;
+        dst[b] = left >= 8 ? 0xff : uint8_t((1u << left) - 1);
+    }
+}
+
+template <typename T, int kPer>
+__device__ __forceinline__ void write_dense_column(const OutColumns& cols, const OutColumn& oc, uint32_t pidx,
+                                                   uint8_t* __restrict__ dst) {
+    const SlotSource& s = oc.slot;
+    if (s.kind != 0) {  // a word of the matched entry: its key, or a payload slot
+        const HTView& ht = cols.ps.ht[s.probe];
+        const uint32_t stride = 1 + ht.width;
+        const uint64_t* word = ht.ent + (s.kind == 2 ? 0 : 1 + s.slot);
+        write_dense_page<T, kPer>(cols.items.ents[s.probe], cols.nrows, oc.rpp, pidx, dst,
+                                  [&](uint32_t e) { return *reinterpret_cast<const T*>(word + size_t(e) * stride); });
+    } else if (s.col.rpp && !(s.col.flags & (kColNulls | kColLongStrings))) {
+        const uint8_t* values = s.col.pages + sizeof(T);
+        write_dense_page<T, kPer>(cols.items.rows, cols.nrows, oc.rpp, pidx, dst, [&](uint32_t row) {
+            const uint32_t p = page_of_row(s.col, row);
+            return *reinterpret_cast<const T*>(values + size_t(p) * kPageSize + sizeof(T) * (row - p * s.col.rpp));
+        });
+    } else {
+        write_dense_page<T, kPer>(cols.items.rows, cols.nrows, oc.rpp, pidx, dst, [&](uint32_t row) {
+            uint64_t v = 0;
+            column_value(s.col, row, v);
+            return T(v);
+        });
+    }
 }
 
 // Byte range of a short string (page p, value d) in its source page.
@@ -387,16 +453,21 @@ __device__ __forceinline__ bool cta_page(const OutColumns& cols, uint32_t g, int
 }
 
 // Every page of the result, all columns, one CTA per page in cta_page's order.
-__global__ void __launch_bounds__(256) k_write_pages(OutColumns cols, uint8_t* __restrict__ out,
+__global__ void __launch_bounds__(256) k_write_pages(OutColumns cols, uint8_t* out, uint8_t* const* out_at,
                                                      uint32_t* __restrict__ err) {
     __shared__ __align__(16) uint8_t page[kPageSize];
     int k = 0;
     uint32_t p = 0;
     if (!cta_page(cols, blockIdx.x, k, p)) return;
     const OutColumn& oc = cols.c[k];
-    uint8_t* dst = out + size_t(oc.page_base + p) * kPageSize;
+    uint8_t* dst = (out_at ? *out_at + cols.out_offset : out) + size_t(oc.page_base + p) * kPageSize;
     if (oc.type != kVarchar) {
-        if (oc.direct) {
+        if (oc.direct == 2) {
+            if (oc.type == kInt32)
+                write_dense_column<uint32_t, 8>(cols, oc, p, dst);
+            else
+                write_dense_column<uint64_t, 4>(cols, oc, p, dst);
+        } else if (oc.direct) {
             // Values straight from the items (every item is one output row).
             write_fixed_page(
                 [&](uint64_t r0, uint32_t lo, uint32_t nr, uint64_t(&v8)[8]) {
@@ -427,6 +498,21 @@ __global__ void __launch_bounds__(256) k_write_pages(OutColumns cols, uint8_t* _
         d.chunk = 0xffffffffu;
     }
     write_string_page(oc.vals, oc.valid, oc.lens, oc.src, d, page, dst, err);
+}
+
+// The same when every column is fixed width and none of its values can be
+// NULL: without the other forms' registers and shared memory twice as many
+// pages are in flight, which is what the gathers' latency asks for.
+__global__ void __launch_bounds__(256, 8) k_write_dense(OutColumns cols, uint8_t* out, uint8_t* const* out_at) {
+    int k = 0;
+    uint32_t p = 0;
+    if (!cta_page(cols, blockIdx.x, k, p)) return;
+    const OutColumn& oc = cols.c[k];
+    uint8_t* dst = (out_at ? *out_at + cols.out_offset : out) + size_t(oc.page_base + p) * kPageSize;
+    if (oc.type == kInt32)
+        write_dense_column<uint32_t, 8>(cols, oc, p, dst);
+    else
+        write_dense_column<uint64_t, 4>(cols, oc, p, dst);
 }
 
 // Parallel page assignment for VARCHAR columns ("floor packing"). With S_i
@@ -469,8 +555,8 @@ int string_pack(const uint32_t* lens, const uint8_t* valid, uint64_t n, int pass
     return 1;
 }
 
-int write_pages(const OutColumns& cols_in, uint32_t total_pages, uint8_t* out_pages, uint32_t* err,
-                cudaStream_t st) {
+int write_pages(const OutColumns& cols_in, uint32_t total_pages, uint8_t* out_pages, uint8_t* const* out_at,
+                uint32_t* err, cudaStream_t st) {
     if (!total_pages || cols_in.n <= 0) return 0;
     OutColumns cols = cols_in;
     cols.nfixed = 0;
@@ -483,13 +569,25 @@ int write_pages(const OutColumns& cols_in, uint32_t total_pages, uint8_t* out_pa
             continue;
         }
         if (!oc.npages || !oc.rpp) continue;
+        if (oc.direct) {
+            // A slot that cannot be NULL: see write_dense_column.
+            const SlotSource& sl = oc.slot;
+            const bool nulls = sl.kind == 0 ? (sl.col.flags & kColNulls) != 0
+                                            : sl.kind == 1 && cols.ps.ht[sl.probe].pnull != nullptr;
+            cols.c[c].direct = nulls ? 1u : 2u;
+        }
         cols.fixed_col[cols.nfixed++] = c;
         if (!cols.base_rpp || oc.rpp < cols.base_rpp) cols.base_rpp = oc.rpp;
     }
     cols.rounds = cols.nfixed ? uint32_t((cols.nrows + cols.base_rpp - 1) / cols.base_rpp) : 0u;
     const uint64_t ctas = uint64_t(cols.nfixed) * cols.rounds + varchar_pages;
     if (ctas > 0x7fffffffull) throw std::length_error("result pages beyond one launch");
-    k_write_pages<<<unsigned(ctas), 256, 0, st>>>(cols, out_pages, err);
+    bool dense = varchar_pages == 0;
+    for (int c = 0; c < cols.n; c++) dense = dense && (cols.c[c].type == kVarchar || cols.c[c].direct == 2);
+    if (dense)
+        k_write_dense<<<unsigned(ctas), 256, 0, st>>>(cols, out_pages, out_at);
+    else
+        k_write_pages<<<unsigned(ctas), 256, 0, st>>>(cols, out_pages, out_at, err);
     return 1;
 }
 

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(256) k_probe_stage(Items in, DevColumn key, HT
             out.rows[o] = row;
             for (int p = 0; p < in.nprobes; p++) out.ents[p][o] = in.ents[p][i];
             out.ents[in.nprobes][o] = e;
-            out.mult[o] = m * ht_mult(ht, e);
+            if (out.mult) out.mult[o] = m * ht_mult(ht, e);
             o++;
             return true;
         });

@@ -539,7 +539,8 @@ int string_floor_first(const FloorCols& cols, uint64_t n, cudaStream_t st);
 struct OutColumn {
     int32_t type;
     uint32_t floor;
-    uint32_t direct;            // fixed width: values from `slot` of the items, not vals/valid
+    uint32_t direct;            // fixed width: values from `slot` of the items, not vals/valid (2, set by
+                                // write_pages: and none can be NULL)
     SlotSource slot;
     const uint64_t* vals;       // values, or string handles into src
     const uint8_t* valid;
@@ -565,7 +566,11 @@ struct OutColumns {
     uint32_t base_rpp;
     uint32_t rounds;
     int32_t fixed_col[kMaxOut];
+    size_t out_offset;  // of these columns' pages from *out_at
 };
-int write_pages(const OutColumns& cols, uint32_t total_pages, uint8_t* out_pages, uint32_t* err, cudaStream_t st);
+// The pages go to out_pages, or (out_at not null) to the address that *out_at,
+// in device memory, holds when the kernel runs, plus cols.out_offset.
+int write_pages(const OutColumns& cols, uint32_t total_pages, uint8_t* out_pages, uint8_t* const* out_at,
+                uint32_t* err, cudaStream_t st);
 
 } // namespace bj

@@ -114,3 +114,52 @@ def test_builds(pkg, ctx, oracle, rows, copies, wide):
     b = p.new_scan_node(1, [(0, kt), (1, pkg.INT64), (2, pkg.FP64)])
     p.root = p.new_join_node(False, a, b, 0, 0, [(0, kt), (1, pkg.INT32), (3, pkg.INT64), (4, pkg.FP64)])
     check(pkg, ctx, oracle, pkg.CPlan(p), f"rows {rows} copies {copies} wide {wide}")
+
+
+def _lookup(pkg, fact, null_payload):
+    """Every fact row finds one row; INT32, INT64 and FP64 results from the fact and from the build."""
+    rng = np.random.default_rng(fact)
+    valid = (rng.random(97) >= 0.5).astype(np.uint8) if null_payload else None
+    p = pkg.Plan()
+    p.new_input(pkg.ColumnarTable(fact, [
+        column(pkg, pkg.INT32, rng.integers(0, 97, fact, dtype=np.int32)),
+        column(pkg, pkg.INT32, np.arange(fact, dtype=np.int32)), column(pkg, pkg.FP64, rng.random(fact))]))
+    p.new_input(pkg.ColumnarTable(97, [
+        column(pkg, pkg.INT32, rng.permutation(97).astype(np.int32)),
+        column(pkg, pkg.INT64, rng.integers(0, 1 << 60, 97), valid),
+        column(pkg, pkg.INT32, rng.integers(0, 1 << 30, 97, dtype=np.int32))]))
+    a = p.new_scan_node(0, [(0, pkg.INT32), (1, pkg.INT32), (2, pkg.FP64)])
+    b = p.new_scan_node(1, [(0, pkg.INT32), (1, pkg.INT64), (2, pkg.INT32)])
+    p.root = p.new_join_node(False, a, b, 0, 0, [(0, pkg.INT32), (1, pkg.INT32), (2, pkg.FP64), (4, pkg.INT64),
+                                                 (5, pkg.INT32)])
+    return pkg.CPlan(p)
+
+
+# Result sizes: part threads of a page, page edges (1,984 INT32 rows, 1,007 INT64 and FP64 rows), several pages.
+@pytest.mark.parametrize("rows", [1, 8, 255, 257, 1007, 1008, 1984, 1985, 2014, 2015, 9000])
+@pytest.mark.parametrize("null_payload", [False, True])
+def test_result_pages(pkg, ctx, oracle, rows, null_payload):
+    check(pkg, ctx, oracle, _lookup(pkg, rows, null_payload), f"rows {rows} null {null_payload}")
+
+
+@pytest.mark.parametrize("null_payload", [False, True])
+def test_device_results_of_replays_in_flight(pkg, oracle, null_payload):
+    """Replays write their pages into memory of their own: several in flight, each complete."""
+    cp = _lookup(pkg, 5000, null_payload)
+    want = oracle.execute(cp.ref())
+    with pkg.Context(0) as c:
+        res = [c.upload(cp.struct.inputs[i]) for i in range(2)]
+        for run in range(2):  # recorded, captured
+            c.execute_resident(cp, res, pkg.RESULT_DEVICE).free()
+        flying = [c.execute_resident(cp, res, pkg.RESULT_DEVICE | pkg.RESULT_ASYNC) for _ in range(4)]
+        at = [pkg.lib().bj_result_device_page(r.handle, 0, 0) for r in flying]
+        assert len(set(at)) == 4
+        for r in flying:
+            r.wait()
+            t = pkg.Plan()
+            t.new_input(r.to_table())
+            got = pkg.CPlan(t)
+            oracle_lib.assert_same_rows(oracle, ctypes.byref(got.struct.inputs[0]), want.view(), "device result")
+            r.free()
+        for x in res:
+            x.free()
