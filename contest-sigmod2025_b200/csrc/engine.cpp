@@ -699,6 +699,16 @@ class Executor {
         }
     }
 
+    // A scan stage of probe k that runs as a probe stage over the table's rows
+    // (probe_stage): repeated build keys, pages in device memory, and no long
+    // filtered scan (the lines of direct_scan).
+    bool rows_stage(const PipelinePlan& pp, uint32_t k, double rate) const {
+        const BuiltHT& bh = hts_[pp.probes[k].child];
+        const DevColumn& key = col(pp.probes[k].probe_attr);
+        return !bh.unique && !(key.flags & kColHostPages) &&
+               !(bh.view.bloom && rate < 0.5 && key.npages > kDirectFilterPages);
+    }
+
     // The scan stage as scan_probe_direct (k_direct.cu) with the unique-key
     // stages after it, when that form takes it: updates s and items. Not
     // taken: repeated build keys, pages in host memory (their loads are sized
@@ -755,18 +765,20 @@ class Executor {
     }
     // The same for counts of items (rows of an intermediate result), which are
     // 32-bit: the counts are also summed in 64 bits, and a join step whose
-    // result would not fit fails with kItemOverflow instead of wrapping.
+    // result would not fit fails with item_overflow instead of wrapping.
     uint32_t item_total(const uint32_t* in, uint32_t* out, size_t n) {
         launched(scan_exclusive_u32(in, out, n, A_, st_));
         auto* wide = reinterpret_cast<unsigned long long*>(alloc<uint64_t>(1));
         launched(sum_u32_wide(in, n, wide, st_));
-        stash_u32(ctx_, out + n, 0);
-        stash_u64(ctx_, reinterpret_cast<const uint64_t*>(wide), 1);
+        return read_item_total(wide);
+    }
+    uint32_t read_item_total(const unsigned long long* wide) {
+        stash_u64(ctx_, reinterpret_cast<const uint64_t*>(wide), 0);
         stash_err(ctx_);
-        readback(ctx_, 2);
-        if (ctx_->h_small[1] > 0xfffffffeull) {
+        readback(ctx_, 1);
+        if (ctx_->h_small[0] > 0xfffffffeull) {
             ctx_->item_overflow = true;
-            throw Fail{BJ_ERR_UNSUPPORTED, "a join step yields " + std::to_string(ctx_->h_small[1]) +
+            throw Fail{BJ_ERR_UNSUPPORTED, "a join step yields " + std::to_string(ctx_->h_small[0]) +
                                                " intermediate rows, more than 2^32 - 2"};
         }
         return uint32_t(ctx_->h_small[0]);
@@ -879,7 +891,8 @@ class Executor {
             uint32_t k = order[s];
             const HTView& ht = by_stage[s];
             if (direct_scan(pp, order, by_stage, rate, s, items)) continue;
-            if (items.rows == nullptr && col(pp.probes[k].probe_attr).type == kInt32) {
+            if (items.rows == nullptr && col(pp.probes[k].probe_attr).type == kInt32 &&
+                !rows_stage(pp, k, rate[k])) {
                 // Scan stage: stream the key pages of the scanned table. (An
                 // INT64 key column takes the item stages below, over the
                 // implicit items 0..rows-1.)
@@ -993,18 +1006,22 @@ class Executor {
             }
             resolve(items);
             if (items.count == 0) return false;
-            uint32_t tiles = (items.count + kTile - 1) / kTile;
-            uint32_t* tc = alloc<uint32_t>(tiles);
-            uint32_t* toff = alloc<uint32_t>(tiles + 1);
-            ItemsOut none{};
-            launched(probe_stage(items, key, ht, 0, tc, nullptr, none, bloom, ctx_->d_err, st_, 0xffffffffu, ksrc));
-            uint32_t total = item_total(tc, toff, tiles);
+            // The count sizes the items' buffers; a captured query has it on
+            // its tape, so its graph only appends.
+            auto* wide = reinterpret_cast<unsigned long long*>(alloc<uint64_t>(1));
+            if (ctx_->tape_mode != 2) {
+                BJ_CK(cudaMemsetAsync(wide, 0, sizeof(uint64_t), st_));
+                launched(probe_stage_count(items, key, ht, bloom, ksrc, wide, ctx_->d_err, st_));
+            }
+            const uint32_t total = read_item_total(wide);
             if (total == 0) return false;
             ItemsOut out{};
             out.rows = alloc<uint32_t>(total);
             for (size_t j = 0; j <= s; j++) out.ents[j] = alloc<uint32_t>(total);
             out.mult = !items.mult && bh.unit_mult ? nullptr : alloc<uint64_t>(total);
-            launched(probe_stage(items, key, ht, 1, nullptr, toff, out, bloom, ctx_->d_err, st_, total, ksrc));
+            uint32_t* cursor = alloc<uint32_t>(1);
+            BJ_CK(cudaMemsetAsync(cursor, 0, sizeof(uint32_t), st_));
+            launched(probe_stage(items, key, ht, bloom, ksrc, out, cursor, total, ctx_->d_err, st_));
             Items next{};
             next.rows = out.rows;
             for (size_t j = 0; j <= s; j++) next.ents[j] = out.ents[j];

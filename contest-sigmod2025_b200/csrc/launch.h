@@ -107,7 +107,6 @@ struct ItemsOut {
     uint32_t* ents[kMaxProbes];
     uint64_t* mult;
 };
-constexpr uint32_t kTile = 256;  // items per CTA tile in stage kernels (one per thread)
 // Where a stage's probe key comes from: a column of the scanned input at the
 // item's row (stage < 0), or payload slot `slot` of the entry that an earlier
 // stage `stage` matched (table ht), an attribute of an input probed before.
@@ -118,14 +117,14 @@ struct KeySource {
 };
 
 
-// Probe stage: for each item, read the key `key` at its row, probe `ht`,
-// and emit one item per matching entry. mode 0 counts matches per tile into
-// tile_counts; mode 1 writes items at tile_offsets (exclusive scan of counts).
-// Mode 0 saturates a tile's count at 2^32 - 1 (recording kErrCapacity);
-// mode 1 writes at most `capacity` items (more record kErrCapacity).
-int probe_stage(const Items& in, const DevColumn& key, const HTView& ht, int mode, uint32_t* tile_counts,
-                const uint32_t* tile_offsets, ItemsOut out, bool use_bloom, uint32_t* err, cudaStream_t st,
-                uint32_t capacity = 0xffffffffu, KeySource src = KeySource{-1, 0, HTView{}});
+// Probe stage: for each item, read the key `key` at its row (or its source
+// src), probe `ht`, and append one item per matching entry at *cursor (zero
+// before; past `capacity` items: kErrCapacity). probe_stage_count only adds
+// the number of matches to *total, in 64 bits.
+int probe_stage_count(const Items& in, const DevColumn& key, const HTView& ht, bool use_bloom, const KeySource& src,
+                      unsigned long long* total, uint32_t* err, cudaStream_t st);
+int probe_stage(const Items& in, const DevColumn& key, const HTView& ht, bool use_bloom, const KeySource& src,
+                const ItemsOut& out, uint32_t* cursor, uint32_t capacity, uint32_t* err, cudaStream_t st);
 
 // Consecutive probe stages against tables with unique keys (at most one
 // match per item and stage), fused: an item probes the stages in order and

@@ -163,3 +163,20 @@ def test_device_results_of_replays_in_flight(pkg, oracle, null_payload):
             r.free()
         for x in res:
             x.free()
+
+
+# Keys that repeat: few, more than a bucket entry's bit mask (33 and more), more matches than a block collects (4,096),
+# a stage over a scan's rows and one over items; NULL keys.
+@pytest.mark.parametrize("copies,rows", [(2, 3000), (33, 3000), (70, 2100), (400, 800)])
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("dims", [1, 2])
+def test_repeated_keys(pkg, ctx, oracle, copies, rows, wide, dims):
+    fact = 1300 if dims == 2 and copies > 33 else 5000
+    sizes = [rows // copies, 40][:dims]
+    check(pkg, ctx, oracle, star(pkg, copies, fact, sizes, 1.0, 0.1, wide, copies if dims == 1 else min(copies, 40)),
+          f"copies {copies} wide {wide} dims {dims}")
+
+
+@pytest.mark.parametrize("fact", [511, 512, 513, 512 * 1984, 512 * 1984 + 1])
+def test_repeated_keys_sizes(pkg, ctx, oracle, fact):
+    check(pkg, ctx, oracle, star(pkg, fact, fact, [4000], 0.03, 0.0, False, 3), f"fact {fact}")
