@@ -395,13 +395,23 @@ struct bj_estimator {
         cap = rows;
     }
 
-    // Forward over n_pad rows of X (a multiple of 64); outputs y.
-    void forward(int n_pad) {
+    // The batch's features: row i is row idx[i] (null: i) of X, zeros from
+    // n_real on.
+    struct Rows {
+        const uint16_t* X;
+        const uint32_t* idx;
+        int n_real;
+    };
+
+    // Forward over n_pad rows (a multiple of 64); outputs H1 and H2.
+    void forward(const Rows& in, int n_pad) {
         using namespace bj;
         GemmArgs g{};
-        g.A = static_cast<uint16_t*>(X.p);
+        g.A = in.X;
         g.a_rs = kF;
         g.a_cs = 1;
+        g.a_idx = in.idx;
+        g.a_there = in.n_real;
         g.B = WB() + kOffW1;
         g.b_rs = kH;
         g.b_cs = 1;
@@ -415,6 +425,8 @@ struct bj_estimator {
         gemm_bf16(g, stream);
         g.A = static_cast<uint16_t*>(H1.p);
         g.a_rs = kH;
+        g.a_idx = nullptr;
+        g.a_there = n_pad;
         g.B = WB() + kOffW2;
         g.K = kH;
         g.bias = WB() + kOffB2;
@@ -422,28 +434,28 @@ struct bj_estimator {
         gemm_bf16(g, stream);
     }
 
-    // Forward, loss and gradients over a batch of n_real rows (padded to
-    // n_pad) whose features are in X and targets in t.
-    void forward_backward(int n_real, int n_pad) {
+    // Forward, loss and gradients over a batch of in.n_real rows (padded to
+    // n_pad) with targets T (indexed as the rows are).
+    void forward_backward(const Rows& in, const float* T, int n_pad) {
         using namespace bj;
-        forward(n_pad);
-        EST_CK(cudaMemsetAsync(grad.p, 0, sizeof(float) * kParams, stream));
+        forward(in, n_pad);
         MlpHeadArgs h{};
         h.H2 = static_cast<uint16_t*>(H2.p);
         h.w3 = WB() + kOffW3;
         h.b3 = WB() + kOffB3;
-        h.t = static_cast<float*>(t.p);
-        h.y = static_cast<float*>(y.p);
+        h.t = T;
+        h.idx = in.idx;
         h.loss = static_cast<float*>(loss.p);
         h.dy = static_cast<float*>(dy.p);
         h.dH2 = static_cast<uint16_t*>(dH2.p);
-        h.n_real = n_real;
+        h.n_real = in.n_real;
         mlp_head(h, n_pad, stream);
         GemmArgs g{};
         // dW2 = H1^T dH2
         g.A = static_cast<uint16_t*>(H1.p);
         g.a_rs = 1;
         g.a_cs = kH;
+        g.a_there = n_pad;
         g.B = static_cast<uint16_t*>(dH2.p);
         g.b_rs = kH;
         g.b_cs = 1;
@@ -454,14 +466,12 @@ struct bj_estimator {
         g.Cf = G() + kOffW2;
         g.ldc = kH;
         gemm_bf16(g, stream);
-        colsum(static_cast<uint16_t*>(dH2.p), nullptr, n_pad, kH, G() + kOffB2, stream);
-        colsum(static_cast<uint16_t*>(H2.p), static_cast<float*>(dy.p), n_pad, kH, G() + kOffW3, stream);
-        sum_f32(static_cast<float*>(dy.p), n_pad, G() + kOffB3, stream);
         // dH1 = (dH2 W2^T) * [H1 > 0]
         g = GemmArgs{};
         g.A = static_cast<uint16_t*>(dH2.p);
         g.a_rs = kH;
         g.a_cs = 1;
+        g.a_there = n_pad;
         g.B = WB() + kOffW2;
         g.b_rs = 1;
         g.b_cs = kH;
@@ -475,9 +485,11 @@ struct bj_estimator {
         gemm_bf16(g, stream);
         // dW1 = X^T dH1
         g = GemmArgs{};
-        g.A = static_cast<uint16_t*>(X.p);
+        g.A = in.X;
         g.a_rs = 1;
         g.a_cs = kF;
+        g.a_idx = in.idx;
+        g.a_there = in.n_real;
         g.B = static_cast<uint16_t*>(dH1.p);
         g.b_rs = kH;
         g.b_cs = 1;
@@ -488,7 +500,17 @@ struct bj_estimator {
         g.Cf = G() + kOffW1;
         g.ldc = kH;
         gemm_bf16(g, stream);
-        colsum(static_cast<uint16_t*>(dH1.p), nullptr, n_pad, kH, G() + kOffB1, stream);
+        RowSumArgs r{};
+        r.dH1 = static_cast<uint16_t*>(dH1.p);
+        r.dH2 = static_cast<uint16_t*>(dH2.p);
+        r.H2 = static_cast<uint16_t*>(H2.p);
+        r.dy = static_cast<float*>(dy.p);
+        r.rows = n_pad;
+        r.b1 = G() + kOffB1;
+        r.b2 = G() + kOffB2;
+        r.w3 = G() + kOffW3;
+        r.b3 = G() + kOffB3;
+        row_sums(r, stream);
     }
 
     void adam(float lr) {
@@ -557,7 +579,7 @@ struct bj_estimator {
     // Forward and head over the pad rows in X; the first `rows` predictions to out.
     void run_head(int pad, int rows, float* out) {
         using namespace bj;
-        forward(pad);
+        forward({static_cast<uint16_t*>(X.p), nullptr, rows}, pad);
         MlpHeadArgs h{};
         h.H2 = static_cast<uint16_t*>(H2.p);
         h.w3 = WB() + kOffW3;
@@ -576,15 +598,7 @@ struct bj_estimator {
             const int rows = int(std::min<uint64_t>(kChunk, n - i0));
             const int pad = (rows + 63) & ~63;
             upload_features(f + i0 * kF, rows, pad);
-            forward(pad);
-            MlpHeadArgs h{};
-            h.H2 = static_cast<uint16_t*>(H2.p);
-            h.w3 = WB() + kOffW3;
-            h.b3 = WB() + kOffB3;
-            h.y = static_cast<float*>(y.p);
-            mlp_head(h, rows, stream);
-            EST_CK(cudaMemcpyAsync(out + i0, y.p, sizeof(float) * rows, cudaMemcpyDeviceToHost, stream));
-            EST_CK(cudaStreamSynchronize(stream));
+            run_head(pad, rows, out + i0);
         }
     }
 };
@@ -816,6 +830,7 @@ BJ_API int bj_estimator_create(int device, uint64_t seed, bj_estimator** out) {
         e->mo.alloc<float>(kParams);
         e->vo.alloc<float>(kParams);
         e->grad.alloc<float>(kParams);
+        EST_CK(cudaMemsetAsync(e->grad.p, 0, sizeof(float) * kParams, e->stream));  // (the padding's stays zero)
         // He-uniform weights (ReLU layers), zero biases.
         std::vector<float> p(kParams, 0.f);
         std::mt19937_64 rng(seed);
@@ -910,9 +925,7 @@ BJ_API int bj_estimator_train(bj_estimator* e, const float* features, const floa
             for (uint64_t b0 = 0; b0 < n; b0 += batch) {
                 const int rows = int(std::min<uint64_t>(batch, n - b0));
                 const int pad = (rows + 63) & ~63;
-                gather_rows(X, T, perm + b0, rows, pad, kF, static_cast<uint16_t*>(e->X.p), static_cast<float*>(e->t.p),
-                            e->stream);
-                e->forward_backward(rows, pad);
+                e->forward_backward({X, perm + b0, rows}, T, pad);
                 // Cosine decay from lr to lr / 10.
                 const double frac = double(done++) / std::max(1.0, total);
                 e->adam(float(lr * (0.1 + 0.9 * 0.5 * (1.0 + std::cos(M_PI * frac)))));
@@ -955,7 +968,7 @@ BJ_API int bj_estimator_gradients(bj_estimator* e, const float* features, const 
         std::copy(targets, targets + n, t.begin());
         EST_CK(cudaMemcpyAsync(e->t.p, t.data(), sizeof(float) * pad, cudaMemcpyHostToDevice, e->stream));
         EST_CK(cudaMemsetAsync(e->loss.p, 0, sizeof(float), e->stream));
-        e->forward_backward(int(n), pad);
+        e->forward_backward({static_cast<uint16_t*>(e->X.p), nullptr, int(n)}, static_cast<float*>(e->t.p), pad);
         EST_CK(cudaMemcpyAsync(grads, e->G(), sizeof(float) * kParams, cudaMemcpyDeviceToHost, e->stream));
         EST_CK(cudaMemcpyAsync(loss, e->loss.p, sizeof(float), cudaMemcpyDeviceToHost, e->stream));
         EST_CK(cudaStreamSynchronize(e->stream));

@@ -426,9 +426,10 @@ int sample_edges(const SampleEdges& e, uint32_t nsample, uint32_t* hits, cudaStr
 // BF16 matrices are passed as raw 16-bit words. C (M x N) = A (M x K) B (K x N)
 // on the tensor cores, FP32 accumulation; A(m, k) = A[m * a_rs + k * a_cs],
 // B(k, n) = B[k * b_rs + n * b_cs], one stride of each being 1 and the other
-// a multiple of 8. K must be a multiple of 32 and N of 64; an operand whose
+// a multiple of 8. K and N must be multiples of 64; an operand whose
 // contiguous dimension is its rows (m for A, n for B) needs those rows a
-// multiple of 8.
+// multiple of 8. A's other dimension (m, or k) may be indirect: its position i
+// is a_idx[i] (null: i), and positions from a_there on read zeros.
 constexpr int kMlpHidden = 256;
 enum GemmEpi : int {
     kEpiBiasRelu = 0,  // Cb = bf16(relu(acc + bias[n]))
@@ -438,6 +439,8 @@ enum GemmEpi : int {
 struct GemmArgs {
     const uint16_t* A;
     long a_rs, a_cs;
+    const uint32_t* a_idx;
+    int a_there;
     const uint16_t* B;
     long b_rs, b_cs;
     int M, N, K;
@@ -458,6 +461,7 @@ struct MlpHeadArgs {
     const uint16_t* w3;
     const uint16_t* b3;
     const float* t;
+    const uint32_t* idx;  // row m's target is t[idx[m]] (null: t[m])
     float* y;
     float* loss;
     float* dy;
@@ -465,22 +469,30 @@ struct MlpHeadArgs {
     int n_real;
 };
 int mlp_head(const MlpHeadArgs& a, int rows, cudaStream_t st);
-// out[n] += sum over rows of X[m][n] (times dy[m] when dy is given).
-int colsum(const uint16_t* X, const float* dy, int rows, int cols, float* out, cudaStream_t st);
-int sum_f32(const float* v, int n, float* out, cudaStream_t st);
+// Bias and output-layer gradients of a batch of `rows` rows (see k_row_sums).
+struct RowSumArgs {
+    const uint16_t* dH1;
+    const uint16_t* dH2;
+    const uint16_t* H2;
+    const float* dy;
+    int rows;
+    float* b1;
+    float* b2;
+    float* w3;
+    float* b3;
+};
+int row_sums(const RowSumArgs& a, cudaStream_t st);
 struct AdamArgs {
     float* w;
     uint16_t* wb;
     const float* grad;
     float* m;
     float* v;
-    long n;
+    long n;  // a multiple of 4
     float lr, beta1, beta2, eps, bc1, bc2;  // bc: 1 - beta^t
 };
 int adam_step(const AdamArgs& a, cudaStream_t st);
 int f32_to_bf16(const float* in, uint16_t* out, long n, cudaStream_t st);
-int gather_rows(const uint16_t* src, const float* tsrc, const uint32_t* idx, int n, int n_pad, int cols, uint16_t* dst,
-                float* tdst, cudaStream_t st);
 
 // ---- output pages (k_output.cu) ----
 // Page descriptors of a VARCHAR column.
