@@ -20,6 +20,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -51,7 +52,11 @@ inline size_t full_page_rows(size_t width) {
 class ThreadPool {
     public:
     explicit ThreadPool(unsigned n) {
-        for (unsigned i = 0; i < n; i++) workers_.emplace_back([this] { loop(); });
+        try {
+            for (unsigned i = 0; i < n; i++) workers_.emplace_back([this] { loop(); });
+        } catch (const std::system_error&) {
+            // No more threads to be had: the pool works with those it got.
+        }
     }
     ~ThreadPool() {
         {
