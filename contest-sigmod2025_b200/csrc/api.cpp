@@ -174,6 +174,7 @@ BJ_API void bj_context_destroy(bj_context* ctx) {
     if (ctx->h_small) cudaFreeHost(ctx->h_small);
     if (ctx->d_small) cudaFree(ctx->d_small);
     if (ctx->d_result) cudaFree(ctx->d_result);
+    if (ctx->d_counts) cudaFree(ctx->d_counts);
     if (ctx->d_err) cudaFree(ctx->d_err);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);

@@ -391,6 +391,24 @@ struct bj_context {
     std::vector<uint32_t> free_slots;
     std::vector<cudaEvent_t> free_done;
 
+    // n device words for sub-plan counts, kept and grown from call to call.
+    unsigned long long* d_counts = nullptr;
+    size_t counts_cap = 0;
+    unsigned long long* count_words(size_t n) {
+        if (n > counts_cap) {
+            if (d_counts) cudaFree(d_counts);
+            d_counts = nullptr;
+            counts_cap = 0;
+            if (cudaMalloc(reinterpret_cast<void**>(&d_counts), n * sizeof(*d_counts)) != cudaSuccess) {
+                cudaGetLastError();
+                d_counts = nullptr;
+                throw bj::Fail{BJ_ERR_OOM, "device memory for sub-plan counts"};
+            }
+            counts_cap = n;
+        }
+        return d_counts;
+    }
+
     // `n` events without timing, created once and reused across calls.
     cudaEvent_t* events(std::vector<cudaEvent_t>& v, size_t n) {
         while (v.size() < n) {

@@ -106,8 +106,7 @@ ColStats& column_stats_of(bj_context* ctx, bj_resident* r, uint32_t c) {
     if (dc.type != kInt32 && dc.type != kInt64) throw Fail{BJ_ERR_UNSUPPORTED, "join keys must be INT32 or INT64"};
     const uint32_t log2cap = std::max<uint32_t>(4, bit_width(uint64_t(dc.nrows) * 2));
     s.map.log2cap = log2cap;
-    s.map.keys = static_cast<unsigned long long*>(r->mem.alloc(sizeof(uint64_t) << log2cap));
-    s.map.vals = static_cast<unsigned long long*>(r->mem.alloc(sizeof(uint64_t) * ((size_t(1) << log2cap) + 1)));
+    s.map.slots = static_cast<ulonglong2*>(r->mem.alloc(sizeof(ulonglong2) * ((size_t(1) << log2cap) + 1)));
     struct Out {
         uint32_t hist[kHistBins];
         unsigned int totals[2];
@@ -213,77 +212,189 @@ void enumerate_subplans(const Graph& G, uint32_t max_tables, std::vector<uint32_
         if (uint32_t(__builtin_popcount(m)) <= max_tables && G.connected(m)) out.push_back(m);
 }
 
-// Exact cardinalities of sub-plans (device counts by weights).
+// Exact cardinalities of sub-plans (device counts by weights). The map of a
+// table with a sub-tree below it is built once for all sub-plans that have
+// that sub-tree there, and the sub-plans with the same root are counted in
+// passes they share.
+class Counter {
+    public:
+    Counter(bj_context* ctx, const Graph& G, const uint32_t* masks, uint64_t n)
+        : ctx_(ctx), G_(G), masks_(masks), n_(n) {}
+
+    void run(double* out) {
+        // Per sub-plan its total and, in the low half of the word after all
+        // totals, its overflow flag.
+        tot_ = ctx_->count_words(2 * n_ + 1);
+        EST_CK(cudaMemsetAsync(tot_, 0, sizeof(unsigned long long) * (2 * n_ + 1), ctx_->stream));
+        EST_CK(cudaMemsetAsync(ctx_->d_err, 0, sizeof(uint32_t), ctx_->stream));
+        for (uint64_t i = 0; i < n_; i++)
+            if (!G_.connected(masks_[i])) throw Fail{BJ_ERR_INVALID, "sub-plan inputs are not connected"};
+        for (uint32_t root = 0; root < G_.n(); root++) {
+            for (uint64_t i = 0; i < n_; i++)
+                if (uint32_t(__builtin_ctz(masks_[i])) == root && __builtin_popcount(masks_[i]) > 1) add(root, i);
+            flush(root);
+        }
+        std::vector<unsigned long long> h(2 * n_);
+        uint32_t code = 0;
+        EST_CK(cudaMemcpyAsync(h.data(), tot_, sizeof(unsigned long long) * 2 * n_, cudaMemcpyDeviceToHost, ctx_->stream));
+        EST_CK(cudaMemcpyAsync(&code, ctx_->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx_->stream));
+        EST_CK(cudaStreamSynchronize(ctx_->stream));
+        ctx_->arena.reset();
+        if (code) throw Fail{BJ_ERR_INVALID, std::string("sub-plan count: ") + dev_error_text(code)};
+        for (uint64_t i = 0; i < n_; i++) {
+            if (__builtin_popcount(masks_[i]) == 1)
+                out[i] = double(G_.g.inputs[__builtin_ctz(masks_[i])].rows);  // a lone input: its rows
+            else
+                out[i] = h[n_ + i] ? INFINITY : double(h[i]);
+        }
+    }
+
+    private:
+    // Device memory of maps kept for later sub-plans; past it they are dropped.
+    static constexpr size_t kKeptMaps = size_t(768) << 20;
+
+    // The inputs of `mask` on input y's side of edge e.
+    uint32_t side(uint32_t y, uint32_t e, uint32_t mask) const {
+        uint32_t seen = 1u << y;
+        std::vector<std::pair<uint32_t, uint32_t>> stack{{y, e}};
+        while (!stack.empty()) {
+            const auto [x, from] = stack.back();
+            stack.pop_back();
+            for (auto [z, f] : G_.adj[x])
+                if (f != from && (mask >> z & 1) && !(seen >> z & 1)) {
+                    seen |= 1u << z;
+                    stack.push_back({z, f});
+                }
+        }
+        return seen;
+    }
+
+    // Input x's key -> weight map on edge pe for the sub-tree `sub` (x and
+    // inputs behind it).
+    KeyMap node_map(uint32_t x, uint32_t pe, uint32_t sub) {
+        const uint32_t pc = G_.col(x, pe);
+        const ColStats& ps = column_stats_of(ctx_, G_.res[x], pc);
+        if (sub == 1u << x) return ps.map;  // a leaf: its key -> count map
+        for (const Made& m : made_)
+            if (m.x == x && m.pe == pe && m.sub == sub) return m.map;
+        CountNode nd{};
+        for (auto [y, e] : G_.adj[x]) {
+            if (e == pe || !(sub >> y & 1)) continue;
+            if (nd.nch == kMaxCountChildren) throw Fail{BJ_ERR_UNSUPPORTED, "a table with too many joins"};
+            const KeyMap below = node_map(y, e, side(y, e, sub));
+            nd.ch[nd.nch].key = G_.dcol(x, e);
+            nd.ch[nd.nch++].map = below;
+        }
+        nd.nrows = uint32_t(G_.g.inputs[x].rows);
+        nd.pkey = G_.res[x]->table.cols[pc];
+        const uint64_t keys = std::max<uint64_t>(1, std::min<uint64_t>(nd.nrows, ps.distinct + 1));
+        nd.out.log2cap = std::max<uint32_t>(4, bit_width(keys * 2));
+        nd.out.slots = static_cast<ulonglong2*>(ctx_->arena.alloc(sizeof(ulonglong2) * ((size_t(1) << nd.out.log2cap) + 1)));
+        ctx_->launches += uint64_t(map_clear(nd.out, ctx_->stream));
+        ctx_->launches += uint64_t(count_node(nd, ctx_->d_err, ctx_->num_sms, ctx_->stream));
+        made_.push_back({x, pe, sub, nd.out});
+        return nd.out;
+    }
+
+    // Queues sub-plan i, rooted at `root`, for a shared pass.
+    void add(uint32_t root, uint64_t i) {
+        struct Need {
+            uint32_t e, y, sub;
+        };
+        std::vector<Need> needs;
+        for (auto [y, e] : G_.adj[root])
+            if (masks_[i] >> y & 1) needs.push_back({e, y, side(y, e, masks_[i])});
+        if (needs.size() > size_t(kMaxCountChildren)) throw Fail{BJ_ERR_UNSUPPORTED, "a table with too many joins"};
+        auto option = [&](const Need& nd) {
+            for (size_t o = 0; o < opts_.size(); o++)
+                if (opts_[o].e == nd.e && opts_[o].sub == nd.sub) return int(o);
+            return -1;
+        };
+        size_t fresh = 0;
+        for (const Need& nd : needs) fresh += option(nd) < 0;
+        if (opts_.size() + fresh > size_t(kMaxCountOptions) || tots_.size() == size_t(kMaxCountTotals)) flush(root);
+        if (ctx_->arena.used_total() > kKeptMaps) {
+            flush(root);
+            made_.clear();
+            ctx_->arena.reset();  // (the next maps are written after the kernels that read these)
+        }
+        uint32_t set = 0;
+        for (const Need& nd : needs) {
+            int o = option(nd);
+            if (o < 0) {
+                o = int(opts_.size());
+                opts_.push_back({nd.e, nd.y, nd.sub, node_map(nd.y, nd.e, nd.sub)});
+            }
+            set |= 1u << o;
+        }
+        tots_.push_back({set, uint32_t(i)});
+    }
+
+    // Launches the queued sub-plans' pass over `root`.
+    void flush(uint32_t root) {
+        if (!tots_.empty()) {
+            // Options by edge, a child alone before its sub-trees.
+            std::vector<uint32_t> order(opts_.size());
+            for (size_t o = 0; o < order.size(); o++) order[o] = uint32_t(o);
+            std::sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
+                return opts_[a].e != opts_[b].e ? opts_[a].e < opts_[b].e
+                                                : __builtin_popcount(opts_[a].sub) < __builtin_popcount(opts_[b].sub);
+            });
+            std::vector<uint32_t> place(opts_.size());
+            CountGroup g{};
+            for (uint32_t o : order) {
+                const Option& op = opts_[o];
+                CountOption& c = g.opt[g.nopt];
+                const bool same = g.nopt > 0 && opts_[order[size_t(g.nopt) - 1]].e == op.e;
+                c.key = G_.dcol(root, op.e);
+                c.map = op.map;
+                c.new_edge = same ? 0 : 1;
+                c.leaf = -1;
+                if (same) {
+                    int first = g.nopt - 1;
+                    while (!g.opt[first].new_edge) first--;
+                    if (opts_[order[size_t(first)]].sub == 1u << op.y) c.leaf = first;
+                }
+                place[o] = uint32_t(g.nopt++);
+            }
+            for (const Total& t : tots_) {
+                uint32_t set = 0;
+                for (uint32_t m = t.set; m; m &= m - 1) set |= 1u << place[size_t(__builtin_ctz(m))];
+                g.options[g.ntot] = set;
+                g.slot[g.ntot++] = t.slot;
+            }
+            g.nrows = uint32_t(G_.g.inputs[root].rows);
+            g.total = tot_;
+            g.flags = reinterpret_cast<unsigned int*>(tot_ + n_);
+            ctx_->launches += uint64_t(count_group(g, ctx_->num_sms, ctx_->stream));
+        }
+        opts_.clear();
+        tots_.clear();
+    }
+
+    struct Made {
+        uint32_t x, pe, sub;
+        KeyMap map;
+    };
+    struct Option {
+        uint32_t e, y, sub;
+        KeyMap map;
+    };
+    struct Total {
+        uint32_t set, slot;
+    };
+    bj_context* ctx_;
+    const Graph& G_;
+    const uint32_t* masks_;
+    uint64_t n_;
+    unsigned long long* tot_ = nullptr;
+    std::vector<Made> made_;
+    std::vector<Option> opts_;
+    std::vector<Total> tots_;
+};
+
 void exact_cards(bj_context* ctx, const Graph& G, const uint32_t* masks, uint64_t n, double* out) {
-    DevBuf tot_buf;
-    unsigned long long* tot = tot_buf.alloc<unsigned long long>(2 * n + 1);
-    EST_CK(cudaMemsetAsync(tot, 0, sizeof(unsigned long long) * (2 * n + 1), ctx->stream));
-    EST_CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream));
-    std::vector<uint32_t> order;
-    std::vector<int> parent, pedge;
-    std::vector<KeyMap> child_map(G.n());
-    for (uint64_t i = 0; i < n; i++) {
-        const uint32_t mask = masks[i];
-        if (!G.connected(mask)) throw Fail{BJ_ERR_INVALID, "sub-plan inputs are not connected"};
-        const uint32_t root = __builtin_ctz(mask);
-        G.tree(mask, root, order, parent, pedge, false);
-        if (order.size() == 1) {
-            out[i] = double(G.g.inputs[root].rows);  // a lone input: its rows
-            continue;
-        }
-        // Children before parents.
-        for (size_t oi = order.size(); oi-- > 0;) {
-            const uint32_t x = order[oi];
-            std::vector<std::pair<uint32_t, uint32_t>> kids;  // (child, edge)
-            for (auto [y, e] : G.adj[x])
-                if ((mask >> y & 1) && parent[y] == int(x)) kids.push_back({y, e});
-            if (kids.empty()) {
-                // A leaf: its key -> count map from the column statistics.
-                child_map[x] = column_stats_of(ctx, G.res[x], G.col(x, uint32_t(pedge[x]))).map;
-                continue;
-            }
-            if (kids.size() > size_t(kMaxCountChildren)) throw Fail{BJ_ERR_UNSUPPORTED, "a table with too many joins"};
-            CountNode nd{};
-            nd.nch = int(kids.size());
-            for (size_t j = 0; j < kids.size(); j++) {
-                nd.ch[j].key = G.dcol(x, kids[j].second);
-                nd.ch[j].map = child_map[kids[j].first];
-            }
-            nd.nrows = uint32_t(G.g.inputs[x].rows);
-            nd.flags = reinterpret_cast<unsigned int*>(tot + n + i);
-            if (x == root) {
-                nd.has_out = 0;
-                nd.total = tot + i;
-            } else {
-                nd.has_out = 1;
-                const uint32_t pc = G.col(x, uint32_t(pedge[x]));
-                nd.pkey = G.res[x]->table.cols[pc];
-                const ColStats& ps = column_stats_of(ctx, G.res[x], pc);
-                const uint64_t keys = std::max<uint64_t>(1, std::min<uint64_t>(nd.nrows, ps.distinct + 1));
-                KeyMap m{};
-                m.log2cap = std::max<uint32_t>(4, bit_width(keys * 2));
-                m.keys = static_cast<unsigned long long*>(ctx->arena.alloc(sizeof(uint64_t) << m.log2cap));
-                m.vals = static_cast<unsigned long long*>(ctx->arena.alloc(sizeof(uint64_t) * ((size_t(1) << m.log2cap) + 1)));
-                ctx->launches += uint64_t(map_clear(m, ctx->stream));
-                nd.out = m;
-                child_map[x] = m;
-            }
-            ctx->launches += uint64_t(count_node(nd, ctx->d_err, ctx->num_sms, ctx->stream));
-        }
-        // The maps of this sub-plan are dead once its kernels ran; the next
-        // sub-plan's (stream-ordered after them) may reuse the arena.
-        ctx->arena.reset();
-    }
-    std::vector<unsigned long long> h(2 * n);
-    uint32_t code = 0;
-    EST_CK(cudaMemcpyAsync(h.data(), tot, sizeof(unsigned long long) * 2 * n, cudaMemcpyDeviceToHost, ctx->stream));
-    EST_CK(cudaMemcpyAsync(&code, ctx->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-    EST_CK(cudaStreamSynchronize(ctx->stream));
-    if (code) throw Fail{BJ_ERR_INVALID, std::string("sub-plan count: ") + dev_error_text(code)};
-    for (uint64_t i = 0; i < n; i++) {
-        if (__builtin_popcount(masks[i]) == 1) continue;
-        out[i] = h[n + i] ? INFINITY : double(h[i]);
-    }
+    Counter(ctx, G, masks, n).run(out);
 }
 
 // Join-sample selectivities of every directed edge: sel[2e] for a -> b (rows

@@ -11,12 +11,12 @@
 //  * k_col_stats: per join-key column, a 64-bin histogram of its non-null
 //    values by the top six bits of the key hash, and a key -> count map (the
 //    index the join samples and exact counts look keys up in);
-//  * k_count_node: one table of a connected sub-plan in the exact count of
-//    its join result, by weights instead of rows (a row's weight is the
-//    number of join results it takes part in below it): children's maps are
-//    looked up, weights multiplied, and summed into the parent-edge key's
-//    map, or into the total at the root, so a count never materialises a
-//    join result;
+//  * k_count_node, k_count_group: exact counts of join results, by weights
+//    instead of rows (a row's weight is the number of join results it takes
+//    part in below it): children's maps are looked up, weights multiplied, and
+//    summed into the parent-edge key's map (an inner table), or into the
+//    totals of the sub-plans that have the table at their root, so a count
+//    never materialises a join result;
 //  * k_sample_edges: for every directed join edge, how many of 64 sampled
 //    rows of one side find their key in the other side's map (the
 //    reference's join sample).
@@ -33,79 +33,87 @@ __device__ __forceinline__ uint32_t map_slot(uint64_t key, uint32_t log2cap) {
     return uint32_t(mix64(key) >> (64 - log2cap));
 }
 
-// Adds v to key's value (inserting the key). The key ~0ull, which marks empty
-// slots, keeps its value in vals[cap].
-__device__ __forceinline__ void map_add(const KeyMap& m, uint64_t key, unsigned long long v, unsigned int* distinct,
-                                        uint32_t* err) {
+// Adds v to key's value (inserting the key); returns 1 when the key is new. The
+// key ~0ull, which marks empty slots, keeps its value in slot cap.
+__device__ __forceinline__ uint32_t map_add(const KeyMap& m, uint64_t key, unsigned long long v, uint32_t* err) {
     const uint32_t cap = 1u << m.log2cap;
-    if (key == kMapEmpty) {
-        if (atomicAdd(&m.vals[cap], v) == 0 && distinct) atomicAdd(distinct, 1u);
-        return;
-    }
-    uint32_t pos = map_slot(key, m.log2cap);
+    if (key == kMapEmpty) return atomicAdd(&m.slots[cap].y, v) == 0 ? 1u : 0u;
+    uint32_t pos = map_slot(key, m.log2cap), added = 0;
     for (uint32_t step = 0; step < cap; step++) {
-        unsigned long long cur = m.keys[pos];
+        unsigned long long cur = m.slots[pos].x;
         if (cur == kMapEmpty) {
-            cur = atomicCAS(&m.keys[pos], kMapEmpty, key);
+            cur = atomicCAS(&m.slots[pos].x, kMapEmpty, key);
             if (cur == kMapEmpty) {
-                if (distinct) atomicAdd(distinct, 1u);
+                added = 1;
                 cur = key;
             }
         }
         if (cur == key) {
-            atomicAdd(&m.vals[pos], v);
-            return;
+            atomicAdd(&m.slots[pos].y, v);
+            return added;
         }
         pos = (pos + 1) & (cap - 1);
     }
     record_error(err, kErrCapacity);
+    return 0;
 }
 
+// Key's value in a finished map (0 when it is not there): key and value in one
+// 16-byte load.
 __device__ __forceinline__ unsigned long long map_get(const KeyMap& m, uint64_t key) {
     const uint32_t cap = 1u << m.log2cap;
-    if (key == kMapEmpty) return m.vals[cap];
+    if (key == kMapEmpty) return m.slots[cap].y;
     uint32_t pos = map_slot(key, m.log2cap);
     for (uint32_t step = 0; step < cap; step++) {
-        const unsigned long long cur = m.keys[pos];
-        if (cur == key) return m.vals[pos];
-        if (cur == kMapEmpty) return 0;
+        const ulonglong2 cur = __ldg(m.slots + pos);
+        if (cur.x == key) return cur.y;
+        if (cur.x == kMapEmpty) return 0;
         pos = (pos + 1) & (cap - 1);
     }
     return 0;
 }
 
-__global__ void k_map_clear(KeyMap m) {
-    const uint32_t cap = 1u << m.log2cap;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= cap; i += gridDim.x * blockDim.x) {
-        if (i < cap) m.keys[i] = kMapEmpty;
-        m.vals[i] = 0;
-    }
+__device__ __forceinline__ bool map_overflowed(const KeyMap& m) {
+    return m.slots[1u << m.log2cap].x != kMapEmpty;
 }
 
-// One CTA per page (grid-stride): a page stores its non-null values densely,
-// so the histogram and the map need neither the bitmap nor the row index.
-__global__ void __launch_bounds__(256) k_col_stats(DevColumn c, KeyMap m, uint32_t* hist, unsigned int* totals,
-                                                   uint32_t* err) {
+__global__ void k_map_clear(KeyMap m) {
+    const uint32_t cap = 1u << m.log2cap;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= cap; i += gridDim.x * blockDim.x)
+        m.slots[i] = make_ulonglong2(kMapEmpty, 0);
+}
+
+// `parts` CTAs per page (grid-stride): a page stores its non-null values
+// densely, so the histogram and the map need neither the bitmap nor the row
+// index. A column of few pages is split further: its CTAs' chains of atomics
+// are what it takes (45K rows in 23 pages: 33 us whole, 13 us in eight parts).
+__global__ void __launch_bounds__(256) k_col_stats(DevColumn c, uint32_t parts, KeyMap m, uint32_t* hist,
+                                                   unsigned int* totals, uint32_t* err) {
     __shared__ uint32_t h[kHistBins];
     for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) h[i] = 0;
     __syncthreads();
     const uint32_t width = c.type == kInt32 ? 4 : 8;
-    uint32_t nonnull = 0;
-    for (uint32_t p = blockIdx.x; p < c.npages; p += gridDim.x) {
+    uint32_t nonnull = 0, distinct = 0;
+    for (uint32_t u = blockIdx.x; u < c.npages * parts; u += gridDim.x) {
+        const uint32_t p = u / parts;
         const uint8_t* pg = c.pages + size_t(p) * kPageSize;
         const uint32_t hd = c.hdr ? c.hdr[p] : *reinterpret_cast<const uint32_t*>(pg);
         const uint32_t nn = hd >> 16;
         const uint32_t base = width;  // values start at byte 4 (INT32) or 8 (INT64)
-        for (uint32_t i = threadIdx.x; i < nn; i += blockDim.x) {
+        for (uint32_t i = (u % parts) * blockDim.x + threadIdx.x; i < nn; i += parts * blockDim.x) {
             uint64_t key = width == 4 ? uint64_t(*reinterpret_cast<const uint32_t*>(pg + base + 4 * i))
                                       : *reinterpret_cast<const uint64_t*>(pg + base + 8 * size_t(i));
             atomicAdd(&h[key_hash_any(key, c.type) >> 58], 1u);
-            map_add(m, key, 1ull, &totals[1], err);
+            distinct += map_add(m, key, 1ull, err);
             nonnull++;
         }
     }
-    for (int o = 16; o > 0; o >>= 1) nonnull += __shfl_down_sync(0xffffffffu, nonnull, o);
+    for (int o = 16; o > 0; o >>= 1) {
+        nonnull += __shfl_down_sync(0xffffffffu, nonnull, o);
+        distinct += __shfl_down_sync(0xffffffffu, distinct, o);
+    }
     if ((threadIdx.x & 31) == 0 && nonnull) atomicAdd(&totals[0], nonnull);
+    if ((threadIdx.x & 31) == 0 && distinct) atomicAdd(&totals[1], distinct);
     __syncthreads();
     for (int i = threadIdx.x; i < kHistBins; i += blockDim.x)
         if (h[i]) atomicAdd(&hist[i], h[i]);
@@ -120,8 +128,8 @@ __device__ __forceinline__ unsigned long long mul_sat(unsigned long long a, unsi
     return a * b;
 }
 
+// An inner table's map: each row's weight, summed into its parent-edge key.
 __global__ void __launch_bounds__(256) k_count_node(CountNode n, uint32_t* err) {
-    unsigned long long local = 0;
     bool over = false;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n.nrows; r += gridDim.x * blockDim.x) {
         unsigned long long w = 1;
@@ -134,20 +142,100 @@ __global__ void __launch_bounds__(256) k_count_node(CountNode n, uint32_t* err) 
             w = mul_sat(w, map_get(n.ch[j].map, k), over);
         }
         if (!w) continue;
-        if (n.has_out) {
-            uint64_t k;
-            if (col_get(n.pkey, r, k)) map_add(n.out, k, w, nullptr, err);
-        } else {
-            const unsigned long long s = local + w;
-            if (s < local) over = true;
-            local = s;
+        uint64_t k;
+        if (col_get(n.pkey, r, k)) map_add(n.out, k, w, err);
+    }
+    if (blockIdx.x == 0 && threadIdx.x < uint32_t(n.nch)) over = over || map_overflowed(n.ch[threadIdx.x].map);
+    if (over) n.out.slots[1u << n.out.log2cap].x = 0;
+}
+
+// The totals of sub-plans with the same root table, in one pass over it. A
+// tile's rows look up every option (a child edge with the sub-tree below it
+// that some sub-plan has there) once. A row whose options are all 0 or 1 (keys
+// unique on the child's side) counts 1 in every total whose options it has, so
+// only its set of options is counted, and the sets' counts go into the totals
+// at the end; the other rows' options are multiplied, a warp a total, a lane a
+// row. The pass, its keys and the lookups' random sectors are paid once for up
+// to kMaxCountTotals sub-plans instead of for each.
+// The 26 totals over the 1.5M-row root of a seven-table query on a B200: 93
+// us, where a pass a total took 26 x 40 us; every row multiplied: 191 us.
+__global__ void __launch_bounds__(256) k_count_group(CountGroup g) {
+    extern __shared__ uint32_t sets[];  // rows by set of options, 1 << nopt
+    __shared__ unsigned long long w[kMaxCountOptions][256];
+    __shared__ uint32_t heavy[256];  // per row: its options when one is above 1, else 0
+    constexpr int kPerWarp = kMaxCountTotals / 8;
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    unsigned long long acc[kPerWarp] = {};
+    uint32_t over = 0;  // bit i: this warp's i-th total passed 2^64 - 1
+    for (uint32_t m = t; m < 1u << g.nopt; m += 256) sets[m] = 0;
+    __syncthreads();
+    for (uint32_t r0 = blockIdx.x * 256; r0 < g.nrows; r0 += gridDim.x * 256) {
+        const uint32_t r = r0 + t;
+        uint64_t key = 0;
+        bool ok = false, above = false;
+        uint32_t have = 0;
+        for (int o = 0; o < g.nopt; o++) {
+            const CountOption& op = g.opt[o];
+            if (op.new_edge) ok = r < g.nrows && col_get(op.key, r, key);
+            // A key that the child's own rows lack is in none of its sub-trees' maps.
+            const bool gone = op.leaf >= 0 && !((have >> op.leaf) & 1);
+            const unsigned long long v = ok && !gone ? map_get(op.map, key) : 0ull;
+            w[o][t] = v;
+            above = above || v > 1;
+            if (v) have |= 1u << o;
         }
+        heavy[t] = above ? have : 0u;
+        const uint32_t same = __match_any_sync(0xffffffffu, above ? 0u : have);
+        if (!above && have && lane == uint32_t(__ffs(same) - 1)) atomicAdd(&sets[have], __popc(same));
+        if (!__syncthreads_or(above)) continue;
+#pragma unroll
+        for (int i = 0; i < kPerWarp; i++) {
+            const int s = int(warp) + 8 * i;
+            if (s >= g.ntot) continue;
+            const uint32_t set = g.options[s];
+            for (int j = 0; j < 8; j++) {
+                if ((heavy[32 * j + lane] & set) != set) continue;
+                unsigned long long v = 1;
+                bool o1 = false;
+                for (uint32_t m = set; m; m &= m - 1) {
+                    const unsigned long long x = w[__ffs(m) - 1][32 * j + lane];
+                    v = (v | x) >> 32 ? mul_sat(v, x, o1) : static_cast<unsigned long long>(uint32_t(v)) * uint32_t(x);
+                }
+                const unsigned long long sum = acc[i] + v;
+                if (o1 || sum < v) over |= 1u << i;
+                acc[i] = sum;
+            }
+        }
+        __syncthreads();
     }
-    if (!n.has_out) {
-        for (int o = 16; o > 0; o >>= 1) local += __shfl_down_sync(0xffffffffu, local, o);
-        if ((threadIdx.x & 31) == 0 && local) atomicAdd(n.total, local);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kPerWarp; i++) {
+        const int s = int(warp) + 8 * i;
+        if (s >= g.ntot) continue;
+        const uint32_t set = g.options[s];
+        unsigned long long v = acc[i];
+        bool o1 = (over >> i) & 1;
+        for (uint32_t m = lane; m < 1u << g.nopt; m += 32)
+            if ((m & set) == set) {
+                const unsigned long long sum = v + sets[m];
+                o1 = o1 || sum < v;
+                v = sum;
+            }
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long u = __shfl_xor_sync(0xffffffffu, v, o);
+            o1 = o1 || v + u < v;
+            v += u;
+        }
+        o1 = __any_sync(0xffffffffu, o1);
+        if (lane == 0 && v) {
+            const unsigned long long old = atomicAdd(g.total + g.slot[s], v);
+            o1 = o1 || old + v < old;
+        }
+        if (blockIdx.x == 0)
+            for (uint32_t m = set; m; m &= m - 1) o1 = o1 || map_overflowed(g.opt[__ffs(m) - 1].map);
+        if (lane == 0 && o1) atomicOr(g.flags + 2 * g.slot[s], 1u);
     }
-    if (over) atomicOr(n.flags, 1u);
 }
 
 // Row i of a sample: a seeded position (the reference samples 64 rows with
@@ -178,8 +266,8 @@ int map_clear(const KeyMap& m, cudaStream_t st) {
 int column_stats(const DevColumn& c, const KeyMap& m, uint32_t* hist, unsigned int* totals, uint32_t* err, int num_sms,
                  cudaStream_t st) {
     if (!c.npages) return 0;
-    const uint32_t blocks = std::min<uint32_t>(c.npages, uint32_t(num_sms) * 8);
-    k_col_stats<<<blocks, 256, 0, st>>>(c, m, hist, totals, err);
+    const uint32_t most = uint32_t(num_sms) * 8, parts = std::min<uint32_t>(8, std::max<uint32_t>(1, most / c.npages));
+    k_col_stats<<<std::min<uint32_t>(c.npages * parts, most), 256, 0, st>>>(c, parts, m, hist, totals, err);
     return 1;
 }
 
@@ -187,6 +275,13 @@ int count_node(const CountNode& n, uint32_t* err, int num_sms, cudaStream_t st) 
     if (!n.nrows) return 0;
     const uint32_t blocks = std::min<uint32_t>((n.nrows + 255) / 256, uint32_t(num_sms) * 8);
     k_count_node<<<blocks, 256, 0, st>>>(n, err);
+    return 1;
+}
+
+int count_group(const CountGroup& g, int num_sms, cudaStream_t st) {
+    if (!g.nrows || !g.ntot) return 0;
+    const uint32_t blocks = std::min<uint32_t>((g.nrows + 255) / 256, uint32_t(num_sms) * 8);
+    k_count_group<<<blocks, 256, sizeof(uint32_t) << g.nopt, st>>>(g);
     return 1;
 }
 

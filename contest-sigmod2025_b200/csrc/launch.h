@@ -371,12 +371,12 @@ struct SampleSet {
 int sample_probes(const SampleSet& set, uint32_t nsample, uint32_t* hits, cudaStream_t st);
 
 // ---- join-ordering statistics (k_stats.cu) ----
-// Open-addressing map from a key slot (u64) to a u64 value: keys[i] = ~0ull
-// marks an empty slot; the key ~0ull itself keeps its value in vals[cap].
-// cap = 1 << log2cap; keys has cap words, vals cap + 1.
+// Open-addressing map from a key slot (u64) to a u64 value: slot = (key, value);
+// the key ~0ull marks an empty slot, and itself keeps its value in slot cap,
+// whose key word tells an overflow: other than ~0ull, some value of the map
+// passed 2^64 - 1. cap = 1 << log2cap; cap + 1 slots.
 struct KeyMap {
-    unsigned long long* keys;
-    unsigned long long* vals;
+    ulonglong2* slots;
     uint32_t log2cap;
 };
 constexpr int kHistBins = 64;
@@ -387,11 +387,10 @@ int map_clear(const KeyMap& m, cudaStream_t st);
 // keys (both zero before).
 int column_stats(const DevColumn& c, const KeyMap& m, uint32_t* hist, unsigned int* totals, uint32_t* err,
                  int num_sms, cudaStream_t st);
-// One table of a sub-plan's exact count. For every row r: w = product over
+// An inner table of sub-plans' exact counts. For every row r: w = product over
 // the children j of ch[j].map[value of ch[j].key at r] (0 when the value is
-// NULL or absent); then, with has_out, out[value of pkey at r] += w (rows
-// with a NULL pkey skipped), else *total += w. flags[0] |= 1 when a weight
-// or the total passes 2^64 - 1.
+// NULL or absent); out[value of pkey at r] += w (rows with a NULL pkey
+// skipped). A weight past 2^64 - 1, here or in a child's map, marks `out`.
 constexpr int kMaxCountChildren = 12;
 struct CountChild {
     DevColumn key;  // this table's column on the edge to the child
@@ -400,14 +399,37 @@ struct CountChild {
 struct CountNode {
     CountChild ch[kMaxCountChildren];
     int nch;
-    int has_out;
     DevColumn pkey;  // this table's column on the edge to its parent
     KeyMap out;
+    uint32_t nrows;
+};
+int count_node(const CountNode& n, uint32_t* err, int num_sms, cudaStream_t st);
+// The root table of several sub-plans. Option o of a row: opt[o].map[value of
+// opt[o].key] (0 when the value is NULL or absent). For sub-plan s: *(total +
+// slot[s]) += the sum over the rows of the product of the options in
+// options[s]; word 2 slot[s] of flags |= 1 when a product, the total or a value
+// of one of its maps passes 2^64 - 1. Options of one edge lie side by side, new_edge set on the first;
+// leaf: an earlier option of the same edge whose map holds every key of this
+// one's (-1: none).
+constexpr int kMaxCountOptions = kMaxCountChildren;
+constexpr int kMaxCountTotals = 64;
+struct CountOption {
+    DevColumn key;
+    KeyMap map;
+    int new_edge;
+    int leaf;
+};
+struct CountGroup {
+    CountOption opt[kMaxCountOptions];
+    int nopt;
+    int ntot;
+    uint32_t options[kMaxCountTotals];
+    uint32_t slot[kMaxCountTotals];
     uint32_t nrows;
     unsigned long long* total;
     unsigned int* flags;
 };
-int count_node(const CountNode& n, uint32_t* err, int num_sms, cudaStream_t st);
+int count_group(const CountGroup& g, int num_sms, cudaStream_t st);
 // Join samples: for directed edge d, hits[d] (zero before) = how many of
 // nsample seeded rows of e[d].key have a non-null value present in e[d].map.
 constexpr int kMaxSampleEdges = 24;
