@@ -124,14 +124,13 @@ BJ_API int bj_context_create(int device, bj_context** out) {
         if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return BJ_ERR_CUDA;
     if (cudaStreamCreateWithFlags(&ctx->copy, cudaStreamNonBlocking) != cudaSuccess) return BJ_ERR_CUDA;
     if (cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess) return BJ_ERR_CUDA;
-    if (cudaMalloc(&ctx->d_err, 256) != cudaSuccess) return BJ_ERR_OOM;
+    if (cudaMalloc(&ctx->d_err, sizeof(uint32_t) * bj_context::kWords) != cudaSuccess) return BJ_ERR_OOM;
     ctx->arena.err = ctx->d_err;
-    if (cudaMalloc(&ctx->d_small, sizeof(uint64_t) * 64) != cudaSuccess) return BJ_ERR_OOM;
     if (cudaMalloc(&ctx->d_result, 256) != cudaSuccess) return BJ_ERR_OOM;
     if (cudaHostAlloc(reinterpret_cast<void**>(&ctx->h_small), sizeof(uint64_t) * 64, cudaHostAllocDefault) != cudaSuccess)
         return BJ_ERR_OOM;
-    cudaMemset(ctx->d_err, 0, 256);
-    cudaMemset(ctx->d_small, 0, sizeof(uint64_t) * 64);
+    cudaMemset(ctx->d_err, 0, sizeof(uint32_t) * bj_context::kWords);
+    std::memset(ctx->h_small, 0, sizeof(uint64_t) * 64);
     if (cudaHostAlloc(reinterpret_cast<void**>(&ctx->async_err), sizeof(uint32_t) * bj_context::kAsyncSlots,
                       cudaHostAllocDefault) != cudaSuccess)
         return BJ_ERR_OOM;
@@ -172,7 +171,6 @@ BJ_API void bj_context_destroy(bj_context* ctx) {
     for (auto& b : ctx->pinned_free) cudaFreeHost(b.p);
     if (ctx->stage.p) cudaFreeHost(ctx->stage.p);
     if (ctx->h_small) cudaFreeHost(ctx->h_small);
-    if (ctx->d_small) cudaFree(ctx->d_small);
     if (ctx->d_result) cudaFree(ctx->d_result);
     if (ctx->d_counts) cudaFree(ctx->d_counts);
     if (ctx->d_err) cudaFree(ctx->d_err);

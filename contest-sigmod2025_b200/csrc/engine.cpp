@@ -55,8 +55,6 @@ void phase_stats(const std::vector<cudaEvent_t>& marks, bj_stats& st) {
 }
 
 
-// Reads back `n` u64 slots of ctx->d_small after the stream drains; checks the
-// device error word.
 // Host-side trace of a call (B200JOIN_TRACE=1): milliseconds since the call
 // began and since the previous mark, to stderr. B200JOIN_TRACE=2 drains the
 // call's stream at every mark first, so that a mark's delta is the device
@@ -86,6 +84,8 @@ void trace(const char* what) {
     g_trace_last = now;
 }
 
+// Reads back the queued values (into h_small) after the stream drains; checks the
+// device error word.
 void readback(bj_context* ctx, int n) {
     (void)n;
     if (ctx->tape_mode == 2) {
@@ -94,9 +94,10 @@ void readback(bj_context* ctx, int n) {
         std::memcpy(ctx->h_small, t.slots[t.pos++].data(), sizeof(uint64_t) * 64);
         return;
     }
-    ctx->launches += uint64_t(gather_values(ctx->gather, ctx->d_small, ctx->stream));
+    // The kernel writes the pinned slots themselves (unified addressing): no
+    // copy follows it.
+    ctx->launches += uint64_t(gather_values(ctx->gather, ctx->h_small, ctx->stream));
     ctx->gather.n = 0;
-    BJ_CK(cudaMemcpyAsync(ctx->h_small, ctx->d_small, sizeof(uint64_t) * 64, cudaMemcpyDeviceToHost, ctx->stream));
     trace("read-back issued");
     BJ_CK(cudaStreamSynchronize(ctx->stream));
     trace("read-back done");
@@ -275,8 +276,11 @@ void index_columns(bj_context* ctx, std::vector<ColumnJob>& jobs, Scratch& mem) 
     for (size_t i0 = 0; i0 < jobs.size(); i0 += 15) {
         const size_t i1 = std::min(jobs.size(), i0 + 15);
         PageIndexBatch b{};
-        uint32_t* flags = static_cast<uint32_t*>(sc.alloc(sizeof(uint32_t) * (i1 - i0)));
-        BJ_CK(cudaMemsetAsync(flags, 0, sizeof(uint32_t) * (i1 - i0), ctx->stream));
+        uint32_t* flags = ctx->take_words(i1 - i0);
+        if (!flags) {
+            flags = static_cast<uint32_t*>(sc.alloc(sizeof(uint32_t) * (i1 - i0)));
+            BJ_CK(cudaMemsetAsync(flags, 0, sizeof(uint32_t) * (i1 - i0), ctx->stream));
+        }
         for (size_t i = i0; i < i1; i++) {
             const uint32_t np = uint32_t(jobs[i].src ? jobs[i].src->num_pages : 0);
             PageIndexCol& c = b.c[b.n++];
@@ -344,8 +348,9 @@ struct BuiltHT {
     HTView view{};
     bool empty = true;
     uint32_t* dflags = nullptr;  // device: [0] some key repeats, [1] some multiplicity > 1
-    bool unique = false;         // host copies, valid once the parent pipeline read them back
+    bool unique = false;         // host copies, valid once read back (flags_known)
     bool unit_mult = false;
+    bool flags_known = false;
 };
 
 // A scan that tests a filter runs in the direct form below this many key
@@ -355,6 +360,11 @@ struct BuiltHT {
 // filter the direct form is never slower: 100K keys of which 35% are kept,
 // all matching: 1M rows 36 / 18 us.
 constexpr uint32_t kDirectFilterPages = 512;
+
+// Builds fed by probes of inputs up to this many rows are sized by the rows:
+// at most 2.6 MB of buckets and counts too many, 1-2 us, for a read-back of
+// about 20 us.
+constexpr uint32_t kBoundedBuild = 65536;
 
 // Streamed scans (Executor::streamed_scan): windows of 16 MiB, three in flight.
 constexpr uint32_t kWindowPages = 2048;
@@ -525,6 +535,7 @@ class Executor {
                     batched[p] = 1;
                     batched_[p] = 1;
                 }
+                read_leaf_flags();
             }
         }
         for (size_t p = 0; p < np; p++) {
@@ -563,6 +574,15 @@ class Executor {
     template <typename T>
     T* alloc(size_t n) {
         return static_cast<T*>(A_.alloc(sizeof(T) * std::max<size_t>(n, 1)));
+    }
+    // n zero words on the current stream.
+    uint32_t* zero_words(size_t n) {
+        uint32_t* p = ctx_->take_words(n);
+        if (!p) {
+            p = alloc<uint32_t>(n);
+            BJ_CK(cudaMemsetAsync(p, 0, sizeof(uint32_t) * n, st_));
+        }
+        return p;
     }
     void launched(int n) { ctx_->launches += uint64_t(n); }
     void record_timed() {
@@ -629,8 +649,7 @@ class Executor {
         r.out.rows = alloc<uint32_t>(r.cap);
         for (size_t j = 0; j < s2; j++) r.out.ents[j] = alloc<uint32_t>(r.cap);
         r.out.mult = unit ? nullptr : alloc<uint64_t>(r.cap);
-        r.cursor = alloc<uint32_t>(1);
-        BJ_CK(cudaMemsetAsync(r.cursor, 0, sizeof(uint32_t), st_));
+        r.cursor = zero_words(1);
         r.result.rows = r.out.rows;
         for (size_t j = 0; j < s2; j++) r.result.ents[j] = r.out.ents[j];
         r.result.mult = r.out.mult;
@@ -699,6 +718,37 @@ class Executor {
         }
     }
 
+    // Whether the probe's column is scanned in the direct form with or without a
+    // filter.
+    bool small_scan(const PipelinePlan::Probe& pr) const {
+        const DevColumn& key = col(pr.probe_attr);
+        return pr.key_probe < 0 && !(key.flags & kColHostPages) && key.npages <= kDirectFilterPages;
+    }
+
+    // Reads back the flags of the leaves that pipelines of one short scan probe
+    // (one read-back for all, where each such pipeline had its own).
+    void read_leaf_flags() {
+        std::vector<size_t> want;
+        for (size_t p = 0; p + 1 < ex_.pipelines.size(); p++) {
+            const PipelinePlan& pp = ex_.pipelines[p];
+            if (pp.probes.size() == 1 && batched_[pp.probes[0].child] && small_scan(pp.probes[0]) && want.size() < 30)
+                want.push_back(pp.probes[0].child);
+        }
+        if (want.empty()) return;
+        for (size_t i = 0; i < want.size(); i++) {
+            stash_u32(ctx_, hts_[want[i]].dflags, int(2 * i));
+            stash_u32(ctx_, hts_[want[i]].dflags + 1, int(2 * i + 1));
+        }
+        stash_err(ctx_);
+        readback(ctx_, int(2 * want.size()));
+        for (size_t i = 0; i < want.size(); i++) {
+            BuiltHT& t = hts_[want[i]];
+            t.unique = ctx_->h_small[2 * i] == 0;
+            t.unit_mult = ctx_->h_small[2 * i + 1] == 0;
+            t.flags_known = true;
+        }
+    }
+
     // A scan stage of probe k that runs as a probe stage over the table's rows
     // (probe_stage): repeated build keys, pages in device memory, and no long
     // filtered scan (the lines of direct_scan).
@@ -741,9 +791,8 @@ class Executor {
             next.rows = out.rows = alloc<uint32_t>(key.nrows);
             next.ents[0] = out.ents[0] = alloc<uint32_t>(key.nrows);
             next.mult = out.mult = bh.unit_mult ? nullptr : alloc<uint64_t>(key.nrows);
-            cursor = alloc<uint32_t>(1);
+            cursor = zero_words(1);
             next.dcount = cursor;
-            BJ_CK(cudaMemsetAsync(cursor, 0, sizeof(uint32_t), st_));
         }
         if (ctx_->profile) begin_timed();
         launched(scan_probe_direct(key, ht, bloom, fuse ? &chain.ch : nullptr, out, cursor, key.nrows, ctx_->d_err,
@@ -816,13 +865,16 @@ class Executor {
         std::vector<uint32_t> order(np);
         std::iota(order.begin(), order.end(), 0u);
         std::vector<double> rate(np, 1.0);
-        if (np) {
+        if (np == 1 && !root && hts_[pp.probes[0].child].flags_known && small_scan(pp.probes[0])) {
+            // One probe, one order; a scan this short takes the same form
+            // whatever its hit rate, which nothing else needs to know.
+        } else if (np) {
             // Sample rows read from pinned host memory cross the host link one
             // by one, beside the scan windows' copies: fewer of them there.
             bool host_keys = false;
             for (size_t k = 0; k < np; k++) host_keys = host_keys || (col(pp.probes[k].probe_attr).flags & kColHostPages);
             uint32_t nsample = uint32_t(std::min<uint64_t>(in.rows, host_keys ? 1024 : 4096));
-            uint32_t* hits = alloc<uint32_t>(np);
+            uint32_t* hits = ctx_->tape_mode != 2 ? zero_words(np) : nullptr;
             SampleSet set{};
             set.n = int(np);
             for (size_t k = 0; k < np; k++) {
@@ -846,6 +898,7 @@ class Executor {
                 BuiltHT& child = hts_[pp.probes[k].child];
                 child.unique = ctx_->h_small[16 + 2 * k] == 0;
                 child.unit_mult = ctx_->h_small[17 + 2 * k] == 0;
+                child.flags_known = true;
             }
             // A table whose build was restricted by another probed here holds
             // only keys that one's filter passes, so it can only look more
@@ -907,8 +960,7 @@ class Executor {
                     out.rows = alloc<uint32_t>(cap);
                     out.ents[0] = alloc<uint32_t>(cap);
                     out.mult = bh.unit_mult ? nullptr : alloc<uint64_t>(cap);
-                    uint32_t* cursor = alloc<uint32_t>(2);  // item cursor, candidate count (split scan)
-                    BJ_CK(cudaMemsetAsync(cursor, 0, 2 * sizeof(uint32_t), st_));
+                    uint32_t* cursor = zero_words(2);  // item cursor, candidate count (split scan)
                     // The next stage reads the count on the device.
                     Items next{};
                     next.rows = out.rows;
@@ -1008,9 +1060,9 @@ class Executor {
             if (items.count == 0) return false;
             // The count sizes the items' buffers; a captured query has it on
             // its tape, so its graph only appends.
-            auto* wide = reinterpret_cast<unsigned long long*>(alloc<uint64_t>(1));
+            unsigned long long* wide = nullptr;
             if (ctx_->tape_mode != 2) {
-                BJ_CK(cudaMemsetAsync(wide, 0, sizeof(uint64_t), st_));
+                wide = reinterpret_cast<unsigned long long*>(zero_words(2));
                 launched(probe_stage_count(items, key, ht, bloom, ksrc, wide, ctx_->d_err, st_));
             }
             const uint32_t total = read_item_total(wide);
@@ -1019,8 +1071,7 @@ class Executor {
             out.rows = alloc<uint32_t>(total);
             for (size_t j = 0; j <= s; j++) out.ents[j] = alloc<uint32_t>(total);
             out.mult = !items.mult && bh.unit_mult ? nullptr : alloc<uint64_t>(total);
-            uint32_t* cursor = alloc<uint32_t>(1);
-            BJ_CK(cudaMemsetAsync(cursor, 0, sizeof(uint32_t), st_));
+            uint32_t* cursor = zero_words(1);
             launched(probe_stage(items, key, ht, bloom, ksrc, out, cursor, total, ctx_->d_err, st_));
             Items next{};
             next.rows = out.rows;
@@ -1030,7 +1081,10 @@ class Executor {
             next.nprobes = int(s + 1);
             items = next;
         }
-        resolve(items);
+        // A build of few items is sized by their bound instead of their count
+        // (which the device has): no read-back.
+        const bool bounded = pp.build_key >= 0 && items.dcount && items.count <= kBoundedBuild;
+        if (!bounded) resolve(items);
         if (items.count == 0) return false;
 
         SlotSources src{};
@@ -1633,7 +1687,7 @@ int execute_common(bj_context* ctx, const bj_plan* plan, bj_resident* const* res
         ctx->tune = tune_for(ctx, ex);
         res->types = ex.out_types;
         uint64_t launches0 = ctx->launches;
-        BJ_CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream));
+        ctx->begin_words();
         BJ_CK(cudaEventRecord(ctx->ev0, ctx->stream));
         std::vector<DevTable> owned;
         std::vector<const DevTable*> tables(plan->num_inputs, nullptr);

@@ -335,10 +335,27 @@ struct bj_context {
     std::vector<bj::PinnedBlock> pinned_free;
     std::unique_ptr<bj::ThreadPool> pool;
     std::string last_error;
-    uint32_t* d_err = nullptr;         // device error word
+    // Device words: the error word, then words that a call finds zero and takes
+    // for its counters (begin_words clears them all with one memset).
+    static constexpr uint32_t kWords = 256;
+    uint32_t* d_err = nullptr;
+    uint32_t words_taken = 2;
+    void begin_words() {
+        using bj::Fail;
+        BJ_CK(cudaMemsetAsync(d_err, 0, sizeof(uint32_t) * kWords, stream));
+        words_taken = 2;
+    }
+    // n zero words, 8-byte aligned, for work ordered after begin_words on the
+    // call's stream; null when the call has taken them all.
+    uint32_t* take_words(size_t n) {
+        n = (n + 1) & ~size_t(1);
+        if (words_taken + n > kWords) return nullptr;
+        uint32_t* p = d_err + words_taken;
+        words_taken += uint32_t(n);
+        return p;
+    }
     uint8_t** d_result = nullptr;      // device word: where a replayed graph writes its result pages
-    uint64_t* h_small = nullptr;       // pinned readback slots
-    uint64_t* d_small = nullptr;       // device readback slots
+    uint64_t* h_small = nullptr;       // pinned readback slots, written by the device
     bj::GatherList gather{};               // values queued for the next read-back
     uint64_t launches = 0;
     std::atomic<uint64_t> live_results{0};

@@ -70,9 +70,10 @@ bool capture_graph(bj_context* ctx, GraphEntry& g, const bj_plan* plan, bj_resid
         ctx->graph_output = true;
         BJ_CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
         capturing = true;
-        // The graph clears the device error word first and copies it to the
-        // pinned read-back slot last, so a replay needs no other call.
-        BJ_CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream));
+        // The graph clears the device error word (and its counters) first and
+        // copies it to the pinned read-back slot last, so a replay needs no
+        // other call.
+        ctx->begin_words();
         uint64_t pipelines = 0;
         const bool nonempty = run_pipelines(ctx, ex, tables, res, flags, pipelines);
         BJ_CK(cudaMemcpyAsync(&ctx->h_small[63], ctx->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));

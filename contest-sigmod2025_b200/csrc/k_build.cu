@@ -161,7 +161,13 @@ __device__ __forceinline__ void emit_tuple(const BuildArgs& a, uint32_t i) {
 
 __global__ void __launch_bounds__(256) k_emit(BuildArgs a) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < a.tb.count) emit_tuple(a, i);
+    if (i >= a.tb.count) return;
+    if (a.in.dcount && i >= *a.in.dcount) {  // beyond the items: represents nothing
+        a.rank1[i] = 0;
+        a.tb.mult[i] = 0;
+        return;
+    }
+    emit_tuple(a, i);
 }
 
 __global__ void __launch_bounds__(256) k_aggregate(BuildArgs a) {
@@ -443,7 +449,6 @@ int build_leaves(const LeafBatch& batch, cudaStream_t st) {
 }
 
 int sample_probes(const SampleSet& set, uint32_t nsample, uint32_t* hits, cudaStream_t st) {
-    cudaMemsetAsync(hits, 0, sizeof(uint32_t) * std::max(set.n, 1), st);
     if (!nsample || set.n <= 0) return 0;
     k_sample_probes<<<dim3((nsample + 255) / 256, unsigned(set.n)), 256, 0, st>>>(set, nsample, hits);
     return 1;

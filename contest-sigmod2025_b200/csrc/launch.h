@@ -358,7 +358,7 @@ int build_cluster_leaves(const LeafBatch& batch, cudaStream_t st);
 // (both words must be zero before).
 int ht_flags(HTView ht, uint32_t nbuckets, uint32_t* flags, int num_sms, cudaStream_t st);
 // Counts, for nsample evenly spaced rows of each probe's key column, how many
-// hit its table: hits[p] for probe p, all probes in one launch (the role of
+// hit its table: hits[p] (zero before) for probe p, all in one launch (the role of
 // the reference's 64-row join samples, engine/query/QueryPlan.cpp:719-746).
 struct SampleProbe {
     DevColumn key;

@@ -44,7 +44,7 @@ BJ_API int bj_resident_upload(bj_context* ctx, const bj_table* table, bj_residen
         } else {
             for (uint64_t c = 0; c < table->num_columns; c++) d.present[c] = 1;
         }
-        BJ_CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream));
+        ctx->begin_words();
         upload_pages(ctx, jobs);
         index_columns(ctx, jobs, r->mem);
         BJ_CK(cudaStreamSynchronize(ctx->stream));

@@ -180,3 +180,27 @@ def test_repeated_keys(pkg, ctx, oracle, copies, rows, wide, dims):
 @pytest.mark.parametrize("fact", [511, 512, 513, 512 * 1984, 512 * 1984 + 1])
 def test_repeated_keys_sizes(pkg, ctx, oracle, fact):
     check(pkg, ctx, oracle, star(pkg, fact, fact, [4000], 0.03, 0.0, False, 3), f"fact {fact}")
+
+
+# Builds fed by probes: sized by the input's rows up to 65,536, by their counted items beyond; none, some and all rows
+# surviving; the sub-dimension's keys unique and repeated.
+@pytest.mark.parametrize("rows", [1, 300, 65_536, 65_537])
+@pytest.mark.parametrize("keep", [0.0, 0.4, 1.0])
+@pytest.mark.parametrize("copies", [1, 2])
+def test_fed_builds(pkg, ctx, oracle, rows, keep, copies):
+    rng = np.random.default_rng(rows + copies)
+    fact, sub = (100_003 if rows > 300 else 2003), max(1, rows // 7)
+    p = pkg.Plan()
+    i32 = lambda v: column(pkg, pkg.INT32, np.asarray(v, dtype=np.int32))  # noqa: E731
+    some = (rng.random(rows) >= 0.05).astype(np.uint8)
+    p.new_input(pkg.ColumnarTable(fact, [i32(np.arange(fact)), i32(rng.integers(0, rows, fact))]))
+    p.new_input(pkg.ColumnarTable(rows, [i32(rng.permutation(rows)),
+                                         column(pkg, pkg.INT32, rng.integers(0, sub, rows).astype(np.int32), some)]))
+    own = np.repeat(rng.permutation(sub)[:max(1, int(sub * keep))] + (0 if keep else 2 * sub), copies)
+    p.new_input(pkg.ColumnarTable(len(own), [i32(own), i32(rng.integers(0, 1 << 30, len(own)))]))
+    f = p.new_scan_node(0, [(0, pkg.INT32), (1, pkg.INT32)])
+    d = p.new_scan_node(1, [(0, pkg.INT32), (1, pkg.INT32)])
+    s = p.new_scan_node(2, [(0, pkg.INT32), (1, pkg.INT32)])
+    j = p.new_join_node(False, f, d, 1, 0, [(0, pkg.INT32), (3, pkg.INT32)])
+    p.root = p.new_join_node(False, j, s, 1, 0, [(0, pkg.INT32), (3, pkg.INT32)])
+    check(pkg, ctx, oracle, pkg.CPlan(p), f"rows {rows} keep {keep} copies {copies}")
