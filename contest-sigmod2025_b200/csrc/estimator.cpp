@@ -95,6 +95,81 @@ struct DevBuf {
     }
 };
 
+// The way of feature rows to a device, shared by its estimators and freed with
+// the last of them: a small pinned ring (pinning costs a millisecond or more a
+// MB), the events of its slots' copies and the threads that convert into it.
+class RowStage {
+    public:
+    static std::shared_ptr<RowStage> of(int device) {
+        static std::mutex m;
+        static std::vector<std::weak_ptr<RowStage>> stages;
+        std::lock_guard<std::mutex> g(m);
+        if (stages.size() <= size_t(device)) stages.resize(size_t(device) + 1);
+        std::shared_ptr<RowStage> s = stages[size_t(device)].lock();
+        if (!s) stages[size_t(device)] = s = std::make_shared<RowStage>(device);
+        return s;
+    }
+
+    explicit RowStage(int device)
+        : device_(device), pool_(std::min(std::max(1u, std::thread::hardware_concurrency()), 8u) - 1) {
+        void* p = nullptr;
+        EST_CK(cudaHostAlloc(&p, sizeof(uint16_t) * kSlots * kSlotWords, cudaHostAllocDefault));
+        ring_ = static_cast<uint16_t*>(p);
+        for (cudaEvent_t& e : done_)
+            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+                free_all();
+                throw Fail{BJ_ERR_CUDA, "event creation failed"};
+            }
+    }
+    ~RowStage() {
+        for (cudaEvent_t e : done_) cudaEventSynchronize(e);
+        free_all();
+    }
+
+    // Host threads take slots of rows in order, convert them into the ring and
+    // start their copies on `stream`, each after the copy that used its place
+    // before. Bound: the host reading its FP32 rows. A whole prediction of 6,000
+    // rows on a 16-core B200 host: 1.5 ms, where one thread converting every
+    // row into pageable memory before their copy made it 8.4 ms.
+    void upload(const float* f, uint64_t n, uint16_t* dst, cudaStream_t stream) {
+        std::lock_guard<std::mutex> g(m_);
+        std::atomic<uint64_t> copying[kSlots];  // slots taken from the ring's place whose copy is enqueued
+        for (auto& c : copying) c = 0;
+        std::atomic<int> failed{cudaSuccess};
+        pool_.parallel_for((n + kSlotRows - 1) / kSlotRows, [&](size_t i) {
+            const size_t s = i % kSlots, turn = i / kSlots;
+            // The slot's earlier turns were taken by threads already at work.
+            while (copying[s].load(std::memory_order_acquire) < turn) std::this_thread::yield();
+            cudaError_t e = cudaSetDevice(device_);
+            if (e == cudaSuccess) e = cudaEventSynchronize(done_[s]);
+            if (e == cudaSuccess) {
+                const uint64_t r0 = i * kSlotRows, rows = std::min(kSlotRows, n - r0);
+                uint16_t* to = ring_ + s * kSlotWords;
+                to_bf16_n(f + r0 * kF, to, rows * kF);
+                e = cudaMemcpyAsync(dst + r0 * kF, to, sizeof(uint16_t) * rows * kF, cudaMemcpyHostToDevice, stream);
+                if (e == cudaSuccess) e = cudaEventRecord(done_[s], stream);
+            }
+            if (e != cudaSuccess) failed = e;
+            copying[s].store(turn + 1, std::memory_order_release);
+        });
+        EST_CK(cudaError_t(failed.load()));
+    }
+
+    private:
+    static constexpr uint64_t kSlots = 8, kSlotRows = 64;
+    static constexpr size_t kSlotWords = kSlotRows * kF;
+    void free_all() {
+        for (cudaEvent_t e : done_)
+            if (e) cudaEventDestroy(e);
+        cudaFreeHost(ring_);
+    }
+    int device_;
+    std::mutex m_;
+    uint16_t* ring_ = nullptr;
+    cudaEvent_t done_[kSlots] = {};
+    ThreadPool pool_;
+};
+
 // Statistics of column c of a resident table, computed on first use.
 ColStats& column_stats_of(bj_context* ctx, bj_resident* r, uint32_t c) {
     std::lock_guard<std::mutex> g(r->stats_m);
@@ -506,7 +581,9 @@ struct bj_estimator {
     long step = 0;
     // Batch scratch for up to cap rows.
     int cap = 0;
-    bj::DevBuf X, H1, H2, dH2, dH1, y, t, dy, loss, idx;
+    bj::DevBuf batch;  // one allocation for all of them
+    uint16_t *X = nullptr, *H1 = nullptr, *H2 = nullptr, *dH2 = nullptr, *dH1 = nullptr;
+    float *y = nullptr, *t = nullptr, *dy = nullptr, *loss = nullptr;
     // The training set (BF16 rows, targets, the epoch's order), kept for the
     // next call up to kKeptSet bytes of rows.
     bj::DevBuf set_rows, set_targets, set_order;
@@ -514,40 +591,34 @@ struct bj_estimator {
 
     // Pinned BF16 feature rows of a planned query's sub-plans (kPredictChunk).
     uint16_t* hx = nullptr;
-    // Rows on their way to the device (upload_rows): a small pinned ring (pinning
-    // costs about 1 ms a MB), the events of its slots' copies, and the threads
-    // that convert into it.
-    static constexpr uint64_t kSlots = 8, kSlotRows = 64;
-    uint16_t* ring = nullptr;
-    cudaEvent_t slot_done[kSlots] = {};
-    std::unique_ptr<bj::ThreadPool> pool;
+    std::shared_ptr<bj::RowStage> stage;  // of the device, with its other estimators
 
     ~bj_estimator() {
         if (stream) cudaStreamSynchronize(stream);
         if (hx) cudaFreeHost(hx);
-        if (ring) cudaFreeHost(ring);
-        for (cudaEvent_t e : slot_done)
-            if (e) cudaEventDestroy(e);
         if (stream) cudaStreamDestroy(stream);
     }
     float* W() { return static_cast<float*>(w.p); }
     uint16_t* WB() { return static_cast<uint16_t*>(wb.p); }
     float* G() { return static_cast<float*>(grad.p); }
 
-    void reserve(int rows) {
-        if (rows <= cap) return;
+    void reserve(uint64_t rows) {
         using namespace bj;
-        X.alloc<uint16_t>(size_t(rows) * kF);
-        H1.alloc<uint16_t>(size_t(rows) * kH);
-        H2.alloc<uint16_t>(size_t(rows) * kH);
-        dH2.alloc<uint16_t>(size_t(rows) * kH);
-        dH1.alloc<uint16_t>(size_t(rows) * kH);
-        y.alloc<float>(rows);
-        t.alloc<float>(rows);
-        dy.alloc<float>(rows);
-        loss.alloc<float>(4);
-        idx.alloc<uint32_t>(rows);
-        cap = rows;
+        if (rows <= uint64_t(cap)) return;
+        size_t n = 64;
+        while (n < rows) n *= 2;
+        cap = 0;
+        uint16_t* p = batch.alloc<uint16_t>(n * (kF + 4 * kH) + 2 * (3 * n + 4));
+        X = p;
+        H1 = X + n * kF;
+        H2 = H1 + n * kH;
+        dH2 = H2 + n * kH;
+        dH1 = dH2 + n * kH;
+        y = reinterpret_cast<float*>(dH1 + n * kH);
+        t = y + n;
+        dy = t + n;
+        loss = dy + n;
+        cap = int(n);
     }
 
     // The batch's features: row i is row idx[i] (null: i) of X, zeros from
@@ -575,17 +646,17 @@ struct bj_estimator {
         g.K = kF;
         g.epi = kEpiBiasRelu;
         g.bias = WB() + kOffB1;
-        g.Cb = static_cast<uint16_t*>(H1.p);
+        g.Cb = H1;
         g.ldc = kH;
         gemm_bf16(g, stream);
-        g.A = static_cast<uint16_t*>(H1.p);
+        g.A = H1;
         g.a_rs = kH;
         g.a_idx = nullptr;
         g.a_there = n_pad;
         g.B = WB() + kOffW2;
         g.K = kH;
         g.bias = WB() + kOffB2;
-        g.Cb = static_cast<uint16_t*>(H2.p);
+        g.Cb = H2;
         gemm_bf16(g, stream);
     }
 
@@ -595,23 +666,23 @@ struct bj_estimator {
         using namespace bj;
         forward(in, n_pad);
         MlpHeadArgs h{};
-        h.H2 = static_cast<uint16_t*>(H2.p);
+        h.H2 = H2;
         h.w3 = WB() + kOffW3;
         h.b3 = WB() + kOffB3;
         h.t = T;
         h.idx = in.idx;
-        h.loss = static_cast<float*>(loss.p);
-        h.dy = static_cast<float*>(dy.p);
-        h.dH2 = static_cast<uint16_t*>(dH2.p);
+        h.loss = loss;
+        h.dy = dy;
+        h.dH2 = dH2;
         h.n_real = in.n_real;
         mlp_head(h, n_pad, stream);
         GemmArgs g{};
         // dW2 = H1^T dH2
-        g.A = static_cast<uint16_t*>(H1.p);
+        g.A = H1;
         g.a_rs = 1;
         g.a_cs = kH;
         g.a_there = n_pad;
-        g.B = static_cast<uint16_t*>(dH2.p);
+        g.B = dH2;
         g.b_rs = kH;
         g.b_cs = 1;
         g.M = kH;
@@ -623,7 +694,7 @@ struct bj_estimator {
         gemm_bf16(g, stream);
         // dH1 = (dH2 W2^T) * [H1 > 0]
         g = GemmArgs{};
-        g.A = static_cast<uint16_t*>(dH2.p);
+        g.A = dH2;
         g.a_rs = kH;
         g.a_cs = 1;
         g.a_there = n_pad;
@@ -634,8 +705,8 @@ struct bj_estimator {
         g.N = kH;
         g.K = kH;
         g.epi = kEpiReluMask;
-        g.mask = static_cast<uint16_t*>(H1.p);
-        g.Cb = static_cast<uint16_t*>(dH1.p);
+        g.mask = H1;
+        g.Cb = dH1;
         g.ldc = kH;
         gemm_bf16(g, stream);
         // dW1 = X^T dH1
@@ -645,7 +716,7 @@ struct bj_estimator {
         g.a_cs = kF;
         g.a_idx = in.idx;
         g.a_there = in.n_real;
-        g.B = static_cast<uint16_t*>(dH1.p);
+        g.B = dH1;
         g.b_rs = kH;
         g.b_cs = 1;
         g.M = kF;
@@ -656,10 +727,10 @@ struct bj_estimator {
         g.ldc = kH;
         gemm_bf16(g, stream);
         RowSumArgs r{};
-        r.dH1 = static_cast<uint16_t*>(dH1.p);
-        r.dH2 = static_cast<uint16_t*>(dH2.p);
-        r.H2 = static_cast<uint16_t*>(H2.p);
-        r.dy = static_cast<float*>(dy.p);
+        r.dH1 = dH1;
+        r.dH2 = dH2;
+        r.H2 = H2;
+        r.dy = dy;
         r.rows = n_pad;
         r.b1 = G() + kOffB1;
         r.b2 = G() + kOffB2;
@@ -697,43 +768,10 @@ struct bj_estimator {
         step = 0;
     }
 
-    // Brings n feature rows (f32 host) to dst as BF16: host threads take slots
-    // of rows in order, convert them into the ring and start their copies, each
-    // after the copy that used its place before. Bound: the host reading its
-    // FP32 rows. A whole prediction of 6,000 rows on a 16-core B200 host: 1.5
-    // ms, where one thread converting every row into pageable memory before
-    // their copy made it 8.4 ms.
+    // Brings n feature rows (f32 host) to dst as BF16.
     void upload_rows(const float* f, uint64_t n, uint16_t* dst) {
-        using namespace bj;
-        constexpr size_t kSlotWords = kSlotRows * kF;
-        if (!ring) {
-            void* p = nullptr;
-            EST_CK(cudaHostAlloc(&p, sizeof(uint16_t) * kSlots * kSlotWords, cudaHostAllocDefault));
-            ring = static_cast<uint16_t*>(p);
-        }
-        for (cudaEvent_t& e : slot_done)
-            if (!e) EST_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        if (!pool) pool = std::make_unique<ThreadPool>(std::min(std::max(1u, std::thread::hardware_concurrency()), 8u) - 1);
-        std::atomic<uint64_t> copying[kSlots];  // slots taken from the ring's place whose copy is enqueued
-        for (auto& c : copying) c = 0;
-        std::atomic<int> failed{cudaSuccess};
-        pool->parallel_for((n + kSlotRows - 1) / kSlotRows, [&](size_t i) {
-            const size_t s = i % kSlots, turn = i / kSlots;
-            // The slot's earlier turns were taken by threads already at work.
-            while (copying[s].load(std::memory_order_acquire) < turn) std::this_thread::yield();
-            cudaError_t e = cudaSetDevice(device);
-            if (e == cudaSuccess) e = cudaEventSynchronize(slot_done[s]);
-            if (e == cudaSuccess) {
-                const uint64_t r0 = i * kSlotRows, rows = std::min(kSlotRows, n - r0);
-                uint16_t* to = ring + s * kSlotWords;
-                to_bf16_n(f + r0 * kF, to, rows * kF);
-                e = cudaMemcpyAsync(dst + r0 * kF, to, sizeof(uint16_t) * rows * kF, cudaMemcpyHostToDevice, stream);
-                if (e == cudaSuccess) e = cudaEventRecord(slot_done[s], stream);
-            }
-            if (e != cudaSuccess) failed = e;
-            copying[s].store(turn + 1, std::memory_order_release);
-        });
-        EST_CK(cudaError_t(failed.load()));
+        if (!stage) stage = bj::RowStage::of(device);
+        stage->upload(f, n, dst, stream);
     }
 
     static constexpr int kPredictChunk = 4096;
@@ -744,7 +782,7 @@ struct bj_estimator {
     template <typename Fill>
     void predict_rows(uint64_t n, float* out, Fill&& fill) {
         using namespace bj;
-        reserve(kPredictChunk);
+        reserve(std::min<uint64_t>(n, kPredictChunk));
         if (!hx) {
             void* p = nullptr;
             EST_CK(cudaHostAlloc(&p, sizeof(uint16_t) * size_t(kPredictChunk) * kF, cudaHostAllocDefault));
@@ -753,7 +791,7 @@ struct bj_estimator {
         for (uint64_t i0 = 0; i0 < n; i0 += kPredictChunk) {
             const int rows = int(std::min<uint64_t>(kPredictChunk, n - i0));
             fill(i0, rows, hx);
-            EST_CK(cudaMemcpyAsync(X.p, hx, sizeof(uint16_t) * size_t(rows) * kF, cudaMemcpyHostToDevice, stream));
+            EST_CK(cudaMemcpyAsync(X, hx, sizeof(uint16_t) * size_t(rows) * kF, cudaMemcpyHostToDevice, stream));
             run_head(rows, out + i0);
         }
     }
@@ -761,23 +799,23 @@ struct bj_estimator {
     // Predictions of the first `rows` rows of X to out.
     void run_head(int rows, float* out) {
         using namespace bj;
-        forward({static_cast<uint16_t*>(X.p), nullptr, rows}, (rows + 63) & ~63);
+        forward({X, nullptr, rows}, (rows + 63) & ~63);
         MlpHeadArgs h{};
-        h.H2 = static_cast<uint16_t*>(H2.p);
+        h.H2 = H2;
         h.w3 = WB() + kOffW3;
         h.b3 = WB() + kOffB3;
-        h.y = static_cast<float*>(y.p);
+        h.y = y;
         mlp_head(h, rows, stream);
-        EST_CK(cudaMemcpyAsync(out, y.p, sizeof(float) * rows, cudaMemcpyDeviceToHost, stream));
+        EST_CK(cudaMemcpyAsync(out, y, sizeof(float) * rows, cudaMemcpyDeviceToHost, stream));
         EST_CK(cudaStreamSynchronize(stream));
     }
 
     void predict(const float* f, uint64_t n, float* out) {
         using namespace bj;
-        reserve(kPredictChunk);
+        reserve(std::min<uint64_t>(n, kPredictChunk));
         for (uint64_t i0 = 0; i0 < n; i0 += kPredictChunk) {
             const int rows = int(std::min<uint64_t>(kPredictChunk, n - i0));
-            upload_rows(f + i0 * kF, rows, static_cast<uint16_t*>(X.p));
+            upload_rows(f + i0 * kF, rows, X);
             run_head(rows, out + i0);
         }
     }
@@ -1092,7 +1130,7 @@ BJ_API int bj_estimator_train(bj_estimator* e, const float* features, const floa
         for (uint32_t ep = 0; ep < epochs; ep++) {
             std::shuffle(order.begin(), order.end(), rng);
             EST_CK(cudaMemcpyAsync(perm, order.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, e->stream));
-            EST_CK(cudaMemsetAsync(e->loss.p, 0, sizeof(float), e->stream));
+            EST_CK(cudaMemsetAsync(e->loss, 0, sizeof(float), e->stream));
             for (uint64_t b0 = 0; b0 < n; b0 += batch) {
                 const int rows = int(std::min<uint64_t>(batch, n - b0));
                 const int pad = (rows + 63) & ~63;
@@ -1102,7 +1140,7 @@ BJ_API int bj_estimator_train(bj_estimator* e, const float* features, const floa
                 e->adam(float(lr * (0.1 + 0.9 * 0.5 * (1.0 + std::cos(M_PI * frac)))));
             }
             float l = 0;
-            EST_CK(cudaMemcpyAsync(&l, e->loss.p, sizeof(float), cudaMemcpyDeviceToHost, e->stream));
+            EST_CK(cudaMemcpyAsync(&l, e->loss, sizeof(float), cudaMemcpyDeviceToHost, e->stream));
             EST_CK(cudaStreamSynchronize(e->stream));
             if (epoch_loss) epoch_loss[ep] = l / float(n);
         }
@@ -1140,14 +1178,14 @@ BJ_API int bj_estimator_gradients(bj_estimator* e, const float* features, const 
     try {
         const int pad = int((n + 63) & ~63ull);
         e->reserve(pad);
-        e->upload_rows(features, n, static_cast<uint16_t*>(e->X.p));
+        e->upload_rows(features, n, e->X);
         std::vector<float> t(pad, 0.f);
         std::copy(targets, targets + n, t.begin());
-        EST_CK(cudaMemcpyAsync(e->t.p, t.data(), sizeof(float) * pad, cudaMemcpyHostToDevice, e->stream));
-        EST_CK(cudaMemsetAsync(e->loss.p, 0, sizeof(float), e->stream));
-        e->forward_backward({static_cast<uint16_t*>(e->X.p), nullptr, int(n)}, static_cast<float*>(e->t.p), pad);
+        EST_CK(cudaMemcpyAsync(e->t, t.data(), sizeof(float) * pad, cudaMemcpyHostToDevice, e->stream));
+        EST_CK(cudaMemsetAsync(e->loss, 0, sizeof(float), e->stream));
+        e->forward_backward({e->X, nullptr, int(n)}, e->t, pad);
         EST_CK(cudaMemcpyAsync(grads, e->G(), sizeof(float) * kParams, cudaMemcpyDeviceToHost, e->stream));
-        EST_CK(cudaMemcpyAsync(loss, e->loss.p, sizeof(float), cudaMemcpyDeviceToHost, e->stream));
+        EST_CK(cudaMemcpyAsync(loss, e->loss, sizeof(float), cudaMemcpyDeviceToHost, e->stream));
         EST_CK(cudaStreamSynchronize(e->stream));
         *loss /= float(n);
     } catch (const Fail&) {
