@@ -548,8 +548,9 @@ class Executor {
                 st_ = ctx_->side[next_side++ % bj_context::kSideStreams];
                 BJ_CK(cudaStreamWaitEvent(st_, start, 0));
             } else {
-                st_ = main;
-                for (const auto& pr : pp.probes) BJ_CK(cudaStreamWaitEvent(main, ctx_->pipe_event(pr.child), 0));
+                // A build that needs no read-back runs beside the others.
+                st_ = quiet_build(p) ? ctx_->side[next_side++ % bj_context::kSideStreams] : main;
+                for (const auto& pr : pp.probes) BJ_CK(cudaStreamWaitEvent(st_, ctx_->pipe_event(pr.child), 0));
             }
             bool ok = p + 1 < np ? run_pipeline(p, nullptr, 0) : run_pipeline(p, &res, flags);
             trace(leaf ? "leaf pipeline enqueued" : "pipeline done");
@@ -723,6 +724,16 @@ class Executor {
     bool small_scan(const PipelinePlan::Probe& pr) const {
         const DevColumn& key = col(pr.probe_attr);
         return pr.key_probe < 0 && !(key.flags & kColHostPages) && key.npages <= kDirectFilterPages;
+    }
+
+    // A build fed by one short scan of a batched leaf's table with unique keys,
+    // sized by its bound: nothing of it is read back.
+    bool quiet_build(size_t p) const {
+        const PipelinePlan& pp = ex_.pipelines[p];
+        if (p + 1 == ex_.pipelines.size() || pp.probes.size() != 1) return false;
+        const BuiltHT& child = hts_[pp.probes[0].child];
+        return child.flags_known && child.unique && small_scan(pp.probes[0]) &&
+               ex_.inputs[pp.input].rows <= kBoundedBuild && !(ctx_->scan_split && ctx_->tune.scan_split);
     }
 
     // Reads back the flags of the leaves that pipelines of one short scan probe
@@ -1242,8 +1253,13 @@ class Executor {
             ba.rlog2w = hts_[size_t(r)].view.bloom_log2;
             restricted_by_[pi] = r;
         }
+        // One launch while launches cost the host more than the barriers cost the
+        // device: not in a captured graph, and only small builds (a few more
+        // where builds run beside each other).
+        const bool whole = ctx_->tape_mode != 2 &&
+                           items.count <= (st_ == ctx_->stream ? kClusterTuples : 2 * kClusterTuples);
         uint8_t* z = alloc<uint8_t>(pb.zbytes);
-        BJ_CK(cudaMemsetAsync(z, 0, pb.zbytes, st_));
+        if (!whole) BJ_CK(cudaMemsetAsync(z, 0, pb.zbytes, st_));
         place_zero(pb, z);
         ba.table = pb.table;
         ba.tlog2 = pb.tlog2;
@@ -1253,6 +1269,11 @@ class Executor {
         ba.bloom = pb.bloom;
         ba.err = ctx_->d_err;
         ba.distinct = leaf ? 1u : 0u;
+        if (whole) {
+            launched(build_fed_cluster(FedBuild{ba, pb.nb, pb.dflags, ctx_->tape_mode != 2 ? 1 : 0}, st_));
+            publish(pi, pb);
+            return true;
+        }
         launched(emit_aggregate(ba, st_));
         launched(place_tuples(tb, pb.rank1, pb.counts, pb.dflags + 2, pb.nb, pb.ht, ctx_->d_err, st_));
         publish(pi, pb);

@@ -175,19 +175,24 @@ __global__ void __launch_bounds__(256) k_aggregate(BuildArgs a) {
     if (i < a.tb.count) aggregate_tuple(a, i);
 }
 
-// Places the representatives as entries of their buckets.
-__global__ void __launch_bounds__(256) k_place(TupleBuf t, const uint32_t* __restrict__ rank1, HTView ht,
-                                               uint32_t* __restrict__ err) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= t.count) return;
+// Places representative i as an entry of its bucket. (Its multiplicity grew by
+// atomics, perhaps earlier in this launch: read through L2.)
+__device__ __forceinline__ void place_tuple(const TupleBuf& t, const uint32_t* rank1, const HTView& ht, uint32_t* err,
+                                            uint32_t i) {
     const uint32_t r1 = rank1[i];
     uint32_t pos;
     if (!r1 || !place_key(ht, t.keys[i], r1 - 1, err, pos)) return;
-    const_cast<uint64_t*>(ht.mult)[pos] = t.mult[i];
+    const_cast<uint64_t*>(ht.mult)[pos] = __ldcg(t.mult + i);
     if (ht.pnull) const_cast<uint32_t*>(ht.pnull)[pos] = t.pnull[i];
     uint64_t* dst = const_cast<uint64_t*>(ht.ent) + size_t(pos) * (1 + ht.width) + 1;
     const uint64_t* src = t.pay + size_t(i) * t.width;
     for (uint32_t j = 0; j < t.width; j++) dst[j] = src[j];
+}
+
+__global__ void __launch_bounds__(256) k_place(TupleBuf t, const uint32_t* __restrict__ rank1, HTView ht,
+                                               uint32_t* __restrict__ err) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < t.count) place_tuple(t, rank1, ht, err, i);
 }
 
 __device__ __forceinline__ int leaf_of(const uint32_t* start, int n, uint32_t x) {
@@ -245,7 +250,7 @@ __device__ __forceinline__ void flag_bucket(const HTView& ht, uint32_t b, uint32
     const uint4 k = __ldcg(ht.buckets + b);
     if (ht.mult)
         for (uint32_t j = 0; j < k.y; j++)
-            if (ht.mult[k.x + j] > 1) flags[1] = 1;
+            if (__ldcg(ht.mult + k.x + j) > 1) flags[1] = 1;
     if (k.y < 2) return;
     if (k.y > 256) {
         flags[0] = 1;  // long bucket: assume repeats (only steers capacity choices)
@@ -265,6 +270,62 @@ __device__ __forceinline__ void flag_bucket(const HTView& ht, uint32_t b, uint32
 __global__ void __launch_bounds__(256) k_ht_flags(HTView ht, uint32_t nbuckets, uint32_t* __restrict__ flags) {
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nbuckets; b += gridDim.x * blockDim.x)
         flag_bucket(ht, b, flags);
+}
+
+// The same by a cluster: thread t of `all`, a warp a run of 32 buckets (or all
+// 16), each run's entries reserved with one atomic.
+__device__ __forceinline__ void cluster_ranges(const uint32_t* counts, const HTView& ht, uint32_t nb, uint32_t* entries,
+                                               uint32_t t, uint32_t all) {
+    uint4* buckets = const_cast<uint4*>(ht.buckets);
+    const uint32_t lane = t & 31;
+    for (uint32_t w = t >> 5; w * 32 < nb; w += all / 32) {
+        const uint32_t b = w * 32 + lane;
+        const uint32_t n = b < nb ? __ldcg(counts + b) : 0u;
+        uint32_t inc = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= uint32_t(o)) inc += u;
+        }
+        uint32_t first = 0;
+        if (lane == 31 && inc) first = atomicAdd(entries, inc);
+        first = __shfl_sync(0xffffffffu, first, 31);
+        if (b < nb) buckets[b] = make_uint4(first + inc - n, n, 0, 0);
+    }
+}
+__device__ __forceinline__ void cluster_zero(uint32_t* p, uint32_t words, uint32_t t, uint32_t all) {  // 16-byte multiples
+    for (uint32_t i = t; i < words / 4; i += all) reinterpret_cast<uint4*>(p)[i] = make_uint4(0, 0, 0, 0);
+}
+
+// A small build fed by probes, whole: the passes above (zeroing, emit,
+// aggregation, ranges, places, flags) in one launch, with a cluster barrier
+// where they have a launch. Five launches and a memset cost the host about 20
+// us a build when a query is not replayed. Bound: the passes' latencies, each
+// row's chain of atomics among them, over the cluster's 8,192 threads.
+constexpr int kFedCtas = 8, kFedThreads = 1024;
+__global__ void __cluster_dims__(kFedCtas, 1, 1) __launch_bounds__(kFedThreads) k_fed_cluster(FedBuild f) {
+    const cg::cluster_group cluster = cg::this_cluster();
+    const BuildArgs& a = f.a;
+    constexpr uint32_t all = kFedCtas * kFedThreads;
+    const uint32_t t = blockIdx.x * kFedThreads + threadIdx.x;
+    const uint32_t n = a.in.dcount ? min(a.tb.count, *a.in.dcount) : a.tb.count;
+    if (!a.distinct) cluster_zero(a.table, 1u << a.tlog2, t, all);
+    cluster_zero(a.counts, f.nb, t, all);
+    if (a.bloom) cluster_zero(a.bloom, 1u << a.ht.bloom_log2, t, all);
+    if (t < 3) f.dflags[t] = 0;
+    if (a.distinct) cluster.sync();  // the emit counts
+    for (uint32_t i = t; i < n; i += all) emit_tuple(a, i);
+    cluster.sync();
+    if (!a.distinct) {
+        for (uint32_t i = t; i < n; i += all) aggregate_tuple(a, i);
+        cluster.sync();
+    }
+    cluster_ranges(a.counts, a.ht, f.nb, f.dflags + 2, t, all);
+    cluster.sync();
+    for (uint32_t i = t; i < n; i += all) place_tuple(a.tb, a.rank1, a.ht, a.err, i);
+    if (!f.flags) return;
+    cluster.sync();
+    for (uint32_t b = t; b < f.nb; b += all) flag_bucket(a.ht, b, f.dflags);
 }
 
 // ---- leaf builds of a query, batched ----
@@ -342,10 +403,8 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     const LeafBuild& L = B.l[blockIdx.x / kClusterCtas];
     const uint32_t all = kClusterCtas * kClusterThreads;
     const uint32_t t = (blockIdx.x % kClusterCtas) * kClusterThreads + threadIdx.x;
-    uint4* counts4 = reinterpret_cast<uint4*>(L.counts);
-    for (uint32_t i = t; i < L.nb / 4; i += all) counts4[i] = make_uint4(0, 0, 0, 0);
-    if (L.bloom)
-        for (uint32_t i = t; i < 1u << L.ht.bloom_log2; i += all) L.bloom[i] = 0;
+    cluster_zero(L.counts, L.nb, t, all);
+    if (L.bloom) cluster_zero(L.bloom, 1u << L.ht.bloom_log2, t, all);
     if (t < 3) L.dflags[t] = 0;
     cluster.sync();
     for (uint32_t i = t; i < L.rows; i += all) {
@@ -353,21 +412,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
         L.rank1[i] = leaf_key(L, i, kv) ? count_key(L.counts, L.ht, L.bloom, kv) : 0u;
     }
     cluster.sync();
-    uint4* buckets = const_cast<uint4*>(L.ht.buckets);
-    for (uint32_t w = t >> 5; w * 32 < L.nb; w += all / 32) {  // a warp a run of 32 buckets (or all 16)
-        const uint32_t b = w * 32 + (t & 31);
-        const uint32_t n = b < L.nb ? __ldcg(L.counts + b) : 0u;
-        uint32_t inc = n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
-            if ((t & 31) >= uint32_t(o)) inc += u;
-        }
-        uint32_t first = 0;
-        if ((t & 31) == 31 && inc) first = atomicAdd(L.dflags + 2, inc);
-        first = __shfl_sync(0xffffffffu, first, 31);
-        if (b < L.nb) buckets[b] = make_uint4(first + inc - n, n, 0, 0);
-    }
+    cluster_ranges(L.counts, L.ht, L.nb, L.dflags + 2, t, all);
     cluster.sync();
     for (uint32_t i = t; i < L.rows; i += all) {
         const uint32_t r1 = L.rank1[i];  // this thread's own
@@ -403,6 +448,12 @@ int emit_aggregate(const BuildArgs& a, cudaStream_t st) {
     if (a.distinct) return 1;
     k_aggregate<<<blocks, 256, 0, st>>>(a);
     return 2;
+}
+
+int build_fed_cluster(const FedBuild& f, cudaStream_t st) {
+    if (!f.a.tb.count) return 0;
+    k_fed_cluster<<<kFedCtas, kFedThreads, 0, st>>>(f);
+    return 1;
 }
 
 int place_tuples(const TupleBuf& t, const uint32_t* rank1, const uint32_t* counts, uint32_t* entries, uint32_t nb,

@@ -52,17 +52,6 @@ __device__ __forceinline__ uint64_t load_value(const uint8_t* pg, uint32_t d) {
     return __ldg(reinterpret_cast<const uint32_t*>(pg + 4) + d);
 }
 
-// Bitmap bits of rows 32 w .. 32 w + 31 of a page whose nbytes bitmap bytes
-// end the page (bits beyond the page's rows are garbage).
-__device__ __forceinline__ uint32_t bitmap_word(const uint8_t* pg, uint32_t nbytes, uint32_t w) {
-    const uint32_t byte = kPageSize - nbytes + 4 * w;
-    const uint32_t lo = byte & ~3u;
-    if (lo >= kPageSize) return 0;
-    const uint32_t a = *reinterpret_cast<const uint32_t*>(pg + lo);
-    const uint32_t b = lo + 4 < kPageSize ? *reinterpret_cast<const uint32_t*>(pg + lo + 4) : 0u;
-    return __funnelshift_r(a, b, 8 * (byte & 3));
-}
-
 // The entry each of a lane's kGroups keys matches (unique keys: at most one).
 // `valid` flags the keys present; the result flags the matches in e.
 template <bool kWide>
@@ -163,7 +152,7 @@ __device__ __forceinline__ uint32_t load_groups(const DirectArgs& a, const uint8
     // The value index of a row comes from the page index and the bitmap.
     uint32_t word = 0;
     if (lane < kGroups && r0 + 32 * lane < end) {
-        word = bitmap_word(pg, (s.n + 7) >> 3, r0 / 32 + lane);
+        word = page_bitmap_word(pg, (s.n + 7) >> 3, r0 / 32 + lane);
         const uint32_t left = end - (r0 + 32 * lane);
         if (left < 32) word &= (1u << left) - 1;
     }
