@@ -16,18 +16,21 @@
 //    two funnel shifts and a logic op (bloom_bits_fast), spread over the
 //    multiply and integer pipes; the lane's survivors form a 32-bit mask, so
 //    a unit costs one vote and at most one warp prefix sum;
-//  * a page with NULLs is read in blocks of 1024 rows, 32 per lane: the null
-//    bitmap word of a lane's rows gives their validity, and the page index's
-//    dense base of their 64-row chunk plus a popcount the value index of
-//    each (units split a page's rows the same way);
+//  * a page with NULLs stores its values densely, so with a filter it is read
+//    the same way, and the survivors find their rows through the page index
+//    and the null bitmap. Without one (every row probes) it is read in blocks
+//    of 1024 rows, 32 per lane: the null bitmap word of a lane's rows gives
+//    their validity, and the page index's dense base of their 64-row chunk
+//    plus a popcount the value index of each (units split the rows so);
 //  * the hash table's bloom filter (up to 128 KiB) is staged once per CTA in
 //    shared memory; one CTA of 32 warps runs per SM;
-//  * bloom survivors are recorded as (key, row) in a per-warp buffer in
-//    shared memory (the key read again from the page just loaded, a cache
-//    hit); the buffer is probed 128 entries at a time, four independent
-//    bucket lookups per lane, so the latency of the probes is paid once per
-//    batch instead of once per hit. Without a bloom filter (a probe that is
-//    not selective) every lane probes its own rows directly, four at a time;
+//  * bloom survivors are recorded by their place (page and value in it) in a
+//    per-warp buffer in shared memory, a candidate of every lane a turn; the
+//    buffer is probed 128 entries at a time, four keys (read again from pages
+//    just loaded, a cache hit) and four independent bucket lookups per lane,
+//    so the latency of the probes is paid once per batch instead of once per
+//    hit. Without a bloom filter (a probe that is not selective) every lane
+//    probes its own rows directly, four at a time;
 //  * matches become items (row, entry, mult). With unique build keys a row
 //    has at most one match: items are appended with one atomicAdd per batch
 //    and the buffer carries over from unit to unit (mode 2). Otherwise a
@@ -122,8 +125,8 @@ __device__ __forceinline__ uint32_t warp_excl(uint32_t v, uint32_t& total) {
 }
 
 struct WarpState {
-    uint32_t* bkey;     // candidate buffer: key
-    uint32_t* brow;     // row of the scanned table
+    uint32_t* bpage;    // candidate buffer: page
+    uint32_t* bval;     // value index in the page
     uint32_t n;         // entries buffered (warp-uniform)
     uint32_t page_cnt;  // matches counted / written for the current unit (modes 0 and 1)
 };
@@ -194,7 +197,39 @@ __device__ __forceinline__ void probe_batch(const ScanArgs& a, WarpState& w, con
     w.page_cnt += total;
 }
 
-// Probes every buffered candidate.
+// First row of page p (of a window of a column, when rows follow from rpp).
+__device__ __forceinline__ uint32_t first_row(const ScanArgs& a, uint32_t p) {
+    return a.key.rpp ? a.row_base + p * a.key.rpp : __ldg(a.key.row_start + p);
+}
+
+// Row in page p of its value d, when the page has NULLs: the 64-row chunk that
+// holds the value by the page index, then the bit of the chunk's bitmap.
+__device__ __forceinline__ uint32_t row_of_value(const DevColumn& c, const uint8_t* pg, uint32_t p, uint32_t n, uint32_t d) {
+    const uint32_t c0 = __ldg(c.chunk_base + p);
+    uint32_t lo = 0, hi = (n + 63) / 64 - 1;  // the last chunk with at most d values before it
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) / 2;
+        if (__ldg(c.dense_base + c0 + mid) <= d)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    uint32_t k = d - __ldg(c.dense_base + c0 + lo);  // set bits of the chunk before the value's
+    const uint32_t nbytes = (n + 7) >> 3;
+    uint32_t w = page_bitmap_word(pg, nbytes, 2 * lo), r = 64 * lo;
+    if (k >= __popc(w)) {
+        k -= __popc(w);
+        w = page_bitmap_word(pg, nbytes, 2 * lo + 1);
+        r += 32;
+    }
+    for (; k; k--) w &= w - 1;
+    return r + (w ? __ffs(w) - 1 : 0);
+}
+
+// Probes every buffered candidate: the keys are read again from their pages,
+// just loaded by this warp, four at a time a lane. (kNulls: the column has
+// pages with NULLs.)
+template <bool kNulls>
 __device__ __forceinline__ void flush(const ScanArgs& a, WarpState& w, uint32_t unit) {
     if (w.n == 0) return;
     __syncwarp();
@@ -205,8 +240,15 @@ __device__ __forceinline__ void flush(const ScanArgs& a, WarpState& w, uint32_t 
         const uint32_t h = lane + 32 * i;
         key[i] = row[i] = 0;
         if (h < w.n) {
-            key[i] = w.bkey[h];
-            row[i] = w.brow[h];
+            const uint32_t p = w.bpage[h], d = w.bval[h];
+            const uint32_t* pg = reinterpret_cast<const uint32_t*>(a.key.pages + size_t(p) * kPageSize);
+            key[i] = __ldg(pg + 1 + d);
+            uint32_t r = d;
+            if (kNulls) {
+                const uint32_t hdr = __ldg(pg), n = hdr & 0xffff;
+                if (hdr >> 16 != n) r = row_of_value(a.key, reinterpret_cast<const uint8_t*>(pg), p, n, d);
+            }
+            row[i] = first_row(a, p) + r;
             has |= 1u << i;
         }
     }
@@ -238,37 +280,24 @@ __device__ __forceinline__ void probe_bits(const ScanArgs& a, WarpState& w, uint
     }
 }
 
-// Buffers the candidates flagged in `take` (up to 32 per lane): map(c, key,
-// row) gives candidate c's key and row. Candidates are numbered across the
-// warp in lane order; when they do not fit, the buffer is filled, probed and
-// refilled until all are in.
-template <typename Map>
-__device__ __forceinline__ void push_bits(const ScanArgs& a, WarpState& w, uint32_t take, uint32_t p, Map&& map) {
-    if (!__any_sync(0xffffffffu, take != 0)) return;
-    uint32_t total;
-    const uint32_t cnt = __popc(take);
-    const uint32_t off = warp_excl(cnt, total);
-    for (uint32_t done = 0;;) {
-        const uint32_t room = kBatch - w.n;
-        // This lane's candidates are numbered [off, off + cnt); only those in
-        // the window [done, done + room) go into the buffer this round.
-        if (off + cnt > done && off < done + room) {
-            uint32_t t = take, j = off;
-            for (; j < done; j++) t &= t - 1;  // skip the ones already buffered
-            for (; t && j < done + room; j++) {
-                const uint32_t c = __ffs(t) - 1;
-                t &= t - 1;
-                uint32_t key, row;
-                map(c, key, row);
-                w.bkey[w.n + j - done] = key;
-                w.brow[w.n + j - done] = row;
-            }
+// Buffers the candidates flagged in `take` (up to 32 per lane) of page p:
+// at(c) gives candidate c's value index in the page. A turn
+// of the loop takes one candidate of every lane that has one left, at most 32,
+// so the buffer is probed and emptied whenever a turn would not fit.
+template <bool kNulls, typename At>
+__device__ __forceinline__ void push_bits(const ScanArgs& a, WarpState& w, uint32_t take, uint32_t unit, uint32_t p,
+                                          At&& at) {
+    const uint32_t below = (1u << lane_id()) - 1;
+    for (uint32_t m; (m = __ballot_sync(0xffffffffu, take != 0)) != 0;) {
+        const uint32_t k = __popc(m);
+        if (w.n + k > kBatch) flush<kNulls>(a, w, unit);
+        if (take) {
+            const uint32_t o = w.n + __popc(m & below);
+            w.bpage[o] = p;
+            w.bval[o] = at(__ffs(take) - 1);
+            take &= take - 1;
         }
-        const uint32_t took = min(room, total - done);
-        w.n += took;
-        done += took;
-        if (done >= total) break;
-        flush(a, w, p);
+        w.n += k;
     }
 }
 
@@ -295,23 +324,22 @@ __device__ __forceinline__ void append_bits(const ScanArgs& a, uint32_t take, Ma
     }
 }
 
-// Candidates of one step of a page without NULLs: bit c of `take` is value
-// vi0 + 128 (c / 4) + c % 4 of the page of unit p (values at vals, first row
-// row0); the key is read again from the page, which this warp has just loaded.
-template <bool kFilter>
+// Candidates of one step of page p, without NULLs: bit c of `take` is value
+// vi0 + 128 (c / 4) + c % 4 of the page (values at vals, first row row0).
+template <bool kFilter, bool kNulls>
 __device__ __forceinline__ void push_step(const ScanArgs& a, WarpState& w, uint32_t take, int vi0,
-                                          const uint32_t* vals, uint32_t row0, uint32_t p, bool dense) {
+                                          const uint32_t* vals, uint32_t row0, uint32_t unit, uint32_t p, bool dense) {
+    auto index = [&](uint32_t c) { return uint32_t(vi0 + 128 * int(c >> 2) + int(c & 3)); };
     auto cand = [&](uint32_t c, uint32_t& key, uint32_t& row) {
-        const uint32_t vi = uint32_t(vi0 + 128 * int(c >> 2) + int(c & 3));
-        key = __ldg(vals + vi);
-        row = row0 + vi;
+        key = __ldg(vals + index(c));
+        row = row0 + index(c);
     };
     if (kFilter)
         append_bits(a, take, cand);
     else if (dense)
-        probe_bits(a, w, take, p, cand);
+        probe_bits(a, w, take, unit, cand);
     else
-        push_bits(a, w, take, p, cand);
+        push_bits<kNulls>(a, w, take, unit, p, index);
 }
 
 __device__ __forceinline__ bool bloom_pass(const ScanArgs& a, const uint32_t* bloom, uint32_t key) {
@@ -391,7 +419,7 @@ __device__ __forceinline__ void scan_rows_nulls(const ScanArgs& a, WarpState& w,
         // comes from a malformed page (reported by the page index) and is not read.
         if (d0 + __popc(wb) > 2047) wb = 0;
         uint32_t take = wb;
-        if (use_bloom && wb) {
+        if (kFilter && use_bloom && wb) {
             take = 0;
             uint32_t t = wb, d = d0;
             while (t) {
@@ -407,8 +435,6 @@ __device__ __forceinline__ void scan_rows_nulls(const ScanArgs& a, WarpState& w,
         };
         if (kFilter)
             append_bits(a, take, cand);
-        else if (use_bloom)
-            push_bits(a, w, take, unit, cand);
         else
             probe_bits(a, w, take, unit, cand);
     }
@@ -416,11 +442,14 @@ __device__ __forceinline__ void scan_rows_nulls(const ScanArgs& a, WarpState& w,
 
 // kFilter: the filter kernel of the split form (no probes; survivors go to
 // the candidate list). Otherwise the fused scan-side probe.
-template <bool kFilter>
+// kNulls: a column with NULLs (page index at hand), taken by its values when
+// there is a filter; its survivors' row search is kept out of the other form
+// (registers: 54 against 56 us for 24M rows without NULLs).
+template <bool kFilter, bool kNulls>
 __global__ void __launch_bounds__(kCtaThreads, 1) k_scan_probe(ScanArgs a) {
     extern __shared__ uint4 bloom4[];
-    __shared__ uint32_t bkey[kFilter ? 1 : kWarpsPerCta][kFilter ? 1 : kBatch];
-    __shared__ uint32_t brow[kFilter ? 1 : kWarpsPerCta][kFilter ? 1 : kBatch];
+    __shared__ uint32_t bpage[kFilter ? 1 : kWarpsPerCta][kFilter ? 1 : kBatch];
+    __shared__ uint32_t bval[kFilter ? 1 : kWarpsPerCta][kFilter ? 1 : kBatch];
     const uint32_t* bloom = reinterpret_cast<const uint32_t*>(bloom4);
     const bool use_bloom = a.use_bloom != 0;
     const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
@@ -440,9 +469,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) k_scan_probe(ScanArgs a) {
 #pragma unroll
         for (int i = 0; i < kStepWords; i++) q[i] = ld_stream(pw + (u % kUnitsPerPage) * kWordsPerStep + lane + 32 * i, pol);
         hdr = lane == 0 ? __ldg(reinterpret_cast<const uint32_t*>(pw)) : 0;
-        row0 = lane == 0 ? (a.key.rpp ? a.row_base + (u / kUnitsPerPage) * a.key.rpp
-                                      : __ldg(a.key.row_start + u / kUnitsPerPage))
-                         : 0;
+        row0 = lane == 0 ? first_row(a, u / kUnitsPerPage) : 0;
     };
     uint4 q[kStepWords];
     uint32_t hdr_l = 0, row0_l = 0;
@@ -461,7 +488,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) k_scan_probe(ScanArgs a) {
     }
     __syncthreads();
 
-    WarpState w{bkey[kFilter ? 0 : warp], brow[kFilter ? 0 : warp], 0, 0};
+    WarpState w{bpage[kFilter ? 0 : warp], bval[kFilter ? 0 : warp], 0, 0};
     for (uint32_t u = first; u < nunits; u += total_warps) {
         const uint32_t p = u / kUnitsPerPage, part = u % kUnitsPerPage;
         load_unit(u, q, hdr_l, row0_l);
@@ -484,11 +511,13 @@ __global__ void __launch_bounds__(kCtaThreads, 1) k_scan_probe(ScanArgs a) {
         const uint32_t n = hdr & 0xffff, nn = hdr >> 16;
         const uint32_t* vals = reinterpret_cast<const uint32_t*>(a.key.pages + size_t(p) * kPageSize) + 1;
         w.page_cnt = 0;
-        if (nn == n) {
+        // With a filter, NULLs do not matter: the page's values are tested as
+        // they lie, and the few that pass find their rows (flush).
+        if (nn == n || (kNulls && use_bloom)) {
             const int vi0 = 4 * int(lane) - 1 + int(part * 4 * kWordsPerStep);
-            if (vi0 - int(lane) * 4 < int(n))  // some value of the unit is below n
-                push_step<kFilter>(a, w, step_take(a, q, bloom, use_bloom) & step_valid(vi0, n), vi0, vals, row0,
-                                   u, !use_bloom);
+            if (vi0 - int(lane) * 4 < int(nn))  // some value of the unit is below nn
+                push_step<kFilter, kNulls>(a, w, step_take(a, q, bloom, use_bloom) & step_valid(vi0, nn), vi0, vals, row0,
+                                   u, p, !use_bloom);
         } else {
             // A page with NULLs: unit k takes rows [1024 k, 1024 (k + 1)), the
             // last unit every row from there on.
@@ -497,11 +526,11 @@ __global__ void __launch_bounds__(kCtaThreads, 1) k_scan_probe(ScanArgs a) {
             if (r_begin < r_end) scan_rows_nulls<kFilter>(a, w, bloom, use_bloom, u, p, n, row0, r_begin, r_end);
         }
         if (!kFilter && a.mode != 2) {
-            flush(a, w, u);
+            flush<kNulls>(a, w, u);
             if (a.mode == 0 && lane == 0) a.page_counts[u] = w.page_cnt;
         }
     }
-    if (!kFilter && a.mode == 2) flush(a, w, 0);
+    if (!kFilter && a.mode == 2) flush<kNulls>(a, w, 0);
 }
 
 // The probe kernel of the split form: every candidate of the list, 128 per
@@ -529,22 +558,22 @@ __global__ void __launch_bounds__(256) k_probe_candidates(ScanArgs a) {
     }
 }
 
-template <bool kFilter>
+template <bool kFilter, bool kNulls>
 void launch_scan(const ScanArgs& a, size_t bloom_bytes, int num_sms, cudaStream_t st) {
     // Once per process and form (thread-safe static initialisation; server
     // workers launch from several threads).
     static const bool configured = [] {
-        cudaFuncSetAttribute(k_scan_probe<kFilter>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBloomSmemMax));
+        cudaFuncSetAttribute(k_scan_probe<kFilter, kNulls>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBloomSmemMax));
         return true;
     }();
     (void)configured;
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scan_probe<kFilter>, kCtaThreads, bloom_bytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scan_probe<kFilter, kNulls>, kCtaThreads, bloom_bytes);
     per_sm = std::max(1, per_sm);
     const uint64_t ctas =
         std::min<uint64_t>((uint64_t(kUnitsPerPage) * a.key.npages + kWarpsPerCta - 1) / kWarpsPerCta,
                            uint64_t(num_sms) * per_sm);
-    k_scan_probe<kFilter><<<unsigned(ctas), kCtaThreads, bloom_bytes, st>>>(a);
+    k_scan_probe<kFilter, kNulls><<<unsigned(ctas), kCtaThreads, bloom_bytes, st>>>(a);
 }
 
 } // namespace
@@ -570,7 +599,10 @@ int scan_probe(const DevColumn& key, const HTView& ht, int mode, bool bloom_smem
                ht.bloom_log2 ? (1u << ht.bloom_log2) : 0u, 1u << 27,
                page_counts, page_off, cursor, out_rows, out_ents, out_mult, capacity, err, row_base,
                nullptr, nullptr, nullptr, 0};
-    launch_scan<false>(a, bloom_bytes, num_sms, st);
+    if ((key.flags & kColNulls) && key.chunk_base && key.dense_base)
+        launch_scan<false, true>(a, bloom_bytes, num_sms, st);
+    else
+        launch_scan<false, false>(a, bloom_bytes, num_sms, st);
     return 1;
 }
 
@@ -585,7 +617,7 @@ int scan_probe_split(const DevColumn& key, const HTView& ht, uint32_t* cursor, u
                ht.bloom_log2 ? (1u << ht.bloom_log2) : 0u, 1u << 27,
                nullptr, nullptr, cursor, out_rows, out_ents, out_mult, capacity, err, row_base,
                cand_key, cand_row, cand_count, cand_cap};
-    launch_scan<true>(a, bloom_bytes, num_sms, st);
+    launch_scan<true, false>(a, bloom_bytes, num_sms, st);
     k_probe_candidates<<<unsigned(num_sms) * 8, 256, 0, st>>>(a);  // 64 warps per SM (32 registers)
     return 2;
 }

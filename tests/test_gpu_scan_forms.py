@@ -204,3 +204,12 @@ def test_fed_builds(pkg, ctx, oracle, rows, keep, copies):
     j = p.new_join_node(False, f, d, 1, 0, [(0, pkg.INT32), (3, pkg.INT32)])
     p.root = p.new_join_node(False, j, s, 1, 0, [(0, pkg.INT32), (3, pkg.INT32)])
     check(pkg, ctx, oracle, pkg.CPlan(p), f"rows {rows} keep {keep} copies {copies}")
+
+
+# The staged filter over pages with NULLs: survivors find their rows from their values' places (pages of few and of
+# many NULLs, all-NULL chunks, a page's last value), over more than 512 pages.
+@pytest.mark.parametrize("nulls", [0.02, 0.5, 0.97])
+@pytest.mark.parametrize("keep", [0.02, 0.3])
+def test_filter_over_nulls(pkg, ctx, oracle, nulls, keep):
+    fact = int(1_100_000 / (1 - nulls)) if nulls < 0.9 else 8_000_000
+    check(pkg, ctx, oracle, star(pkg, 3, fact, [20_000], keep, nulls, False), f"nulls {nulls} keep {keep}")
