@@ -255,11 +255,16 @@ uint64_t upload_pages(bj_context* ctx, const std::vector<ColumnJob>& jobs) {
             staging_fence();  // this thread's streaming stores are in memory before the DMA is issued
         });
         // Consecutive pages of one column (one device allocation) become one
-        // copy; a copy never spans two allocations.
+        // copy, and columns side by side in a chunk of the arena (a chunk is one
+        // allocation) too; a copy never spans two allocations.
         size_t i = c0;
         while (i < c1) {
             size_t k = i + 1;
-            while (k < c1 && all[k].job == all[i].job && all[k].dst == all[k - 1].dst + kPageSize) k++;
+            while (k < c1 && all[k].dst == all[k - 1].dst + kPageSize &&
+                   (all[k].job == all[k - 1].job ||
+                    (jobs[all[k].job].in_arena && jobs[all[k - 1].job].in_arena &&
+                     ctx->arena.same_chunk(all[k].dst, all[k - 1].dst))))
+                k++;
             BJ_CK(cudaMemcpyAsync(all[i].dst, stage + i * kPageSize, (k - i) * kPageSize, cudaMemcpyHostToDevice,
                                   ctx->stream));
             i = k;
@@ -1756,7 +1761,7 @@ int execute_common(bj_context* ctx, const bj_plan* plan, bj_resident* const* res
                         continue;
                     }
                     uint8_t* dp = static_cast<uint8_t*>(ctx->arena.alloc(std::max<uint64_t>(hc.num_pages, 1) * kPageSize));
-                    jobs.push_back(ColumnJob{&hc, dp, t.num_rows, &d.cols[c], false, pinned});
+                    jobs.push_back(ColumnJob{&hc, dp, t.num_rows, &d.cols[c], false, pinned, true});
                 }
             }
             trace("plan and input columns");

@@ -153,6 +153,12 @@ class Arena : public Scratch {
         cur_ = chunks_.size() - 1;
         return p;
     }
+    // Whether two addresses of the arena lie in one allocation.
+    bool same_chunk(const uint8_t* a, const uint8_t* b) const {
+        for (const auto& c : chunks_)
+            if (a >= c.p && a < c.p + c.size) return b >= c.p && b < c.p + c.size;
+        return false;
+    }
     void reset() {
         for (auto& c : chunks_) c.used = 0;
         cur_ = 0;
@@ -285,6 +291,7 @@ struct ColumnJob {
     DevColumn* out;
     bool in_place = false; // pages are read where they are (pinned host memory): no copy
     const uint8_t* pinned = nullptr;  // pages back to back in pinned host memory: one DMA from here
+    bool in_arena = false; // dpages lies in the context's arena
 };
 
 // The host address of a column's pages when they lie back to back in pinned

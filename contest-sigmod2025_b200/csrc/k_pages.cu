@@ -4,10 +4,9 @@
 // (TableScan::prepareColumn / makeSearchVector, engine/op/TableScan.cpp:546-582:
 // an exclusive prefix of rows per page used by the readers' exponential page
 // search) and the popcount-to-dense-index step of its readers
-// (TableScan.cpp:113-238, 287-292). Pass 1 reads every page header (one
-// thread per page), validates it against the page format and writes the
-// page's contained rows and 64-row chunk count; two scans turn those into
-// row_start / chunk_base. Pass 2 writes the dense-value base of every chunk
+// (TableScan.cpp:113-238, 287-292). Pass 1 reads every page header, validates
+// it against the page format and writes the page's contained rows and 64-row
+// chunk count; two scans turn those into row_start / chunk_base. Pass 2 writes the dense-value base of every chunk
 // and the page of every 1024-row block.
 #include "launch.h"
 
@@ -16,80 +15,93 @@
 namespace bj {
 namespace {
 
-__global__ void k_page_headers(PageIndexBatch batch, uint32_t* __restrict__ err) {
+// A warp takes `per` pages: their headers together, then what a page holds
+// beside the header (null bitmap, string offsets), the lanes side by side. (A
+// thread a page walked them byte by byte: 4,041 pages with NULLs took 32 us on
+// a B200, 9 pages of strings 25; now 7 and 7.5.) One page a warp until the
+// pages fill the chip, four beyond.
+__global__ void __launch_bounds__(256) k_page_headers(PageIndexBatch batch, uint32_t per, uint32_t* __restrict__ err) {
     const PageIndexCol& col = batch.c[blockIdx.y];
     const uint8_t* __restrict__ pages = col.pages;
     const uint32_t npages = col.npages;
     const int32_t type = col.type;
-    uint32_t* __restrict__ hdr = col.hdr;
-    uint32_t* __restrict__ rows = col.rows;
-    uint32_t* __restrict__ chunks = col.chunks;
-    uint32_t* __restrict__ flags = col.flags;
-    if (blockIdx.x * blockDim.x >= npages) return;  // whole CTA beyond this column
+    const uint32_t lane = threadIdx.x & 31, p0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * per;
+    if (blockIdx.x * 8 * per >= npages) return;  // whole CTA beyond this column
     // Page 0's header, read once per CTA (pages may be in host memory).
     __shared__ uint32_t s_h0;
     if (threadIdx.x == 0) s_h0 = *reinterpret_cast<const uint32_t*>(pages);
     __syncthreads();
-    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= npages) return;
-    const uint8_t* pg = pages + size_t(p) * kPageSize;
-    const uint32_t h = *reinterpret_cast<const uint32_t*>(pg);
-    hdr[p] = h;
-    uint32_t n = h & 0xffff, nn = h >> 16;
-    uint32_t r = n, c = (n + 63) >> 6;
-    uint32_t f = 0;
-    if (type == kVarchar && n >= 0xfffe) {
-        // Long-string page: 1 row for the first page of the run, 0 for the rest.
-        r = n == 0xffff ? 1 : 0;
-        c = 0;
-        f |= 2;
-        if (nn > kPageSize - 4) record_error(err, kErrLongString);
-        if (n == 0xfffe && (p == 0 || ld16(pages + size_t(p - 1) * kPageSize) < 0xfffe)) record_error(err, kErrLongString);
-    } else {
-        // Every later read of this page (values by dense index, string offsets)
-        // stays inside it once these hold: bitmap and header fit, the bitmap's
-        // population equals the non-null count, values / offsets / bytes fit.
-        uint32_t nbytes = (n + 7) >> 3;
-        bool ok = nn <= n && 4 + nbytes <= kPageSize;
-        if (ok && nn != n) {
-            f |= 1;
-            const uint8_t* bm = pg + kPageSize - nbytes;
-            uint32_t pop = 0;
-            for (uint32_t b = 0; b < nbytes; b++) {
-                uint32_t byte = bm[b];
-                if (b == nbytes - 1 && (n & 7)) byte &= (1u << (n & 7)) - 1;
-                pop += __popc(byte);
+    if (p0 >= npages) return;  // whole warp
+    const uint32_t mine = p0 + lane;
+    const bool own = lane < per && mine < npages;
+    const uint32_t h_own = own ? *reinterpret_cast<const uint32_t*>(pages + size_t(mine) * kPageSize) : 0u;
+    uint32_t r = 0, c = 0, f = 0;  // of this lane's page
+    for (uint32_t j = 0; j < per && p0 + j < npages; j++) {
+        const uint32_t p = p0 + j, h = __shfl_sync(0xffffffffu, h_own, j), n = h & 0xffff, nn = h >> 16;
+        const uint8_t* pg = pages + size_t(p) * kPageSize;
+        uint32_t rj = n, cj = (n + 63) >> 6, fj = 0;
+        if (type == kVarchar && n >= 0xfffe) {
+            // Long-string page: 1 row for the first page of the run, 0 for the rest.
+            rj = n == 0xffff ? 1 : 0;
+            cj = 0;
+            fj |= 2;
+            if (lane == 0) {
+                if (nn > kPageSize - 4) record_error(err, kErrLongString);
+                if (n == 0xfffe && (p == 0 || ld16(pages + size_t(p - 1) * kPageSize) < 0xfffe))
+                    record_error(err, kErrLongString);
             }
-            ok = pop == nn;
-        }
-        if (ok && type == kVarchar) {
-            ok = 4 + 2 * nn + nbytes <= kPageSize;
-            uint32_t prev = 0;
-            for (uint32_t k = 0; ok && k < nn; k++) {
-                uint32_t e = ld16(pg + 4 + 2 * k);
-                ok = e >= prev;
-                prev = e;
+        } else {
+            // Every later read of this page (values by dense index, string offsets)
+            // stays inside it once these hold: bitmap and header fit, the bitmap's
+            // population equals the non-null count, values / offsets / bytes fit.
+            const uint32_t nbytes = (n + 7) >> 3;
+            bool ok = nn <= n && 4 + nbytes <= kPageSize;
+            if (ok && nn != n) {
+                fj |= 1;
+                uint32_t pop = 0;
+                for (uint32_t w = lane; 32 * w < n; w += 32) {
+                    uint32_t bits = page_bitmap_word(pg, nbytes, w);
+                    if (n - 32 * w < 32) bits &= (1u << (n - 32 * w)) - 1;
+                    pop += __popc(bits);
+                }
+                ok = __reduce_add_sync(0xffffffffu, pop) == nn;
             }
-            ok = ok && 4 + 2 * nn + prev + nbytes <= kPageSize;
-        } else if (ok) {
-            uint32_t w = type == kInt32 ? 4 : 8;
-            uint32_t begin = type == kInt32 ? 4 : 8;
-            ok = begin + nn * w + nbytes <= kPageSize;
+            if (ok && type == kVarchar) {
+                ok = 4 + 2 * nn + nbytes <= kPageSize;
+                if (ok) {
+                    bool rising = true;
+                    for (uint32_t k = lane + 1; k < nn; k += 32) rising = rising && ld16(pg + 4 + 2 * k) >= ld16(pg + 2 + 2 * k);
+                    const uint32_t last = nn ? ld16(pg + 2 + 2 * nn) : 0u;
+                    ok = __all_sync(0xffffffffu, rising) && 4 + 2 * nn + last + nbytes <= kPageSize;
+                }
+            } else if (ok) {
+                const uint32_t w = type == kInt32 ? 4 : 8;
+                ok = w + nn * w + nbytes <= kPageSize;  // values begin at byte 4 (INT32) or 8
+            }
+            if (!ok) {
+                if (lane == 0) record_error(err, kErrPageHeader);
+                rj = 0;
+                cj = 0;
+            }
         }
-        if (!ok) {
-            record_error(err, kErrPageHeader);
-            r = 0;
-            c = 0;
+        // Uniform pages: every page but the last holds as many rows as page 0,
+        // the last at most that many.
+        const uint32_t h0 = s_h0;
+        const uint32_t r0 = (type == kVarchar && (h0 & 0xffff) >= 0xfffe) ? 0u : (h0 & 0xffff);
+        if (r0 == 0 || (rj != r0 && (p + 1 < npages || rj > r0)) || (fj & 2)) fj |= kColRaggedPages;
+        if (lane == j) {
+            r = rj;
+            c = cj;
+            f = fj;
         }
     }
-    // Uniform pages: every page but the last holds as many rows as page 0,
-    // the last at most that many.
-    const uint32_t h0 = s_h0;
-    const uint32_t r0 = (type == kVarchar && (h0 & 0xffff) >= 0xfffe) ? 0u : (h0 & 0xffff);
-    if (r0 == 0 || (r != r0 && (p + 1 < npages || r > r0)) || (f & 2)) f |= kColRaggedPages;
-    rows[p] = r;
-    chunks[p] = c;
-    if (f) atomicOr(flags, f);
+    if (own) {
+        col.hdr[mine] = h_own;
+        col.rows[mine] = r;
+        col.chunks[mine] = c;
+    }
+    f = __reduce_or_sync(0xffffffffu, f);
+    if (lane == 0 && f) atomicOr(col.flags, f);
 }
 
 // One warp per page: dense base of each 64-row chunk (a running popcount of
@@ -177,7 +189,8 @@ int page_index_pass1(const PageIndexBatch& b, uint32_t* err, Scratch& s, cudaStr
     }
     int launches = 0;
     if (max_np) {
-        k_page_headers<<<dim3((max_np + 255) / 256, unsigned(b.n)), 256, 0, st>>>(b, err);
+        const uint32_t per = max_np > 148 * 8 * 4 ? 4 : 1;
+        k_page_headers<<<dim3((max_np + 8 * per - 1) / (8 * per), unsigned(b.n)), 256, 0, st>>>(b, per, err);
         launches++;
     }
     return launches + scan_exclusive_u32_segs(segs, s, st);
