@@ -648,7 +648,7 @@ struct bj_estimator {
         g.bias = WB() + kOffB1;
         g.Cb = H1;
         g.ldc = kH;
-        gemm_bf16(g, stream);
+        gemm_forward(g, stream);
         g.A = H1;
         g.a_rs = kH;
         g.a_idx = nullptr;
@@ -657,7 +657,7 @@ struct bj_estimator {
         g.K = kH;
         g.bias = WB() + kOffB2;
         g.Cb = H2;
-        gemm_bf16(g, stream);
+        gemm_forward(g, stream);
     }
 
     // Forward, loss and gradients over a batch of in.n_real rows (padded to
@@ -691,7 +691,7 @@ struct bj_estimator {
         g.epi = kEpiStoreF32;
         g.Cf = G() + kOffW2;
         g.ldc = kH;
-        gemm_bf16(g, stream);
+        const GemmArgs dw2 = g;
         // dH1 = (dH2 W2^T) * [H1 > 0]
         g = GemmArgs{};
         g.A = dH2;
@@ -708,7 +708,7 @@ struct bj_estimator {
         g.mask = H1;
         g.Cb = dH1;
         g.ldc = kH;
-        gemm_bf16(g, stream);
+        gemm_backward(dw2, g, stream);
         // dW1 = X^T dH1
         g = GemmArgs{};
         g.A = in.X;
@@ -725,7 +725,6 @@ struct bj_estimator {
         g.epi = kEpiStoreF32;
         g.Cf = G() + kOffW1;
         g.ldc = kH;
-        gemm_bf16(g, stream);
         RowSumArgs r{};
         r.dH1 = dH1;
         r.dH2 = dH2;
@@ -736,7 +735,7 @@ struct bj_estimator {
         r.b2 = G() + kOffB2;
         r.w3 = G() + kOffW3;
         r.b3 = G() + kOffB3;
-        row_sums(r, stream);
+        gemm_row_sums(g, r, stream);
     }
 
     void adam(float lr) {

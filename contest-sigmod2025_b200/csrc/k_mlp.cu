@@ -18,16 +18,25 @@
 // chain of accumulations in ascending k, whatever the tile.
 //
 // The products are small (256 to 4096 rows, 256 columns, K up to 1792), so
-// what bounds them is the length of that chain: 112 dependent steps at
-// K = 1792. tcgen05's 128-row tiles would leave them on a handful of SMs, and
-// its accumulation order is not this one. Measured on a B200 (one slice of 32
-// at a time, loaded and waited for, in 64 x 64 tiles, against this): 256 x 256
-// x 1792 about 110 -> 12 us; the two products of 4096 rows 147 -> 43 us; a
-// whole training step of 256 rows 215 -> 67 us.
+// what bounds them is the length of that chain, 28 slices at K = 1792: a
+// barrier, the copies' and ldmatrix's issue and the slice's MMAs, with one warp
+// a scheduler to overlap them; a deeper ring (8 or 10 stages) measures the
+// same. tcgen05's 128-row tiles would leave them on a handful of SMs, and its
+// accumulation order is not this one. Measured on a B200 (one slice of 32 at a
+// time, loaded and waited for, in 64 x 64 tiles, against this): 256 x 256 x
+// 1792 about 110 -> 9 us; the two products of 4096 rows 147 -> 43 us.
+//
+// A training step of 256 rows: nine launches 215 us with the former products;
+// eight launches 50 us with these; 37 us now, with six launches (products that
+// do not read each other share one, row sums run beside a product), each put
+// on the chip while the one before it ends (after.cuh).
+#include "after.cuh"
 #include "launch.h"
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 namespace bj {
 namespace {
@@ -121,16 +130,61 @@ constexpr size_t gemm_smem() {
     return sizeof(uint16_t) * kStages * size_t(Slice<T, kAt>::kWords + Slice<T, kBt>::kWords);
 }
 
-// kAt: A stored with m contiguous; kBt: B stored with n contiguous.
+// A warp's operands of one slice, in registers.
+template <int T>
+struct Fragments {
+    static constexpr int kMI = T / 32, kNJ = T / 16;  // its 16-row and 8-column MMA tiles
+    uint32_t a[kBK / 16][kMI][4], b[kBK / 16][kNJ][2];
+    template <bool kAt, bool kBt>
+    __device__ __forceinline__ void load(const uint16_t* sA, const uint16_t* sB, int wm, int wn, int lane) {
+        constexpr int kLdA = Slice<T, kAt>::kLd, kLdB = Slice<T, kBt>::kLd;
+#pragma unroll
+        for (int s = 0; s < kBK / 16; s++) {
+            const int kk = s * 16;
+#pragma unroll
+            for (int i = 0; i < kMI; i++) {
+                const int m = wm + i * 16;
+                if (kAt)
+                    ldmatrix_x4_trans(a[s][i][0], a[s][i][1], a[s][i][2], a[s][i][3],
+                                      sA + (kk + (lane >> 4) * 8 + (lane & 7)) * kLdA + m + ((lane >> 3) & 1) * 8);
+                else
+                    ldmatrix_x4(a[s][i][0], a[s][i][1], a[s][i][2], a[s][i][3],
+                                sA + (m + (lane & 15)) * kLdA + kk + (lane >> 4) * 8);
+            }
+#pragma unroll
+            for (int j = 0; j < kNJ; j += 2) {
+                const int n = wn + j * 8;
+                if (kBt)
+                    ldmatrix_x4_trans(b[s][j][0], b[s][j][1], b[s][j + 1][0], b[s][j + 1][1],
+                                      sB + (kk + ((lane >> 3) & 1) * 8 + (lane & 7)) * kLdB + n + (lane >> 4) * 8);
+                else
+                    ldmatrix_x4(b[s][j][0], b[s][j][1], b[s][j + 1][0], b[s][j + 1][1],
+                                sB + (n + (lane & 7) + (lane >> 4) * 8) * kLdB + kk + ((lane >> 3) & 1) * 8);
+            }
+        }
+    }
+    __device__ __forceinline__ void multiply(float (&acc)[kMI][kNJ][4]) const {
+#pragma unroll
+        for (int s = 0; s < kBK / 16; s++)
+#pragma unroll
+            for (int i = 0; i < kMI; i++)
+#pragma unroll
+                for (int j = 0; j < kNJ; j++) mma_bf16(acc[i][j], a[s][i], b[s][j][0], b[s][j][1]);
+    }
+};
+
+// Tile (m0, n0) of g, by a block of 128 threads. kAt: A stored with m
+// contiguous; kBt: B stored with n contiguous. While a slice is multiplied the
+// next one's operands are on their way to registers, so what a slice takes is
+// its chain of MMAs.
 template <int T, bool kAt, bool kBt>
-__global__ void __launch_bounds__(128) k_gemm_bf16(GemmArgs g) {
-    extern __shared__ __align__(16) uint16_t gemm_ring[];
+__device__ __forceinline__ void gemm_tile(const GemmArgs& g, int m0, int n0, uint16_t* ring) {
     using SA = Slice<T, kAt>;
     using SB = Slice<T, kBt>;
-    constexpr int kMI = T / 32, kNJ = T / 16;  // a warp's 16-row and 8-column MMA tiles
-    uint16_t* ringA = gemm_ring;
-    uint16_t* ringB = gemm_ring + kStages * SA::kWords;
-    const int m0 = blockIdx.y * T, n0 = blockIdx.x * T;
+    using F = Fragments<T>;
+    constexpr int kMI = F::kMI, kNJ = F::kNJ;
+    uint16_t* ringA = ring;
+    uint16_t* ringB = ring + kStages * SA::kWords;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wm = (warp >> 1) * (T / 2), wn = (warp & 1) * (T / 2);
     const int slices = g.K / kBK;
@@ -145,41 +199,26 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(GemmArgs g) {
     };
     for (int t = 0; t < kStages - 1; t++) fetch(t);
     float acc[kMI][kNJ][4] = {};
-    for (int t = 0; t < slices; t++) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
-        __syncthreads();  // slice t is there, and slice t - 1's stage is free
+    F now, next;
+    auto take = [&](F& f, int t) {
+        f.template load<kAt, kBt>(ringA + (t % kStages) * SA::kWords, ringB + (t % kStages) * SB::kWords, wm, wn, lane);
+    };
+    auto slice = [&](const F& cur, F& other, int t) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 3) : "memory");
+        __syncthreads();  // slice t + 1 is there, and slice t - 1's stage is free
         fetch(t + kStages - 1);
-        const uint16_t* sA = ringA + (t % kStages) * SA::kWords;
-        const uint16_t* sB = ringB + (t % kStages) * SB::kWords;
-#pragma unroll
-        for (int kk = 0; kk < kBK; kk += 16) {
-            uint32_t a[kMI][4], b[kNJ][2];
-#pragma unroll
-            for (int i = 0; i < kMI; i++) {
-                const int m = wm + i * 16;
-                if (kAt)
-                    ldmatrix_x4_trans(a[i][0], a[i][1], a[i][2], a[i][3],
-                                      sA + (kk + (lane >> 4) * 8 + (lane & 7)) * SA::kLd + m + ((lane >> 3) & 1) * 8);
-                else
-                    ldmatrix_x4(a[i][0], a[i][1], a[i][2], a[i][3],
-                                sA + (m + (lane & 15)) * SA::kLd + kk + (lane >> 4) * 8);
-            }
-#pragma unroll
-            for (int j = 0; j < kNJ; j += 2) {
-                const int n = wn + j * 8;
-                if (kBt)
-                    ldmatrix_x4_trans(b[j][0], b[j][1], b[j + 1][0], b[j + 1][1],
-                                      sB + (kk + ((lane >> 3) & 1) * 8 + (lane & 7)) * SB::kLd + n + (lane >> 4) * 8);
-                else
-                    ldmatrix_x4(b[j][0], b[j][1], b[j + 1][0], b[j + 1][1],
-                                sB + (n + (lane & 7) + (lane >> 4) * 8) * SB::kLd + kk + ((lane >> 3) & 1) * 8);
-            }
-#pragma unroll
-            for (int i = 0; i < kMI; i++)
-#pragma unroll
-                for (int j = 0; j < kNJ; j++) mma_bf16(acc[i][j], a[i], b[j][0], b[j][1]);
-        }
+        if (t + 1 < slices) take(other, t + 1);
+        cur.multiply(acc);
+    };
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    __syncthreads();
+    if (slices) take(now, 0);
+    int t = 0;
+    for (; t + 2 <= slices; t += 2) {
+        slice(now, next, t);
+        slice(next, now, t + 1);
     }
+    if (t < slices) slice(now, next, t);
     asm volatile("cp.async.wait_all;" ::: "memory");
     // Epilogue: acc[i][j] covers rows wm + 16 i + lane / 4 (+ 8) and columns
     // wn + 8 j + 2 (lane % 4) (+ 1).
@@ -210,10 +249,35 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(GemmArgs g) {
             }
 }
 
+template <int T, bool kAt, bool kBt>
+__global__ void __launch_bounds__(128) k_gemm_bf16(GemmArgs g) {
+    extern __shared__ __align__(16) uint16_t gemm_ring[];
+    begin_after_previous();
+    gemm_tile<T, kAt, kBt>(g, blockIdx.y * T, blockIdx.x * T, gemm_ring);
+}
+
+// Two products of one step that do not read each other, in one launch: g's
+// 32 x 32 tiles (A and B stored transposed: a weight gradient), then h's T x T
+// ones (a row gradient). Alone, either is 64 blocks at 256 rows.
+template <int T>
+__global__ void __launch_bounds__(128) k_gemm_pair(GemmArgs g, GemmArgs h, int g_tiles) {
+    extern __shared__ __align__(16) uint16_t gemm_ring[];
+    begin_after_previous();
+    const int b = blockIdx.x;
+    if (b < g_tiles) {
+        const int wide = (g.N + 31) / 32;
+        gemm_tile<32, true, true>(g, b / wide * 32, b % wide * 32, gemm_ring);
+    } else {
+        const int wide = (h.N + T - 1) / T;
+        gemm_tile<T, false, false>(h, (b - g_tiles) / wide * T, (b - g_tiles) % wide * T, gemm_ring);
+    }
+}
+
 // Output layer and its gradient, one CTA of 256 threads per batch row:
 // y = H2 . w3 + b3; with targets, loss += (y - t)^2, dy = 2 (y - t) / n_real,
 // dH2 = bf16(dy * w3 * [H2 > 0]); rows at or beyond n_real get dy = 0.
 __global__ void __launch_bounds__(256) k_mlp_head(MlpHeadArgs a) {
+    begin_after_previous();
     const int m = blockIdx.x, n = threadIdx.x;
     const float h = bf2f(a.H2[long(m) * kMlpHidden + n]);
     const float w = bf2f(a.w3[n]);
@@ -240,43 +304,59 @@ __global__ void __launch_bounds__(256) k_mlp_head(MlpHeadArgs a) {
     if (a.dH2) a.dH2[long(m) * kMlpHidden + n] = f2bf(h > 0.f ? dy_s * w : 0.f);
 }
 
-// The gradients that are sums over the batch's rows, one launch: b2 (columns
-// of dH2), w3 (columns of H2 times dy) and b1 (columns of dH1), 32 columns a
-// block, and b3 (dy). Rows are summed in chunks (32 rows or more, at most 64
-// chunks) and the chunks' sums in order, so the result does not depend on
-// scheduling.
-__global__ void __launch_bounds__(256) k_row_sums(RowSumArgs a) {
-    constexpr int kBlocks = kMlpHidden / 32;
-    __shared__ float part[64][32];
-    const int which = blockIdx.x / kBlocks, t = threadIdx.x;
+// The gradients that are sums over the batch's rows: b2 (columns of dH2), w3
+// (columns of H2 times dy) and b1 (columns of dH1), 32 columns a block of 128
+// threads, and b3 (dy), a block. Rows are summed in chunks (32 rows or more, at
+// most 64 chunks) and the chunks' sums in order, so the result does not depend
+// on scheduling. part: 64 x 32.
+constexpr int kSumColumns = 32, kRowSumBlocks = 3 * (kMlpHidden / kSumColumns) + 1;
+__device__ __forceinline__ void row_sum_block(const RowSumArgs& a, int block, float (*part)[kSumColumns]) {
+    constexpr int kBlocks = kMlpHidden / kSumColumns;
+    const int which = block / kBlocks, t = threadIdx.x;
     if (which == 3) {
-        float s = 0.f;
-        for (int i = t; i < a.rows; i += 256) s += a.dy[i];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if ((t & 31) == 0) part[0][t >> 5] = s;
+        float s[2] = {};
+        for (int j = 0; j < 2; j++) {
+            for (int i = t + 128 * j; i < a.rows; i += 256) s[j] += a.dy[i];
+            for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_down_sync(0xffffffffu, s[j], o);
+            if ((t & 31) == 0) part[(t >> 5) + 4 * j][0] = s[j];
+        }
         __syncthreads();
         if (t == 0) {
-            for (int w = 1; w < 8; w++) s += part[0][w];
-            *a.b3 = s;
+            float sum = s[0];
+            for (int w = 1; w < 8; w++) sum += part[w][0];
+            *a.b3 = sum;
         }
         return;
     }
     const uint16_t* X = which == 0 ? a.dH2 : which == 1 ? a.H2 : a.dH1;
     float* out = which == 0 ? a.b2 : which == 1 ? a.w3 : a.b1;
-    const int n = (blockIdx.x % kBlocks) * 32 + (t & 31);
+    const int n = (block % kBlocks) * kSumColumns + t % kSumColumns;
     const int chunks = max(1, min(64, a.rows / 32)), per = (a.rows + chunks - 1) / chunks;
-    for (int c = t >> 5; c < chunks; c += 8) {
+    for (int c = t / kSumColumns; c < chunks; c += 128 / kSumColumns) {
         float s = 0.f;
-#pragma unroll 16
+#pragma unroll 32
         for (int m = c * per; m < min(a.rows, c * per + per); m++)
             s += bf2f(X[long(m) * kMlpHidden + n]) * (which == 1 ? a.dy[m] : 1.f);
-        part[c][t & 31] = s;
+        part[c][t % kSumColumns] = s;
     }
     __syncthreads();
-    if (t >= 32) return;
+    if (t >= kSumColumns) return;
     float s = 0.f;
     for (int c = 0; c < chunks; c++) s += part[c][t];
     out[n] = s;
+}
+
+// The first layer's weight gradient (g: 32 x 32 tiles, A and B stored
+// transposed) and the row sums, which its other blocks hide.
+__global__ void __launch_bounds__(128) k_gemm_row_sums(GemmArgs g, RowSumArgs r) {
+    extern __shared__ __align__(16) uint16_t gemm_ring[];
+    begin_after_previous();
+    if (blockIdx.x < kRowSumBlocks) {
+        row_sum_block(r, blockIdx.x, reinterpret_cast<float(*)[kSumColumns]>(gemm_ring));
+        return;
+    }
+    const int b = blockIdx.x - kRowSumBlocks, wide = (g.N + 31) / 32;
+    gemm_tile<32, true, true>(g, b / wide * 32, b % wide * 32, gemm_ring);
 }
 
 // Adam (Kingma & Ba 2015) over every parameter, four a thread; the BF16 copy
@@ -292,6 +372,7 @@ __device__ __forceinline__ void adam_one(const AdamArgs& a, float g, float& am, 
     wb = f2bf(p);
 }
 __global__ void __launch_bounds__(128) k_adam(AdamArgs a) {
+    begin_after_previous();
     const long i = 4 * (blockIdx.x * 128l + threadIdx.x);
     if (i >= a.n) return;  // n is a multiple of 4
     const float4 g = *reinterpret_cast<const float4*>(a.grad + i);
@@ -309,6 +390,7 @@ __global__ void __launch_bounds__(128) k_adam(AdamArgs a) {
 }
 
 __global__ void k_f32_to_bf16(const float* in, uint16_t* out, long n) {
+    begin_after_previous();
     for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < n; i += long(gridDim.x) * blockDim.x)
         out[i] = f2bf(in[i]);
 }
@@ -316,55 +398,72 @@ __global__ void k_f32_to_bf16(const float* in, uint16_t* out, long n) {
 } // namespace
 
 namespace {
-template <int T, bool kAt, bool kBt>
-void launch_gemm(const GemmArgs& g, cudaStream_t st) {
-    static const bool configured = [] {  // once per process
-        cudaFuncSetAttribute(k_gemm_bf16<T, kAt, kBt>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(gemm_smem<T, kAt, kBt>()));
+// Kernels with more than the default 48 KiB of dynamic shared memory say so
+// once per process.
+template <auto kKernel>
+void allow_smem(size_t bytes) {
+    static const bool configured = [bytes] {
+        cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
         return true;
     }();
     (void)configured;
-    k_gemm_bf16<T, kAt, kBt><<<dim3((g.N + T - 1) / T, (g.M + T - 1) / T), 128, gemm_smem<T, kAt, kBt>(), st>>>(g);
+}
+template <int T, bool kAt, bool kBt>
+void launch_gemm(const GemmArgs& g, cudaStream_t st) {
+    allow_smem<k_gemm_bf16<T, kAt, kBt>>(gemm_smem<T, kAt, kBt>());
+    launch_after(k_gemm_bf16<T, kAt, kBt>, dim3((g.N + T - 1) / T, (g.M + T - 1) / T), 128, gemm_smem<T, kAt, kBt>(),
+                 st, g);
 }
 template <int T>
-void launch_gemm(const GemmArgs& g, cudaStream_t st) {
-    const bool at = g.a_cs != 1, bt = g.b_rs != 1;
-    if (at)
-        bt ? launch_gemm<T, true, true>(g, st) : launch_gemm<T, true, false>(g, st);
-    else
-        bt ? launch_gemm<T, false, true>(g, st) : launch_gemm<T, false, false>(g, st);
+void launch_pair(const GemmArgs& g, const GemmArgs& h, cudaStream_t st) {
+    constexpr size_t smem = std::max(gemm_smem<32, true, true>(), gemm_smem<T, false, false>());
+    allow_smem<k_gemm_pair<T>>(smem);
+    const int g_tiles = (g.M + 31) / 32 * ((g.N + 31) / 32), h_tiles = (h.M + T - 1) / T * ((h.N + T - 1) / T);
+    launch_after(k_gemm_pair<T>, g_tiles + h_tiles, 128, smem, st, g, h, g_tiles);
 }
+// 64 x 64 tiles where they fill the chip (half the operand traffic), else
+// 32 x 32 ones, four times the CTAs: the chain is as long in either.
+bool wide_tiles(const GemmArgs& g) { return long((g.M + 63) / 64) * ((g.N + 63) / 64) >= 148; }
 } // namespace
 
-int gemm_bf16(const GemmArgs& g, cudaStream_t st) {
+int gemm_forward(const GemmArgs& g, cudaStream_t st) {
     if (g.M <= 0 || g.N <= 0) return 0;
-    // 64 x 64 tiles where they fill the chip (half the operand traffic), else
-    // 32 x 32 ones, four times the CTAs: the chain is as long in either.
-    if (long((g.M + 63) / 64) * ((g.N + 63) / 64) >= 148)
-        launch_gemm<64>(g, st);
+    if (wide_tiles(g))
+        launch_gemm<64, false, true>(g, st);
     else
-        launch_gemm<32>(g, st);
+        launch_gemm<32, false, true>(g, st);
+    return 1;
+}
+
+int gemm_backward(const GemmArgs& dw, const GemmArgs& dh, cudaStream_t st) {
+    if (wide_tiles(dh))
+        launch_pair<64>(dw, dh, st);
+    else
+        launch_pair<32>(dw, dh, st);
+    return 1;
+}
+
+int gemm_row_sums(const GemmArgs& dw, const RowSumArgs& r, cudaStream_t st) {
+    constexpr size_t smem = gemm_smem<32, true, true>();
+    static_assert(smem >= 64 * kSumColumns * sizeof(float));
+    allow_smem<k_gemm_row_sums>(smem);
+    launch_after(k_gemm_row_sums, kRowSumBlocks + (dw.M + 31) / 32 * ((dw.N + 31) / 32), 128, smem, st, dw, r);
     return 1;
 }
 
 int mlp_head(const MlpHeadArgs& a, int rows, cudaStream_t st) {
     if (rows <= 0) return 0;
-    k_mlp_head<<<rows, kMlpHidden, 0, st>>>(a);
-    return 1;
-}
-
-int row_sums(const RowSumArgs& a, cudaStream_t st) {
-    k_row_sums<<<3 * (kMlpHidden / 32) + 1, 256, 0, st>>>(a);
+    launch_after(k_mlp_head, rows, kMlpHidden, 0, st, a);
     return 1;
 }
 
 int adam_step(const AdamArgs& a, cudaStream_t st) {
-    k_adam<<<unsigned((a.n / 4 + 127) / 128), 128, 0, st>>>(a);
+    launch_after(k_adam, unsigned((a.n / 4 + 127) / 128), 128, 0, st, a);
     return 1;
 }
 
 int f32_to_bf16(const float* in, uint16_t* out, long n, cudaStream_t st) {
-    k_f32_to_bf16<<<592, 256, 0, st>>>(in, out, n);
+    launch_after(k_f32_to_bf16, 592, 256, 0, st, in, out, n);
     return 1;
 }
 

@@ -486,7 +486,10 @@ struct GemmArgs {
     float* Cf;
     long ldc;
 };
-int gemm_bf16(const GemmArgs& g, cudaStream_t st);
+int gemm_forward(const GemmArgs& g, cudaStream_t st);  // A with k contiguous, B with n contiguous
+// A weight gradient (A with m contiguous, B with n contiguous) and the gradient
+// of a layer's rows (A and B with k contiguous) in one launch.
+int gemm_backward(const GemmArgs& dw, const GemmArgs& dh, cudaStream_t st);
 // Output layer (one CTA per row): y = H2 . w3 + b3; with targets t, loss +=
 // (y - t)^2 and, for rows below n_real, dy = 2 (y - t) / n_real and dH2 =
 // bf16(dy * w3 * [H2 > 0]) (zero for the other rows). Optional outputs may
@@ -504,7 +507,8 @@ struct MlpHeadArgs {
     int n_real;
 };
 int mlp_head(const MlpHeadArgs& a, int rows, cudaStream_t st);
-// Bias and output-layer gradients of a batch of `rows` rows (see k_row_sums).
+// Bias and output-layer gradients of a batch of `rows` rows, in one launch with
+// a weight gradient (A with m contiguous, B with n contiguous).
 struct RowSumArgs {
     const uint16_t* dH1;
     const uint16_t* dH2;
@@ -516,7 +520,7 @@ struct RowSumArgs {
     float* w3;
     float* b3;
 };
-int row_sums(const RowSumArgs& a, cudaStream_t st);
+int gemm_row_sums(const GemmArgs& dw, const RowSumArgs& r, cudaStream_t st);
 struct AdamArgs {
     float* w;
     uint16_t* wb;
