@@ -7,7 +7,7 @@
 // The matrix products run on the tensor cores through mma.sync m16n8k16
 // (BF16 in, FP32 accumulate): a CTA of four warps computes a 32 x 32 or 64 x
 // 64 tile of C = A B from 64-deep slices of A and B, which cp.async brings
-// into a ring of four shared-memory stages (rows padded by 16 bytes, so
+// into a ring of shared-memory stages (rows padded by 16 bytes, so
 // ldmatrix reads are free of bank conflicts). A and B may each be stored with
 // either dimension contiguous (the backward pass reads the forward operands
 // transposed); a slice keeps its operand's own order in shared memory and
@@ -18,16 +18,16 @@
 // chain of accumulations in ascending k, whatever the tile.
 //
 // The products are small (256 to 4096 rows, 256 columns, K up to 1792), so
-// what bounds them is the length of that chain, 28 slices at K = 1792: a
-// barrier, the copies' and ldmatrix's issue and the slice's MMAs, with one warp
-// a scheduler to overlap them; a deeper ring (8 or 10 stages) measures the
-// same. tcgen05's 128-row tiles would leave them on a handful of SMs, and its
-// accumulation order is not this one. Measured on a B200 (one slice of 32 at a
-// time, loaded and waited for, in 64 x 64 tiles, against this): 256 x 256 x
-// 1792 about 110 -> 9 us; the two products of 4096 rows 147 -> 43 us.
+// what bounds them is the length of that chain, 28 slices at K = 1792: with one
+// warp a scheduler, a barrier, the copies' and ldmatrix's issue and the slice's
+// MMAs (20 cycles each in a chain) follow one another. tcgen05's 128-row tiles
+// would leave them on a handful of SMs, and its accumulation order is not this
+// one. Measured on a B200 (one slice of 32 at a time, loaded and waited for, in
+// 64 x 64 tiles, against this): 256 x 256 x 1792 about 110 -> 8 us; the two
+// products of 4096 rows 147 -> 43 us.
 //
 // A training step of 256 rows: nine launches 215 us with the former products;
-// eight launches 50 us with these; 37 us now, with six launches (products that
+// eight launches 50 us with these; 35 us now, with six launches (products that
 // do not read each other share one, row sums run beside a product), each put
 // on the chip while the one before it ends (after.cuh).
 #include "after.cuh"
@@ -41,7 +41,15 @@
 namespace bj {
 namespace {
 
-constexpr int kBK = 64, kPad = 8, kStages = 4;
+constexpr int kBK = 64, kPad = 8;
+// Stages of the ring. The forward products' 32 x 32 tiles have 28 slices and an
+// SM each: 8 stages cover the way from L2 (a step of 256 rows 34.7 us; 4: 38.4;
+// 6 and 10: 38.6 and 38.2, their remainders cost what they gain). 64 x 64 tiles
+// share an SM, and the backward products have 4 slices.
+template <int T>
+constexpr int kForwardStages = T == 32 ? 8 : 4;
+constexpr int kBackwardStages = 4;
+constexpr int kMaxBatch = 8192;  // rows of a batch (see bj_estimator_train)
 
 __device__ __forceinline__ float bf2f(uint16_t v) { return __uint_as_float(uint32_t(v) << 16); }
 __device__ __forceinline__ uint16_t f2bf(float f) {
@@ -82,50 +90,60 @@ __device__ __forceinline__ void copy16(void* dst, const void* src, bool there) {
 // kBK. kRowsContiguous: stored with the rows contiguous in memory, kept as
 // [k][row]; else [row][k]. Element (row, k) is at p[row + k * stride] or p[row
 // * stride + k]; the dimension that is not contiguous goes through idx when
-// given, and from position `there` on it reads zeros (rows: from `rows` on).
+// given (in shared memory when that is k), and from position `there` on it
+// reads zeros (rows: from `rows` on). load() takes the slices in order.
 template <int R, bool kRowsContiguous>
 struct Slice {
     static constexpr int kLd = (kRowsContiguous ? R : kBK) + kPad;
     static constexpr int kWords = kLd * (kRowsContiguous ? kBK : R);
     static constexpr int kCopies = R * kBK / 8 / 128;  // 16-byte copies a thread and slice
-    const uint16_t* p;
+    const uint16_t* from[kCopies];  // this thread's part of the next slice (its rows' start, under idx in k)
+    int left[kCopies];              // positions before `there`, in the dimension that is not contiguous
     const uint32_t* idx;
     long stride;
-    int there;
-    bool in_rows;                    // [k][row]: this thread's rows exist
-    const uint16_t* from[kCopies];   // [row][k]: this thread's rows, at its k (null: zeros)
-    __device__ __forceinline__ Slice(const uint16_t* p_, long stride_, const uint32_t* idx_, int there_, int r0, int rows)
-        : p(p_), idx(idx_), stride(stride_), there(there_), in_rows(false) {
-        if (kRowsContiguous) {
-            const int r = r0 + (threadIdx.x % (R / 8)) * 8;
-            in_rows = r < rows;
-            p += in_rows ? r : 0;
-        } else {
+    int to;                         // this thread's first element of a slice
+    __device__ __forceinline__ Slice(const uint16_t* p, long stride_, const uint32_t* idx_, int there, int r0, int rows)
+        : idx(idx_), stride(stride_) {
+        constexpr int kLine = (kRowsContiguous ? R : kBK) / 8;  // copies a line
+        const int line = threadIdx.x / kLine, at = threadIdx.x % kLine * 8;
+        to = line * kLd + at;
 #pragma unroll
-            for (int i = 0; i < kCopies; i++) {
-                const int r = r0 + threadIdx.x / (kBK / 8) + i * (128 / (kBK / 8));
-                const bool ok = r < min(there, rows);
-                from[i] = ok ? p + (idx ? long(idx[r]) : long(r)) * stride + (threadIdx.x % (kBK / 8)) * 8 : nullptr;
+        for (int i = 0; i < kCopies; i++) {
+            const int l = line + i * (128 / kLine);
+            if (kRowsContiguous) {
+                left[i] = r0 + at < rows ? there - l : 0;
+                from[i] = p + (left[i] > 0 ? r0 + at + (idx ? 0 : l * stride) : 0);
+                idx = idx_ ? idx_ + line : nullptr;
+            } else {
+                const int r = r0 + l;
+                left[i] = r < min(there, rows) ? 1 : 0;
+                from[i] = p + (left[i] ? (idx ? long(idx[r]) : long(r)) * stride + at : 0);
             }
         }
     }
-    __device__ __forceinline__ void load(uint16_t* s, int k0) const {
+    __device__ __forceinline__ void load(uint16_t* s) {
+        constexpr int kStep = 128 / ((kRowsContiguous ? R : kBK) / 8);  // lines between a thread's copies
 #pragma unroll
         for (int i = 0; i < kCopies; i++) {
-            const int c = threadIdx.x + 128 * i;
+            const bool there = left[i] > 0;
+            const uint16_t* src = from[i];
             if (kRowsContiguous) {
-                const int k = c / (R / 8);
-                const bool ok = in_rows && k0 + k < there;
-                copy16(s + k * kLd + (c % (R / 8)) * 8, p + (ok ? (idx ? long(idx[k0 + k]) : long(k0 + k)) * stride : 0),
-                       ok);
-            } else {
-                copy16(s + (c / (kBK / 8)) * kLd + (c % (kBK / 8)) * 8, from[i] ? from[i] + k0 : p, from[i] != nullptr);
+                if (idx) {
+                    if (there) src += idx[i * kStep] * stride;
+                } else if (left[i] > kBK) {
+                    from[i] += kBK * stride;
+                }
+                left[i] -= kBK;
+            } else if (there) {
+                from[i] += kBK;
             }
+            copy16(s + to + i * kStep * kLd, src, there);
         }
+        if (kRowsContiguous && idx) idx += kBK;
     }
 };
 
-template <int T, bool kAt, bool kBt>
+template <int T, bool kAt, bool kBt, int kStages>
 constexpr size_t gemm_smem() {
     return sizeof(uint16_t) * kStages * size_t(Slice<T, kAt>::kWords + Slice<T, kBt>::kWords);
 }
@@ -177,8 +195,15 @@ struct Fragments {
 // contiguous; kBt: B stored with n contiguous. While a slice is multiplied the
 // next one's operands are on their way to registers, so what a slice takes is
 // its chain of MMAs.
-template <int T, bool kAt, bool kBt>
+template <int T, bool kAt, bool kBt, int kStages>
 __device__ __forceinline__ void gemm_tile(const GemmArgs& g, int m0, int n0, uint16_t* ring) {
+    const uint32_t* picked = g.a_idx;
+    if (kAt && picked) {  // a slice's rows would wait for their numbers
+        uint32_t* const numbers = reinterpret_cast<uint32_t*>(ring + gemm_smem<T, kAt, kBt, kStages>() / sizeof(uint16_t));
+        for (int k = threadIdx.x; k < g.a_there; k += 128) numbers[k] = picked[k];
+        __syncthreads();
+        picked = numbers;
+    }
     using SA = Slice<T, kAt>;
     using SB = Slice<T, kBt>;
     using F = Fragments<T>;
@@ -188,12 +213,12 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& g, int m0, int n0, uin
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wm = (warp >> 1) * (T / 2), wn = (warp & 1) * (T / 2);
     const int slices = g.K / kBK;
-    const SA from_a(g.A, kAt ? g.a_cs : g.a_rs, g.a_idx, g.a_there, m0, g.M);
-    const SB from_b(g.B, kBt ? g.b_rs : g.b_cs, nullptr, kBt ? g.K : g.N, n0, g.N);
+    SA from_a(g.A, kAt ? g.a_cs : g.a_rs, picked, g.a_there, m0, g.M);
+    SB from_b(g.B, kBt ? g.b_rs : g.b_cs, nullptr, kBt ? g.K : g.N, n0, g.N);
     auto fetch = [&](int t) {
         if (t < slices) {
-            from_a.load(ringA + (t % kStages) * SA::kWords, t * kBK);
-            from_b.load(ringB + (t % kStages) * SB::kWords, t * kBK);
+            from_a.load(ringA + (t % kStages) * SA::kWords);
+            from_b.load(ringB + (t % kStages) * SB::kWords);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -253,7 +278,7 @@ template <int T, bool kAt, bool kBt>
 __global__ void __launch_bounds__(128) k_gemm_bf16(GemmArgs g) {
     extern __shared__ __align__(16) uint16_t gemm_ring[];
     begin_after_previous();
-    gemm_tile<T, kAt, kBt>(g, blockIdx.y * T, blockIdx.x * T, gemm_ring);
+    gemm_tile<T, kAt, kBt, kForwardStages<T>>(g, blockIdx.y * T, blockIdx.x * T, gemm_ring);
 }
 
 // Two products of one step that do not read each other, in one launch: g's
@@ -266,10 +291,10 @@ __global__ void __launch_bounds__(128) k_gemm_pair(GemmArgs g, GemmArgs h, int g
     const int b = blockIdx.x;
     if (b < g_tiles) {
         const int wide = (g.N + 31) / 32;
-        gemm_tile<32, true, true>(g, b / wide * 32, b % wide * 32, gemm_ring);
+        gemm_tile<32, true, true, kBackwardStages>(g, b / wide * 32, b % wide * 32, gemm_ring);
     } else {
         const int wide = (h.N + T - 1) / T;
-        gemm_tile<T, false, false>(h, (b - g_tiles) / wide * T, (b - g_tiles) % wide * T, gemm_ring);
+        gemm_tile<T, false, false, kBackwardStages>(h, (b - g_tiles) / wide * T, (b - g_tiles) % wide * T, gemm_ring);
     }
 }
 
@@ -356,7 +381,7 @@ __global__ void __launch_bounds__(128) k_gemm_row_sums(GemmArgs g, RowSumArgs r)
         return;
     }
     const int b = blockIdx.x - kRowSumBlocks, wide = (g.N + 31) / 32;
-    gemm_tile<32, true, true>(g, b / wide * 32, b % wide * 32, gemm_ring);
+    gemm_tile<32, true, true, kBackwardStages>(g, b / wide * 32, b % wide * 32, gemm_ring);
 }
 
 // Adam (Kingma & Ba 2015) over every parameter, four a thread; the BF16 copy
@@ -410,13 +435,14 @@ void allow_smem(size_t bytes) {
 }
 template <int T, bool kAt, bool kBt>
 void launch_gemm(const GemmArgs& g, cudaStream_t st) {
-    allow_smem<k_gemm_bf16<T, kAt, kBt>>(gemm_smem<T, kAt, kBt>());
-    launch_after(k_gemm_bf16<T, kAt, kBt>, dim3((g.N + T - 1) / T, (g.M + T - 1) / T), 128, gemm_smem<T, kAt, kBt>(),
-                 st, g);
+    constexpr size_t smem = gemm_smem<T, kAt, kBt, kForwardStages<T>>();
+    allow_smem<k_gemm_bf16<T, kAt, kBt>>(smem);
+    launch_after(k_gemm_bf16<T, kAt, kBt>, dim3((g.N + T - 1) / T, (g.M + T - 1) / T), 128, smem, st, g);
 }
 template <int T>
 void launch_pair(const GemmArgs& g, const GemmArgs& h, cudaStream_t st) {
-    constexpr size_t smem = std::max(gemm_smem<32, true, true>(), gemm_smem<T, false, false>());
+    constexpr size_t smem =
+        std::max(gemm_smem<32, true, true, kBackwardStages>(), gemm_smem<T, false, false, kBackwardStages>());
     allow_smem<k_gemm_pair<T>>(smem);
     const int g_tiles = (g.M + 31) / 32 * ((g.N + 31) / 32), h_tiles = (h.M + T - 1) / T * ((h.N + T - 1) / T);
     launch_after(k_gemm_pair<T>, g_tiles + h_tiles, 128, smem, st, g, h, g_tiles);
@@ -444,9 +470,10 @@ int gemm_backward(const GemmArgs& dw, const GemmArgs& dh, cudaStream_t st) {
 }
 
 int gemm_row_sums(const GemmArgs& dw, const RowSumArgs& r, cudaStream_t st) {
-    constexpr size_t smem = gemm_smem<32, true, true>();
-    static_assert(smem >= 64 * kSumColumns * sizeof(float));
-    allow_smem<k_gemm_row_sums>(smem);
+    constexpr size_t ring = gemm_smem<32, true, true, kBackwardStages>();
+    static_assert(ring >= 64 * kSumColumns * sizeof(float));
+    const size_t smem = ring + (dw.a_idx ? sizeof(uint32_t) * size_t(dw.a_there) : 0);  // at most 8,192 rows a batch
+    allow_smem<k_gemm_row_sums>(ring + sizeof(uint32_t) * kMaxBatch);
     launch_after(k_gemm_row_sums, kRowSumBlocks + (dw.M + 31) / 32 * ((dw.N + 31) / 32), 128, smem, st, dw, r);
     return 1;
 }
