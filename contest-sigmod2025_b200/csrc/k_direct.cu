@@ -8,7 +8,8 @@
 // takes one by one), and a table of a few hundred pages, which there runs on
 // a handful of warps, each working through a long chain of dependent loads.
 //
-// Here a CTA of 256 threads takes a page. Lane l of a warp has row l of a
+// Here a CTA of 256 threads takes a page, or an eighth, quarter or half of one
+// where pages are few. Lane l of a warp has row l of a
 // group of 32 rows, so keys, items and the null bitmap are read and written
 // coalesced, and four groups at a time are probed with their bucket loads in
 // flight together. Matches leave in one append (one global atomic a page),
@@ -34,11 +35,13 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kGroups = 4;             // groups of 32 rows probed together by a warp
 constexpr uint32_t kPageValues = 2048; // more than the values of any page
+constexpr uint32_t kMaxParts = 8;      // blocks a page at most
 
 struct DirectArgs {
     DevColumn key;
     HTView ht;
     uint32_t use_bloom;  // test ht.bloom (in global memory) before the bucket
+    uint32_t parts;      // blocks a page
     ProbeChain chain;
     ItemsOut out;
     uint32_t* cursor;
@@ -129,6 +132,14 @@ __device__ __forceinline__ PageShape page_shape(const DevColumn& c, uint32_t p) 
     return s;
 }
 
+// This block's rows of its page: [first, end), first a multiple of 64; empty
+// beyond the page's rows.
+__device__ __forceinline__ void block_rows(const DirectArgs& a, const PageShape& s, uint32_t& first, uint32_t& end) {
+    const uint32_t span = (s.n + 64 * a.parts - 1) / (64 * a.parts) * 64;
+    first = blockIdx.x % a.parts * span;
+    end = min(first + span, s.n);
+}
+
 // The keys of kGroups groups of 32 rows of a page from row r0 (a multiple of
 // 64, below `end`), a row a lane, none at or beyond row `end`; the result
 // flags the lanes' rows that have one.
@@ -179,14 +190,17 @@ __global__ void __launch_bounds__(kThreads, 5) k_scan_direct(DirectArgs a) {
     __shared__ uint32_t count[kWarps], base;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t below = (1u << lane) - 1;
-    const uint32_t p = blockIdx.x;
+    const uint32_t p = blockIdx.x / a.parts;
     const uint8_t* pg = a.key.pages + size_t(p) * kPageSize;
     const PageShape s = page_shape(a.key, p);
+    uint32_t from, to;
+    block_rows(a, s, from, to);
+    if (from >= to) return;
     // Rows a warp, in chunks of 64: 256 on a full page without NULLs, more on
-    // one with; a page of more than 3,072 rows takes several turns.
-    const uint32_t share = min((s.n + 64 * kWarps - 1) / (64 * kWarps) * 64, uint32_t(kRounds * kGroups * 32));
-    for (uint32_t span = 0; span < s.n; span += share * kWarps) {
-        const uint32_t first = span + warp * share, end = min(first + share, s.n);
+    // one with; more than 3,072 rows take several turns.
+    const uint32_t share = min((to - from + 64 * kWarps - 1) / (64 * kWarps) * 64, uint32_t(kRounds * kGroups * 32));
+    for (uint32_t span = from; span < to; span += share * kWarps) {
+        const uint32_t first = span + warp * share, end = min(first + share, to);
         uint32_t e[kRounds][kGroups], hit[kRounds], total = 0;
 #pragma unroll
         for (int h = 0; h < kRounds; h++) {
@@ -242,15 +256,19 @@ __global__ void __launch_bounds__(kThreads, 6) k_scan_chain(DirectArgs a) {
     __shared__ uint32_t nfound, base, nkept[2];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t below = (1u << lane) - 1;
-    const uint32_t p = blockIdx.x;
+    const uint32_t p = blockIdx.x / a.parts;
     if (threadIdx.x == 0) nfound = 0;
     __syncthreads();
     const uint8_t* pg = a.key.pages + size_t(p) * kPageSize;
     const PageShape s = page_shape(a.key, p);
-    for (uint32_t r0 = warp * (32 * kGroups); r0 < s.n; r0 += kWarps * 32 * kGroups) {
+    uint32_t from, to;
+    block_rows(a, s, from, to);
+    if (from >= to) return;
+    const uint32_t share = to - from <= 64 * kWarps ? 64u : 32u * kGroups;  // rows a warp
+    for (uint32_t r0 = from + warp * share; r0 < to; r0 += kWarps * share) {
         uint64_t key[kGroups];
         uint32_t e[kGroups];
-        const uint32_t valid = load_groups<kWide>(a, pg, s, r0, s.n, key);
+        const uint32_t valid = load_groups<kWide>(a, pg, s, r0, min(r0 + share, to), key);
         const uint32_t hit = probe_groups<kWide>(a, key, valid, e);
         uint32_t m[kGroups], total = 0;
 #pragma unroll
@@ -335,7 +353,14 @@ int scan_probe_direct(const DevColumn& key, const HTView& ht, bool use_bloom, co
     a.capacity = capacity;
     a.err = err;
     if (chain) a.chain = *chain;
-    const uint32_t blocks = key.npages;
+    // Few pages: several blocks a page while all are resident together (six an
+    // SM), since a block's warps take their rows, and its matches their stages,
+    // one after another. The scan of 30K rows with one stage after it 26 -> 18
+    // us; at 445 pages and more a block has a page, as its atomic and header
+    // then cost more than the rows it shares.
+    a.parts = kMaxParts;
+    while (a.parts > 1 && uint64_t(key.npages) * a.parts > uint64_t(num_sms) * 6) a.parts /= 2;
+    const uint32_t blocks = key.npages * a.parts;
     const bool wide = key.type == kInt64;
     if (chain && chain->n > 0)
         wide ? k_scan_chain<true><<<blocks, kThreads, 0, st>>>(a) : k_scan_chain<false><<<blocks, kThreads, 0, st>>>(a);
