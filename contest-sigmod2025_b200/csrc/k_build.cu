@@ -245,31 +245,52 @@ __global__ void __launch_bounds__(256) k_bucket_ranges(BucketTiles t) {
     out[3] = make_uint4(run + c.x + c.y + c.z, c.w, 0, 0);
 }
 
-// Flags of bucket b's entries (see ht_flags).
-__device__ __forceinline__ void flag_bucket(const HTView& ht, uint32_t b, uint32_t* __restrict__ flags) {
-    const uint4 k = __ldcg(ht.buckets + b);
-    if (ht.mult)
-        for (uint32_t j = 0; j < k.y; j++)
-            if (__ldcg(ht.mult + k.x + j) > 1) flags[1] = 1;
-    if (k.y < 2) return;
-    if (k.y > 256) {
-        flags[0] = 1;  // long bucket: assume repeats (only steers capacity choices)
-        return;
+// Flags of the entries of the warp's buckets (see ht_flags), a bucket a lane;
+// all lanes together, those without a bucket with there = false. A bucket of
+// more than kLaneBucket entries is the whole warp's: Zipf-repeated keys held
+// single lanes for 9.7 ms; the query that has them takes 1.0 ms in all on its
+// first run now.
+constexpr uint32_t kLaneBucket = 8;
+__device__ __forceinline__ bool repeats(const HTView& ht, uint32_t first, uint32_t i) {  // entry first + i, of those before
+    const uint64_t key = __ldcg(ht.ent + size_t(first + i) * (1 + ht.width));
+    for (uint32_t j = 0; j < i; j++)
+        if (__ldcg(ht.ent + size_t(first + j) * (1 + ht.width)) == key) return true;
+    return false;
+}
+__device__ __forceinline__ void flag_buckets(const HTView& ht, uint32_t b, bool there, uint32_t* flags) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint4 k = there ? __ldcg(ht.buckets + b) : make_uint4(0, 0, 0, 0);
+    if (k.y <= kLaneBucket) {
+        if (ht.mult)
+            for (uint32_t j = 0; j < k.y; j++)
+                if (__ldcg(ht.mult + k.x + j) > 1) flags[1] = 1;
+        if (k.y > 2 || (k.y == 2 && k.z == k.w))
+            for (uint32_t i = 1; i < k.y; i++)
+                if (repeats(ht, k.x, i)) {
+                    flags[0] = 1;
+                    break;
+                }
     }
-    if (k.y == 2 && k.z != k.w) return;
-    for (uint32_t i = 1; i < k.y; i++) {
-        const uint64_t key = __ldcg(ht.ent + size_t(k.x + i) * (1 + ht.width));
-        for (uint32_t j = 0; j < i; j++)
-            if (__ldcg(ht.ent + size_t(k.x + j) * (1 + ht.width)) == key) {
-                flags[0] = 1;
-                return;
-            }
+    for (uint32_t left = __ballot_sync(0xffffffffu, k.y > kLaneBucket); left; left &= left - 1) {
+        const int src = __ffs(left) - 1;
+        const uint32_t x = __shfl_sync(0xffffffffu, k.x, src), y = __shfl_sync(0xffffffffu, k.y, src);
+        if (ht.mult && !__ldcg(flags + 1))
+            for (uint32_t j = lane; j < y; j += 32)
+                if (__ldcg(ht.mult + x + j) > 1) flags[1] = 1;
+        if (y > 256) {
+            if (lane == 0) flags[0] = 1;  // long bucket: assume repeats (only steers capacity choices)
+        } else if (!__ldcg(flags)) {
+            for (uint32_t i = lane; i < y; i += 32)
+                if (repeats(ht, x, i)) flags[0] = 1;
+        }
+        __syncwarp();
     }
 }
 
-__global__ void __launch_bounds__(256) k_ht_flags(HTView ht, uint32_t nbuckets, uint32_t* __restrict__ flags) {
-    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nbuckets; b += gridDim.x * blockDim.x)
-        flag_bucket(ht, b, flags);
+__global__ void __launch_bounds__(256) k_ht_flags(HTView ht, uint32_t nbuckets, uint32_t* flags) {
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b - lane < nbuckets; b += gridDim.x * blockDim.x)
+        flag_buckets(ht, b, b < nbuckets, flags);
 }
 
 // The same by a cluster: thread t of `all`, a warp a run of 32 buckets (or all
@@ -325,7 +346,7 @@ __global__ void __cluster_dims__(kFedCtas, 1, 1) __launch_bounds__(kFedThreads) 
     for (uint32_t i = t; i < n; i += all) place_tuple(a.tb, a.rank1, a.ht, a.err, i);
     if (!f.flags) return;
     cluster.sync();
-    for (uint32_t b = t; b < f.nb; b += all) flag_bucket(a.ht, b, f.dflags);
+    for (uint32_t b = t; b - (t & 31) < f.nb; b += all) flag_buckets(a.ht, b, b < f.nb, f.dflags);
 }
 
 // ---- leaf builds of a query, batched ----
@@ -392,7 +413,7 @@ __global__ void __launch_bounds__(256) k_leaf_flags(LeafBatch B) {
     const int b = leaf_of(B.tile_start, B.n, tile);
     const LeafBuild& L = B.l[b];
     const uint32_t i = (tile - B.tile_start[b]) * kBucketTile + (blockIdx.x % (kBucketTile / 256)) * 256 + threadIdx.x;
-    if (i < L.nb) flag_bucket(L.ht, i, L.dflags);
+    flag_buckets(L.ht, i, i < L.nb, L.dflags);
 }
 
 // Leaves of at most kClusterLeafRows rows: a cluster of eight CTAs builds one
@@ -425,7 +446,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     }
     if (!B.flags) return;
     cluster.sync();
-    for (uint32_t b = t; b < L.nb; b += all) flag_bucket(L.ht, b, L.dflags);
+    for (uint32_t b = t; b - (t & 31) < L.nb; b += all) flag_buckets(L.ht, b, b < L.nb, L.dflags);
 }
 
 // Hit counts of evenly spaced sample rows against every probe of a pipeline:
