@@ -223,10 +223,11 @@ __global__ void __launch_bounds__(kThreads, 5) k_scan_direct(DirectArgs a) {
             all += count[w];
         }
         if (threadIdx.x == 0 && all) base = atomicAdd(a.cursor, all);
-        __syncthreads();
+        __syncthreads();  // (also before count is written again)
+        if (!all) continue;  // no items were reserved: base is not this turn's
         o += base;
         if (base + all > a.capacity || base + all < all) {
-            if (threadIdx.x == 0 && all) record_error(a.err, kErrCapacity);
+            if (threadIdx.x == 0) record_error(a.err, kErrCapacity);
             return;
         }
 #pragma unroll
