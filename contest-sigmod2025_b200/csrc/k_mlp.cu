@@ -32,6 +32,7 @@
 // on the chip while the one before it ends (after.cuh).
 #include "after.cuh"
 #include "launch.h"
+#include "smem.h"
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -423,16 +424,6 @@ __global__ void k_f32_to_bf16(const float* in, uint16_t* out, long n) {
 } // namespace
 
 namespace {
-// Kernels with more than the default 48 KiB of dynamic shared memory say so
-// once per process.
-template <auto kKernel>
-void allow_smem(size_t bytes) {
-    static const bool configured = [bytes] {
-        cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-        return true;
-    }();
-    (void)configured;
-}
 template <int T, bool kAt, bool kBt>
 void launch_gemm(const GemmArgs& g, cudaStream_t st) {
     constexpr size_t smem = gemm_smem<T, kAt, kBt, kForwardStages<T>>();

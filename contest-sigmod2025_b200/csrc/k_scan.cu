@@ -38,6 +38,7 @@
 //    writes at the units' offsets (mode 1); the buffer is emptied at the end
 //    of every unit.
 #include "launch.h"
+#include "smem.h"
 
 #include <algorithm>
 #include <cstdlib>
@@ -589,13 +590,7 @@ __global__ void __launch_bounds__(256) k_probe_candidates(ScanArgs a) {
 
 template <bool kFilter, bool kNulls>
 void launch_scan(const ScanArgs& a, size_t bloom_bytes, int num_sms, cudaStream_t st) {
-    // Once per process and form (thread-safe static initialisation; server
-    // workers launch from several threads).
-    static const bool configured = [] {
-        cudaFuncSetAttribute(k_scan_probe<kFilter, kNulls>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBloomSmemMax));
-        return true;
-    }();
-    (void)configured;
+    allow_smem<k_scan_probe<kFilter, kNulls>>(kBloomSmemMax);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scan_probe<kFilter, kNulls>, kCtaThreads, bloom_bytes);
     per_sm = std::max(1, per_sm);

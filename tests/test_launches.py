@@ -1,0 +1,22 @@
+"""Host side of kernel launches, on the CPU: shared-memory attributes are kept for each device."""
+import glob
+import os
+import subprocess
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "contest-sigmod2025_b200", "csrc")
+CUDA = os.environ.get("CUDA", "/usr/local/cuda")
+
+
+def _run(tmp_path, name):
+    exe = str(tmp_path / name)
+    subprocess.run(["g++", "-std=c++20", "-O1", "-pthread", "-I", CSRC, "-I", os.path.join(CUDA, "include"), "-o", exe,
+                    os.path.join(HERE, "cpp", name + ".cpp")], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_shared_memory_attribute_is_set_on_every_device(tmp_path):
+    _run(tmp_path, "smem_attribute")
+    for path in glob.glob(os.path.join(CSRC, "*.cu")):  # no launcher keeps its own once-flag
+        assert "cudaFuncSetAttribute" not in open(path).read(), path
