@@ -16,8 +16,9 @@ __device__ __forceinline__ void begin_after_previous() {
     cudaTriggerProgrammaticLaunchCompletion();
 }
 
+// The launch's status: a refused launch is reported here and nowhere else.
 template <typename... P, typename... A>
-void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+[[nodiscard]] cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchAttribute overlap{};
     overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     overlap.val.programmaticStreamSerializationAllowed = 1;
@@ -28,7 +29,7 @@ void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cuda
     c.stream = st;
     c.attrs = &overlap;
     c.numAttrs = 1;
-    cudaLaunchKernelEx(&c, kernel, P(args)...);
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
 }
 
 } // namespace bj

@@ -648,7 +648,7 @@ struct bj_estimator {
         g.bias = WB() + kOffB1;
         g.Cb = H1;
         g.ldc = kH;
-        gemm_forward(g, stream);
+        EST_CK(gemm_forward(g, stream));
         g.A = H1;
         g.a_rs = kH;
         g.a_idx = nullptr;
@@ -657,7 +657,7 @@ struct bj_estimator {
         g.K = kH;
         g.bias = WB() + kOffB2;
         g.Cb = H2;
-        gemm_forward(g, stream);
+        EST_CK(gemm_forward(g, stream));
     }
 
     // Forward, loss and gradients over a batch of in.n_real rows (padded to
@@ -675,7 +675,7 @@ struct bj_estimator {
         h.dy = dy;
         h.dH2 = dH2;
         h.n_real = in.n_real;
-        mlp_head(h, n_pad, stream);
+        EST_CK(mlp_head(h, n_pad, stream));
         GemmArgs g{};
         // dW2 = H1^T dH2
         g.A = H1;
@@ -708,7 +708,7 @@ struct bj_estimator {
         g.mask = H1;
         g.Cb = dH1;
         g.ldc = kH;
-        gemm_backward(dw2, g, stream);
+        EST_CK(gemm_backward(dw2, g, stream));
         // dW1 = X^T dH1
         g = GemmArgs{};
         g.A = in.X;
@@ -735,7 +735,7 @@ struct bj_estimator {
         r.b2 = G() + kOffB2;
         r.w3 = G() + kOffW3;
         r.b3 = G() + kOffB3;
-        gemm_row_sums(g, r, stream);
+        EST_CK(gemm_row_sums(g, r, stream));
     }
 
     void adam(float lr) {
@@ -754,13 +754,13 @@ struct bj_estimator {
         a.eps = 1e-8f;
         a.bc1 = float(1.0 - std::pow(0.9, double(step)));
         a.bc2 = float(1.0 - std::pow(0.999, double(step)));
-        adam_step(a, stream);
+        EST_CK(adam_step(a, stream));
     }
 
     void upload_params(const float* p) {
         using namespace bj;
         EST_CK(cudaMemcpyAsync(W(), p, sizeof(float) * kParams, cudaMemcpyHostToDevice, stream));
-        f32_to_bf16(W(), WB(), kParams, stream);
+        EST_CK(f32_to_bf16(W(), WB(), kParams, stream));
         EST_CK(cudaMemsetAsync(mo.p, 0, sizeof(float) * kParams, stream));
         EST_CK(cudaMemsetAsync(vo.p, 0, sizeof(float) * kParams, stream));
         EST_CK(cudaStreamSynchronize(stream));
@@ -804,7 +804,7 @@ struct bj_estimator {
         h.w3 = WB() + kOffW3;
         h.b3 = WB() + kOffB3;
         h.y = y;
-        mlp_head(h, rows, stream);
+        EST_CK(mlp_head(h, rows, stream));
         EST_CK(cudaMemcpyAsync(out, y, sizeof(float) * rows, cudaMemcpyDeviceToHost, stream));
         EST_CK(cudaStreamSynchronize(stream));
     }
@@ -1115,7 +1115,7 @@ BJ_API int bj_estimator_train(bj_estimator* e, const float* features, const floa
         const float b3 = float(mean / double(n));
         if (e->step == 0) {
             EST_CK(cudaMemcpyAsync(e->W() + kOffB3, &b3, sizeof(float), cudaMemcpyHostToDevice, e->stream));
-            f32_to_bf16(e->W() + kOffB3, e->WB() + kOffB3, 1, e->stream);
+            EST_CK(f32_to_bf16(e->W() + kOffB3, e->WB() + kOffB3, 1, e->stream));
         }
         const int bpad = int((batch + 63) & ~63u);
         e->reserve(bpad);

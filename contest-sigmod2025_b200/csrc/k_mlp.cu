@@ -425,64 +425,52 @@ __global__ void k_f32_to_bf16(const float* in, uint16_t* out, long n) {
 
 namespace {
 template <int T, bool kAt, bool kBt>
-void launch_gemm(const GemmArgs& g, cudaStream_t st) {
+cudaError_t launch_gemm(const GemmArgs& g, cudaStream_t st) {
     constexpr size_t smem = gemm_smem<T, kAt, kBt, kForwardStages<T>>();
-    allow_smem<k_gemm_bf16<T, kAt, kBt>>(smem);
-    launch_after(k_gemm_bf16<T, kAt, kBt>, dim3((g.N + T - 1) / T, (g.M + T - 1) / T), 128, smem, st, g);
+    if (const cudaError_t e = allow_smem<k_gemm_bf16<T, kAt, kBt>>(smem); e != cudaSuccess) return e;
+    return launch_after(k_gemm_bf16<T, kAt, kBt>, dim3((g.N + T - 1) / T, (g.M + T - 1) / T), 128, smem, st, g);
 }
 template <int T>
-void launch_pair(const GemmArgs& g, const GemmArgs& h, cudaStream_t st) {
+cudaError_t launch_pair(const GemmArgs& g, const GemmArgs& h, cudaStream_t st) {
     constexpr size_t smem =
         std::max(gemm_smem<32, true, true, kBackwardStages>(), gemm_smem<T, false, false, kBackwardStages>());
-    allow_smem<k_gemm_pair<T>>(smem);
+    if (const cudaError_t e = allow_smem<k_gemm_pair<T>>(smem); e != cudaSuccess) return e;
     const int g_tiles = (g.M + 31) / 32 * ((g.N + 31) / 32), h_tiles = (h.M + T - 1) / T * ((h.N + T - 1) / T);
-    launch_after(k_gemm_pair<T>, g_tiles + h_tiles, 128, smem, st, g, h, g_tiles);
+    return launch_after(k_gemm_pair<T>, g_tiles + h_tiles, 128, smem, st, g, h, g_tiles);
 }
 // 64 x 64 tiles where they fill the chip (half the operand traffic), else
 // 32 x 32 ones, four times the CTAs: the chain is as long in either.
 bool wide_tiles(const GemmArgs& g) { return long((g.M + 63) / 64) * ((g.N + 63) / 64) >= 148; }
 } // namespace
 
-int gemm_forward(const GemmArgs& g, cudaStream_t st) {
-    if (g.M <= 0 || g.N <= 0) return 0;
-    if (wide_tiles(g))
-        launch_gemm<64, false, true>(g, st);
-    else
-        launch_gemm<32, false, true>(g, st);
-    return 1;
+cudaError_t gemm_forward(const GemmArgs& g, cudaStream_t st) {
+    if (g.M <= 0 || g.N <= 0) return cudaSuccess;
+    return wide_tiles(g) ? launch_gemm<64, false, true>(g, st) : launch_gemm<32, false, true>(g, st);
 }
 
-int gemm_backward(const GemmArgs& dw, const GemmArgs& dh, cudaStream_t st) {
-    if (wide_tiles(dh))
-        launch_pair<64>(dw, dh, st);
-    else
-        launch_pair<32>(dw, dh, st);
-    return 1;
+cudaError_t gemm_backward(const GemmArgs& dw, const GemmArgs& dh, cudaStream_t st) {
+    return wide_tiles(dh) ? launch_pair<64>(dw, dh, st) : launch_pair<32>(dw, dh, st);
 }
 
-int gemm_row_sums(const GemmArgs& dw, const RowSumArgs& r, cudaStream_t st) {
+cudaError_t gemm_row_sums(const GemmArgs& dw, const RowSumArgs& r, cudaStream_t st) {
     constexpr size_t ring = gemm_smem<32, true, true, kBackwardStages>();
     static_assert(ring >= 64 * kSumColumns * sizeof(float));
     const size_t smem = ring + (dw.a_idx ? sizeof(uint32_t) * size_t(dw.a_there) : 0);  // at most 8,192 rows a batch
-    allow_smem<k_gemm_row_sums>(ring + sizeof(uint32_t) * kMaxBatch);
-    launch_after(k_gemm_row_sums, kRowSumBlocks + (dw.M + 31) / 32 * ((dw.N + 31) / 32), 128, smem, st, dw, r);
-    return 1;
+    if (const cudaError_t e = allow_smem<k_gemm_row_sums>(ring + sizeof(uint32_t) * kMaxBatch); e != cudaSuccess) return e;
+    return launch_after(k_gemm_row_sums, kRowSumBlocks + (dw.M + 31) / 32 * ((dw.N + 31) / 32), 128, smem, st, dw, r);
 }
 
-int mlp_head(const MlpHeadArgs& a, int rows, cudaStream_t st) {
-    if (rows <= 0) return 0;
-    launch_after(k_mlp_head, rows, kMlpHidden, 0, st, a);
-    return 1;
+cudaError_t mlp_head(const MlpHeadArgs& a, int rows, cudaStream_t st) {
+    if (rows <= 0) return cudaSuccess;
+    return launch_after(k_mlp_head, rows, kMlpHidden, 0, st, a);
 }
 
-int adam_step(const AdamArgs& a, cudaStream_t st) {
-    launch_after(k_adam, unsigned((a.n / 4 + 127) / 128), 128, 0, st, a);
-    return 1;
+cudaError_t adam_step(const AdamArgs& a, cudaStream_t st) {
+    return launch_after(k_adam, unsigned((a.n / 4 + 127) / 128), 128, 0, st, a);
 }
 
-int f32_to_bf16(const float* in, uint16_t* out, long n, cudaStream_t st) {
-    launch_after(k_f32_to_bf16, 592, 256, 0, st, in, out, n);
-    return 1;
+cudaError_t f32_to_bf16(const float* in, uint16_t* out, long n, cudaStream_t st) {
+    return launch_after(k_f32_to_bf16, 592, 256, 0, st, in, out, n);
 }
 
 } // namespace bj

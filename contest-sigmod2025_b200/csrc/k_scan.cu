@@ -41,6 +41,7 @@
 #include "smem.h"
 
 #include <algorithm>
+#include <stdexcept>
 #include <cstdlib>
 
 namespace bj {
@@ -590,7 +591,8 @@ __global__ void __launch_bounds__(256) k_probe_candidates(ScanArgs a) {
 
 template <bool kFilter, bool kNulls>
 void launch_scan(const ScanArgs& a, size_t bloom_bytes, int num_sms, cudaStream_t st) {
-    allow_smem<k_scan_probe<kFilter, kNulls>>(kBloomSmemMax);
+    if (allow_smem<k_scan_probe<kFilter, kNulls>>(kBloomSmemMax) != cudaSuccess)
+        throw std::runtime_error("the staged scan's filter was refused its shared memory");
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scan_probe<kFilter, kNulls>, kCtaThreads, bloom_bytes);
     per_sm = std::max(1, per_sm);

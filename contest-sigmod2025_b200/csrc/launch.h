@@ -464,7 +464,8 @@ int sample_edges(const SampleEdges& e, uint32_t nsample, uint32_t* hits, cudaStr
 // a multiple of 8. K and N must be multiples of 64; an operand whose
 // contiguous dimension is its rows (m for A, n for B) needs those rows a
 // multiple of 8. A's other dimension (m, or k) may be indirect: its position i
-// is a_idx[i] (null: i), and positions from a_there on read zeros.
+// is a_idx[i] (null: i), and positions from a_there on read zeros. The
+// estimator's launchers return the launch's status.
 constexpr int kMlpHidden = 256;
 enum GemmEpi : int {
     kEpiBiasRelu = 0,  // Cb = bf16(relu(acc + bias[n]))
@@ -486,10 +487,10 @@ struct GemmArgs {
     float* Cf;
     long ldc;
 };
-int gemm_forward(const GemmArgs& g, cudaStream_t st);  // A with k contiguous, B with n contiguous
+[[nodiscard]] cudaError_t gemm_forward(const GemmArgs& g, cudaStream_t st);  // A with k contiguous, B with n contiguous
 // A weight gradient (A with m contiguous, B with n contiguous) and the gradient
 // of a layer's rows (A and B with k contiguous) in one launch.
-int gemm_backward(const GemmArgs& dw, const GemmArgs& dh, cudaStream_t st);
+[[nodiscard]] cudaError_t gemm_backward(const GemmArgs& dw, const GemmArgs& dh, cudaStream_t st);
 // Output layer (one CTA per row): y = H2 . w3 + b3; with targets t, loss +=
 // (y - t)^2 and, for rows below n_real, dy = 2 (y - t) / n_real and dH2 =
 // bf16(dy * w3 * [H2 > 0]) (zero for the other rows). Optional outputs may
@@ -506,7 +507,7 @@ struct MlpHeadArgs {
     uint16_t* dH2;
     int n_real;
 };
-int mlp_head(const MlpHeadArgs& a, int rows, cudaStream_t st);
+[[nodiscard]] cudaError_t mlp_head(const MlpHeadArgs& a, int rows, cudaStream_t st);
 // Bias and output-layer gradients of a batch of `rows` rows, in one launch with
 // a weight gradient (A with m contiguous, B with n contiguous).
 struct RowSumArgs {
@@ -520,7 +521,7 @@ struct RowSumArgs {
     float* w3;
     float* b3;
 };
-int gemm_row_sums(const GemmArgs& dw, const RowSumArgs& r, cudaStream_t st);
+[[nodiscard]] cudaError_t gemm_row_sums(const GemmArgs& dw, const RowSumArgs& r, cudaStream_t st);
 struct AdamArgs {
     float* w;
     uint16_t* wb;
@@ -530,8 +531,8 @@ struct AdamArgs {
     long n;  // a multiple of 4
     float lr, beta1, beta2, eps, bc1, bc2;  // bc: 1 - beta^t
 };
-int adam_step(const AdamArgs& a, cudaStream_t st);
-int f32_to_bf16(const float* in, uint16_t* out, long n, cudaStream_t st);
+[[nodiscard]] cudaError_t adam_step(const AdamArgs& a, cudaStream_t st);
+[[nodiscard]] cudaError_t f32_to_bf16(const float* in, uint16_t* out, long n, cudaStream_t st);
 
 // ---- output pages (k_output.cu) ----
 // Page descriptors of a VARCHAR column.

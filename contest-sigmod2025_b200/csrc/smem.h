@@ -14,7 +14,7 @@ namespace bj {
 // current device. The attribute belongs to the kernel on one device: it is set
 // on the first launch there (threads that race for it set the same value).
 template <auto kKernel>
-cudaError_t allow_smem(size_t bytes) {
+[[nodiscard]] cudaError_t allow_smem(size_t bytes) {
     static std::atomic<uint64_t> allowed{0};  // bit d: device d; devices from 64 on are set each time
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);

@@ -1,4 +1,5 @@
-"""Host side of kernel launches, on the CPU: shared-memory attributes are kept for each device."""
+"""Host side of kernel launches, on the CPU: shared-memory attributes are kept for each device, a refused launch is
+reported to the caller."""
 import glob
 import os
 import subprocess
@@ -20,3 +21,7 @@ def test_shared_memory_attribute_is_set_on_every_device(tmp_path):
     _run(tmp_path, "smem_attribute")
     for path in glob.glob(os.path.join(CSRC, "*.cu")):  # no launcher keeps its own once-flag
         assert "cudaFuncSetAttribute" not in open(path).read(), path
+
+
+def test_refused_launch_is_reported(tmp_path):
+    _run(tmp_path, "launch_status")
