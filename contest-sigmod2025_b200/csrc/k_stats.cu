@@ -33,11 +33,20 @@ __device__ __forceinline__ uint32_t map_slot(uint64_t key, uint32_t log2cap) {
     return uint32_t(mix64(key) >> (64 - log2cap));
 }
 
+// *y += v for v > 0; a sum past 2^64 - 1 stays at ~0ull. Whoever sees the word
+// wrap puts it there, and an addition that comes after wraps again and does the
+// same, so in any order the last write leaves ~0ull. Returns what was there.
+__device__ __forceinline__ unsigned long long add_sat(unsigned long long* y, unsigned long long v) {
+    const unsigned long long old = atomicAdd(y, v);
+    if (old + v < old) atomicMax(y, ~0ull);
+    return old;
+}
+
 // Adds v to key's value (inserting the key); returns 1 when the key is new. The
 // key ~0ull, which marks empty slots, keeps its value in slot cap.
 __device__ __forceinline__ uint32_t map_add(const KeyMap& m, uint64_t key, unsigned long long v, uint32_t* err) {
     const uint32_t cap = 1u << m.log2cap;
-    if (key == kMapEmpty) return atomicAdd(&m.slots[cap].y, v) == 0 ? 1u : 0u;
+    if (key == kMapEmpty) return add_sat(&m.slots[cap].y, v) == 0 ? 1u : 0u;
     uint32_t pos = map_slot(key, m.log2cap), added = 0;
     for (uint32_t step = 0; step < cap; step++) {
         unsigned long long cur = m.slots[pos].x;
@@ -49,7 +58,7 @@ __device__ __forceinline__ uint32_t map_add(const KeyMap& m, uint64_t key, unsig
             }
         }
         if (cur == key) {
-            atomicAdd(&m.slots[pos].y, v);
+            add_sat(&m.slots[pos].y, v);
             return added;
         }
         pos = (pos + 1) & (cap - 1);
@@ -71,10 +80,6 @@ __device__ __forceinline__ unsigned long long map_get(const KeyMap& m, uint64_t 
         pos = (pos + 1) & (cap - 1);
     }
     return 0;
-}
-
-__device__ __forceinline__ bool map_overflowed(const KeyMap& m) {
-    return m.slots[1u << m.log2cap].x != kMapEmpty;
 }
 
 __global__ void k_map_clear(KeyMap m) {
@@ -119,18 +124,14 @@ __global__ void __launch_bounds__(256) k_col_stats(DevColumn c, uint32_t parts, 
         if (h[i]) atomicAdd(&hist[i], h[i]);
 }
 
-// Saturating u64 product (a count beyond 2^64 - 1 sets the overflow flag).
-__device__ __forceinline__ unsigned long long mul_sat(unsigned long long a, unsigned long long b, bool& over) {
-    if (a && b && __umul64hi(a, b)) {
-        over = true;
-        return ~0ull;
-    }
-    return a * b;
+// Saturating u64 product: ~0ull stands for a weight past 2^64 - 1 and stays that
+// unless the other factor is 0.
+__device__ __forceinline__ unsigned long long mul_sat(unsigned long long a, unsigned long long b) {
+    return __umul64hi(a, b) ? ~0ull : a * b;
 }
 
 // An inner table's map: each row's weight, summed into its parent-edge key.
 __global__ void __launch_bounds__(256) k_count_node(CountNode n, uint32_t* err) {
-    bool over = false;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n.nrows; r += gridDim.x * blockDim.x) {
         unsigned long long w = 1;
         for (int j = 0; j < n.nch && w; j++) {
@@ -139,14 +140,12 @@ __global__ void __launch_bounds__(256) k_count_node(CountNode n, uint32_t* err) 
                 w = 0;
                 break;
             }
-            w = mul_sat(w, map_get(n.ch[j].map, k), over);
+            w = mul_sat(w, map_get(n.ch[j].map, k));
         }
         if (!w) continue;
         uint64_t k;
         if (col_get(n.pkey, r, k)) map_add(n.out, k, w, err);
     }
-    if (blockIdx.x == 0 && threadIdx.x < uint32_t(n.nch)) over = over || map_overflowed(n.ch[threadIdx.x].map);
-    if (over) n.out.slots[1u << n.out.log2cap].x = 0;
 }
 
 // The totals of sub-plans with the same root table, in one pass over it. A
@@ -196,13 +195,12 @@ __global__ void __launch_bounds__(256) k_count_group(CountGroup g) {
             for (int j = 0; j < 8; j++) {
                 if ((heavy[32 * j + lane] & set) != set) continue;
                 unsigned long long v = 1;
-                bool o1 = false;
                 for (uint32_t m = set; m; m &= m - 1) {
                     const unsigned long long x = w[__ffs(m) - 1][32 * j + lane];
-                    v = (v | x) >> 32 ? mul_sat(v, x, o1) : static_cast<unsigned long long>(uint32_t(v)) * uint32_t(x);
+                    v = (v | x) >> 32 ? mul_sat(v, x) : static_cast<unsigned long long>(uint32_t(v)) * uint32_t(x);
                 }
                 const unsigned long long sum = acc[i] + v;
-                if (o1 || sum < v) over |= 1u << i;
+                if (v == ~0ull || sum < v) over |= 1u << i;
                 acc[i] = sum;
             }
         }
@@ -232,8 +230,6 @@ __global__ void __launch_bounds__(256) k_count_group(CountGroup g) {
             const unsigned long long old = atomicAdd(g.total + g.slot[s], v);
             o1 = o1 || old + v < old;
         }
-        if (blockIdx.x == 0)
-            for (uint32_t m = set; m; m &= m - 1) o1 = o1 || map_overflowed(g.opt[__ffs(m) - 1].map);
         if (lane == 0 && o1) atomicOr(g.flags + 2 * g.slot[s], 1u);
     }
 }

@@ -385,9 +385,9 @@ int sample_probes(const SampleSet& set, uint32_t nsample, uint32_t* hits, cudaSt
 
 // ---- join-ordering statistics (k_stats.cu) ----
 // Open-addressing map from a key slot (u64) to a u64 value: slot = (key, value);
-// the key ~0ull marks an empty slot, and itself keeps its value in slot cap,
-// whose key word tells an overflow: other than ~0ull, some value of the map
-// passed 2^64 - 1. cap = 1 << log2cap; cap + 1 slots.
+// the key ~0ull marks an empty slot, and itself keeps its value in slot cap.
+// The value ~0ull stands for a sum past 2^64 - 1. cap = 1 << log2cap; cap + 1
+// slots.
 struct KeyMap {
     ulonglong2* slots;
     uint32_t log2cap;
@@ -403,7 +403,7 @@ int column_stats(const DevColumn& c, const KeyMap& m, uint32_t* hist, unsigned i
 // An inner table of sub-plans' exact counts. For every row r: w = product over
 // the children j of ch[j].map[value of ch[j].key at r] (0 when the value is
 // NULL or absent); out[value of pkey at r] += w (rows with a NULL pkey
-// skipped). A weight past 2^64 - 1, here or in a child's map, marks `out`.
+// skipped). A weight or sum past 2^64 - 1 is ~0ull.
 constexpr int kMaxCountChildren = 12;
 struct CountChild {
     DevColumn key;  // this table's column on the edge to the child
@@ -420,10 +420,10 @@ int count_node(const CountNode& n, uint32_t* err, int num_sms, cudaStream_t st);
 // The root table of several sub-plans. Option o of a row: opt[o].map[value of
 // opt[o].key] (0 when the value is NULL or absent). For sub-plan s: *(total +
 // slot[s]) += the sum over the rows of the product of the options in
-// options[s]; word 2 slot[s] of flags |= 1 when a product, the total or a value
-// of one of its maps passes 2^64 - 1. Options of one edge lie side by side, new_edge set on the first;
-// leaf: an earlier option of the same edge whose map holds every key of this
-// one's (-1: none).
+// options[s]; word 2 slot[s] of flags |= 1 when that sum passes 2^64 - 1.
+// Options of one edge lie side by side, new_edge set on the first; leaf: an
+// earlier option of the same edge whose map holds every key of this one's (-1:
+// none).
 constexpr int kMaxCountOptions = kMaxCountChildren;
 constexpr int kMaxCountTotals = 64;
 struct CountOption {
