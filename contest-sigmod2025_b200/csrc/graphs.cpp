@@ -123,7 +123,7 @@ bool capture_graph(bj_context* ctx, GraphEntry& g, const bj_plan* plan, bj_resid
         ctx->prof_bytes = 0;
         ctx->arena.reset();
         return true;
-    } catch (const Fail&) {
+    } catch (...) {  // not only Fail: the launchers throw standard exceptions, and the capture must end
         if (capturing) {
             cudaGraph_t gr = nullptr;
             cudaStreamEndCapture(ctx->stream, &gr);
