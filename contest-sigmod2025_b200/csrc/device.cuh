@@ -113,17 +113,6 @@ __device__ __forceinline__ uint64_t load_bits64(const uint8_t* bm, uint32_t k, u
     return w;
 }
 
-// Bitmap bits of rows 32 w .. 32 w + 31 of a page whose nbytes bitmap bytes
-// end the page (bits beyond the page's rows are garbage).
-__device__ __forceinline__ uint32_t page_bitmap_word(const uint8_t* pg, uint32_t nbytes, uint32_t w) {
-    const uint32_t byte = kPageSize - nbytes + 4 * w;
-    const uint32_t lo = byte & ~3u;
-    if (lo >= kPageSize) return 0;
-    const uint32_t a = *reinterpret_cast<const uint32_t*>(pg + lo);
-    const uint32_t b = lo + 4 < kPageSize ? *reinterpret_cast<const uint32_t*>(pg + lo + 4) : 0u;
-    return __funnelshift_r(a, b, 8 * (byte & 3));
-}
-
 // Reads the value of `row` as a 64-bit slot. Returns false for NULL.
 // INT32 is zero-extended, INT64/FP64 are raw bits, VARCHAR yields a handle.
 // row / c.rpp for c.rpp != 0: floor(rpp_m * row / 2^64) from 32-bit halves

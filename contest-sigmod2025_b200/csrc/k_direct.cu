@@ -25,6 +25,7 @@
 // 28 -> 16 us; 8M rows with 10% NULLs 145 -> 63 us (75 us with the matches
 // staged in shared memory and 1,184 CTAs looping over the pages).
 #include "launch.h"
+#include "page_rows.cuh"
 
 #include <algorithm>
 

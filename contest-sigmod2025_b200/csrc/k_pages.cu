@@ -9,6 +9,7 @@
 // chunk count; two scans turn those into row_start / chunk_base. Pass 2 writes the dense-value base of every chunk
 // and the page of every 1024-row block.
 #include "launch.h"
+#include "page_rows.cuh"
 
 #include <algorithm>
 

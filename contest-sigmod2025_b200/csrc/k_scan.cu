@@ -38,6 +38,7 @@
 //    writes at the units' offsets (mode 1); the buffer is emptied at the end
 //    of every unit.
 #include "launch.h"
+#include "page_rows.cuh"
 #include "smem.h"
 
 #include <algorithm>
@@ -233,30 +234,6 @@ __device__ __forceinline__ uint32_t first_row(const ScanArgs& a, uint32_t p) {
     return a.key.rpp ? a.row_base + p * a.key.rpp : __ldg(a.key.row_start + p);
 }
 
-// Row in page p of its value d, when the page has NULLs: the 64-row chunk that
-// holds the value by the page index, then the bit of the chunk's bitmap.
-__device__ __forceinline__ uint32_t row_of_value(const DevColumn& c, const uint8_t* pg, uint32_t p, uint32_t n, uint32_t d) {
-    const uint32_t c0 = __ldg(c.chunk_base + p);
-    uint32_t lo = 0, hi = (n + 63) / 64 - 1;  // the last chunk with at most d values before it
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) / 2;
-        if (__ldg(c.dense_base + c0 + mid) <= d)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    uint32_t k = d - __ldg(c.dense_base + c0 + lo);  // set bits of the chunk before the value's
-    const uint32_t nbytes = (n + 7) >> 3;
-    uint32_t w = page_bitmap_word(pg, nbytes, 2 * lo), r = 64 * lo;
-    if (k >= __popc(w)) {
-        k -= __popc(w);
-        w = page_bitmap_word(pg, nbytes, 2 * lo + 1);
-        r += 32;
-    }
-    for (; k; k--) w &= w - 1;
-    return r + (w ? __ffs(w) - 1 : 0);
-}
-
 // Probes every buffered candidate: the keys are read again from their pages,
 // just loaded by this warp, four at a time a lane. (kNulls: the column has
 // pages with NULLs.)
@@ -277,7 +254,8 @@ __device__ __forceinline__ void flush(const ScanArgs& a, WarpState& w, uint32_t 
             uint32_t r = d;
             if (kNulls) {
                 const uint32_t hdr = __ldg(pg), n = hdr & 0xffff;
-                if (hdr >> 16 != n) r = row_of_value(a.key, reinterpret_cast<const uint8_t*>(pg), p, n, d);
+                if (hdr >> 16 != n)
+                    r = row_of_value(reinterpret_cast<const uint8_t*>(pg), n, a.key.dense_base + __ldg(a.key.chunk_base + p), d);
             }
             row[i] = first_row(a, p) + r;
             has |= 1u << i;
