@@ -10,6 +10,7 @@
 // cardinalities it is given: the reference's row-count model, join samples,
 // or the learned MLP (kernels in k_mlp.cu), with sampling as its fallback.
 #include "engine.h"
+#include "row_stage.h"
 
 #include <cmath>
 #include <cstdio>
@@ -50,20 +51,6 @@ uint16_t to_bf16(float f) {
     return uint16_t(u >> 16);
 }
 
-// The same for n values; runs as wide as the host's vectors (the branch of the
-// scalar form becomes a select).
-#if defined(__x86_64__) && defined(__GNUC__) && !defined(__clang__)
-__attribute__((target_clones("avx512f", "avx2", "default")))
-#endif
-void to_bf16_n(const float* in, uint16_t* out, size_t n) {
-    for (size_t i = 0; i < n; i++) {
-        uint32_t u;
-        std::memcpy(&u, in + i, 4);
-        const uint32_t r = (u + 0x7fffu + ((u >> 16) & 1u)) >> 16, nan = (u >> 16) | 0x40u;
-        out[i] = uint16_t((u & 0x7fffffffu) > 0x7f800000u ? nan : r);
-    }
-}
-
 // Device buffer freed with the owner.
 struct DevBuf {
     void* p = nullptr;
@@ -93,81 +80,6 @@ struct DevBuf {
         EST_CK(cudaMalloc(&p, std::max<size_t>(n * sizeof(T), 256)));
         return static_cast<T*>(p);
     }
-};
-
-// The way of feature rows to a device, shared by its estimators and freed with
-// the last of them: a small pinned ring (pinning costs a millisecond or more a
-// MB), the events of its slots' copies and the threads that convert into it.
-class RowStage {
-    public:
-    static std::shared_ptr<RowStage> of(int device) {
-        static std::mutex m;
-        static std::vector<std::weak_ptr<RowStage>> stages;
-        std::lock_guard<std::mutex> g(m);
-        if (stages.size() <= size_t(device)) stages.resize(size_t(device) + 1);
-        std::shared_ptr<RowStage> s = stages[size_t(device)].lock();
-        if (!s) stages[size_t(device)] = s = std::make_shared<RowStage>(device);
-        return s;
-    }
-
-    explicit RowStage(int device)
-        : device_(device), pool_(std::min(std::max(1u, std::thread::hardware_concurrency()), 8u) - 1) {
-        void* p = nullptr;
-        EST_CK(cudaHostAlloc(&p, sizeof(uint16_t) * kSlots * kSlotWords, cudaHostAllocDefault));
-        ring_ = static_cast<uint16_t*>(p);
-        for (cudaEvent_t& e : done_)
-            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
-                free_all();
-                throw Fail{BJ_ERR_CUDA, "event creation failed"};
-            }
-    }
-    ~RowStage() {
-        for (cudaEvent_t e : done_) cudaEventSynchronize(e);
-        free_all();
-    }
-
-    // Host threads take slots of rows in order, convert them into the ring and
-    // start their copies on `stream`, each after the copy that used its place
-    // before. Bound: the host reading its FP32 rows. A whole prediction of 6,000
-    // rows on a 16-core B200 host: 1.5 ms, where one thread converting every
-    // row into pageable memory before their copy made it 8.4 ms.
-    void upload(const float* f, uint64_t n, uint16_t* dst, cudaStream_t stream) {
-        std::lock_guard<std::mutex> g(m_);
-        std::atomic<uint64_t> copying[kSlots];  // slots taken from the ring's place whose copy is enqueued
-        for (auto& c : copying) c = 0;
-        std::atomic<int> failed{cudaSuccess};
-        pool_.parallel_for((n + kSlotRows - 1) / kSlotRows, [&](size_t i) {
-            const size_t s = i % kSlots, turn = i / kSlots;
-            // The slot's earlier turns were taken by threads already at work.
-            while (copying[s].load(std::memory_order_acquire) < turn) std::this_thread::yield();
-            cudaError_t e = cudaSetDevice(device_);
-            if (e == cudaSuccess) e = cudaEventSynchronize(done_[s]);
-            if (e == cudaSuccess) {
-                const uint64_t r0 = i * kSlotRows, rows = std::min(kSlotRows, n - r0);
-                uint16_t* to = ring_ + s * kSlotWords;
-                to_bf16_n(f + r0 * kF, to, rows * kF);
-                e = cudaMemcpyAsync(dst + r0 * kF, to, sizeof(uint16_t) * rows * kF, cudaMemcpyHostToDevice, stream);
-                if (e == cudaSuccess) e = cudaEventRecord(done_[s], stream);
-            }
-            if (e != cudaSuccess) failed = e;
-            copying[s].store(turn + 1, std::memory_order_release);
-        });
-        EST_CK(cudaError_t(failed.load()));
-    }
-
-    private:
-    static constexpr uint64_t kSlots = 8, kSlotRows = 64;
-    static constexpr size_t kSlotWords = kSlotRows * kF;
-    void free_all() {
-        for (cudaEvent_t e : done_)
-            if (e) cudaEventDestroy(e);
-        cudaFreeHost(ring_);
-    }
-    int device_;
-    std::mutex m_;
-    uint16_t* ring_ = nullptr;
-    cudaEvent_t done_[kSlots] = {};
-    ThreadPool pool_;
 };
 
 // Statistics of column c of a resident table, computed on first use.
