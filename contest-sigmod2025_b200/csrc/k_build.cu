@@ -260,23 +260,15 @@ __device__ __forceinline__ bool repeats(const HTView& ht, uint32_t first, uint32
 __device__ __forceinline__ void flag_buckets(const HTView& ht, uint32_t b, bool there, uint32_t* flags) {
     const uint32_t lane = threadIdx.x & 31;
     const uint4 k = there ? __ldcg(ht.buckets + b) : make_uint4(0, 0, 0, 0);
-    if (k.y <= kLaneBucket) {
-        if (ht.mult)
-            for (uint32_t j = 0; j < k.y; j++)
-                if (__ldcg(ht.mult + k.x + j) > 1) flags[1] = 1;
-        if (k.y > 2 || (k.y == 2 && k.z == k.w))
-            for (uint32_t i = 1; i < k.y; i++)
-                if (repeats(ht, k.x, i)) {
-                    flags[0] = 1;
-                    break;
-                }
-    }
+    if (k.y <= kLaneBucket && (k.y > 2 || (k.y == 2 && k.z == k.w)))
+        for (uint32_t i = 1; i < k.y; i++)
+            if (repeats(ht, k.x, i)) {
+                flags[0] = 1;
+                break;
+            }
     for (uint32_t left = __ballot_sync(0xffffffffu, k.y > kLaneBucket); left; left &= left - 1) {
         const int src = __ffs(left) - 1;
         const uint32_t x = __shfl_sync(0xffffffffu, k.x, src), y = __shfl_sync(0xffffffffu, k.y, src);
-        if (ht.mult && !__ldcg(flags + 1))
-            for (uint32_t j = lane; j < y; j += 32)
-                if (__ldcg(ht.mult + x + j) > 1) flags[1] = 1;
         if (y > 256) {
             if (lane == 0) flags[0] = 1;  // long bucket: assume repeats (only steers capacity choices)
         } else if (!__ldcg(flags)) {
@@ -286,11 +278,20 @@ __device__ __forceinline__ void flag_buckets(const HTView& ht, uint32_t b, bool 
         __syncwarp();
     }
 }
+// The flag of the multiplicities, by entries (flags[2] of them, placed): with
+// their buckets, one of two million entries was one warp's for 20 ms.
+__device__ __forceinline__ void flag_mults(const HTView& ht, uint32_t t, uint32_t all, uint32_t* flags) {
+    if (!ht.mult) return;
+    const uint32_t n = min(__ldcg(flags + 2), ht.nentries);
+    bool above = false;
+    for (uint32_t e = t; e < n; e += all) above = above || __ldcg(ht.mult + e) > 1;
+    if (above) flags[1] = 1;
+}
 
 __global__ void __launch_bounds__(256) k_ht_flags(HTView ht, uint32_t nbuckets, uint32_t* flags) {
-    const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b - lane < nbuckets; b += gridDim.x * blockDim.x)
-        flag_buckets(ht, b, b < nbuckets, flags);
+    const uint32_t lane = threadIdx.x & 31, t = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
+    for (uint32_t b = t; b - lane < nbuckets; b += all) flag_buckets(ht, b, b < nbuckets, flags);
+    flag_mults(ht, t, all, flags);
 }
 
 // The same by a cluster: thread t of `all`, a warp a run of 32 buckets (or all
@@ -347,6 +348,7 @@ __global__ void __cluster_dims__(kFedCtas, 1, 1) __launch_bounds__(kFedThreads) 
     if (!f.flags) return;
     cluster.sync();
     for (uint32_t b = t; b - (t & 31) < f.nb; b += all) flag_buckets(a.ht, b, b < f.nb, f.dflags);
+    flag_mults(a.ht, t, all, f.dflags);
 }
 
 // ---- leaf builds of a query, batched ----

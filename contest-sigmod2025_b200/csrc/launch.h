@@ -368,7 +368,7 @@ constexpr uint32_t kClusterLeafRows = 4096;
 int build_cluster_leaves(const LeafBatch& batch, cudaStream_t st);
 
 // Flags of a built table: [0] = 1 if some key repeats, [1] = 1 if some mult > 1
-// (both words must be zero before).
+// (both words must be zero before; [2]: the entries placed).
 int ht_flags(HTView ht, uint32_t nbuckets, uint32_t* flags, int num_sms, cudaStream_t st);
 // Counts, for nsample evenly spaced rows of each probe's key column, how many
 // hit its table: hits[p] (zero before) for probe p, all in one launch (the role of

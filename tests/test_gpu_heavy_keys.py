@@ -1,0 +1,70 @@
+"""Keys that a large part of a table has: what the table's flags, the probes of its long bucket and the writing of its
+matches cost, and their results at the sizes where the stage divides its items differently, against the oracle."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle_lib
+from test_gpu_scan_forms import check, column
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def plain(pkg):
+    """A context that does not replay queries."""
+    c = pkg.Context(0)
+    c.set_graphs(False)
+    yield c
+    c.close()
+
+
+def timed(pkg, ctx, oracle, cp, label):
+    """The shortest device time of five runs, the result checked."""
+    want = oracle.execute(cp.ref())
+    plan = cp.struct
+    res = [ctx.upload(plan.inputs[i]) for i in range(plan.num_inputs)]
+    try:
+        best = 1e9
+        for _ in range(5):
+            with ctx.execute_resident(cp, res) as r:
+                best = min(best, r.stats().device_ms)
+                got, keep = r.table_struct()
+                oracle_lib.assert_same_rows(oracle, ctypes.byref(got), want.view(), label)
+        return best
+    finally:
+        for x in res:
+            x.free()
+
+
+def ints(pkg, values):
+    return column(pkg, pkg.INT32, np.asarray(values, np.int32))
+
+
+def bucket(keys):
+    """The bucket of INT32 keys in a table of 2^20 buckets (in a larger one, keys of two of these are apart too)."""
+    return (np.asarray(keys, np.uint64) * np.uint64(0x9E3779B97F4A7C15)) >> np.uint64(44)
+
+
+def one_key_table(pkg, rows=2_000_000):
+    """A table of one key, its rows fed by a probe, probed by a larger one that does not have the key."""
+    rng = np.random.default_rng(1)
+    i32 = pkg.INT32
+    p = pkg.Plan()
+    top = rng.integers(100, 1 << 28, rows * 3 // 2)
+    top = top[bucket(top) != bucket(7)]
+    p.new_input(pkg.ColumnarTable(len(top), [ints(pkg, top), ints(pkg, np.arange(len(top)))]))
+    p.new_input(pkg.ColumnarTable(rows, [ints(pkg, np.full(rows, 7)), ints(pkg, np.arange(rows)),
+                                         ints(pkg, rng.integers(0, 500, rows))]))
+    p.new_input(pkg.ColumnarTable(500, [ints(pkg, np.arange(500))]))
+    a = p.new_scan_node(0, [(0, i32), (1, i32)])
+    b = p.new_scan_node(1, [(0, i32), (1, i32), (2, i32)])
+    fed = p.new_join_node(False, b, p.new_scan_node(2, [(0, i32)]), 2, 0, [(0, i32), (1, i32)])
+    p.root = p.new_join_node(False, a, fed, 0, 0, [(1, i32), (3, i32)])
+    return pkg.CPlan(p)
+
+
+def test_flags_of_a_table_of_one_key(pkg, plain, oracle):
+    # The flags were one warp's work: 62,500 steps of a load, 20 ms of 22.
+    assert timed(pkg, plain, oracle, one_key_table(pkg), "one key") < 10.0
