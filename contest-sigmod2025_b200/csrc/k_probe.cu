@@ -97,19 +97,23 @@ __device__ __forceinline__ uint32_t match_mask(const HTView& ht, const uint4& b,
 
 // The entries from the 33rd of the warp's long buckets, 32 lanes on a bucket:
 // a key that repeats thousands of times would otherwise hold its lane, and the
-// warp, for as many dependent steps. fn(src, e, hit) is called by all lanes
-// together for the item of lane src: entry e + 32 u matches when bit u of the
-// caller's hit is set. The stages of a schema20 query with Zipf-repeated keys:
-// 8.0 ms with the buckets of a warp walked in step, 2.7 ms with each lane
-// walking its own, 0.25 ms now.
+// warp, for as many dependent steps. Lanes with the same key share a walk (a key
+// that repeats in the build often does in the probe): fn(group, e, hit) is
+// called by all lanes together for the items of the lanes in group: entry e +
+// 32 u matches when bit u of the caller's hit is set. The stages of a schema20
+// query with Zipf-repeated keys: 8.0 ms with the buckets of a warp walked in
+// step, 2.7 ms with each lane walking its own, 0.25 ms now. 116M items that find
+// a long bucket of other keys: 235 ms with a walk an item, 8 ms.
 constexpr int kLongStep = 2;  // entries a lane has in flight (4 spill at 40 registers)
 template <typename Fn>
 __device__ __forceinline__ void long_buckets(const HTView& ht, const uint4& b, uint64_t key, Fn&& fn) {
     const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t left = __ballot_sync(0xffffffffu, b.y > 32); left; left &= left - 1) {
+    for (uint32_t left = __ballot_sync(0xffffffffu, b.y > 32); left;) {
         const int src = __ffs(left) - 1;
         const uint32_t x = __shfl_sync(0xffffffffu, b.x, src), y = __shfl_sync(0xffffffffu, b.y, src);
         const uint64_t k = __shfl_sync(0xffffffffu, key, src);
+        const uint32_t group = __ballot_sync(0xffffffffu, b.y > 32 && key == k);
+        left &= ~group;
         for (uint32_t j0 = 32; j0 < y; j0 += 32 * kLongStep) {
             uint64_t q[kLongStep];
 #pragma unroll
@@ -121,7 +125,7 @@ __device__ __forceinline__ void long_buckets(const HTView& ht, const uint4& b, u
 #pragma unroll
             for (int u = 0; u < kLongStep; u++)
                 if (q[u] == k) hit |= 1u << u;
-            fn(src, x + j0 + lane, hit);
+            fn(group, x + j0 + lane, hit);
         }
     }
 }
@@ -135,7 +139,8 @@ __global__ void __launch_bounds__(256) k_stage_count(Items in, DevColumn key, HT
 #pragma unroll
     for (int k = 0; k < kPer; k++) {
         mine += __popc(match_mask(ht, it.bucket[k], it.key[k]));
-        long_buckets(ht, it.bucket[k], it.key[k], [&](int, uint32_t, uint32_t hit) { mine += __popc(hit); });
+        long_buckets(ht, it.bucket[k], it.key[k],
+                     [&](uint32_t group, uint32_t, uint32_t hit) { mine += __popc(hit) * __popc(group); });
     }
     for (int o = 16; o > 0; o >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, o);
     __shared__ unsigned long long part[8];
@@ -166,7 +171,7 @@ __device__ __forceinline__ void walk_stage(const StageItems& it, const HTView& h
         if (lane == 31 && inc) o = atomicAdd(counter, inc);
         o = __shfl_sync(0xffffffffu, o, 31) + inc - cnt;
         for (; m; m &= m - 1) fn(o++, 256 * k + threadIdx.x, it.bucket[k].x + __ffs(m) - 1);
-        long_buckets(ht, it.bucket[k], it.key[k], [&](int src, uint32_t e, uint32_t hit) {
+        long_buckets(ht, it.bucket[k], it.key[k], [&](uint32_t group, uint32_t e, uint32_t hit) {
             uint32_t m[kLongStep], all = 0;
 #pragma unroll
             for (int u = 0; u < kLongStep; u++) {
@@ -175,12 +180,15 @@ __device__ __forceinline__ void walk_stage(const StageItems& it, const HTView& h
             }
             if (!all) return;
             uint32_t at = 0;
-            if (lane == 0) at = atomicAdd(counter, all);
+            if (lane == 0) at = atomicAdd(counter, all * __popc(group));
             at = __shfl_sync(0xffffffffu, at, 0);
+            for (; group; group &= group - 1) {
+                const uint32_t item = 256 * k + (threadIdx.x & ~31u) + __ffs(group) - 1;
 #pragma unroll
-            for (int u = 0; u < kLongStep; u++) {
-                if ((hit >> u) & 1) fn(at + __popc(m[u] & ((1u << lane) - 1)), 256 * k + (threadIdx.x & ~31u) + src, e + 32 * u);
-                at += __popc(m[u]);
+                for (int u = 0; u < kLongStep; u++) {
+                    if ((hit >> u) & 1) fn(at + __popc(m[u] & ((1u << lane) - 1)), item, e + 32 * u);
+                    at += __popc(m[u]);
+                }
             }
         });
     }
@@ -192,8 +200,9 @@ __device__ __forceinline__ void walk_stage(const StageItems& it, const HTView& h
 // entries of 100K INT64 keys, 4.2M matches, on a B200: 71 us; the two passes
 // over tiles, each lane walking its bucket and writing its own matches, took
 // 128 us (82 of them the second), lanes walking in step with one shared
-// atomic a step 91 us, this kernel at 64 registers 77 us.
-__global__ void __launch_bounds__(256, 6) k_stage_emit(Items in, DevColumn key, HTView ht, int use_bloom, KeySource src,
+// atomic a step 91 us. Five blocks an SM: at six, 40 registers spill what the
+// walks share, and the whole query takes 154 us replayed, not 131.
+__global__ void __launch_bounds__(256, 5) k_stage_emit(Items in, DevColumn key, HTView ht, int use_bloom, KeySource src,
                                                     ItemsOut out, uint32_t* cursor, uint32_t capacity, uint32_t* err) {
     __shared__ uint2 found[kStageMatches];  // (item of the block, entry)
     __shared__ uint32_t count, base;

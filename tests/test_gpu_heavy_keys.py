@@ -68,3 +68,31 @@ def one_key_table(pkg, rows=2_000_000):
 def test_flags_of_a_table_of_one_key(pkg, plain, oracle):
     # The flags were one warp's work: 62,500 steps of a load, 20 ms of 22.
     assert timed(pkg, plain, oracle, one_key_table(pkg), "one key") < 10.0
+
+
+def two_tables(pkg, probe, build):
+    """probe(key, row) joined with build(key, row): the build's keys repeat."""
+    i32 = pkg.INT32
+    p = pkg.Plan()
+    p.new_input(pkg.ColumnarTable(len(probe), [ints(pkg, probe), ints(pkg, np.arange(len(probe)))]))
+    p.new_input(pkg.ColumnarTable(len(build), [ints(pkg, build), ints(pkg, np.arange(len(build)))]))
+    a = p.new_scan_node(0, [(0, i32), (1, i32)])
+    b = p.new_scan_node(1, [(0, i32), (1, i32)])
+    p.root = p.new_join_node(False, a, b, 0, 0, [(1, i32), (3, i32)])
+    return pkg.CPlan(p)
+
+
+def other_key(pkg):
+    # (A build above 131,072 rows has no filter that would drop the probes.)
+    keys = np.arange(1, 1 << 24)
+    first, other = keys[bucket(keys) == bucket(12345)][:2]  # one bucket
+    rng = np.random.default_rng(2)
+    build = np.concatenate([np.full(40_000, first), rng.integers(1 << 27, 1 << 28, 100_000)])
+    probe = np.full(4_000_000, other)
+    probe[:: 500_000] = build[-8:]
+    return two_tables(pkg, probe, rng.permutation(build))
+
+
+def test_probes_of_another_keys_bucket(pkg, plain, oracle):
+    # Each probe walked the bucket's 40,000 entries by itself: 210 ms.
+    assert timed(pkg, plain, oracle, other_key(pkg), "other key") < 70.0
