@@ -47,8 +47,9 @@ __device__ __forceinline__ bool stage_key(const DevColumn& key, const KeySource&
 }
 
 // Probe stage against a table whose keys may repeat: any number of matches per
-// item. A block takes kStageItems items, kPer a thread, whose buckets load
-// together; a lane then finds all matches of an item as one bit mask.
+// item. A block takes `span` items: kStageItems, kPer a thread, whose buckets
+// load together, or fewer where each has many matches; a lane then finds all
+// matches of an item as one bit mask.
 constexpr int kPer = 2;
 constexpr uint32_t kStageItems = 256 * kPer;
 constexpr uint32_t kStageMatches = 4096;  // matches of a block collected in shared memory
@@ -56,15 +57,22 @@ constexpr uint32_t kStageMatches = 4096;  // matches of a block collected in sha
 struct StageItems {
     uint64_t key[kPer];
     uint4 bucket[kPer];  // empty for an item without a key
+    // Item k of lane l of this warp is number 256 k + first + l stride of the
+    // block: fewer than a block's threads are dealt to its warps in turn.
+    uint32_t first, stride;
+    __device__ __forceinline__ uint32_t number(int k, uint32_t lane) const { return 256 * k + first + lane * stride; }
 };
-__device__ __forceinline__ void load_stage(StageItems& it, const Items& in, const DevColumn& key, const HTView& ht,
-                                           int use_bloom, const KeySource& src, uint32_t* err) {
+__device__ __forceinline__ void load_stage(StageItems& it, const Items& in, uint32_t span, const DevColumn& key,
+                                           const HTView& ht, int use_bloom, const KeySource& src, uint32_t* err) {
     bool ok[kPer];
+    const uint32_t warp = threadIdx.x >> 5;
+    it.first = span == kStageItems ? 32 * warp : warp;
+    it.stride = span == kStageItems ? 1 : 8;
 #pragma unroll
     for (int k = 0; k < kPer; k++) {
-        const uint32_t i = blockIdx.x * kStageItems + 256 * k + threadIdx.x;
+        const uint32_t local = it.number(k, threadIdx.x & 31), i = blockIdx.x * span + local;
         it.key[k] = 0;
-        ok[k] = i < in.count && stage_key(key, src, in, i, item_row(in, i), err, it.key[k]);
+        ok[k] = local < span && i < in.count && stage_key(key, src, in, i, item_row(in, i), err, it.key[k]);
     }
 #pragma unroll
     for (int k = 0; k < kPer; k++) {
@@ -134,7 +142,7 @@ __device__ __forceinline__ void long_buckets(const HTView& ht, const uint4& b, u
 __global__ void __launch_bounds__(256) k_stage_count(Items in, DevColumn key, HTView ht, int use_bloom, KeySource src,
                                                      unsigned long long* total, uint32_t* err) {
     StageItems it;
-    load_stage(it, in, key, ht, use_bloom, src, err);
+    load_stage(it, in, kStageItems, key, ht, use_bloom, src, err);
     unsigned long long mine = 0;
 #pragma unroll
     for (int k = 0; k < kPer; k++) {
@@ -170,7 +178,7 @@ __device__ __forceinline__ void walk_stage(const StageItems& it, const HTView& h
         uint32_t o = 0;
         if (lane == 31 && inc) o = atomicAdd(counter, inc);
         o = __shfl_sync(0xffffffffu, o, 31) + inc - cnt;
-        for (; m; m &= m - 1) fn(o++, 256 * k + threadIdx.x, it.bucket[k].x + __ffs(m) - 1);
+        for (; m; m &= m - 1) fn(o++, it.number(k, lane), it.bucket[k].x + __ffs(m) - 1);
         long_buckets(ht, it.bucket[k], it.key[k], [&](uint32_t group, uint32_t e, uint32_t hit) {
             uint32_t m[kLongStep], all = 0;
 #pragma unroll
@@ -183,7 +191,7 @@ __device__ __forceinline__ void walk_stage(const StageItems& it, const HTView& h
             if (lane == 0) at = atomicAdd(counter, all * __popc(group));
             at = __shfl_sync(0xffffffffu, at, 0);
             for (; group; group &= group - 1) {
-                const uint32_t item = 256 * k + (threadIdx.x & ~31u) + __ffs(group) - 1;
+                const uint32_t item = it.number(k, __ffs(group) - 1);
 #pragma unroll
                 for (int u = 0; u < kLongStep; u++) {
                     if ((hit >> u) & 1) fn(at + __popc(m[u] & ((1u << lane) - 1)), item, e + 32 * u);
@@ -202,13 +210,14 @@ __device__ __forceinline__ void walk_stage(const StageItems& it, const HTView& h
 // 128 us (82 of them the second), lanes walking in step with one shared
 // atomic a step 91 us. Five blocks an SM: at six, 40 registers spill what the
 // walks share, and the whole query takes 154 us replayed, not 131.
-__global__ void __launch_bounds__(256, 5) k_stage_emit(Items in, DevColumn key, HTView ht, int use_bloom, KeySource src,
-                                                    ItemsOut out, uint32_t* cursor, uint32_t capacity, uint32_t* err) {
+__global__ void __launch_bounds__(256, 5) k_stage_emit(Items in, uint32_t span, DevColumn key, HTView ht, int use_bloom,
+                                                       KeySource src, ItemsOut out, uint32_t* cursor, uint32_t capacity,
+                                                       uint32_t* err) {
     __shared__ uint2 found[kStageMatches];  // (item of the block, entry)
     __shared__ uint32_t count, base;
     if (threadIdx.x == 0) count = 0;
     StageItems it;
-    load_stage(it, in, key, ht, use_bloom, src, err);
+    load_stage(it, in, span, key, ht, use_bloom, src, err);
     __syncthreads();
     walk_stage(it, ht, &count, [&](uint32_t o, uint32_t local, uint32_t e) {
         if (o < kStageMatches) found[o] = make_uint2(local, e);
@@ -224,7 +233,7 @@ __global__ void __launch_bounds__(256, 5) k_stage_emit(Items in, DevColumn key, 
         return;
     }
     auto write = [&](uint32_t o, uint32_t local, uint32_t e) {
-        const uint32_t i = blockIdx.x * kStageItems + local;
+        const uint32_t i = blockIdx.x * span + local;
         out.rows[o] = item_row(in, i);
         for (int p = 0; p < in.nprobes; p++) out.ents[p][o] = in.ents[p][i];
         out.ents[in.nprobes][o] = e;
@@ -339,8 +348,14 @@ int probe_stage_count(const Items& in, const DevColumn& key, const HTView& ht, b
 int probe_stage(const Items& in, const DevColumn& key, const HTView& ht, bool use_bloom, const KeySource& src,
                 const ItemsOut& out, uint32_t* cursor, uint32_t capacity, uint32_t* err, cudaStream_t st) {
     if (!in.count) return 0;
-    k_stage_emit<<<(in.count - 1) / kStageItems + 1, 256, 0, st>>>(in, key, ht, use_bloom, src, out, cursor, capacity,
-                                                                  err);
+    // `capacity` is the matches there are. A block whose items have more than it
+    // collects walks their buckets twice, and a few hundred items with thousands
+    // each would be one block's: fewer items a block then (2,000 items with 1,000
+    // matches each: the query 1.15 ms with 512 a block, 0.11 with 8).
+    uint32_t span = kStageItems;
+    while (span > 8 && uint64_t(span) * capacity > uint64_t(in.count) * (kStageMatches / 2)) span /= 2;
+    k_stage_emit<<<(in.count - 1) / span + 1, 256, 0, st>>>(in, span, key, ht, use_bloom, src, out, cursor, capacity,
+                                                            err);
     return 1;
 }
 

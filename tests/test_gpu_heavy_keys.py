@@ -93,6 +93,40 @@ def other_key(pkg):
     return two_tables(pkg, probe, rng.permutation(build))
 
 
+def hot_keys(pkg):
+    # 2,000 rows that find 1,000 rows each.
+    rng = np.random.default_rng(3)
+    return two_tables(pkg, np.concatenate([rng.integers(0, 2, 2000), np.arange(10, 1500)]),
+                      rng.permutation(np.repeat([0, 1], 1000)))
+
+
 def test_probes_of_another_keys_bucket(pkg, plain, oracle):
     # Each probe walked the bucket's 40,000 entries by itself: 210 ms.
     assert timed(pkg, plain, oracle, other_key(pkg), "other key") < 70.0
+
+
+def test_few_rows_with_many_matches(pkg, plain, oracle):
+    # All matches were a few blocks' to write, each walking its buckets twice: 1.15 ms.
+    assert timed(pkg, plain, oracle, hot_keys(pkg), "hot keys") < 0.5
+
+
+# Probe rows around a block's and a warp's shares, by the matches of each (a block takes 512 rows, fewer from four matches on):
+# `rows` of a table's 10,000 rows pass a first probe and reach the one whose keys repeat.
+@pytest.mark.parametrize("copies", [3, 5, 40, 300])
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 63, 65, 255, 257, 511, 513, 1100])
+@pytest.mark.parametrize("wide", [False, True])
+def test_shares_of_a_block(pkg, ctx, oracle, rows, copies, wide):
+    rng = np.random.default_rng(rows * 1000 + copies)
+    i32, (kt, kn) = pkg.INT32, (pkg.INT64, np.int64) if wide else (pkg.INT32, np.int32)
+    high = (3 << 32) if wide else 0
+    passes = rng.permutation(np.concatenate([np.arange(rows), np.arange(20_000, 30_000 - rows)]))
+    key = (rng.integers(0, 9, 10_000) | high).astype(kn)  # 0 to 5 are there, each `copies` times
+    own = rng.permutation(np.concatenate([np.repeat(np.arange(6), copies), np.arange(100, 300)]) | high).astype(kn)
+    p = pkg.Plan()
+    p.new_input(pkg.ColumnarTable(10_000, [ints(pkg, passes), column(pkg, kt, key), ints(pkg, np.arange(10_000))]))
+    p.new_input(pkg.ColumnarTable(rows, [ints(pkg, rng.permutation(rows))]))
+    p.new_input(pkg.ColumnarTable(len(own), [column(pkg, kt, own), ints(pkg, np.arange(len(own)))]))
+    a = p.new_scan_node(0, [(0, i32), (1, kt), (2, i32)])
+    first = p.new_join_node(False, a, p.new_scan_node(1, [(0, i32)]), 0, 0, [(1, kt), (2, i32)])
+    p.root = p.new_join_node(False, first, p.new_scan_node(2, [(0, kt), (1, i32)]), 0, 0, [(1, i32), (3, i32)])
+    check(pkg, ctx, oracle, pkg.CPlan(p), f"rows {rows} copies {copies} wide {wide}")
