@@ -906,9 +906,14 @@ class Executor {
                 stash_u32(ctx_, hits + k, int(k));
                 stash_u32(ctx_, child.dflags, int(16 + 2 * k));
                 stash_u32(ctx_, child.dflags + 1, int(17 + 2 * k));
+                if (k < 15) stash_u32(ctx_, child.dflags + 2, int(48 + k));  // (slot 63 is the error word's)
             }
             stash_err(ctx_);
             readback(ctx_, int(np));
+            // Nothing joins an empty table (a build that was sized by its bound may
+            // turn out to be one): the rest need not run.
+            for (size_t k = 0; k < std::min<size_t>(np, 15); k++)
+                if (ctx_->h_small[48 + k] == 0) return false;
             for (size_t k = 0; k < np; k++) {
                 rate[k] = nsample ? double(ctx_->h_small[k]) / nsample : 1.0;
                 BuiltHT& child = hts_[pp.probes[k].child];
