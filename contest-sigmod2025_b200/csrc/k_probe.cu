@@ -112,7 +112,9 @@ __device__ __forceinline__ uint32_t match_mask(const HTView& ht, const uint4& b,
 // query with Zipf-repeated keys: 8.0 ms with the buckets of a warp walked in
 // step, 2.7 ms with each lane walking its own, 0.25 ms now. 116M items that find
 // a long bucket of other keys: 235 ms with a walk an item, 8 ms.
-constexpr int kLongStep = 2;  // entries a lane has in flight (4 spill at 40 registers)
+// Entries a lane has in flight, at five blocks an SM: a replayed query that walks
+// much 7.3 ms with 2, 4.4 with 4 (which spill at six blocks' 40 registers).
+constexpr int kLongStep = 4;
 template <typename Fn>
 __device__ __forceinline__ void long_buckets(const HTView& ht, const uint4& b, uint64_t key, Fn&& fn) {
     const uint32_t lane = threadIdx.x & 31;
@@ -139,7 +141,7 @@ __device__ __forceinline__ void long_buckets(const HTView& ht, const uint4& b, u
 }
 
 // Counts the matches: *total (zero before) += them, in 64 bits.
-__global__ void __launch_bounds__(256) k_stage_count(Items in, DevColumn key, HTView ht, int use_bloom, KeySource src,
+__global__ void __launch_bounds__(256, 5) k_stage_count(Items in, DevColumn key, HTView ht, int use_bloom, KeySource src,
                                                      unsigned long long* total, uint32_t* err) {
     StageItems it;
     load_stage(it, in, kStageItems, key, ht, use_bloom, src, err);
