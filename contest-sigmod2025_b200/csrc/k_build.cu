@@ -253,8 +253,12 @@ __global__ void __launch_bounds__(256) k_bucket_ranges(BucketTiles t) {
 constexpr uint32_t kLaneBucket = 8;
 __device__ __forceinline__ bool repeats(const HTView& ht, uint32_t first, uint32_t i) {  // entry first + i, of those before
     const uint64_t key = __ldcg(ht.ent + size_t(first + i) * (1 + ht.width));
-    for (uint32_t j = 0; j < i; j++)
-        if (__ldcg(ht.ent + size_t(first + j) * (1 + ht.width)) == key) return true;
+    for (uint32_t j = 0; j < i; j += 4) {
+        uint64_t q[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) q[u] = j + u < i ? __ldcg(ht.ent + size_t(first + j + u) * (1 + ht.width)) : ~key;
+        if (q[0] == key || q[1] == key || q[2] == key || q[3] == key) return true;
+    }
     return false;
 }
 __device__ __forceinline__ void flag_buckets(const HTView& ht, uint32_t b, bool there, uint32_t* flags) {
@@ -269,10 +273,11 @@ __device__ __forceinline__ void flag_buckets(const HTView& ht, uint32_t b, bool 
     for (uint32_t left = __ballot_sync(0xffffffffu, k.y > kLaneBucket); left; left &= left - 1) {
         const int src = __ffs(left) - 1;
         const uint32_t x = __shfl_sync(0xffffffffu, k.x, src), y = __shfl_sync(0xffffffffu, k.y, src);
-        if (y > 256) {
-            if (lane == 0) flags[0] = 1;  // long bucket: assume repeats (only steers capacity choices)
-        } else if (!__ldcg(flags)) {
-            for (uint32_t i = lane; i < y; i += 32)
+        // Long bucket: assume repeats (only steers capacity choices).
+        if (y > 256 || (!ht.wide && __shfl_sync(0xffffffffu, k.z, src) == __shfl_sync(0xffffffffu, k.w, src))) {
+            if (lane == 0) flags[0] = 1;
+        } else {
+            for (uint32_t i = lane; i < y && !__ldcg(flags); i += 32)
                 if (repeats(ht, x, i)) flags[0] = 1;
         }
         __syncwarp();
@@ -290,8 +295,8 @@ __device__ __forceinline__ void flag_mults(const HTView& ht, uint32_t t, uint32_
 
 __global__ void __launch_bounds__(256) k_ht_flags(HTView ht, uint32_t nbuckets, uint32_t* flags) {
     const uint32_t lane = threadIdx.x & 31, t = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
-    for (uint32_t b = t; b - lane < nbuckets; b += all) flag_buckets(ht, b, b < nbuckets, flags);
     flag_mults(ht, t, all, flags);
+    for (uint32_t b = t; b - lane < nbuckets; b += all) flag_buckets(ht, b, b < nbuckets, flags);
 }
 
 // The same by a cluster: thread t of `all`, a warp a run of 32 buckets (or all
@@ -347,8 +352,8 @@ __global__ void __cluster_dims__(kFedCtas, 1, 1) __launch_bounds__(kFedThreads) 
     for (uint32_t i = t; i < n; i += all) place_tuple(a.tb, a.rank1, a.ht, a.err, i);
     if (!f.flags) return;
     cluster.sync();
-    for (uint32_t b = t; b - (t & 31) < f.nb; b += all) flag_buckets(a.ht, b, b < f.nb, f.dflags);
     flag_mults(a.ht, t, all, f.dflags);
+    for (uint32_t b = t; b - (t & 31) < f.nb; b += all) flag_buckets(a.ht, b, b < f.nb, f.dflags);
 }
 
 // ---- leaf builds of a query, batched ----
