@@ -344,9 +344,11 @@ class Counter {
                 }
                 place[o] = uint32_t(g.nopt++);
             }
+            g.all = ~0u;
             for (const Total& t : tots_) {
                 uint32_t set = 0;
                 for (uint32_t m = t.set; m; m &= m - 1) set |= 1u << place[size_t(__builtin_ctz(m))];
+                g.all &= set;
                 g.options[g.ntot] = set;
                 g.slot[g.ntot++] = t.slot;
             }

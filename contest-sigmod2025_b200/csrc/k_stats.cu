@@ -158,68 +158,87 @@ __global__ void __launch_bounds__(256) k_count_node(CountNode n, uint32_t* err) 
 // to kMaxCountTotals sub-plans instead of for each.
 // The 26 totals over the 1.5M-row root of a seven-table query on a B200: 93
 // us, where a pass a total took 26 x 40 us; every row multiplied: 191 us.
+// kFew: at most kFewTotals totals, which would leave most warps to wait for the
+// others: a row's own thread multiplies its options, without a barrier, and looks
+// no further once one that all totals have is 0. One total of four tables over
+// rows that are all multiplied: the call 189 us in the other form, 75 us so.
+constexpr int kFewTotals = kMaxCountTotals / 8;
+template <bool kFew>
 __global__ void __launch_bounds__(256) k_count_group(CountGroup g) {
     extern __shared__ uint32_t sets[];  // rows by set of options, 1 << nopt
     __shared__ unsigned long long w[kMaxCountOptions][256];
-    __shared__ uint32_t heavy[256];  // per row: its options when one is above 1, else 0
+    __shared__ uint32_t heavy[kFew ? 1 : 256];  // per row: its options when one is above 1, else 0
     constexpr int kPerWarp = kMaxCountTotals / 8;
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    // Totals i = 0, 1, ... of this warp: number warp + 8 i, or (kFew) its part of number i.
+    const auto total_of = [&](int i) { return kFew ? i : int(warp) + 8 * i; };
     unsigned long long acc[kPerWarp] = {};
     uint32_t over = 0;  // bit i: this warp's i-th total passed 2^64 - 1
+    const auto add_row = [&](unsigned long long& sum, int i, uint32_t row, uint32_t set) {
+        unsigned long long v = 1;
+        for (uint32_t m = set; m; m &= m - 1) {
+            const unsigned long long x = w[__ffs(m) - 1][row];
+            v = (v | x) >> 32 ? mul_sat(v, x) : static_cast<unsigned long long>(uint32_t(v)) * uint32_t(x);
+        }
+        sum += v;
+        if (v == ~0ull || sum < v) over |= 1u << i;
+    };
     for (uint32_t m = t; m < 1u << g.nopt; m += 256) sets[m] = 0;
     __syncthreads();
     for (uint32_t r0 = blockIdx.x * 256; r0 < g.nrows; r0 += gridDim.x * 256) {
         const uint32_t r = r0 + t;
         uint64_t key = 0;
         bool ok = false, above = false;
+        bool live = r < g.nrows;  // may still be in some total
         uint32_t have = 0;
-        for (int o = 0; o < g.nopt; o++) {
+        for (int o = 0; o < g.nopt; o++) {  // (with one end: lanes that left it earlier would part from the others)
             const CountOption& op = g.opt[o];
-            if (op.new_edge) ok = r < g.nrows && col_get(op.key, r, key);
+            if (op.new_edge) ok = live && col_get(op.key, r, key);
             // A key that the child's own rows lack is in none of its sub-trees' maps.
-            const bool gone = op.leaf >= 0 && !((have >> op.leaf) & 1);
+            const bool gone = (op.leaf >= 0 && !((have >> op.leaf) & 1)) || (kFew && !live);
             const unsigned long long v = ok && !gone ? map_get(op.map, key) : 0ull;
+            if (kFew) live = live && (v || !(g.all >> o & 1));
             w[o][t] = v;
             above = above || v > 1;
             if (v) have |= 1u << o;
         }
-        heavy[t] = above ? have : 0u;
+        if (kFew && !live) have = 0, above = false;
         const uint32_t same = __match_any_sync(0xffffffffu, above ? 0u : have);
         if (!above && have && lane == uint32_t(__ffs(same) - 1)) atomicAdd(&sets[have], __popc(same));
+        if (kFew) {
+            if (!above) continue;
+#pragma unroll
+            for (int i = 0; i < kFewTotals; i++)
+                if (i < g.ntot && (have & g.options[i]) == g.options[i]) add_row(acc[i], i, t, g.options[i]);
+            continue;
+        }
+        heavy[kFew ? 0 : t] = above ? have : 0u;
         if (!__syncthreads_or(above)) continue;
 #pragma unroll
         for (int i = 0; i < kPerWarp; i++) {
-            const int s = int(warp) + 8 * i;
+            const int s = total_of(i);
             if (s >= g.ntot) continue;
             const uint32_t set = g.options[s];
-            for (int j = 0; j < 8; j++) {
-                if ((heavy[32 * j + lane] & set) != set) continue;
-                unsigned long long v = 1;
-                for (uint32_t m = set; m; m &= m - 1) {
-                    const unsigned long long x = w[__ffs(m) - 1][32 * j + lane];
-                    v = (v | x) >> 32 ? mul_sat(v, x) : static_cast<unsigned long long>(uint32_t(v)) * uint32_t(x);
-                }
-                const unsigned long long sum = acc[i] + v;
-                if (v == ~0ull || sum < v) over |= 1u << i;
-                acc[i] = sum;
-            }
+            for (int j = 0; j < 8; j++)
+                if ((heavy[kFew ? 0 : 32 * j + lane] & set) == set) add_row(acc[i], i, 32 * j + lane, set);
         }
         __syncthreads();
     }
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < kPerWarp; i++) {
-        const int s = int(warp) + 8 * i;
+        const int s = total_of(i);
         if (s >= g.ntot) continue;
         const uint32_t set = g.options[s];
         unsigned long long v = acc[i];
         bool o1 = (over >> i) & 1;
-        for (uint32_t m = lane; m < 1u << g.nopt; m += 32)
-            if ((m & set) == set) {
-                const unsigned long long sum = v + sets[m];
-                o1 = o1 || sum < v;
-                v = sum;
-            }
+        if (!kFew || warp == 0)
+            for (uint32_t m = lane; m < 1u << g.nopt; m += 32)
+                if ((m & set) == set) {
+                    const unsigned long long sum = v + sets[m];
+                    o1 = o1 || sum < v;
+                    v = sum;
+                }
         for (int o = 16; o > 0; o >>= 1) {
             const unsigned long long u = __shfl_xor_sync(0xffffffffu, v, o);
             o1 = o1 || v + u < v;
@@ -277,7 +296,8 @@ int count_node(const CountNode& n, uint32_t* err, int num_sms, cudaStream_t st) 
 int count_group(const CountGroup& g, int num_sms, cudaStream_t st) {
     if (!g.nrows || !g.ntot) return 0;
     const uint32_t blocks = std::min<uint32_t>((g.nrows + 255) / 256, uint32_t(num_sms) * 8);
-    k_count_group<<<blocks, 256, sizeof(uint32_t) << g.nopt, st>>>(g);
+    const size_t sets = sizeof(uint32_t) << g.nopt;
+    g.ntot <= kFewTotals ? k_count_group<true><<<blocks, 256, sets, st>>>(g) : k_count_group<false><<<blocks, 256, sets, st>>>(g);
     return 1;
 }
 

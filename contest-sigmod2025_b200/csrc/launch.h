@@ -438,6 +438,7 @@ struct CountGroup {
     int ntot;
     uint32_t options[kMaxCountTotals];
     uint32_t slot[kMaxCountTotals];
+    uint32_t all;  // the options that every sub-plan has
     uint32_t nrows;
     unsigned long long* total;
     unsigned int* flags;

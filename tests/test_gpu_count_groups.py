@@ -1,0 +1,75 @@
+"""Sub-plans that share a pass over their root: few of them and many, rows with options of 0, 1 and more. Against counts in
+Python integers."""
+import time
+
+import numpy as np
+import pytest
+
+from test_gpu_count_limits import plan
+from test_gpu_subplan_counts import _count
+
+pytestmark = pytest.mark.gpu
+
+EDGES = [(0, 1), (0, 2), (2, 3), (0, 4), (4, 5)]
+
+
+def tables(seed, rows, copies, present):
+    """A root with three children, two of them with one of their own; `copies` rows a key, `present` of the keys there."""
+    rng = np.random.default_rng(seed)
+    out = [{} for _ in range(6)]
+    out[0] = {0: rng.integers(0, 40, rows), 1: rng.integers(0, 40, rows), 3: rng.integers(0, 40, rows)}
+    own = lambda: np.repeat(rng.permutation(40)[:int(40 * present)], copies)  # noqa: E731
+    out[1] = {0: own()}
+    for t, up, down in ((2, 1, 2), (4, 3, 4)):
+        keys = own()
+        out[t] = {up: keys, down: rng.integers(0, 40, len(keys))}
+    out[3] = {2: own()}
+    out[5] = {4: own()}
+    return out
+
+
+# Eight totals a pass are the rows' own threads', from nine on a warp a total; tiles of 256 rows.
+@pytest.mark.parametrize("take", [1, 2, 7, 8, 9, 10, 16])
+@pytest.mark.parametrize("rows", [1, 255, 257, 5000])
+@pytest.mark.parametrize("copies,present", [(1, 1.0), (1, 0.5), (3, 0.8)])
+def test_groups(pkg, ctx, take, rows, copies, present):
+    cp, cols, place = plan(pkg, tables(rows + take, rows, copies, present), EDGES)
+    res = [ctx.upload(cp.struct.inputs[i]) for i in range(6)]
+    try:
+        masks = pkg.subplans(cp)
+        rooted = np.array([m for m in masks if m & 1 and m & (m - 1)], masks.dtype)
+        rng = np.random.default_rng(take)
+        for _ in range(3):
+            some = rng.permutation(rooted)[:take]
+            got = ctx.subplan_cards(cp, res, some)
+            for m, g in zip(some, got):
+                assert g == float(_count(cols, place, EDGES, int(m))), f"{int(m):#x}"
+        together = [m for m in rooted if m & 3 == 3][:take]  # a child that all of them have
+        for m, g in zip(together, ctx.subplan_cards(cp, res, np.array(together, masks.dtype))):
+            assert g == float(_count(cols, place, EDGES, int(m))), f"{int(m):#x}"
+    finally:
+        for x in res:
+            x.free()
+
+
+def one_total(pkg, ctx, copies):
+    """The shortest of ten counts of one sub-plan over a root of 3M rows."""
+    cp, _, _ = plan(pkg, tables(5, 3_000_000, copies, 1.0), EDGES)
+    res = [ctx.upload(cp.struct.inputs[i]) for i in range(6)]
+    try:
+        mask = np.array([0x3f], np.uint32)
+        best = 1e9
+        for _ in range(10):
+            t0 = time.perf_counter()
+            ctx.subplan_cards(cp, res, mask)
+            best = min(best, time.perf_counter() - t0)
+        return best * 1e6
+    finally:
+        for x in res:
+            x.free()
+
+
+def test_one_total_of_many_matches(pkg, ctx):
+    """A call whose rows are multiplied takes little longer than one whose rows are counted: 131 to 110 us (169 to 114 while
+    they were one warp's of eight)."""
+    assert one_total(pkg, ctx, 3) < 1.35 * one_total(pkg, ctx, 1)
