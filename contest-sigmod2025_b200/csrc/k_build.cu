@@ -264,24 +264,22 @@ __device__ __forceinline__ bool repeats(const HTView& ht, uint32_t first, uint32
 __device__ __forceinline__ void flag_buckets(const HTView& ht, uint32_t b, bool there, uint32_t* flags) {
     const uint32_t lane = threadIdx.x & 31;
     const uint4 k = there ? __ldcg(ht.buckets + b) : make_uint4(0, 0, 0, 0);
+    // Once it is set there is nothing left to find; a warp sets it once (35,000
+    // buckets of repeated keys each setting it: 150 us, 59 us so).
+    if (__any_sync(0xffffffffu, __ldcg(flags) != 0)) return;
+    bool found = false;
     if (k.y <= kLaneBucket && (k.y > 2 || (k.y == 2 && k.z == k.w)))
-        for (uint32_t i = 1; i < k.y; i++)
-            if (repeats(ht, k.x, i)) {
-                flags[0] = 1;
-                break;
-            }
-    for (uint32_t left = __ballot_sync(0xffffffffu, k.y > kLaneBucket); left; left &= left - 1) {
+        for (uint32_t i = 1; i < k.y && !found; i++) found = repeats(ht, k.x, i);
+    found = __any_sync(0xffffffffu, found);
+    for (uint32_t left = __ballot_sync(0xffffffffu, k.y > kLaneBucket); left && !found; left &= left - 1) {
         const int src = __ffs(left) - 1;
         const uint32_t x = __shfl_sync(0xffffffffu, k.x, src), y = __shfl_sync(0xffffffffu, k.y, src);
         // Long bucket: assume repeats (only steers capacity choices).
-        if (y > 256 || (!ht.wide && __shfl_sync(0xffffffffu, k.z, src) == __shfl_sync(0xffffffffu, k.w, src))) {
-            if (lane == 0) flags[0] = 1;
-        } else {
-            for (uint32_t i = lane; i < y && !__ldcg(flags); i += 32)
-                if (repeats(ht, x, i)) flags[0] = 1;
-        }
-        __syncwarp();
+        found = y > 256 || (!ht.wide && __shfl_sync(0xffffffffu, k.z, src) == __shfl_sync(0xffffffffu, k.w, src));
+        for (uint32_t i = lane; i - lane < y && !found; i += 32)
+            found = __any_sync(0xffffffffu, (i < y && repeats(ht, x, i)) || __ldcg(flags) != 0);
     }
+    if (found && lane == 0) flags[0] = 1;
 }
 // The flag of the multiplicities, by entries (flags[2] of them, placed): with
 // their buckets, one of two million entries was one warp's for 20 ms.
