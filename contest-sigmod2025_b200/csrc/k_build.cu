@@ -245,11 +245,13 @@ __global__ void __launch_bounds__(256) k_bucket_ranges(BucketTiles t) {
     out[3] = make_uint4(run + c.x + c.y + c.z, c.w, 0, 0);
 }
 
-// Flags of the entries of the warp's buckets (see ht_flags), a bucket a lane;
-// all lanes together, those without a bucket with there = false. A bucket of
-// more than kLaneBucket entries is the whole warp's: Zipf-repeated keys held
-// single lanes for 9.7 ms; the query that has them takes 1.0 ms in all on its
-// first run now.
+// Whether a key repeats in the warp's buckets, a bucket a lane; all lanes
+// together, those without a bucket with there = false. A bucket of more than
+// kLaneBucket entries is the whole warp's: Zipf-repeated keys held single lanes
+// for 9.7 ms; the query that has them takes 1.0 ms in all on its first run now.
+// (flags: what other blocks have found, looked at along a long bucket only. A
+// block sets it once, with set_repeats: a store for each of 50,000 buckets of
+// repeated keys, or a look at the word by every warp, is 60 to 270 us.)
 constexpr uint32_t kLaneBucket = 8;
 __device__ __forceinline__ bool repeats(const HTView& ht, uint32_t first, uint32_t i) {  // entry first + i, of those before
     const uint64_t key = __ldcg(ht.ent + size_t(first + i) * (1 + ht.width));
@@ -261,12 +263,9 @@ __device__ __forceinline__ bool repeats(const HTView& ht, uint32_t first, uint32
     }
     return false;
 }
-__device__ __forceinline__ void flag_buckets(const HTView& ht, uint32_t b, bool there, uint32_t* flags) {
+__device__ __forceinline__ bool key_repeats(const HTView& ht, uint32_t b, bool there, const uint32_t* flags) {
     const uint32_t lane = threadIdx.x & 31;
     const uint4 k = there ? __ldcg(ht.buckets + b) : make_uint4(0, 0, 0, 0);
-    // Once it is set there is nothing left to find; a warp sets it once (35,000
-    // buckets of repeated keys each setting it: 150 us, 59 us so).
-    if (__any_sync(0xffffffffu, __ldcg(flags) != 0)) return;
     bool found = false;
     if (k.y <= kLaneBucket && (k.y > 2 || (k.y == 2 && k.z == k.w)))
         for (uint32_t i = 1; i < k.y && !found; i++) found = repeats(ht, k.x, i);
@@ -279,7 +278,10 @@ __device__ __forceinline__ void flag_buckets(const HTView& ht, uint32_t b, bool 
         for (uint32_t i = lane; i - lane < y && !found; i += 32)
             found = __any_sync(0xffffffffu, (i < y && repeats(ht, x, i)) || __ldcg(flags) != 0);
     }
-    if (found && lane == 0) flags[0] = 1;
+    return found;
+}
+__device__ __forceinline__ void set_repeats(bool found, uint32_t* flags) {
+    if (__syncthreads_or(found) && threadIdx.x == 0) flags[0] = 1;
 }
 // The flag of the multiplicities, by entries (flags[2] of them, placed): with
 // their buckets, one of two million entries was one warp's for 20 ms.
@@ -294,7 +296,9 @@ __device__ __forceinline__ void flag_mults(const HTView& ht, uint32_t t, uint32_
 __global__ void __launch_bounds__(256) k_ht_flags(HTView ht, uint32_t nbuckets, uint32_t* flags) {
     const uint32_t lane = threadIdx.x & 31, t = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
     flag_mults(ht, t, all, flags);
-    for (uint32_t b = t; b - lane < nbuckets; b += all) flag_buckets(ht, b, b < nbuckets, flags);
+    bool found = false;
+    for (uint32_t b = t; b - lane < nbuckets && !found; b += all) found = key_repeats(ht, b, b < nbuckets, flags);
+    set_repeats(found, flags);
 }
 
 // The same by a cluster: thread t of `all`, a warp a run of 32 buckets (or all
@@ -351,7 +355,9 @@ __global__ void __cluster_dims__(kFedCtas, 1, 1) __launch_bounds__(kFedThreads) 
     if (!f.flags) return;
     cluster.sync();
     flag_mults(a.ht, t, all, f.dflags);
-    for (uint32_t b = t; b - (t & 31) < f.nb; b += all) flag_buckets(a.ht, b, b < f.nb, f.dflags);
+    bool found = false;
+    for (uint32_t b = t; b - (t & 31) < f.nb && !found; b += all) found = key_repeats(a.ht, b, b < f.nb, f.dflags);
+    set_repeats(found, f.dflags);
 }
 
 // ---- leaf builds of a query, batched ----
@@ -418,7 +424,7 @@ __global__ void __launch_bounds__(256) k_leaf_flags(LeafBatch B) {
     const int b = leaf_of(B.tile_start, B.n, tile);
     const LeafBuild& L = B.l[b];
     const uint32_t i = (tile - B.tile_start[b]) * kBucketTile + (blockIdx.x % (kBucketTile / 256)) * 256 + threadIdx.x;
-    flag_buckets(L.ht, i, i < L.nb, L.dflags);
+    set_repeats(key_repeats(L.ht, i, i < L.nb, L.dflags), L.dflags);
 }
 
 // Leaves of at most kClusterLeafRows rows: a cluster of eight CTAs builds one
@@ -451,7 +457,9 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     }
     if (!B.flags) return;
     cluster.sync();
-    for (uint32_t b = t; b - (t & 31) < L.nb; b += all) flag_buckets(L.ht, b, b < L.nb, L.dflags);
+    bool found = false;
+    for (uint32_t b = t; b - (t & 31) < L.nb && !found; b += all) found = key_repeats(L.ht, b, b < L.nb, L.dflags);
+    set_repeats(found, L.dflags);
 }
 
 // Hit counts of evenly spaced sample rows against every probe of a pipeline:
