@@ -164,7 +164,8 @@ BJ_API void bj_context_destroy(bj_context* ctx) {
     for (cudaEvent_t e : ctx->window_events) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->free_done) cudaEventDestroy(e);
     if (ctx->async_err) cudaFreeHost(ctx->async_err);
-    for (uint8_t* p : ctx->release_dev) cudaFree(p);
+    for (const auto& b : ctx->release_dev) cudaFree(b.p);
+    for (const auto& b : ctx->spare_dev) cudaFree(b.p);
     for (cudaStream_t s : ctx->side)
         if (s) cudaStreamDestroy(s);
     if (ctx->copy) cudaStreamDestroy(ctx->copy);
@@ -369,7 +370,7 @@ BJ_API void bj_result_free(bj_result* r) {
     bj_result_wait(r);
     if (r->ctx) {
         if (r->dev) {
-            r->ctx->release_device(r->dev);
+            r->ctx->release_device(r->dev, r->dev_size);
             r->dev = nullptr;
         }
         if (r->host.p) r->ctx->give_pinned(r->host);

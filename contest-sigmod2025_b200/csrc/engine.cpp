@@ -1494,7 +1494,7 @@ class Executor {
             dst = alloc<uint8_t>(total * kPageSize);
             res.arena_pages = dst;
         } else if (flags & BJ_RESULT_DEVICE) {
-            if (total) BJ_CK(cudaMallocAsync(reinterpret_cast<void**>(&res.dev), total * kPageSize, st_));
+            if (total) res.dev = ctx_->take_result(total * kPageSize, res.dev_size);
             dst = res.dev;
         } else {
             dst = alloc<uint8_t>(total * kPageSize);
@@ -1592,6 +1592,7 @@ bool run_pipelines(bj_context* ctx, const ExecPlan& ex, const std::vector<const 
 
 int fail_to_status(bj_context* ctx, const Fail& f) {
     ctx->last_error = f.msg;
+    ctx->free_spares();
     ctx->gather.n = 0;
     for (cudaEvent_t e : ctx->prof_events) cudaEventDestroy(e);
     ctx->prof_events.clear();
@@ -1824,6 +1825,7 @@ int execute_common(bj_context* ctx, const bj_plan* plan, bj_resident* const* res
             pipes = exe.pipelines_run();
         }
         end_window_prefetch(ctx, ctx->stream);
+        ctx->free_spares();
         if (!nonempty) {
             if (res->dev) cudaFreeAsync(res->dev, ctx->stream);
             res->dev = nullptr;

@@ -473,29 +473,68 @@ struct bj_context {
     // while one of its streams may be capturing a graph (a free enqueued on
     // a capturing stream would land in the graph).
     std::mutex release_m;
-    std::vector<uint8_t*> release_dev;
-    void release_device(uint8_t* p) {
+    struct DevBlock {
+        uint8_t* p;
+        size_t size;
+    };
+    std::vector<DevBlock> release_dev;
+    void release_device(uint8_t* p, size_t size) {
         std::lock_guard<std::mutex> g(release_m);
-        release_dev.push_back(p);
+        release_dev.push_back({p, size});
     }
     // On the context's own thread, outside stream capture.
     void drain_releases() {
-        std::vector<uint8_t*> dev;
         std::vector<bj::PinnedBlock> excess;
         {
             std::lock_guard<std::mutex> g(release_m);
-            dev.swap(release_dev);
+            spare_dev.insert(spare_dev.end(), release_dev.begin(), release_dev.end());
+            release_dev.clear();
             while (pinned_free.size() > 4) {
                 excess.push_back(pinned_free.front());
                 pinned_free.erase(pinned_free.begin());
             }
         }
-        for (uint8_t* p : dev) cudaFreeAsync(p, stream);
         if (!excess.empty()) {
             cudaStreamSynchronize(stream);
             for (const bj::PinnedBlock& b : excess) cudaFreeHost(b.p);
         }
     }
+
+    // Device memory of results that were freed, for this call's result: its
+    // stream runs behind whatever read them. What the call does not take goes
+    // back to the pool at its end.
+    std::vector<DevBlock> spare_dev;
+    void free_spares() {
+        for (const DevBlock& b : spare_dev) cudaFreeAsync(b.p, stream);
+        spare_dev.clear();
+    }
+    // `bytes` of device memory for a result, in the stream's order; `size` is
+    // what there is: the closest spare block not much larger, else the pool's.
+    // (The pool takes 0.4 to 8 ms for a block of another size than the one just
+    // freed, and a replay, which writes in place, waits for its address: three
+    // inputs in turn, 88 MB results 0.02% apart in size, every third call 0.6-8
+    // ms, 0.19 so.)
+    uint8_t* take_result(size_t bytes, size_t& size) {
+        using bj::Fail;
+        size_t best = spare_dev.size();
+        for (size_t i = 0; i < spare_dev.size(); i++)
+            if (spare_dev[i].size >= bytes && spare_dev[i].size <= bytes + bytes / 4 + kResultSlack &&
+                (best == spare_dev.size() || spare_dev[i].size < spare_dev[best].size))
+                best = i;
+        uint8_t* p = nullptr;
+        if (best < spare_dev.size()) {
+            p = spare_dev[best].p;
+            size = spare_dev[best].size;
+            spare_dev.erase(spare_dev.begin() + long(best));
+            free_spares();
+            return p;
+        }
+        free_spares();
+        BJ_CK(cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, stream));
+        size = bytes;
+        return p;
+    }
+    static constexpr size_t kResultSlack = size_t(2) << 20;
 
     bj::PinnedBlock take_pinned(size_t bytes) {
         {
@@ -542,6 +581,7 @@ struct bj_result {
     uint64_t total_pages = 0;
     bj::PinnedBlock host;
     uint8_t* dev = nullptr;
+    size_t dev_size = 0;  // bytes there, at least its pages'
     uint8_t* arena_pages = nullptr;  // capture only: where the graph leaves the result pages
     bool nonempty = false;
     bj_stats stats{};

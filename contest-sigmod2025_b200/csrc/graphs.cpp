@@ -162,9 +162,10 @@ int replay_graph(bj_context* ctx, GraphEntry& g, const std::vector<int32_t>& typ
             // The graph writes the pages where this word says, in stream
             // order (8 pageable bytes: staged by the call, so replays in
             // flight keep theirs).
-            BJ_CK(cudaMallocAsync(reinterpret_cast<void**>(&res->dev), bytes, ctx->stream));
+            res->dev = ctx->take_result(bytes, res->dev_size);
             BJ_CK(cudaMemcpyAsync(ctx->d_result, &res->dev, sizeof(res->dev), cudaMemcpyHostToDevice, ctx->stream));
         }
+        ctx->free_spares();
         BJ_CK(cudaGraphLaunch(g.exec, ctx->stream));
         if (bytes && !(flags & BJ_RESULT_DEVICE)) {
             res->host = ctx->take_pinned(bytes);
