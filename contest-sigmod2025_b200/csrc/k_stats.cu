@@ -158,17 +158,19 @@ __global__ void __launch_bounds__(256) k_count_node(CountNode n, uint32_t* err) 
 // to kMaxCountTotals sub-plans instead of for each.
 // The 26 totals over the 1.5M-row root of a seven-table query on a B200: 93
 // us, where a pass a total took 26 x 40 us; every row multiplied: 191 us.
-// kFew: at most kFewTotals totals, which would leave most warps to wait for the
-// others: a row's own thread multiplies its options, without a barrier, and looks
+// kFew: at most kFewTotals totals, which would leave half of the warps or more to
+// wait for the others: a row's own thread multiplies its options, without a barrier, and looks
 // no further once one that all totals have is 0. One total of four tables over
-// rows that are all multiplied: the call 189 us in the other form, 75 us so.
-constexpr int kFewTotals = kMaxCountTotals / 8;
+// rows that are all multiplied: the call 189 us in the other form, 77 us so. (Eight
+// totals are a warp's each: 91 us for the labels of a 500K-row fact in the other
+// form, 101 so.)
+constexpr int kFewTotals = 4;
 template <bool kFew>
 __global__ void __launch_bounds__(256) k_count_group(CountGroup g) {
     extern __shared__ uint32_t sets[];  // rows by set of options, 1 << nopt
     __shared__ unsigned long long w[kMaxCountOptions][256];
     __shared__ uint32_t heavy[kFew ? 1 : 256];  // per row: its options when one is above 1, else 0
-    constexpr int kPerWarp = kMaxCountTotals / 8;
+    constexpr int kPerWarp = kFew ? kFewTotals : kMaxCountTotals / 8;
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     // Totals i = 0, 1, ... of this warp: number warp + 8 i, or (kFew) its part of number i.
     const auto total_of = [&](int i) { return kFew ? i : int(warp) + 8 * i; };
