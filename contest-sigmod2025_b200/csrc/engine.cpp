@@ -14,6 +14,7 @@
 //    pipeline of the ExecPlan (planner.h) runs as probe stages, then either a
 //    hash build or the result materialisation.
 #include "engine.h"
+#include "string_pages.h"
 
 #include <cuda_runtime.h>
 #if defined(__x86_64__)
@@ -1450,7 +1451,7 @@ class Executor {
             for (size_t i = i0; i < i1; i++) {
                 const StrPlan& q = sp[strcols[i]];
                 const int slot = int(3 * (i - i0));
-                if (N) stash_u64(ctx_, q.start + (N - 1), slot);
+                stash_u64(ctx_, q.start + N, slot);
                 stash_u32(ctx_, q.stats, slot + 1);
                 stash_u32(ctx_, q.stats + 1, slot + 2);
             }
@@ -1459,19 +1460,23 @@ class Executor {
             for (size_t i = i0; i < i1; i++) {
                 StrPlan& q = sp[strcols[i]];
                 const int slot = int(3 * (i - i0));
-                const uint64_t last_start = N ? ctx_->h_small[slot] : 0;
-                const uint64_t maxc = ctx_->h_small[slot + 1];
+                const uint64_t total = ctx_->h_small[slot], maxc = ctx_->h_small[slot + 1];
                 const bool has_long = ctx_->h_small[slot + 2] != 0;
                 // Floor packing while the longest string keeps pages at least ~87% full.
                 if (!has_long && maxc <= kStrPageUnits / 8) {
-                    q.floor = true;
-                    q.cp = kStrPageUnits - maxc;
-                    res.npages[strcols[i]] = N ? last_start / q.cp + 1 : 0;
+                    const FloorPlan f = floor_plan(total, maxc);
+                    q.floor = f.pages > 0 || !N;
+                    q.cp = f.cp;
+                    res.npages[strcols[i]] = f.pages;
                 }
             }
         }
         for (size_t c : strcols) {
             if (sp[c].floor) continue;
+            // The pages of rows packed one by one depend on the rows' order, which
+            // is another in each replay, while a graph's pages are as many as its
+            // recording's: such a query is not captured.
+            if (ctx_->graph_output) throw Fail{BJ_ERR_UNSUPPORTED, "strings packed one by one are not replayed"};
             const uint32_t j = ex_.out_slot[c];
             const size_t nblocks = (N + kStrBlock - 1) / kStrBlock;
             uint32_t* bp = alloc<uint32_t>(nblocks);

@@ -19,7 +19,7 @@
 // between.
 //
 // Bound: the bucket lookups' L2 sectors (8M probes of a 1M-key table: 58 us,
-// 140 G sectors/s), below a few thousand pages the latency of one page.
+// 136 G sectors/s), below a few thousand pages the latency of one page.
 // Measured on a B200 against the staged form, device time of the scan (with
 // the stages after it): 30K rows in 16 pages 30 -> 10 us; 1M rows, two tables
 // 28 -> 16 us; 8M rows with 10% NULLs 145 -> 63 us (75 us with the matches

@@ -516,10 +516,10 @@ __global__ void __launch_bounds__(256, 8) k_write_dense(OutColumns cols, uint8_t
 }
 
 // Parallel page assignment for VARCHAR columns ("floor packing"). With S_i
-// the exclusive prefix of row costs, row i goes to page floor(S_i / Cp),
-// Cp = 65496 - max cost: a page then holds less than 65496 eighth-bytes, i.e.
-// 4 + 2 nv + bytes + ceil(rows / 8) <= 8192, and consecutive rows advance by
-// at most one page, so no page is empty. Used when no string is long
+// the exclusive prefix of row costs, row i goes to page floor(S_i / Cp), Cp at
+// most 65496 - max cost (floor_plan): a page then holds less than 65496
+// eighth-bytes, i.e. 4 + 2 nv + bytes + ceil(rows / 8) <= 8192, and consecutive
+// rows advance by at most one page, so no page is empty. Used when no string is long
 // (> PAGE_SIZE-7) and the longest is short enough to keep pages ~full. This
 // pass records each page's first row (blockIdx.y = column); the page writer
 // takes a page's row count from the next page's first row.

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "device.cuh"
+#include "string_pages.h"
 
 #include <cuda_runtime.h>
 
@@ -575,7 +576,6 @@ int string_pack(const uint32_t* lens, const uint8_t* valid, uint64_t n, int pass
                 const uint32_t* block_page_off, StrPageDesc* descs, cudaStream_t st);
 // Parallel packing: first row of each page from the exclusive scan `start`
 // of the costs for page capacity cp, every floor-packed column in one launch.
-constexpr uint64_t kStrPageUnits = 65496;  // eighth-bytes a page may hold
 struct FloorCols {
     const uint64_t* start[kMaxOut];
     StrPageDesc* descs[kMaxOut];
