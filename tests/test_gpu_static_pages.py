@@ -32,20 +32,24 @@ def test_turns(pkg, pages, build):
 
 
 def test_many_pages_against_a_small_table(pkg):
+    """What 16M rows against 5,000 keys take, by what they take against 262,144, whose slots miss L1."""
     import torch
 
     rng = np.random.default_rng(1)
-    db, nb = _pages(pkg, rng.integers(0, 5000, 5000), np.ones(5000, bool))
     dp, npp = _pages(pkg, rng.integers(0, 10_000, 16_000_000), np.ones(16_000_000, bool))
     out = torch.zeros(1, dtype=torch.int64, device="cuda")
-    best = 1e9
-    for _ in range(20):
-        begin, end = torch.cuda.Event(True), torch.cuda.Event(True)
-        begin.record()
-        # (Not count_static: it waits for the count before the end is recorded.)
-        assert pkg.lib().bj_join_count_static(db.data_ptr(), nb, 5000, dp.data_ptr(), npp, out.data_ptr(), None) == 0
-        end.record()
-        torch.cuda.synchronize()
-        best = min(best, begin.elapsed_time(end) * 1e3)
-    # 54 us; with a block a page, each ending in its own atomics, 87.
-    assert best < 72.0
+    builds = [(n, *_pages(pkg, rng.integers(0, 10_000 if n == 5000 else 1 << 30, n), np.ones(n, bool))) for n in (5000, 262_144)]
+    dq, nq = _pages(pkg, rng.integers(0, 1 << 30, 16_000_000), np.ones(16_000_000, bool))
+    best = [1e9, 1e9]
+    for _ in range(25):
+        for k, (n, db, nb) in enumerate(builds):
+            probe, pages = (dp, npp) if k == 0 else (dq, nq)
+            begin, end = torch.cuda.Event(True), torch.cuda.Event(True)
+            begin.record()
+            # (Not count_static: it waits for the count before the end is recorded.)
+            assert pkg.lib().bj_join_count_static(db.data_ptr(), nb, n, probe.data_ptr(), pages, out.data_ptr(), None) == 0
+            end.record()
+            torch.cuda.synchronize()
+            best[k] = min(best[k], begin.elapsed_time(end) * 1e3)
+    # 54 to 92 us; with a block a page, each ending in its own atomics, 87 to 109.
+    assert best[0] < 0.70 * best[1], best
