@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(256) k_ht_flags(HTView ht, uint32_t nbuckets, 
     set_repeats(found, flags);
 }
 
-// The same by a cluster: thread t of `all`, a warp a run of 32 buckets (or all
+// Bucket ranges by a cluster: thread t of `all`, a warp a run of 32 buckets (or all
 // 16), each run's entries reserved with one atomic.
 __device__ __forceinline__ void cluster_ranges(const uint32_t* counts, const HTView& ht, uint32_t nb, uint32_t* entries,
                                                uint32_t t, uint32_t all) {
